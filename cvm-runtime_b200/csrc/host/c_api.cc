@@ -44,7 +44,9 @@ class Model {
     VERIFY_NE(params.size(), 0U);
     g_.LoadParams(params);
     g_.RaiseRefusal();
-    exec_.reset(new Executor(g_, device_id_));
+    // a single head without post-processing goes out as it is, when its elements have the output's width
+    const bool as_is = out_num_ == 1 && postprocess_ != "argmax" && postprocess_ != "detection";
+    exec_.reset(new Executor(g_, device_id_, as_is ? output_bytes_ : 0));
   }
 
   int GetInputLength() const { return (int)in_size_ * input_bytes_; }
@@ -81,8 +83,8 @@ class Model {
     for (size_t i = 0; i < expected->size(); ++i)
       VERIFY_EQ(in_shape_[i], (*expected)[i]) << "Loaded data shape at index " << i << " with value "
                                               << in_shape_[i] << ", Expected " << (*expected)[i];
-    exec_->Run(input, (size_t)input_len);
-    SaveTensor(output);
+    exec_->Run(input, (size_t)input_len, output);
+    if (!exec_->delivers_output()) SaveTensor(output);
   }
 
   Executor& executor() {

@@ -1395,6 +1395,11 @@ struct Lowering {
     });
   }
 
+  // Outputs of non_max_suppression that hold at most so many bytes of rows per image: images, bytes,
+  // device array of the valid counts.
+  struct Limited { size_t images, live_bytes; const int32_t* valid_count; };
+  std::map<uint32_t, Limited> limited;
+
   void lower_nms(uint32_t nid) {
     const Node& n = g.nodes[nid];
     const std::string label = "non_max_suppression:" + n.name();
@@ -1424,6 +1429,11 @@ struct Lowering {
       VERIFY(own.ptr == x.ptr) << label << ": its input is read again after the operator, which needs the input "
                                << "stored as int32 rows";
       d.x_writeback = (int32_t*)own.ptr;
+    }
+    if (d.top_k > 0 && (size_t)d.B * 4 < (size_t)1 << 20) {   // (a small buffer is not shared: the counts stay to the end)
+      int64_t bound = std::min<int64_t>(d.N, d.top_k);
+      if (d.max_output_size > 0) bound = std::min<int64_t>(bound, d.max_output_size);
+      if (bound < d.N) limited[g.entry_id(nid, 0)] = {(size_t)d.B, (size_t)bound * 24, d.valid_count};
     }
     add_step(label, [d](cudaStream_t s) { return cvmk_non_max_suppression(&d, s); });
   }
@@ -1588,6 +1598,12 @@ struct Lowering {
       h.dtype = c.dtype;
       h.dev = c.ptr;
       h.bytes = c.bytes();
+      auto lim = limited.find(eid);
+      if (lim != limited.end()) {
+        h.images = lim->second.images;
+        h.live_bytes = lim->second.live_bytes;
+        h.valid_count = lim->second.valid_count;
+      }
       CUDA_OK(cudaMallocHost(&h.host, h.bytes));
       ex.pinned_.push_back(h.host);
       ex.heads_.push_back(h);
@@ -1595,7 +1611,7 @@ struct Lowering {
   }
 };
 
-Executor::Executor(const Graph& g, int device_id) : g_(g), device_(device_id) {
+Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g), device_(device_id) {
   int count = 0;
   CUDA_OK(cudaGetDeviceCount(&count));
   CHECK(device_id >= 0 && device_id < count) << "device_id " << device_id << " out of range (" << count << " GPUs)";
@@ -1617,6 +1633,10 @@ Executor::Executor(const Graph& g, int device_id) : g_(g), device_(device_id) {
   }
   Lowering low(*this, g);
   low.run();
+  plain_ = heads_.size() == 1 && heads_[0].dtype == plain_elem_bytes;
+  if (!plain_)
+    for (auto& h : heads_) h.live_bytes = 0;
+  ChooseDownload();
   // One eager pass sets per-kernel attributes and surfaces launch errors before capture.
   Upload(in_host_, stream_);
   Enqueue(stream_);
@@ -1640,7 +1660,15 @@ Executor::Executor(const Graph& g, int device_id) : g_(g), device_(device_id) {
     };
     capture_from(prefix_steps_, &graph_exec_);
     if (prefix_steps_pageable_ != prefix_steps_) capture_from(prefix_steps_pageable_, &graph_exec_pageable_);
+    if (prefix_steps_ > 0) capture_from(0, &graph_exec_device_);
   }
+}
+
+bool Executor::IsDevice(const void* input) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, input) == cudaSuccess) return at.type == cudaMemoryTypeDevice;
+  cudaGetLastError();
+  return false;
 }
 
 bool Executor::IsDirect(const void* input) {
@@ -1716,7 +1744,9 @@ Executor::~Executor() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   if (graph_exec_pageable_) cudaGraphExecDestroy(graph_exec_pageable_);
+  if (graph_exec_device_) cudaGraphExecDestroy(graph_exec_device_);
   if (kernels_exec_) cudaGraphExecDestroy(kernels_exec_);
+  for (auto e : piece_events_) cudaEventDestroy(e);
   for (auto e : chunk_events_) cudaEventDestroy(e);
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
   for (void* p : allocs_) cudaFree(p);
@@ -1729,99 +1759,88 @@ Executor::~Executor() {
   if (stream_) cudaStreamDestroy(stream_);
 }
 
-StagePool::StagePool(int threads) {
-  for (int i = 0; i < threads; ++i) workers_.emplace_back([this] { Work(); });
+// Where the bytes of an input come from.  Page-locked (or device) memory is read where it lies.  A
+// pageable input of up to 1 MiB is copied into the staging buffer by the calling thread (waking
+// helpers costs more than they save: 1 MiB takes about 50 us cold), a larger one by the pool.
+Executor::Source Executor::SourceOf(const void* input) const {
+  if (IsDirect(input)) return Source::kDirect;
+  return in_bytes_ <= ((size_t)1 << 20) ? Source::kSmall : Source::kPool;
 }
 
-StagePool::~StagePool() {
-  {
-    std::lock_guard<std::mutex> lk(mu_);
-    stop_ = true;
-  }
-  cv_.notify_all();
-  for (auto& t : workers_) t.join();
-}
-
-void StagePool::Start(const char* src, char* dst, size_t bytes, size_t piece) {
-  std::lock_guard<std::mutex> lk(mu_);
-  src_ = src; dst_ = dst; bytes_ = bytes; piece_ = piece;
-  pieces_ = (bytes + piece - 1) / piece;
-  if (pieces_ > done_cap_) {
-    done_.reset(new std::atomic<int>[pieces_]);
-    done_cap_ = pieces_;
-  }
-  for (size_t k = 0; k < pieces_; ++k) done_[k].store(0, std::memory_order_relaxed);
-  next_.store(0, std::memory_order_release);
-  ++job_;
-  cv_.notify_all();
-}
-
-void StagePool::Work() {
-  uint64_t seen = 0;
-  for (;;) {
-    {
-      std::unique_lock<std::mutex> lk(mu_);
-      cv_.wait(lk, [&] { return stop_ || job_ != seen; });
-      if (stop_) return;
-      seen = job_;
-    }
-    for (;;) {
-      const size_t k = next_.fetch_add(1, std::memory_order_acq_rel);
-      if (k >= pieces_) break;
-      const size_t off = k * piece_;
-      memcpy(dst_ + off, src_ + off, std::min(piece_, bytes_ - off));
-      done_[k].store(1, std::memory_order_release);
-    }
-  }
-}
-
-void StagePool::WaitPiece(size_t k) {
-  // the caller helps out instead of idling: pieces are small, so this never waits long
-  while (!done_[k].load(std::memory_order_acquire)) {
-    const size_t j = next_.fetch_add(1, std::memory_order_acq_rel);
-    if (j < pieces_) {
-      const size_t off = j * piece_;
-      memcpy(dst_ + off, src_ + off, std::min(piece_, bytes_ - off));
-      done_[j].store(1, std::memory_order_release);
-    } else {
-      std::this_thread::yield();
-    }
-  }
-}
-
-// Queues the upload of one input.  Page-locked (or device) memory is read where it lies; pageable
-// memory goes through the pinned staging buffer in pieces that a few host threads copy in
-// parallel, each piece being sent to the device as soon as it is staged.
-void Executor::Upload(const void* input, cudaStream_t s) { UploadRange(input, 0, in_bytes_, s); }
-
-void Executor::UploadRange(const void* input, size_t begin, size_t bytes, cudaStream_t s) {
-  if (IsDirect(input)) {
-    CUDA_OK(cudaMemcpyAsync((char*)in_dev_ + begin, (const char*)input + begin, bytes, cudaMemcpyDefault, s));
-    return;
-  }
-  const size_t piece = (size_t)1 << 20;
-  if (bytes <= 2 * piece) {   // small inputs: not worth waking anyone
-    memcpy((char*)in_host_ + begin, (const char*)input + begin, bytes);
-    CUDA_OK(cudaMemcpyAsync((char*)in_dev_ + begin, (char*)in_host_ + begin, bytes, cudaMemcpyHostToDevice, s));
-    return;
-  }
-  if (!stage_pool_) {
+HostPool& Executor::pool() {
+  if (!pool_) {
     unsigned hw = std::thread::hardware_concurrency();
     int gpus = 1;
     cudaGetDeviceCount(&gpus);
-    // three helpers beside the calling thread, fewer when the host has few cores per GPU
-    int helpers = hw ? std::max(1, std::min(3, (int)hw / std::max(1, gpus) - 1)) : 1;
-    stage_pool_.reset(new StagePool(helpers));
+    // five helpers beside the calling thread, fewer when the host has few cores per GPU: one core
+    // copies 14 GB/s here, four just reach the link's 55 GB/s, six leave room for a fill beside it
+    pool_.reset(new HostPool(hw ? std::max(1, std::min(5, (int)hw / std::max(1, gpus) - 1)) : 1));
   }
-  stage_pool_->Start((const char*)input + begin, (char*)in_host_ + begin, bytes, piece);
-  // the transfer is issued in groups of four pieces: fewer driver calls, still well pipelined
-  const size_t group = 4;
-  for (size_t k = 0; k < stage_pool_->pieces(); k += group) {
-    const size_t last = std::min(stage_pool_->pieces(), k + group);
-    for (size_t j = k; j < last; ++j) stage_pool_->WaitPiece(j);
-    const size_t off = begin + k * piece;
-    const size_t n = std::min(group * piece, begin + bytes - off);
-    CUDA_OK(cudaMemcpyAsync((char*)in_dev_ + off, (char*)in_host_ + off, n, cudaMemcpyHostToDevice, s));
+  return *pool_;
+}
+
+void Executor::BeginUpload(const void* input, Source src) {
+  if (src != Source::kPool) return;
+  const char* from = (const char*)input;
+  char* to = (char*)in_host_;
+  const size_t bytes = in_bytes_, pieces = (bytes + kStagePiece - 1) / kStagePiece;
+  pool().Start(HostPool::kUpload, pieces, pieces, [from, to, bytes](size_t k) {
+    const size_t off = k * kStagePiece;
+    stream_copy(to + off, from + off, std::min(kStagePiece, bytes - off));
+  });
+}
+
+// Staged bytes are sent in groups of pieces (1 MiB) as soon as they are there: fewer driver calls,
+// still well pipelined.
+void Executor::SendRange(const void* input, Source src, size_t begin, size_t bytes, cudaStream_t s) {
+  char* const dev = (char*)in_dev_;
+  if (src == Source::kDirect) {
+    CUDA_OK(cudaMemcpyAsync(dev + begin, (const char*)input + begin, bytes, cudaMemcpyDefault, s));
+    return;
+  }
+  const size_t group = src == Source::kSmall ? kStagePiece : 4 * kStagePiece;
+  for (size_t off = begin; off < begin + bytes;) {
+    const size_t end = std::min(begin + bytes, (off / group + 1) * group);
+    if (src == Source::kSmall) memcpy((char*)in_host_ + off, (const char*)input + off, end - off);
+    else
+      for (size_t k = off / kStagePiece; k * kStagePiece < end; ++k) pool().WaitPiece(HostPool::kUpload, k);
+    CUDA_OK(cudaMemcpyAsync(dev + off, (char*)in_host_ + off, end - off, cudaMemcpyHostToDevice, s));
+    off = end;
+  }
+}
+
+void Executor::Upload(const void* input, cudaStream_t s) {
+  const Source src = SourceOf(input);
+  if (src == Source::kPool) pool().Begin();
+  BeginUpload(input, src);
+  SendRange(input, src, 0, in_bytes_, s);
+  if (src == Source::kPool) {
+    pool().Finish(HostPool::kUpload);
+    pool().End();
+  }
+}
+
+// Heads of up to 1 MiB in all (8 MiB of an NMS head's rows: fetching its -1 tail too costs more) are
+// written into page-locked memory by one kernel, with the status word: a copy node for each costs 3 us and more
+// and starts only after the kernel before it has drained.  A single larger head whose bytes are
+// the result leaves in pieces (DeliverPieces).
+void Executor::ChooseDownload() {
+  size_t total = 0;
+  for (const auto& h : heads_) total += h.live_bytes ? h.images * h.live_bytes : h.bytes;
+  const size_t small = (size_t)(plain_ && heads_[0].live_bytes ? 8 : 1) << 20;
+  if (total <= small && heads_.size() + 2 <= CVMK_MAX_EXPORT_SEGMENTS) {
+    download_ = Download::kKernel;
+  } else {
+    for (auto& h : heads_) h.live_bytes = 0;
+    download_ = plain_ ? Download::kPieces : Download::kCopies;
+  }
+  if (download_ == Download::kPieces) {
+    piece_events_.resize((heads_[0].bytes + kDownloadPiece - 1) / kDownloadPiece);
+    for (auto& e : piece_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  if (download_ == Download::kKernel && heads_[0].live_bytes) {
+    CUDA_OK(cudaMallocHost((void**)&valid_host_, heads_[0].images * 4));
+    pinned_.push_back(valid_host_);
   }
 }
 
@@ -1831,19 +1850,117 @@ void Executor::Enqueue(cudaStream_t s, size_t first) {
     int rc = st.launch(s);
     CHECK(rc == CVMK_OK) << "step " << st.label << " failed (" << rc << "): " << cvmk_last_error();
   }
-  for (auto& h : heads_) CUDA_OK(cudaMemcpyAsync(h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost, s));
-  CUDA_OK(cudaMemcpyAsync(status_host_, status_dev_, 4, cudaMemcpyDeviceToHost, s));
+  cvmk_export_segment seg[CVMK_MAX_EXPORT_SEGMENTS];
+  int n = 0;
+  auto add = [&](const void* src, void* dst, size_t rows, size_t row_bytes, size_t pitch) {
+    seg[n].src = src; seg[n].dst = dst;
+    seg[n].rows = (int64_t)rows; seg[n].row_bytes = (int64_t)row_bytes; seg[n].src_pitch = (int64_t)pitch;
+    ++n;
+  };
+  add(status_dev_, status_host_, 1, 4, 4);
+  if (download_ == Download::kKernel) {
+    for (auto& h : heads_) {
+      if (h.live_bytes) add(h.dev, h.host, h.images, h.live_bytes, h.bytes / h.images);
+      else add(h.dev, h.host, 1, h.bytes, h.bytes);
+      if (h.live_bytes) add(h.valid_count, valid_host_, 1, h.images * 4, h.images * 4);
+    }
+  } else if (download_ == Download::kCopies) {
+    for (auto& h : heads_) CUDA_OK(cudaMemcpyAsync(h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost, s));
+  }
+  KERNEL_OK(cvmk_export(seg, n, s));
 }
 
-void Executor::Run(const void* input, size_t input_bytes) {
+// The part of an NMS head that is -1 whatever the data says, written while the GPU works.
+void Executor::StartFill(char* out) {
+  const HeadOut& h = heads_[0];
+  const size_t image = h.bytes / h.images, tail = image - h.live_bytes, live = h.live_bytes;
+  const size_t per = std::max<size_t>(1, (tail + kStagePiece - 1) / kStagePiece);
+  const size_t piece = (tail + per - 1) / per;
+  pool().Start(HostPool::kFill, h.images * per, h.images * per, [=](size_t k) {
+    const size_t b = k / per, off = std::min(tail, (k % per) * piece);
+    memset(out + b * image + live + off, 0xff, std::min(piece, tail - off));
+  });
+}
+
+// One large head: the copy engine brings it in pieces, the pool copies every piece that has arrived
+// into the caller's buffer.  A page-locked buffer takes the pieces directly.
+void Executor::DeliverPieces(char* out) {
+  const HeadOut& h = heads_[0];
+  if (IsDirect(out)) {
+    CUDA_OK(cudaMemcpyAsync(out, h.dev, h.bytes, cudaMemcpyDefault, stream_));
+    CUDA_OK(cudaStreamSynchronize(stream_));
+    return;
+  }
+  for (size_t k = 0; k < piece_events_.size(); ++k) {
+    const size_t off = k * kDownloadPiece;
+    CUDA_OK(cudaMemcpyAsync((char*)h.host + off, (const char*)h.dev + off, std::min(kDownloadPiece, h.bytes - off), cudaMemcpyDeviceToHost, stream_));
+    CUDA_OK(cudaEventRecord(piece_events_[k], stream_));
+  }
+  const size_t unit = kStagePiece, units = (h.bytes + unit - 1) / unit, per = kDownloadPiece / unit;
+  const char* from = (const char*)h.host;
+  const size_t bytes = h.bytes;
+  pool().Start(HostPool::kDownload, units, 0, [=](size_t k) { memcpy(out + k * unit, from + k * unit, std::min(unit, bytes - k * unit)); });
+  for (size_t k = 0; k < piece_events_.size(); ++k) {
+    cudaError_t e;
+    while ((e = cudaEventQuery(piece_events_[k])) == cudaErrorNotReady) pool().HelpOnce();
+    if (e != cudaSuccess) {   // nothing more will arrive: let the job end before reporting
+      pool().Release(HostPool::kDownload, units);
+      CUDA_OK(e);
+    }
+    pool().Release(HostPool::kDownload, std::min(units, (k + 1) * per));
+  }
+  pool().Finish(HostPool::kDownload);
+}
+
+// The head is in page-locked memory (and the GPU idle): into the caller's buffer.
+void Executor::DeliverHead(char* out) {
+  const HeadOut& h = heads_[0];
+  if (!h.live_bytes) {
+    memcpy(out, h.host, h.bytes);
+    return;
+  }
+  const size_t image = h.bytes / h.images, live = h.live_bytes;
+  const char* from = (const char*)h.host;
+  pool().Start(HostPool::kDownload, h.images, h.images, [=](size_t b) { memcpy(out + b * image, from + b * live, live); });
+  pool().Finish(HostPool::kDownload);
+  pool().Finish(HostPool::kFill);
+  // The operator's loop ends at the first image without valid boxes; what it leaves in the images
+  // after that one is whatever their memory holds, which is fetched as it is.
+  size_t b = 0;
+  while (b < h.images && valid_host_[b] > 0) ++b;
+  if (b + 1 < h.images) {
+    CUDA_OK(cudaMemcpyAsync(out + (b + 1) * image, (const char*)h.dev + (b + 1) * image, h.bytes - (b + 1) * image, cudaMemcpyDeviceToHost, stream_));
+    CUDA_OK(cudaStreamSynchronize(stream_));
+  }
+}
+
+void Executor::Run(const void* input, size_t input_bytes, char* out) {
   CHECK(input_bytes == in_bytes_) << "input size " << input_bytes << " vs. " << in_bytes_;
   CUDA_OK(cudaSetDevice(device_));
-  const bool pageable = graph_exec_pageable_ && !IsDirect(input);
-  const size_t prefix = pageable ? prefix_steps_pageable_ : prefix_steps_;
+  const Source src = SourceOf(input);
+  const bool on_device = src == Source::kDirect && IsDevice(input);
+  const bool fill = plain_ && heads_[0].live_bytes > 0, pieces = plain_ && download_ == Download::kPieces;
+  // Whatever way this ends, no helper touches the caller's buffers afterwards.
+  struct PoolGuard {
+    HostPool* p = nullptr;
+    ~PoolGuard() {
+      if (!p) return;
+      for (int k = 0; k < HostPool::kSlots; ++k) p->Finish((HostPool::Slot)k);
+      p->End();
+    }
+  } guard;
+  if (src == Source::kPool || fill || pieces) {
+    guard.p = &pool();
+    guard.p->Begin();
+  }
+  BeginUpload(input, src);
+  if (fill) StartFill(out);
+  const bool pageable = graph_exec_pageable_ && src != Source::kDirect;
+  const size_t prefix = on_device ? 0 : (pageable ? prefix_steps_pageable_ : prefix_steps_);
   if (graph_exec_ && prefix > 0) {
     // chunk c of the batch is uploaded on the copy stream while the leading steps run on chunk c - 1
     for (size_t c = 0; c < steps_[0].chunk.size(); ++c) {
-      UploadRange(input, c * chunk_bytes_, chunk_bytes_, copy_stream_);
+      SendRange(input, src, c * chunk_bytes_, chunk_bytes_, copy_stream_);
       CUDA_OK(cudaEventRecord(chunk_events_[c], copy_stream_));
       CUDA_OK(cudaStreamWaitEvent(stream_, chunk_events_[c], 0));
       for (size_t k = 0; k < prefix; ++k) {
@@ -1853,11 +1970,13 @@ void Executor::Run(const void* input, size_t input_bytes) {
     }
     CUDA_OK(cudaGraphLaunch(pageable ? graph_exec_pageable_ : graph_exec_, stream_));
   } else {
-    Upload(input, stream_);
-    if (graph_exec_) CUDA_OK(cudaGraphLaunch(graph_exec_, stream_));
+    SendRange(input, src, 0, in_bytes_, stream_);
+    cudaGraphExec_t whole = on_device && graph_exec_device_ ? graph_exec_device_ : graph_exec_;
+    if (whole) CUDA_OK(cudaGraphLaunch(whole, stream_));
     else Enqueue(stream_);
   }
-  CUDA_OK(cudaStreamSynchronize(stream_));
+  if (pieces) DeliverPieces(out);
+  else CUDA_OK(cudaStreamSynchronize(stream_));
   if (*status_host_ != 0) {
     const int code = *status_host_;
     *status_host_ = 0;
@@ -1865,6 +1984,7 @@ void Executor::Run(const void* input, size_t input_bytes) {
     cudaStreamSynchronize(stream_);
     FATAL() << "a device-side wait ran out (status word 0x" << std::hex << code << ")";
   }
+  if (plain_ && !pieces) DeliverHead(out);
 }
 
 void Executor::SetStatusWord(int code) {

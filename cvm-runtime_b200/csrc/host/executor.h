@@ -15,16 +15,13 @@
 // There is no CPU fallback: every step is a CUDA kernel from this library.
 #pragma once
 #include <cuda_runtime.h>
-#include <atomic>
-#include <condition_variable>
 #include <functional>
 #include <memory>
-#include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 #include "cvmk_kernels.h"
 #include "graph.h"
+#include "host_pool.h"
 
 namespace cvm {
 
@@ -50,43 +47,23 @@ struct HeadOut {
   void* dev = nullptr;       // canonical row-major copy on the device
   void* host = nullptr;      // pinned
   size_t bytes = 0;
-};
-
-// A few host threads that copy a pageable caller buffer into the page-locked staging buffer piece
-// by piece, so that the copy runs at several times one core's memcpy rate and the transfer of a
-// piece to the device starts as soon as that piece is staged.
-class StagePool {
- public:
-  explicit StagePool(int threads);
-  ~StagePool();
-  // Starts copying [src, src + bytes) to dst in pieces of `piece` bytes; returns at once.
-  void Start(const char* src, char* dst, size_t bytes, size_t piece);
-  // Blocks until piece k (0-based) of the current job has been copied.
-  void WaitPiece(size_t k);
-  size_t pieces() const { return pieces_; }
-
- private:
-  void Work();
-  std::vector<std::thread> workers_;
-  std::mutex mu_;
-  std::condition_variable cv_;
-  bool stop_ = false;
-  uint64_t job_ = 0;                 // generation counter: a new value wakes the workers
-  const char* src_ = nullptr;
-  char* dst_ = nullptr;
-  size_t bytes_ = 0, piece_ = 0, pieces_ = 0;
-  std::atomic<size_t> next_{0};
-  std::unique_ptr<std::atomic<int>[]> done_;
-  size_t done_cap_ = 0;
+  // The output of non_max_suppression with a limit on its rows: of every image only the first
+  // live_bytes can hold anything but -1, so only those are downloaded (0: the whole tensor is).
+  size_t images = 1, live_bytes = 0;
+  const int32_t* valid_count = nullptr;   // device, [images]: an image with none ends the operator's loop
 };
 
 class Executor {
  public:
-  Executor(const Graph& g, int device_id);
+  // `plain_elem_bytes`: when not 0, the caller wants a single head's elements as they are, this many
+  // bytes each, and hands Run() the buffer for them (see delivers_output()).
+  Executor(const Graph& g, int device_id, int plain_elem_bytes);
   ~Executor();
   // Runs one inference.  `input` holds the `data` tensor in API form (int8 or int32, row-major).
-  // On return heads()[k].host holds head k (row-major, heads()[k].dtype).
-  void Run(const void* input, size_t input_bytes);
+  // If delivers_output(), the head's bytes are in `out` on return; otherwise heads()[k].host holds
+  // head k (row-major, heads()[k].dtype).
+  void Run(const void* input, size_t input_bytes, char* out);
+  bool delivers_output() const { return plain_; }
   const std::vector<HeadOut>& heads() const { return heads_; }
   size_t num_steps() const { return steps_.size(); }
   size_t device_bytes() const { return device_bytes_; }
@@ -121,6 +98,7 @@ class Executor {
   cudaGraphExec_t graph_exec_pageable_ = nullptr;   // the steps from prefix_steps_pageable_ on
   void ChoosePrefixes();
   static bool IsDirect(const void* input);
+  static bool IsDevice(const void* input);
   size_t chunk_bytes_ = 0;    // input bytes of one batch chunk
   std::vector<HeadOut> heads_;
   std::vector<void*> allocs_;
@@ -140,7 +118,21 @@ class Executor {
   // upload / stem overlap: per-chunk stem plans, the copy stream and one event per chunk
   cudaStream_t copy_stream_ = nullptr;
   std::vector<cudaEvent_t> chunk_events_;
-  std::unique_ptr<StagePool> stage_pool_;   // created by the first inference from pageable memory
+  cudaGraphExec_t graph_exec_device_ = nullptr;   // every step: the input is on the device already
+  std::unique_ptr<HostPool> pool_;   // created by the first inference that has enough bytes to move
+  HostPool& pool();
+  // How the heads reach the host: small ones are written into page-locked memory by a kernel
+  // together with the status word, one large head that goes out as it is by the copy engine in
+  // pieces that host threads move on while the next ones arrive, anything else by one copy each.
+  enum class Download { kKernel, kPieces, kCopies };
+  Download download_ = Download::kCopies;
+  bool plain_ = false;
+  std::vector<cudaEvent_t> piece_events_;
+  int32_t* valid_host_ = nullptr;    // pinned copy of HeadOut::valid_count
+  void ChooseDownload();
+  void StartFill(char* out);
+  void DeliverPieces(char* out);
+  void DeliverHead(char* out);
 
   void* dalloc(size_t bytes);
   // Activation memory.  Every activation buffer gets a virtual address range of its own when the
@@ -169,8 +161,14 @@ class Executor {
   std::vector<PhysBlock> phys_;
   bool vmm_ = false;
   size_t vmm_gran_ = 0;
+  // Uploads: BeginUpload() starts the staging of a pageable input (the whole of it), SendRange()
+  // queues the transfer of a part, Upload() does both for all of it.
+  enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
+  static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
+  Source SourceOf(const void* input) const;
+  void BeginUpload(const void* input, Source src);
+  void SendRange(const void* input, Source src, size_t begin, size_t bytes, cudaStream_t s);
   void Upload(const void* input, cudaStream_t s);
-  void UploadRange(const void* input, size_t begin, size_t bytes, cudaStream_t s);
   void Enqueue(cudaStream_t s, size_t first = 0);
   friend struct Lowering;
 };

@@ -1,0 +1,70 @@
+// A few host threads that move bytes for the calling thread of an inference: a pageable caller
+// buffer into the page-locked staging buffer, downloaded pieces into the caller's output buffer,
+// constant fills.  Each of these is a job cut into pieces; a piece is a call of the job's body.
+//
+// The helpers sleep between inferences.  Begin() wakes them once, and until End() they spin over
+// the jobs, lowest slot first, so that a job that starts while others run is picked up without a
+// wake-up (tens of microseconds, more than many of these jobs take).  The caller helps with every
+// job it waits for.
+#pragma once
+#include <atomic>
+#include <condition_variable>
+#include <cstddef>
+#include <cstdint>
+#include <functional>
+#include <memory>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace cvm {
+
+class HostPool {
+ public:
+  enum Slot { kUpload = 0, kDownload = 1, kFill = 2, kSlots = 3 };   // in order of urgency
+
+  explicit HostPool(int helpers);
+  ~HostPool();
+  HostPool(const HostPool&) = delete;
+  HostPool& operator=(const HostPool&) = delete;
+
+  void Begin();
+  void End();
+  // Starts a job of `pieces` calls body(k).  The slot's previous job must have finished.  The first
+  // `available` pieces may run at once, the others when Release() says so.
+  void Start(Slot slot, size_t pieces, size_t available, std::function<void(size_t)> body);
+  void Release(Slot slot, size_t available);
+  // Waits until piece k has run, running pieces of this job meanwhile.
+  void WaitPiece(Slot slot, size_t k);
+  // Waits until the whole job has run.
+  void Finish(Slot slot);
+  // Runs one piece of any job, if one is free; false if there is none.
+  bool HelpOnce();
+
+ private:
+  struct Job {
+    // (generation << 32 | count): a claim is a compare-exchange of the whole word against `avail` of
+    // the same generation, so a helper that looked at the slot's previous job cannot take a
+    // piece the present one does not have.
+    std::atomic<uint64_t> next{0}, avail{0};
+    std::function<void(size_t)> body;
+    size_t pieces = 0;
+    std::unique_ptr<std::atomic<uint8_t>[]> done;
+    size_t done_cap = 0;
+    std::atomic<size_t> completed{0};
+  };
+  bool RunPiece(Job& j);
+  void Work();
+
+  Job jobs_[kSlots];
+  std::vector<std::thread> workers_;
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::atomic<bool> active_{false}, stop_{false};
+};
+
+// memcpy with stores that bypass the cache: for destinations the CPU does not read soon (the
+// staging buffer the copy engine reads, a large output).
+void stream_copy(char* dst, const char* src, size_t bytes);
+
+}  // namespace cvm

@@ -212,6 +212,18 @@ CVMK_API int cvmk_strided(const cvmk_strided_desc* d, cvmk_stream_t stream);
 CVMK_API int cvmk_strided_batch(const cvmk_strided_desc* d, int32_t n, cvmk_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * Copies up to CVMK_MAX_EXPORT_SEGMENTS row sets in one launch: rows * row_bytes bytes of each segment,
+ * src rows src_pitch bytes apart, dst rows packed.  dst may be page-locked host memory: that is how
+ * small results (and the status word) leave the GPU.
+ * ---------------------------------------------------------------------------------------------- */
+#define CVMK_MAX_EXPORT_SEGMENTS 8
+typedef struct {
+  const void* src; void* dst;
+  int64_t rows, row_bytes, src_pitch;
+} cvmk_export_segment;
+CVMK_API int cvmk_export(const cvmk_export_segment* segments, int32_t n, cvmk_stream_t stream);
+
+/* ------------------------------------------------------------------------------------------------
  * sum / max reduce (cpu/ops/reduce.cc:34-140).  Output point c (up to 6 kept extents, strides into
  * x given per extent) reduces over up to 6 reduced extents.  init_zero = 1 reproduces the
  * reduce-over-everything path, whose accumulator starts at 0 (reduce.cc:41-47); otherwise the

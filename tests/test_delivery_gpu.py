@@ -1,0 +1,53 @@
+"""How inputs reach the GPU and results the caller: every path of the executor against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def copy_case(wl, n):
+    """One operator over n int8 elements: the result is as large as the input."""
+    g = wl.GraphBuilder(3)
+    d = g.var("data", (1, n), 8)
+    y = g.op("clip", [d], (1, n), {"a_min": -100, "a_max": 90})
+    js, pb = g.finish(y)
+    return js, pb, np.random.RandomState(n).randint(-127, 128, size=(1, n)).astype(np.int8)
+
+
+# one kernel writes heads of up to 1 MiB, larger ones leave in 1 MiB pieces; inputs above 1 MiB are
+# staged by the host threads in 256 KiB pieces
+@pytest.mark.parametrize("n", [1, 15, 4099, 1 << 20, (1 << 20) + 1, (3 << 20) + 77])
+@pytest.mark.parametrize("where", ["pageable", "pinned", "device"])
+def test_sizes_and_buffers(n, where, rt, wl, oracle):
+    import torch
+    js, pb, x = copy_case(wl, n)
+    want = oracle.run_model(js, pb, x)
+    net = rt.CVMAPILoadModel(js, pb, 0)
+    try:
+        flat = torch.from_numpy(x.reshape(-1).view(np.uint8).copy())
+        src = {"pageable": flat, "pinned": flat.pin_memory(), "device": flat.cuda()}[where]
+        out = torch.zeros(n, dtype=torch.uint8)
+        for dst in (out, torch.zeros(n, dtype=torch.uint8).pin_memory()):
+            for _ in range(2):
+                dst.zero_()
+                rt.check_call(rt.lib().CVMAPIInference(net, ctypes.c_void_p(src.data_ptr()), n, ctypes.c_void_p(dst.data_ptr())))
+                assert np.array_equal(dst.numpy(), want.view(np.uint8))
+    finally:
+        rt.CVMAPIFreeModel(net)
+
+
+# rows past top_k / max_output_size are not downloaded; the operator's loop ends at an image without
+# valid boxes, whose successors keep what their memory held (zeros in a fresh handle)
+@pytest.mark.parametrize("empty", [None, 0, 1, 3])
+@pytest.mark.parametrize("anchors,top_k,mos", [(1001, 100, -1), (1000, 100, 37), (700, 800, 20), (5003, 1, -1)])
+def test_nms_head(anchors, top_k, mos, empty, gpu_run, wl, oracle):
+    js, pb, x = wl.ssd_tail(batch=4, anchors=anchors, top_k=top_k, max_output_size=mos)
+    if empty is not None:
+        x = x.copy()
+        x[empty, :, 1] = 3
+    got = gpu_run(js, pb, x).view(np.int32).reshape(4, anchors, 6)
+    want = oracle.run_model(js, pb, x).view(np.int32).reshape(4, anchors, 6)
+    last = 4 if empty is None else empty + 1
+    assert np.array_equal(got[:last], want[:last])
