@@ -1,0 +1,42 @@
+// The small-launch form of the tensor-core convolution (conv_small.cu), chosen and prepared by
+// cvmk_conv2d_tc_prepare().
+#pragma once
+#include "tc_common.cuh"
+
+namespace cvmk {
+
+struct SmallConvParams {
+  void* y;
+  int y_dtype;
+  int m_total, oc, oh, ow;
+  int c, kw;
+  int stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
+  int a_mode;                     // 0 plain 2-D tiles (1x1, dense), 1 im2col-mode TMA, 2 spatial patches
+  int patch_w, patch_h, patch_n, patch_w_log2, patch_h_log2, tiles_w, tiles_h;
+  int block_k, block_n, stages;
+  int num_n_tiles;
+  int units;                      // (filter tap, channel block) pairs of the whole reduction
+  int split;                      // CTAs of a cluster, each reducing units / split of them
+  int tmem_cols;
+  tc::FastDiv fd_n_tiles, fd_tiles_w, fd_tiles_h, fd_ohow, fd_ow, fd_cblocks, fd_kw;
+  int* status;
+  const int32_t* bias;
+  int bias_static, first_step;
+  const int8_t* res;              // int8 operand of a fused tensor add / subtract (step res_step), or nullptr
+  int res_step;
+  int fast_variant;               // -1: the chain step by step; else as in conv_tc.cu (+ 8: wide)
+  int f_mul, f_add, f_pre_lo, f_pre_hi;
+  tc::FastQ fq;
+  DevChain chain;
+};
+
+constexpr int SMALL_MAX_STAGES = 12;
+constexpr int SMALL_MAX_N = 128;
+
+// Dynamic shared memory of a launch.
+inline int small_smem_bytes(int block_k, int block_n, int stages, int split) {
+  return 1024 + stages * (tc::BLOCK_M + block_n) * block_k + (split > 1 ? tc::BLOCK_M * block_n * 4 : 0);
+}
+int launch_conv_small(const CUtensorMap& a, const CUtensorMap& b, const SmallConvParams& p, int grid, int smem, cudaStream_t stream);
+
+}  // namespace cvmk

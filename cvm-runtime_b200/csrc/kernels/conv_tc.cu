@@ -35,6 +35,7 @@
 #include <string.h>
 #include <algorithm>
 #include "common.cuh"
+#include "conv_small.cuh"
 #include "tc_common.cuh"
 
 namespace cvmk {
@@ -53,25 +54,6 @@ constexpr int IO_WARP = 2 + NUM_EPI_WARPS;
 constexpr int PRODUCER2_WARP = IO_WARP + 1;
 constexpr int SMEM_DYNAMIC_MAX = 227 * 1024 - 8704;  // 227 KB per CTA minus the static part (bias, barriers)
 constexpr int MAX_BIAS = 2048;          // bias vectors up to this length are staged in shared memory
-
-// Division of a non-negative 31-bit number by a divisor fixed at launch: q = umulhi(n, mul) >> shr
-// (mul = ceil(2^(31 + ceil(log2 d)) / d)); d = 1 is flagged by mul = 0.  Every thread that walks
-// tiles divides several times per tile, and a hardware-emulated 32-bit division is a dependent
-// chain of some twenty instructions.
-struct FastDiv { uint32_t mul, shr; };
-__device__ __forceinline__ int fdiv(int n, const FastDiv& d) {
-  return d.mul ? (int)(__umulhi((uint32_t)n, d.mul) >> d.shr) : n;
-}
-inline FastDiv make_fastdiv(int d) {
-  FastDiv f = {0, 0};
-  if (d <= 1) return f;
-  int lg = 0;
-  while ((1LL << lg) < d) ++lg;
-  const int pw = 31 + lg;
-  f.mul = (uint32_t)((((uint64_t)1 << pw) + (uint64_t)d - 1) / (uint64_t)d);
-  f.shr = (uint32_t)(pw - 32);
-  return f;
-}
 
 struct ConvParams {
   void* y;
@@ -368,13 +350,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
+  if (warp == 1) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);   // before this CTA lets the next kernel start
   // Programmatic dependent launch: the next kernel of the stream may start its own prologue on SMs
   // this grid has left.  Until griddepcontrol.wait returns, the previous kernel of the stream may
   // still be running, so only memory that no kernel writes is touched before it: the tensor maps
   // and the parameter block (both in the kernel's own argument space), the weights, and the bias
   // when it is a model parameter.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (warp == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp == IO_WARP) {
     // Warm the descriptor cache with the tensor maps.
     if (lane < 4) {
@@ -1126,6 +1108,36 @@ bool grouped_supported(const cvmk_conv_desc& d) {
   return halo_tiles_fit(d);
 }
 
+// Which launches go to the small-launch kernel, and how it cuts them.
+struct SmallChoice { int split, block_n, stages; };   // split 0: the persistent kernel
+
+SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int patch_h, int patch_n) {
+  SmallChoice c = {0, 0, 0};
+  if (d.groups > 1 || dev_env("CVM_B200_NO_SMALL")) return c;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaGetLastError();
+  int64_t m_tiles = ((int64_t)d.N * d.OH * d.OW + BLOCK_M - 1) / BLOCK_M;
+  if (a_mode >= 2) {
+    if (a_mode == 3 && !pick_patch(d, &patch_w, &patch_h, &patch_n)) return c;
+    m_tiles = (int64_t)((d.OW + patch_w - 1) / patch_w) * ((d.OH + patch_h - 1) / patch_h) * ((d.N + patch_n - 1) / patch_n);
+  }
+  const int bk = pick_block_k(d.C), units = d.KH * d.KW * (d.C / bk);
+  int bn = d.OC <= 32 ? 32 : 64;
+  if (const char* e = dev_env("CVM_B200_SMALL_N")) bn = atoi(e);
+  const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
+  if (tiles > sms && !dev_env("CVM_B200_SMALL_FORCE")) return c;
+  int split = 1;
+  while (split < 8 && units >= 4 * split && tiles * 2 * split <= sms) split *= 2;
+  if (const char* e = dev_env("CVM_B200_SMALL_SPLIT")) { split = atoi(e); while (split > units) split /= 2; }
+  // half of an SM's shared memory, so that the next layer's CTA fits beside this one
+  int stages = (units + split - 1) / split;
+  if (stages > SMALL_MAX_STAGES) stages = SMALL_MAX_STAGES;
+  while (stages > 1 && small_smem_bytes(bk, bn, stages, split) > 112 * 1024) --stages;
+  c.split = split; c.block_n = bn; c.stages = stages;
+  return c;
+}
+
 }  // namespace
 }  // namespace cvmk
 
@@ -1168,6 +1180,7 @@ static int pick_k_slices(const cvmk_conv_desc& d, int bk, int bn) {
 
 extern "C" int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d) {
   if (!d || !cvmk_conv2d_tc_supported(d)) return 0;
+  if (is_pointwise(*d) && choose_small(*d, 0, 0, 0, 0).split > 0) return 0;   // cut over clusters instead
   const int s = pick_k_slices(*d, pick_block_k(d->C), pick_block_n(d->OC));
   return s > 1 ? (int64_t)d->N * d->OH * d->OW * s * d->OC * 4 : 0;
 }
@@ -1250,6 +1263,16 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
       bk = 64;
     }
   }
+  // The small-launch kernel (conv_small.cu): no halo form, its own tile width and K block.
+  const SmallChoice small = choose_small(*d, plan->a_im2col, patch_w, patch_h, patch_n);
+  if (small.split > 0) {
+    halo = false;
+    bk = pick_block_k(d->C);
+    bn = small.block_n;
+    if (plan->a_im2col == 3) { plan->a_im2col = 2; pick_patch(*d, &patch_w, &patch_h, &patch_n); }
+    plan->block_n = bn;
+  }
+  plan->small_split = small.split;
   plan->reserved[0] = patch_w; plan->reserved[1] = patch_h; plan->reserved[2] = patch_n;
 
   // Output path: int8 tiles leave through shared memory and a TMA store; the first int8 tensor
@@ -1258,11 +1281,11 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   {
     const int ks = pick_k_slices(*d, bk, bn);
     const int64_t need = (int64_t)d->N * d->OH * d->OW * ks * d->OC * 4;
-    plan->k_slices = (ks > 1 && d->workspace && d->workspace_bytes >= need && ((uintptr_t)d->workspace & 15) == 0) ? ks : 1;
+    plan->k_slices = (!small.split && ks > 1 && d->workspace && d->workspace_bytes >= need && ((uintptr_t)d->workspace & 15) == 0) ? ks : 1;
   }
-  plan->tma_out = plan->k_slices == 1 && d->y_dtype == CVMK_I8 && d->OC % 32 == 0 && !dev_env("CVM_B200_NO_TMA_STORE");
+  plan->tma_out = !small.split && plan->k_slices == 1 && d->y_dtype == CVMK_I8 && d->OC % 32 == 0 && !dev_env("CVM_B200_NO_TMA_STORE");
   plan->res_step = -1;
-  if (plan->tma_out) {
+  if (plan->tma_out || (small.split && d->y_dtype == CVMK_I8 && d->OC % 32 == 0)) {
     for (int i = 0; i < d->ep.n; ++i) {
       const cvmk_ep_step& s = d->ep.s[i];
       if ((s.op == CVMK_EP_ADD_T || s.op == CVMK_EP_SUB_T || s.op == CVMK_EP_RSUB_T) &&
@@ -1326,7 +1349,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // (K x block_n bytes) in shared memory; the ring then carries activations only, a third or a
   // fifth of the bytes.  Taken when the weights leave room for a ring of at least four A blocks.
   plan->b_resident = 0;
-  if (plan->a_im2col == 0 && plan->k_slices == 1 && !dev_env("CVM_B200_NO_RESIDENT_B")) {
+  if (!small.split && plan->a_im2col == 0 && plan->k_slices == 1 && !dev_env("CVM_B200_NO_RESIDENT_B")) {
     int sms = 148, dev0 = 0;
     if (cudaGetDevice(&dev0) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev0);
     const int64_t m_tiles = ((int64_t)d->N * d->OH * d->OW + BLOCK_M - 1) / BLOCK_M;
@@ -1360,6 +1383,10 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   plan->stages = stages;
   plan->ring_bytes = resident + stages * stage_bytes;  // resident weights (a_im2col 4) sit in front of the ring
   plan->smem_bytes = plan->ring_bytes + io_bytes + 1024;
+  if (small.split > 0) {
+    plan->stages = small.stages;
+    plan->smem_bytes = small_smem_bytes(bk, bn, small.stages, small.split);
+  }
 
   const int64_t m_total = (int64_t)d->N * d->OH * d->OW;
   const int64_t k_total = (int64_t)d->KH * d->KW * cg;
@@ -1413,6 +1440,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int64_t tiles = num_m_tiles * num_n_tiles * plan->k_slices;
   plan->grid = (int)(tiles < sms ? tiles : sms);
+  if (small.split > 0) plan->grid = (int)(tiles * small.split);
   if (grouped && plan->a_im2col == 4) plan->grid = (int)(plan->grid / num_n_tiles * num_n_tiles);   // tile t + k * grid: same group as t
   return CVMK_OK;
 }
@@ -1516,7 +1544,9 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
 
   // Packed requantisation: chain = [bias] rs_clamp [add_t|sub_t (the TMA-served operand) clip].
   p.fast_mode = 0;
-  if (p.tma_out && d.acc_bound > 0 && d.OC <= MAX_BIAS && !dev_env("CVM_B200_NO_FAST_REQUANT")) {
+  const bool small = plan->small_split > 0;
+  const bool packed_out = small ? (d.y_dtype == CVMK_I8 && d.OC % 32 == 0) : (p.tma_out && d.OC <= MAX_BIAS);
+  if (packed_out && d.acc_bound > 0 && !dev_env("CVM_B200_NO_FAST_REQUANT")) {
     const int i0 = p.first_step;
     const int left = p.chain.n - i0;
     if (left >= 1 && p.chain.s[i0].op == K_RS_CLAMP) {
@@ -1556,6 +1586,36 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
         }
       }
     }
+  }
+
+  if (small) {
+    SmallConvParams q;
+    memset(&q, 0, sizeof(q));
+    q.y = p.y; q.y_dtype = p.y_dtype; q.m_total = p.m_total; q.oc = p.oc; q.oh = p.oh; q.ow = p.ow;
+    q.c = p.c; q.kw = p.kw;
+    q.stride_h = p.stride_h; q.stride_w = p.stride_w; q.pad_h = p.pad_h; q.pad_w = p.pad_w; q.dil_h = p.dil_h; q.dil_w = p.dil_w;
+    q.a_mode = p.a_mode;
+    q.patch_w = p.patch_w; q.patch_h = p.patch_h; q.patch_n = p.patch_n;
+    q.patch_w_log2 = p.patch_w_log2; q.patch_h_log2 = p.patch_h_log2; q.tiles_w = p.tiles_w; q.tiles_h = p.tiles_h;
+    q.block_k = p.block_k; q.block_n = p.block_n; q.stages = p.stages;
+    q.num_n_tiles = p.num_n_tiles; q.units = p.num_units; q.split = plan->small_split;
+    q.tmem_cols = 32;
+    while (q.tmem_cols < q.block_n) q.tmem_cols *= 2;
+    q.fd_n_tiles = p.fd_n_tiles; q.fd_tiles_w = p.fd_tiles_w; q.fd_tiles_h = p.fd_tiles_h; q.fd_ohow = p.fd_ohow; q.fd_ow = p.fd_ow;
+    q.fd_cblocks = make_fastdiv(p.c / p.block_k);
+    q.fd_kw = make_fastdiv(p.kw);
+    q.status = p.status; q.bias = p.bias; q.bias_static = p.bias_static; q.first_step = p.first_step;
+    q.res_step = p.res_step;
+    q.res = p.res_step >= 0 ? reinterpret_cast<const int8_t*>(p.chain.s[p.res_step].ptr) : nullptr;
+    q.fast_variant = p.fast_mode ? p.fast_variant + 8 * p.fast_wide : -1;
+    if (p.fast_mode == 1) q.res = nullptr;
+    q.f_mul = p.f_mul; q.f_add = p.f_add; q.f_pre_lo = p.f_pre_lo; q.f_pre_hi = p.f_pre_hi;
+    q.fq = {p.f_lo1, p.f_hi1, p.f_lo2, p.f_hi2};
+    q.chain = p.chain;
+    CUtensorMap sa, sb;
+    memcpy(&sa, plan->tmap_a, sizeof(sa));
+    memcpy(&sb, plan->tmap_b, sizeof(sb));
+    return launch_conv_small(sa, sb, q, plan->grid, plan->smem_bytes, (cudaStream_t)stream);
   }
 
   static bool attr_set_dev[64] = {false};

@@ -15,6 +15,25 @@ constexpr uint32_t SPIN_LIMIT = 1u << 19;  // x 2 us per hardware wait
 __device__ uint32_t g_wait_hint = 2000u;  // development builds: suspend-time hint of the waits, settable
 #endif
 
+// Division of a non-negative 31-bit number by a divisor fixed at launch: q = umulhi(n, mul) >> shr
+// (mul = ceil(2^(31 + ceil(log2 d)) / d)); d = 1 is flagged by mul = 0.  Every thread that walks
+// tiles divides several times per tile, and a hardware-emulated 32-bit division is a dependent
+// chain of some twenty instructions.
+struct FastDiv { uint32_t mul, shr; };
+__device__ __forceinline__ int fdiv(int n, const FastDiv& d) {
+  return d.mul ? (int)(__umulhi((uint32_t)n, d.mul) >> d.shr) : n;
+}
+inline FastDiv make_fastdiv(int d) {
+  FastDiv f = {0, 0};
+  if (d <= 1) return f;
+  int lg = 0;
+  while ((1LL << lg) < d) ++lg;
+  const int pw = 31 + lg;
+  f.mul = (uint32_t)((((uint64_t)1 << pw) + (uint64_t)d - 1) / (uint64_t)d);
+  f.shr = (uint32_t)(pw - 32);
+  return f;
+}
+
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers
 // ---------------------------------------------------------------------------------------------

@@ -169,7 +169,8 @@ typedef struct __attribute__((aligned(64))) {
   int32_t reserved[4];  /* [0..2] patch width / height / images (a_im2col = 2, 3), [3] (tap, channel block) units per ring stage */
   int32_t k_slices;   /* > 1: the reduction is cut into this many slices (see cvmk_conv_desc.workspace) */
   int32_t b_resident; /* 1: 1x1 layer, every CTA keeps its N tile of the weights in shared memory */
-  int32_t pad_[2];
+  int32_t small_split; /* > 0: the small-launch kernel, each tile's reduction cut over a cluster of so many CTAs */
+  int32_t pad_[1];
 } cvmk_conv_plan;
 
 CVMK_API int cvmk_conv2d_tc_supported(const cvmk_conv_desc* d);
