@@ -5,15 +5,16 @@
 // layer over 512 channels is 36 dependent K blocks, 10 us), and its set-up and hand-overs between
 // eight epilogue warps, staging buffers and the store engine cost several microseconds a launch.
 // What bounds such a layer is latency, so here
-//   - a tile is 128 x 64 (or 32 / 128), one CTA each, and the reduction is cut over a CLUSTER of up
+//   - a tile is 128 x 64 or 128 x 32, one CTA each, and the reduction is cut over a CLUSTER of up
 //     to eight CTAs, each of which multiplies its share of the (filter tap, channel block) units;
 //   - the partial sums (int32: exact in any order) are exchanged through distributed shared memory:
-//     rank r of the cluster finishes rows [r * 128 / split, ...) of the tile, so every CTA of the
-//     cluster has the same share of the requantisation and of the stores;
+//     every rank finishes a run of the tile's rows and receives that run from the others by bulk
+//     copies (8 KB each; written element by element with st.shared::cluster the exchange ran at 16
+//     bytes a clock, 1.2 us), so every CTA of the cluster has the same share of the
+//     requantisation and of the stores, eight columns a thread;
 //   - the weights of the first ring stages are requested BEFORE griddepcontrol.wait (they are model
 //     parameters), i.e. while the previous layer still runs, and so is the bias; a CTA takes at most
 //     half of an SM's shared memory so that two layers fit beside each other;
-//   - results are stored straight from registers.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <string.h>
@@ -24,10 +25,15 @@ namespace {
 
 using namespace tc;
 
-constexpr int THREADS = 192;   // warp 0: TMA, warp 1: MMA + TMEM, warps 2..5: epilogue
+constexpr int THREADS = 320;   // warp 0: TMA, warp 1: MMA + TMEM, warps 2..9: epilogue
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// (relaxed: the barriers' initialisation is released by its own fence, and the second use only says that
+//  memory is no longer read; an arrive with release semantics waited half a microsecond for earlier stores)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// A value that is the same for the whole warp, out of a shuffle: the compiler then keeps it (and what is
+// computed from it) in uniform registers, where TMA and tensor instructions take their operands.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -39,86 +45,98 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
   return d;
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, int a, int b, int c, int d) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+// Copies `bytes` of this CTA's shared memory to `dst` (an address of the cluster window) and reports them
+// to the mbarrier `bar` of the receiving CTA.
+__device__ __forceinline__ void bulk_to_rank(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
 }
 
-template <int RELU1, int KIND>
-__device__ __forceinline__ void requant_case(const SmallConvParams& p, const int32_t (&v)[32], const uint4& r0, const uint4& r1,
-                                             uint4* a, uint4* b) {
-  fast_requant<RELU1, KIND>(p.fq, v, r0, r1, a, b);
-}
-
-// Bias, chain and store of 32 columns of one output row.  `row` is a linear output row inside the
-// tensor; columns past OC (a multiple of 8) are left alone.  r0, r1: the tensor operand's 32 bytes.
-__device__ __forceinline__ void finish_chunk(const SmallConvParams& p, int32_t (&v)[32], int row, int col0, const int32_t* bias_s,
-                                             const uint4& r0, const uint4& r1) {
-  const size_t lin = (size_t)row * p.oc + col0;
+// Packed requantisation of V columns of one row (see fast_requant): OC is a multiple of 32 and the
+// output int8 on this path.  `res`: the tensor operand's bytes.
+template <int V>
+__device__ __forceinline__ void requant(const SmallConvParams& p, const int32_t* v, const int32_t* bias_s, const uint32_t* res, uint32_t* w) {
   const int4* bp = reinterpret_cast<const int4*>(bias_s);
-  if (p.fast_variant >= 0) {   // OC is a multiple of 32 and the output int8 on this path
-    if (p.fast_variant >= 8) {
-      const int lo = p.f_pre_lo, hi = p.f_pre_hi, mul = p.f_mul, am = p.f_add * p.f_mul;
+  const int mul = p.f_mul;
+  const int kind = (p.fast_variant & 7) >> 1;   // 0 no tensor step, 1 and 2 add, 3 subtract
+  const bool wide = p.fast_variant >= 8;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int4 t = bp[j];
-        v[4 * j] = min(max(v[4 * j] + t.x, lo), hi) * mul + am;
-        v[4 * j + 1] = min(max(v[4 * j + 1] + t.y, lo), hi) * mul + am;
-        v[4 * j + 2] = min(max(v[4 * j + 2] + t.z, lo), hi) * mul + am;
-        v[4 * j + 3] = min(max(v[4 * j + 3] + t.w, lo), hi) * mul + am;
-      }
+  for (int q = 0; q < V / 4; ++q) {
+    const int4 t = bp[q];
+    int a = v[4 * q], b = v[4 * q + 1], c = v[4 * q + 2], d = v[4 * q + 3];
+    if (wide) {
+      const int lo = p.f_pre_lo, hi = p.f_pre_hi, am = p.f_add * mul;
+      a = min(max(a + t.x, lo), hi) * mul + am;
+      b = min(max(b + t.y, lo), hi) * mul + am;
+      c = min(max(c + t.z, lo), hi) * mul + am;
+      d = min(max(d + t.w, lo), hi) * mul + am;
     } else {
-      const int mul = p.f_mul;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int4 t = bp[j];
-        v[4 * j] = v[4 * j] * mul + t.x;
-        v[4 * j + 1] = v[4 * j + 1] * mul + t.y;
-        v[4 * j + 2] = v[4 * j + 2] * mul + t.z;
-        v[4 * j + 3] = v[4 * j + 3] * mul + t.w;
-      }
+      a = a * mul + t.x;
+      b = b * mul + t.y;
+      c = c * mul + t.z;
+      d = d * mul + t.w;
     }
-    uint4 a, b;
-    switch (p.fast_variant & 7) {
-      case 0: requant_case<0, 0>(p, v, r0, r1, &a, &b); break;
-      case 1: requant_case<1, 0>(p, v, r0, r1, &a, &b); break;
-      case 2: requant_case<0, 1>(p, v, r0, r1, &a, &b); break;
-      case 3: requant_case<1, 1>(p, v, r0, r1, &a, &b); break;
-      case 4: requant_case<0, 2>(p, v, r0, r1, &a, &b); break;
-      case 5: requant_case<1, 2>(p, v, r0, r1, &a, &b); break;
-      case 6: requant_case<0, 3>(p, v, r0, r1, &a, &b); break;
-      default: requant_case<1, 3>(p, v, r0, r1, &a, &b); break;
+    uint32_t h0 = __byte_perm((uint32_t)a, (uint32_t)b, 0x7632);
+    uint32_t h1 = __byte_perm((uint32_t)c, (uint32_t)d, 0x7632);
+    h0 = __vmaxs2(__vmins2(h0, p.fq.f_hi1), p.fq.f_lo1);
+    h1 = __vmaxs2(__vmins2(h1, p.fq.f_hi1), p.fq.f_lo1);
+    if (kind != 0) {
+      const uint32_t ra = prmt(res[q], 0, 0x9180), rb = prmt(res[q], 0, 0xB3A2);
+      h0 = kind == 3 ? __vsub2(h0, ra) : __vadd2(h0, ra);
+      h1 = kind == 3 ? __vsub2(h1, rb) : __vadd2(h1, rb);
+      h0 = __vmaxs2(__vmins2(h0, p.fq.f_hi2), p.fq.f_lo2);
+      h1 = __vmaxs2(__vmins2(h1, p.fq.f_hi2), p.fq.f_lo2);
     }
-    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<int8_t*>(p.y) + lin);
-    dst[0] = a;
-    dst[1] = b;
-    return;
+    w[q] = __byte_perm(h0, h1, 0x6420);
   }
-  if (p.bias) {
+}
+
+// Bias, chain step by step and store of 8 columns of one output row (OC is a multiple of 8: all of them
+// or none exist).
+template <int V>
+__device__ __forceinline__ void by_steps(const SmallConvParams& p, const int32_t* v, int row, int col0, const int32_t* bias_s) {
+  if (col0 >= p.oc) return;
+  const size_t lin = (size_t)row * p.oc + col0;
+  int32_t t[V];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int4 t = bp[j];
-      v[4 * j] += t.x; v[4 * j + 1] += t.y; v[4 * j + 2] += t.z; v[4 * j + 3] += t.w;
-    }
+  for (int j = 0; j < V; ++j) t[j] = v[j] + bias_s[j];   // zeros without a bias
+  apply_chain<V>(p.chain, t, lin, col0, 1, nullptr, -1, p.first_step);
+  if (p.y_dtype == CVMK_I8) {
+    *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.y) + lin) = make_uint2(pack4(t[0], t[1], t[2], t[3]), pack4(t[4], t[5], t[6], t[7]));
+  } else {
+    int4* dst = reinterpret_cast<int4*>(reinterpret_cast<int32_t*>(p.y) + lin);
+    dst[0] = make_int4(t[0], t[1], t[2], t[3]);
+    dst[1] = make_int4(t[4], t[5], t[6], t[7]);
   }
-  // step by step, eight columns at a time (OC is a multiple of 8: all of them or none exist)
+}
+
+// The products of G units of NK K-steps each, in one straight line behind one predicate: 50 cycles an
+// instruction (its own run time); with a loop in the elected lane's branch it was 80.
+template <int G, int NK>
+__device__ __forceinline__ void issue_steps(bool leader, uint32_t d, uint32_t al, uint32_t hi, uint32_t a_q, uint32_t unit_q, uint32_t idesc,
+                                            uint32_t first) {
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    if (col0 + g * 8 >= p.oc) break;
-    int32_t t[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) t[j] = v[g * 8 + j];
-    apply_chain<8>(p.chain, t, lin + g * 8, col0 + g * 8, 1, nullptr, -1, p.first_step);
-    if (p.y_dtype == CVMK_I8) {
-      uint2 o;
-      o.x = pack4(t[0], t[1], t[2], t[3]);
-      o.y = pack4(t[4], t[5], t[6], t[7]);
-      *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.y) + lin + g * 8) = o;
-    } else {
-      int4* dst = reinterpret_cast<int4*>(reinterpret_cast<int32_t*>(p.y) + lin + g * 8);
-      dst[0] = make_int4(t[0], t[1], t[2], t[3]);
-      dst[1] = make_int4(t[4], t[5], t[6], t[7]);
-    }
+  for (int k = 0; k < G; ++k) {
+    if (leader) mma_i8_k<NK>(d, al, hi, al + a_q, hi, idesc, k == 0 ? first : 1u);
+    al += unit_q;
   }
+}
+template <int G>
+__device__ __forceinline__ void issue_units(bool leader, int nk, uint32_t d, uint32_t al, uint32_t hi, uint32_t a_q, uint32_t unit_q,
+                                            uint32_t idesc, uint32_t first) {
+  if (nk == 4) issue_steps<G, 4>(leader, d, al, hi, a_q, unit_q, idesc, first);
+  else if (nk == 2) issue_steps<G, 2>(leader, d, al, hi, a_q, unit_q, idesc, first);
+  else issue_steps<G, 1>(leader, d, al, hi, a_q, unit_q, idesc, first);
 }
 
 __global__ void __launch_bounds__(THREADS)
@@ -128,6 +146,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __shared__ uint64_t bar_full[SMALL_MAX_STAGES];
   __shared__ uint64_t bar_empty[SMALL_MAX_STAGES];
   __shared__ uint64_t bar_acc;
+  __shared__ uint64_t bar_part;   // this CTA's rows of every rank's partial sums have landed
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   __shared__ __align__(16) int32_t bias_s[SMALL_MAX_N];
@@ -136,28 +155,50 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int split = p.split;
-  const int rank = split > 1 ? (int)cluster_rank() : 0;
-  const int tile = split > 1 ? (int)blockIdx.x / split : (int)blockIdx.x;
+  const int rank = uniform(split > 1 ? (int)cluster_rank() : 0);
+  const int tile = (int)blockIdx.x >> p.split_log2;
   const int a_bytes = BLOCK_M * p.block_k, b_bytes = p.block_n * p.block_k;
-  const int stage_bytes = a_bytes + b_bytes;
-  const int u0 = rank * p.units / split, u1 = (rank + 1) * p.units / split;
-  const int mine = u1 - u0;
+  const int unit_bytes = a_bytes + b_bytes, stage_bytes = p.group * unit_bytes;   // a ring stage is `group` units: one barrier
+  const int u0 = (rank * p.units) >> p.split_log2;
+  const int mine = (((rank + 1) * p.units) >> p.split_log2) - u0;
   // tile origin
-  const int mt = fdiv(tile, p.fd_n_tiles);
+  const int mt = uniform(fdiv(tile, p.fd_n_tiles));
   const int n0 = (tile - mt * p.num_n_tiles) * p.block_n;
   const int m0 = mt * BLOCK_M;
   int cw = 0, ch = 0, cn = 0;
   if (p.a_mode == 2) {
-    const int r = fdiv(mt, p.fd_tiles_w);
+    const int r = uniform(fdiv(mt, p.fd_tiles_w));
     cw = (mt - r * p.tiles_w) * p.patch_w;
-    cn = fdiv(r, p.fd_tiles_h);
+    cn = uniform(fdiv(r, p.fd_tiles_h));
     ch = (r - cn * p.tiles_h) * p.patch_h;
     cn *= p.patch_n;
   }
+  int img = 0, base_w = 0, base_h = 0;
+  if (p.a_mode == 1) {
+    img = uniform(fdiv(m0, p.fd_ohow));
+    const int rem = m0 - img * (p.oh * p.ow);
+    const int oy = uniform(fdiv(rem, p.fd_ow));
+    base_w = (rem - oy * p.ow) * p.stride_w - p.pad_w;
+    base_h = oy * p.stride_h - p.pad_h;
+  }
 
-  if (split > 1) cluster_arrive();   // (waited for before anything is written into another CTA)
+  touch_params(p);
   const bool leader = elect_one();
-  const uint32_t ring = smem_u32(smem);
+  const uint32_t ring = smem_u32(smem), full0 = smem_u32(&bar_full[0]);
+  const int groups = (mine + p.group - 1) / p.group;
+  // announces the bytes of group `g` in ring stage `s` and requests its weights (the elected lane)
+  auto load_b = [&](int s, int g) {
+    const int i0 = g * p.group, n = min(p.group, mine - i0);
+    uint32_t sb = ring + (uint32_t)(s * stage_bytes + a_bytes);
+    const uint32_t bar = full0 + 8u * (uint32_t)s;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(n * unit_bytes)) : "memory");
+    int col = (u0 + i0) * p.block_k;
+    for (int k = 0; k < n; ++k, sb += (uint32_t)unit_bytes, col += p.block_k)
+      asm volatile(
+          "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sb), "l"(reinterpret_cast<uint64_t>(&tmap_b)), "r"(bar), "r"(col), "r"(n0)
+          : "memory");
+  };
   if (warp == 0) {
     if (leader) {
       for (int s = 0; s < p.stages; ++s) {
@@ -165,17 +206,17 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         mbar_init(&bar_empty[s], 1);
       }
       mbar_init(&bar_acc, 1);
+      mbar_init(&bar_part, 1 + (THREADS - 64) / 32);
       abort_flag = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
+    if (leader) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_a)) : "memory");
     // the weights of the first stages: parameters, no kernel writes them
-    const int first = min(p.stages, mine);
-    for (int i = 0; i < first; ++i)
-      if (leader) {
-        mbar_expect_tx(&bar_full[i], (uint32_t)stage_bytes);
-        tma_load_2d(smem + i * stage_bytes + a_bytes, &tmap_b, &bar_full[i], (u0 + i) * p.block_k, n0);
-      }
+    const int first = min(p.stages, groups);
+    if (leader)
+      for (int i = 0; i < first; ++i) load_b(i, i);
+    __syncwarp();
   } else if (warp == 1) {
     // (the next kernel may start only once this CTA has its TMEM columns: it could take them, and then
     //  wait for this kernel's end)
@@ -184,7 +225,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else {
     const bool early = p.bias_static != 0;
     if (!early) pdl_wait();
-    for (int i = (int)threadIdx.x - 64; i < p.block_n; i += 128) {
+    for (int i = (int)threadIdx.x - 64; i < p.block_n; i += THREADS - 64) {
       const int32_t b = (p.bias && n0 + i < p.oc) ? __ldg(p.bias + n0 + i) : 0;
       // packed requantisation: (bias + rounding addend) pre-multiplied, see fast_requant()
       bias_s[i] = (p.fast_variant >= 0 && p.fast_variant < 8) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
@@ -193,177 +234,299 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = (uint32_t)uniform((int)tmem_slot);
+  if (split > 1) cluster_arrive();   // this CTA's barriers exist (waited for before anything is sent to it)
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA
-    int img = 0, base_w = 0, base_h = 0;
-    if (p.a_mode == 1) {
-      img = fdiv(m0, p.fd_ohow);
-      const int rem = m0 - img * (p.oh * p.ow);
-      const int oy = fdiv(rem, p.fd_ow);
-      base_w = (rem - oy * p.ow) * p.stride_w - p.pad_w;
-      base_h = oy * p.stride_h - p.pad_h;
-    }
-    // first unit: filter tap and channel block
-    int tap = fdiv(u0, p.fd_cblocks);
-    int cc = (u0 - tap * (p.c / p.block_k)) * p.block_k;
+    // Units in weight-matrix order: channel blocks, filter columns, filter rows.  The first lap of the
+    // ring, whose stages are free, is a loop of the elected lane with nothing in it but the
+    // load and three counters (about 20 cycles a load; with waits, divisions and the choice of
+    // the load's kind in the loop it took 350, more than the loads themselves).
+    const int tap = fdiv(u0, p.fd_cblocks);
+    int cc = (u0 - tap * p.cblocks) * p.block_k;
     int fy = fdiv(tap, p.fd_kw), fx = tap - fy * p.kw;
-    pdl_wait();
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int i = 0; i < mine; ++i) {
-      uint8_t* sa = smem + stage * stage_bytes;
-      uint64_t* bar = &bar_full[stage];
-      if (i >= p.stages) {
-        if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) break;
-        if (leader) {
-          mbar_expect_tx(bar, (uint32_t)stage_bytes);
-          tma_load_2d(sa + a_bytes, &tmap_b, bar, (u0 + i) * p.block_k, n0);
-        }
-      }
-      if (leader) {
-        const int off_w = fx * p.dil_w, off_h = fy * p.dil_h;
-        if (p.a_mode == 2) tma_load_4d(sa, &tmap_a, bar, cc, cw + off_w - p.pad_w, ch + off_h - p.pad_h, cn);
-        else if (p.a_mode == 1) tma_load_im2col_4d(sa, &tmap_a, bar, cc, base_w, base_h, img, (uint16_t)off_w, (uint16_t)off_h);
-        else tma_load_2d(sa, &tmap_a, bar, cc, m0);
-      }
+    const int lap0 = min(p.stages * p.group, mine);
+    auto step = [&]() {
       cc += p.block_k;
       if (cc >= p.c) { cc = 0; if (++fx == p.kw) { fx = 0; ++fy; } }
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+    };
+    auto patch = [&](uint32_t sa, uint32_t bar) {
+      asm volatile(
+          "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+          " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc),
+          "r"(cw + fx * p.dil_w - p.pad_w), "r"(ch + fy * p.dil_h - p.pad_h), "r"(cn)
+          : "memory");
+    };
+    auto im2col = [&](uint32_t sa, uint32_t bar) {
+      asm volatile(
+          "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+          " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc),
+          "r"(base_w), "r"(base_h), "r"(img), "h"((uint16_t)(fx * p.dil_w)), "h"((uint16_t)(fy * p.dil_h))
+          : "memory");
+    };
+    auto plain = [&](uint32_t sa, uint32_t bar) {
+      asm volatile(
+          "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc), "r"(m0)
+          : "memory");
+    };
+    pdl_wait();
+    if (leader) {
+      uint32_t sa = ring, bar = full0;
+      int k = 0;
+      auto next = [&]() {
+        sa += (uint32_t)unit_bytes;
+        if (++k == p.group) { k = 0; bar += 8; }
+        step();
+      };
+      if (p.a_mode == 2) for (int i = 0; i < lap0; ++i, next()) patch(sa, bar);
+      else if (p.a_mode == 1) for (int i = 0; i < lap0; ++i, next()) im2col(sa, bar);
+      else for (int i = 0; i < lap0; ++i, next()) plain(sa, bar);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int g = p.stages; g < groups; ++g) {
+        if (!mbar_wait(&bar_empty[stage], phase, &abort_flag, 1)) break;
+        load_b(stage, g);
+        sa = ring + (uint32_t)(stage * stage_bytes);
+        bar = full0 + 8u * (uint32_t)stage;
+        for (int i = g * p.group; i < min(mine, (g + 1) * p.group); ++i, sa += (uint32_t)unit_bytes, step()) {
+          if (p.a_mode == 2) patch(sa, bar);
+          else if (p.a_mode == 1) im2col(sa, bar);
+          else plain(sa, bar);
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA
     const uint32_t idesc = umma_idesc_i8(p.block_n);
     const uint64_t desc0 = umma_desc(ring, p.block_k);
     const uint32_t lo0 = (uint32_t)desc0, hi = (uint32_t)(desc0 >> 32);
-    const uint32_t stage_q = (uint32_t)stage_bytes >> 4, a_q = (uint32_t)a_bytes >> 4;
+    const uint32_t stage_q = (uint32_t)stage_bytes >> 4, unit_q = (uint32_t)unit_bytes >> 4, a_q = (uint32_t)a_bytes >> 4;
     const int nk = p.block_k / 32;
     int stage = 0;
     uint32_t phase = 0;
-    for (int i = 0; i < mine; ++i) {
+    // All lanes run this loop, in uniform registers, and one executes the instructions (alone in its
+    // branch); no tcgen05 fence is needed between a TMA load's barrier and the products of its bytes.
+    for (int g = 0, i = 0; g < groups; ++g) {
       if (!mbar_wait(&bar_full[stage], phase, &abort_flag, 3)) break;
-      tc_fence_after();
+      const int n = min(p.group, mine - i);
       const uint32_t al = lo0 + stage_q * (uint32_t)stage;
-      if (leader) {
-        if (nk == 4) mma_i8_k<4>(tmem_base, al, hi, al + a_q, hi, idesc, (uint32_t)i);
-        else if (nk == 2) mma_i8_k<2>(tmem_base, al, hi, al + a_q, hi, idesc, (uint32_t)i);
-        else mma_i8_k<1>(tmem_base, al, hi, al + a_q, hi, idesc, (uint32_t)i);
-        if (i + p.stages < mine) mma_commit(&bar_empty[stage]);   // (nobody waits for the last ones)
-        if (i + 1 == mine) mma_commit(&bar_acc);
+      if (n == 3) issue_units<3>(leader, nk, tmem_base, al, hi, a_q, unit_q, idesc, (uint32_t)i);
+      else if (n == 2) issue_units<2>(leader, nk, tmem_base, al, hi, a_q, unit_q, idesc, (uint32_t)i);
+      else issue_units<1>(leader, nk, tmem_base, al, hi, a_q, unit_q, idesc, (uint32_t)i);
+      i += n;
+      if (g + p.stages < groups) {   // (nobody waits for the last ones)
+        if (leader) mma_commit(&bar_empty[stage]);
       }
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
-    __syncwarp();
+    if (leader) mma_commit(&bar_acc);
   }
-
   __syncwarp();
 
   // ------------------------------------------------------------------ epilogue
-  const int quarter = warp & 3;
-  const int row_in_tile = quarter * 32 + lane;   // epilogue warps 2..5: TMEM lanes of the warp's quarter
-  const int rows_per = BLOCK_M / split;          // rows this CTA finishes
+  // Warps 2..9: two per quarter of the TMEM lanes, each with half of the tile's columns.
+  const int quarter = warp & 3, half = warp >= 6 ? 1 : 0;
+  const int row_in_tile = quarter * 32 + lane;
+  const int half_n = p.block_n >> 1, c_first = half * half_n;
+  const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c_first;
   auto out_row = [&](int r) {                    // linear output row of tile row r; -1 outside the tensor
     if (p.a_mode != 2) return m0 + r < p.m_total ? m0 + r : -1;
     const int ow = cw + (r & (p.patch_w - 1)), q = r >> p.patch_w_log2;
     const int oh = ch + (q & (p.patch_h - 1)), on = cn + (q >> p.patch_h_log2);
     return (ow < p.ow && oh < p.oh && on * p.oh * p.ow < p.m_total) ? (on * p.oh + oh) * p.ow + ow : -1;
   };
-  const uint4 none = make_uint4(0, 0, 0, 0);
-  auto operand = [&](int row, int col, uint4* r0, uint4* r1) {
-    if (p.res == nullptr || p.fast_variant < 0 || row < 0 || col >= p.oc) return;
-    const uint4* q = reinterpret_cast<const uint4*>(p.res + (size_t)row * p.oc + col);
-    *r0 = q[0];
-    *r1 = q[1];
+  const bool with_res = p.res != nullptr;
+  // The epilogue warps report their last TMEM load; the MMA warp then frees the columns while they go on.
+  auto tmem_done = [&]() {
+    tc_fence_before();
+    asm volatile("bar.arrive 1, %0;" ::"r"(THREADS - 32) : "memory");
   };
-  const int chunks = p.block_n >> 5;
+  auto tmem_free = [&]() {
+    asm volatile("bar.sync 1, %0;" ::"r"(THREADS - 32) : "memory");
+    tc_fence_after();
+    tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+  };
   if (warp >= 2) pdl_wait();
   if (split == 1) {
     if (warp >= 2) {
       const int row = out_row(row_in_tile);
-      uint4 r0 = none, r1 = none;
-      operand(row, n0, &r0, &r1);   // the tensor operand travels while the products are computed
+      const bool packed = p.fast_variant >= 0;
+      // Packed results are turned through the idle operand ring so that a store instruction covers whole
+      // rows of the tile: each warp stores 16 rows of its quarter, `cpr` 16-byte chunks a row.
+      const int cpr_log2 = p.block_n == 64 ? 2 : 1, chunk = lane & ((1 << cpr_log2) - 1);
+      const int st0 = quarter * 32 + half * 16 + (lane >> cpr_log2), st1 = st0 + 8;   // (16 rows: two turns of 8 with 64 columns)
+      const int out0 = out_row(st0), out1 = cpr_log2 == 2 ? out_row(st1) : -1;
+      auto slot = [&](int r, int c) { return smem + r * p.block_n + ((c ^ ((r >> 1) & ((1 << cpr_log2) - 1))) << 4); };
+      // the tensor operand travels while the products are computed
+      uint32_t res[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (with_res && row >= 0 && n0 + c_first < p.oc) {
+        const uint4* q = reinterpret_cast<const uint4*>(p.res + (size_t)row * p.oc + n0 + c_first);
+        const uint4 t = q[0];
+        res[0] = t.x; res[1] = t.y; res[2] = t.z; res[3] = t.w;
+        if (half_n == 32) {
+          const uint4 u = q[1];
+          res[4] = u.x; res[5] = u.y; res[6] = u.z; res[7] = u.w;
+        }
+      }
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar_acc, 0u, &abort_flag, 4));
       tc_fence_after();
       if (ok) {
-        const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        for (int c = 0; c < chunks; ++c) {
-          const int col = n0 + c * 32;
-          if (col >= p.oc) break;
-          int32_t v[32];
-          tmem_ld32(tbase + (uint32_t)(c * 32), v);
-          uint4 q0 = r0, q1 = r1;
-          if (c + 1 < chunks) operand(row, col + 32, &r0, &r1);
-          if (row >= 0) finish_chunk(p, v, row, col, bias_s + c * 32, q0, q1);
+        int32_t v[32];
+        if (half_n == 32) tmem_ld32(tbase, v);
+        else {
+          int32_t t[16];
+          tmem_ld16(tbase, t);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = t[j];
         }
+        tmem_done();
+        const int32_t* bp = bias_s + c_first;
+        if (packed) {
+          uint32_t w[8];
+          requant<16>(p, v, bp, res, w);
+          const int c0 = c_first >> 4;
+          *reinterpret_cast<uint4*>(slot(row_in_tile, c0)) = make_uint4(w[0], w[1], w[2], w[3]);
+          if (half_n == 32) {
+            requant<16>(p, v + 16, bp + 16, res + 4, w + 4);
+            *reinterpret_cast<uint4*>(slot(row_in_tile, c0 + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
+          }
+          asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+          const int col = n0 + chunk * 16;
+          if (col < p.oc) {
+            int8_t* y = reinterpret_cast<int8_t*>(p.y) + col;
+            if (out0 >= 0) *reinterpret_cast<uint4*>(y + (size_t)out0 * p.oc) = *reinterpret_cast<const uint4*>(slot(st0, chunk));
+            if (out1 >= 0) *reinterpret_cast<uint4*>(y + (size_t)out1 * p.oc) = *reinterpret_cast<const uint4*>(slot(st1, chunk));
+          }
+        } else if (row >= 0) {
+          by_steps<8>(p, v, row, n0 + c_first, bp);
+          by_steps<8>(p, v + 8, row, n0 + c_first + 8, bp + 8);
+          if (half_n == 32) {
+            by_steps<8>(p, v + 16, row, n0 + c_first + 16, bp + 16);
+            by_steps<8>(p, v + 24, row, n0 + c_first + 24, bp + 24);
+          }
+        }
+      } else {
+        tmem_done();
       }
+    } else if (warp == 1) {
+      tmem_free();
     }
   } else {
-    cluster_wait();   // every CTA of the cluster has started
-    // Partial sums: tile row r goes to rank r / rows_per, as row r % rows_per of its block from
-    // this rank.  16-byte chunks of a row are XORed with its low bits: lanes hold different rows.
-    uint8_t* part = smem + p.stages * stage_bytes;
+    // The tile's rows up to the last one inside the tensor are dealt to the ranks in runs of rows_per.
+    // Each CTA writes its partial sums of all rows into its (now idle) operand ring and sends every
+    // other rank its run; `part` of the receiver holds one block of its rows from each of them.  16-byte
+    // chunks of a row are XORed with the low bits of its number in the run (lanes hold different rows).
+    // All index arithmetic (divisions among it) is done before the waits it would otherwise follow.
+    int rows = min(BLOCK_M, p.m_total - m0);
+    if (p.a_mode == 2) {
+      const int images = p.images - cn;
+      rows = images >= p.patch_n ? BLOCK_M : images << (p.patch_w_log2 + p.patch_h_log2);
+    }
+    const int rows_per = (rows + split - 1) >> p.split_log2;
+    const int row_bytes = p.block_n * 4;
+    uint8_t* part = smem + small_ring_bytes(p.block_k, p.block_n, p.stages * p.group, split);
+    const int mine_rows = max(0, min(rows_per, rows - rank * rows_per));
+    if (warp == 1 && leader) mbar_expect_tx(&bar_part, (uint32_t)((split - 1) * mine_rows * row_bytes));
     if (warp >= 2) {
+      const int rl = row_in_tile % rows_per;
+      uint8_t* const stage_row = smem + row_in_tile * row_bytes;
+      // the runs (one to five) that the quarter's rows belong to
+      const int r_end = min(rows, quarter * 32 + 32), dest0 = (quarter * 32) / rows_per;
+      // this CTA's rows: eight columns a thread and turn
+      const int t = (int)threadIdx.x - 64, per_row_log2 = 31 - __clz(p.block_n >> 3), per_row = 1 << per_row_log2;
+      const int jobs = mine_rows << per_row_log2;
+      int job_rl = t >> per_row_log2, job_q = t & (per_row - 1);
+      int row = -1;
+      uint32_t res[2] = {0, 0};
+      auto job_row = [&]() {
+        row = out_row(rank * rows_per + job_rl);
+        const int col = n0 + job_q * 8;
+        if (col >= p.oc) row = -1;
+        if (!with_res || row < 0) return;
+        const uint2 q = *reinterpret_cast<const uint2*>(p.res + (size_t)row * p.oc + col);
+        res[0] = q.x; res[1] = q.y;
+      };
+      if (t < jobs) job_row();
+      cluster_wait();   // every CTA of the cluster has started and initialised its barriers
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar_acc, 0u, &abort_flag, 4));
       tc_fence_after();
       if (ok) {
-        const int dest = row_in_tile / rows_per, rl = row_in_tile - dest * rows_per;
-        const uint32_t base = map_rank(smem_u32(part) + (uint32_t)((rank * rows_per + rl) * p.block_n * 4), (uint32_t)dest);
-        const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        const bool live = out_row(row_in_tile) >= 0;
-        for (int c = 0; c < chunks; ++c) {
-          int32_t v[32];
-          tmem_ld32(tbase + (uint32_t)(c * 32), v);
-          if (live) {
+        for (int c = 0; c < half_n; c += 16) {
+          int32_t v[16];
+          tmem_ld16(tbase + (uint32_t)c, v);
+          if (row_in_tile < rows) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              st_cluster_v4(base + (uint32_t)(((c * 8 + j) ^ (rl & 7)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < 4; ++j)
+              *reinterpret_cast<int4*>(stage_row + (((((c_first + c) >> 2) + j) ^ (rl & 7)) << 4)) = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          }
+        }
+        fence_async_smem();
+      }
+      tmem_done();
+      // both warps of a quarter have written its 32 rows: one of them sends the runs they belong to
+      asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+      if (lane == 0) mbar_arrive(&bar_part);   // (this CTA's own run is read where it lies)
+      if (half == 0 && ok && leader) {
+        int r = quarter * 32;
+        for (int dest = dest0; r < r_end; ++dest) {
+          const int run = min(r_end, (dest + 1) * rows_per) - r;
+          const int theirs = min(rows_per, rows - dest * rows_per), block = rank - (rank > dest ? 1 : 0);
+          if (dest != rank)
+            bulk_to_rank(map_rank(smem_u32(part) + (uint32_t)((block * theirs + r - dest * rows_per) * row_bytes), (uint32_t)dest),
+                         smem_u32(smem + r * row_bytes), (uint32_t)(run * row_bytes), map_rank(smem_u32(&bar_part), (uint32_t)dest));
+          r += run;
+        }
+      }
+      __syncwarp();
+      const bool landed = mbar_wait(&bar_part, 0u, &abort_flag, 5);
+      __syncwarp();
+      cluster_arrive();   // what was sent here has left its senders' memory
+      if (landed) {
+        for (int k = t; k < jobs; k += THREADS - 64) {
+          if (k != t) {
+            job_rl = k >> per_row_log2; job_q = k & (per_row - 1);
+            job_row();
+          }
+          if (row < 0) continue;
+          const int o0 = ((2 * job_q) ^ (job_rl & 7)) << 4, o1 = ((2 * job_q + 1) ^ (job_rl & 7)) << 4;
+          const uint8_t* src = smem + (rank * rows_per + job_rl) * row_bytes;
+          int4 a = *reinterpret_cast<const int4*>(src + o0), b = *reinterpret_cast<const int4*>(src + o1);
+          int32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          src = part + job_rl * row_bytes;
+#pragma unroll 7
+          for (int s = 1; s < split; ++s, src += mine_rows * row_bytes) {
+            a = *reinterpret_cast<const int4*>(src + o0);
+            b = *reinterpret_cast<const int4*>(src + o1);
+            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+            v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+          }
+          if (p.fast_variant >= 0) {
+            uint32_t w[2];
+            requant<8>(p, v, bias_s + job_q * 8, res, w);
+            *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.y) + (size_t)row * p.oc + n0 + job_q * 8) = make_uint2(w[0], w[1]);
+          } else {
+            by_steps<8>(p, v, row, n0 + job_q * 8, bias_s + job_q * 8);
           }
         }
       }
+    } else {
+      cluster_wait();
+      cluster_arrive();
+      if (warp == 1) tmem_free();
     }
     __syncwarp();
-    cluster_arrive();
-    uint4 r0 = none, r1 = none;
-    const int t = (int)threadIdx.x - 64;
-    const int jobs = rows_per * chunks;
-    auto job_row = [&](int k) { return rank * rows_per + k / chunks; };
-    if (warp >= 2 && t < jobs) operand(out_row(job_row(t)), n0 + (t % chunks) * 32, &r0, &r1);
-    cluster_wait();
-    if (warp >= 2 && !abort_flag) {
-      for (int k = t; k < jobs; k += 128) {
-        const int rl = k / chunks, c = k - rl * chunks, col = n0 + c * 32;
-        const int row = out_row(rank * rows_per + rl);
-        if (row < 0 || col >= p.oc) continue;
-        if (k != t) operand(row, col, &r0, &r1);
-        int32_t v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0;
-        for (int s = 0; s < split; ++s) {
-          const uint8_t* src = part + (size_t)(s * rows_per + rl) * p.block_n * 4;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int4 q = *reinterpret_cast<const int4*>(src + (((c * 8 + j) ^ (rl & 7)) << 4));
-            v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
-          }
-        }
-        finish_chunk(p, v, row, col, bias_s + c * 32, r0, r1);
-      }
-    }
+    cluster_wait();   // nobody still reads this CTA's memory
   }
 
-  // ------------------------------------------------------------------ teardown
+  // Every warp leaves on its own; the TMEM columns have gone back already (tmem_done below).
   __syncwarp();
-  tc_fence_before();
-  __syncthreads();
   if (abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);   // copies in flight land before shared memory is released
-    if (threadIdx.x == 0 && p.status) atomicOr(p.status, 0x200 | abort_flag);
-    __syncthreads();
-  }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+    if (lane == 0 && p.status) atomicOr(p.status, 0x200 | abort_flag);
   }
 }
 

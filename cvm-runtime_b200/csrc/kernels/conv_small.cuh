@@ -9,14 +9,15 @@ struct SmallConvParams {
   void* y;
   int y_dtype;
   int m_total, oc, oh, ow;
-  int c, kw;
+  int c, kw, cblocks;             // cblocks: K blocks per filter tap
   int stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
   int a_mode;                     // 0 plain 2-D tiles (1x1, dense), 1 im2col-mode TMA, 2 spatial patches
   int patch_w, patch_h, patch_n, patch_w_log2, patch_h_log2, tiles_w, tiles_h;
   int block_k, block_n, stages;
-  int num_n_tiles;
+  int group;                      // units that share a ring stage and its barrier
+  int num_n_tiles, images;
   int units;                      // (filter tap, channel block) pairs of the whole reduction
-  int split;                      // CTAs of a cluster, each reducing units / split of them
+  int split, split_log2;          // CTAs of a cluster, each reducing units / split of them
   int tmem_cols;
   tc::FastDiv fd_n_tiles, fd_tiles_w, fd_tiles_h, fd_ohow, fd_ow, fd_cblocks, fd_kw;
   int* status;
@@ -31,11 +32,17 @@ struct SmallConvParams {
 };
 
 constexpr int SMALL_MAX_STAGES = 12;
-constexpr int SMALL_MAX_N = 128;
+constexpr int SMALL_MAX_N = 64;   // tiles are 32 or 64 columns wide
 
-// Dynamic shared memory of a launch.
-inline int small_smem_bytes(int block_k, int block_n, int stages, int split) {
-  return 1024 + stages * (tc::BLOCK_M + block_n) * block_k + (split > 1 ? tc::BLOCK_M * block_n * 4 : 0);
+// Dynamic shared memory of a launch: the operand ring (which also holds the partial sums this CTA sends
+// when the reduction is cut) and, behind it, the ones it receives.
+__host__ __device__ inline int small_ring_bytes(int block_k, int block_n, int units, int split) {   // units in the ring
+  const int ring = units * (tc::BLOCK_M + block_n) * block_k, sums = split > 1 ? tc::BLOCK_M * block_n * 4 : 0;
+  return ring > sums ? ring : sums;
+}
+inline int small_smem_bytes(int block_k, int block_n, int units, int split) {
+  const int rows = split > 1 ? tc::BLOCK_M / split * (split - 1) : 0;   // received from the other ranks, split 2, 4 or 8
+  return 1024 + small_ring_bytes(block_k, block_n, units, split) + rows * block_n * 4;
 }
 int launch_conv_small(const CUtensorMap& a, const CUtensorMap& b, const SmallConvParams& p, int grid, int smem, cudaStream_t stream);
 

@@ -1109,10 +1109,10 @@ bool grouped_supported(const cvmk_conv_desc& d) {
 }
 
 // Which launches go to the small-launch kernel, and how it cuts them.
-struct SmallChoice { int split, block_n, stages; };   // split 0: the persistent kernel
+struct SmallChoice { int split, block_n, stages, group; };   // split 0: the persistent kernel
 
 SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int patch_h, int patch_n) {
-  SmallChoice c = {0, 0, 0};
+  SmallChoice c = {0, 0, 0, 0};
   if (d.groups > 1 || dev_env("CVM_B200_NO_SMALL")) return c;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1123,17 +1123,29 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
     m_tiles = (int64_t)((d.OW + patch_w - 1) / patch_w) * ((d.OH + patch_h - 1) / patch_h) * ((d.N + patch_n - 1) / patch_n);
   }
   const int bk = pick_block_k(d.C), units = d.KH * d.KW * (d.C / bk);
-  int bn = d.OC <= 32 ? 32 : 64;
+  // A tile's products take the same time whatever its width (the tensor core reads 128 rows of A for
+  // them either way), its requantisation and its stores do not: narrow tiles while SMs are free.
+  int bn = m_tiles * ((d.OC + 31) / 32) <= sms ? 32 : 64;
   if (const char* e = dev_env("CVM_B200_SMALL_N")) bn = atoi(e);
   const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
   if (tiles > sms && !dev_env("CVM_B200_SMALL_FORCE")) return c;
+  // Cutting the reduction costs an exchange of partial sums, about as much as ten 24 KB units take.
   int split = 1;
-  while (split < 8 && units >= 4 * split && tiles * 2 * split <= sms) split *= 2;
-  if (const char* e = dev_env("CVM_B200_SMALL_SPLIT")) { split = atoi(e); while (split > units) split /= 2; }
-  // half of an SM's shared memory, so that the next layer's CTA fits beside this one
-  int stages = (units + split - 1) / split;
-  if (stages > SMALL_MAX_STAGES) stages = SMALL_MAX_STAGES;
-  while (stages > 1 && small_smem_bytes(bk, bn, stages, split) > 112 * 1024) --stages;
+  const int unit_bytes = (BLOCK_M + bn) * bk, weight = units * unit_bytes / (24 * 1024);
+  if (weight > 10)
+    while (split < 8 && weight >= 4 * split && tiles * 2 * split <= sms) split *= 2;
+  if (const char* e = dev_env("CVM_B200_SMALL_SPLIT")) { split = atoi(e); while (split > units || split > 8) split /= 2; }
+  // The whole reduction in flight when it fits, even if the next layer's CTA then does not fit beside
+  // this one: a ring that turns costs a load latency (0.65 us) per lap.
+  // Two or three units share a barrier: a wait costs the issuing warp as much as a unit's products.
+  const int per = (units + split - 1) / split;
+  int group = per <= 3 ? per : (per == 4 ? 2 : 3);
+  if (const char* e = dev_env("CVM_B200_SMALL_GROUP")) group = std::min(per, atoi(e));
+  int limit = 208 * 1024;
+  if (const char* e = dev_env("CVM_B200_SMALL_KB")) limit = atoi(e) * 1024;
+  int stages = std::min((per + group - 1) / group, SMALL_MAX_STAGES);
+  while (stages > 1 && small_smem_bytes(bk, bn, stages * group, split) > limit) --stages;
+  c.group = group;
   c.split = split; c.block_n = bn; c.stages = stages;
   return c;
 }
@@ -1385,7 +1397,8 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   plan->smem_bytes = plan->ring_bytes + io_bytes + 1024;
   if (small.split > 0) {
     plan->stages = small.stages;
-    plan->smem_bytes = small_smem_bytes(bk, bn, small.stages, small.split);
+    plan->smem_bytes = small_smem_bytes(bk, bn, small.stages * small.group, small.split);
+    plan->reserved[3] = small.group;
   }
 
   const int64_t m_total = (int64_t)d->N * d->OH * d->OW;
@@ -1597,8 +1610,10 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
     q.a_mode = p.a_mode;
     q.patch_w = p.patch_w; q.patch_h = p.patch_h; q.patch_n = p.patch_n;
     q.patch_w_log2 = p.patch_w_log2; q.patch_h_log2 = p.patch_h_log2; q.tiles_w = p.tiles_w; q.tiles_h = p.tiles_h;
-    q.block_k = p.block_k; q.block_n = p.block_n; q.stages = p.stages;
-    q.num_n_tiles = p.num_n_tiles; q.units = p.num_units; q.split = plan->small_split;
+    q.block_k = p.block_k; q.block_n = p.block_n; q.stages = p.stages; q.group = p.units;
+    q.num_n_tiles = p.num_n_tiles; q.images = d.N; q.units = p.num_units; q.split = plan->small_split;
+    while ((1 << q.split_log2) < q.split) ++q.split_log2;
+    q.cblocks = p.c / p.block_k;
     q.tmem_cols = 32;
     while (q.tmem_cols < q.block_n) q.tmem_cols *= 2;
     q.fd_n_tiles = p.fd_n_tiles; q.fd_tiles_w = p.fd_tiles_w; q.fd_tiles_h = p.fd_tiles_h; q.fd_ohow = p.fd_ohow; q.fd_ow = p.fd_ow;

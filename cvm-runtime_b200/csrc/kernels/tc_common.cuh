@@ -52,6 +52,15 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(pred));
   return pred != 0;
 }
+// Reads one word of every 64-byte line of a kernel parameter.  Parameters are constant memory that no SM
+// has cached when a launch begins: a field first read after a wait costs a trip to L2 (some 300
+// cycles a line) on the critical path; read here, while the warp waits for the previous kernel anyway.
+template <typename T>
+__device__ __forceinline__ void touch_params(const T& p) {
+  const int* w = reinterpret_cast<const int*>(&p);
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 4); i += 16) asm volatile("" ::"r"(w[i]));
+}
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
