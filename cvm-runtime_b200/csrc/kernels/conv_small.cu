@@ -15,6 +15,10 @@
 //   - the weights of the first ring stages are requested BEFORE griddepcontrol.wait (they are model
 //     parameters), i.e. while the previous layer still runs, and so is the bias; a CTA takes at most
 //     half of an SM's shared memory so that two layers fit beside each other;
+//
+// Dense layers of at most 128 rows swap the operands: the weights are the 128-row operand (tile rows are
+// output channels) and the activations the narrow one.  Such a layer is a stream of weights, and this
+// way a tensor instruction takes 4 KB of it and shared memory holds little else.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <string.h>
@@ -120,6 +124,22 @@ __device__ __forceinline__ void by_steps(const SmallConvParams& p, const int32_t
   }
 }
 
+// Swapped operands: 8 output rows (row0 ..) of output channel `ch`.
+__device__ __forceinline__ void store_swapped(const SmallConvParams& p, const int32_t* v, int ch, int row0, int32_t bias) {
+  if (ch >= p.oc) return;
+  int32_t t[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) t[j] = v[j] + bias;
+  apply_chain<8>(p.chain, t, 0, ch, 0, nullptr, -1, p.first_step);   // (no tensor operands: see choose_small)
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (row0 + j < p.m_total) {
+      const size_t lin = (size_t)(row0 + j) * p.oc + ch;
+      if (p.y_dtype == CVMK_I8) reinterpret_cast<int8_t*>(p.y)[lin] = (int8_t)t[j];
+      else reinterpret_cast<int32_t*>(p.y)[lin] = t[j];
+    }
+}
+
 // The products of G units of NK K-steps each, in one straight line behind one predicate: 50 cycles an
 // instruction (its own run time); with a loop in the elected lane's branch it was 80.
 template <int G, int NK>
@@ -139,6 +159,10 @@ __device__ __forceinline__ void issue_units(bool leader, int nk, uint32_t d, uin
   else issue_steps<G, 1>(leader, d, al, hi, a_q, unit_q, idesc, first);
 }
 
+// SWAP: operands swapped (dense).  Whether the reduction is cut stays a run-time choice: with an instance
+// each, consecutive layers alternate between two kernels, and code the SM has not cached costs more than
+// the branches (ResNet-50 batch 1: 213 against 205 us).
+template <bool SWAP>
 __global__ void __launch_bounds__(THREADS)
 conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ SmallConvParams p) {
@@ -149,13 +173,14 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __shared__ uint64_t bar_part;   // this CTA's rows of every rank's partial sums have landed
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
-  __shared__ __align__(16) int32_t bias_s[SMALL_MAX_N];
+  __shared__ __align__(16) int32_t bias_s[BLOCK_M];
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int split = p.split;
-  const int rank = uniform(split > 1 ? (int)cluster_rank() : 0);
+  const bool SPLIT = split > 1;
+  const int rank = uniform(SPLIT ? (int)cluster_rank() : 0);
   const int tile = (int)blockIdx.x >> p.split_log2;
   const int a_bytes = BLOCK_M * p.block_k, b_bytes = p.block_n * p.block_k;
   const int unit_bytes = a_bytes + b_bytes, stage_bytes = p.group * unit_bytes;   // a ring stage is `group` units: one barrier
@@ -189,14 +214,15 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   // announces the bytes of group `g` in ring stage `s` and requests its weights (the elected lane)
   auto load_b = [&](int s, int g) {
     const int i0 = g * p.group, n = min(p.group, mine - i0);
-    uint32_t sb = ring + (uint32_t)(s * stage_bytes + a_bytes);
+    uint32_t sb = ring + (uint32_t)(s * stage_bytes + (SWAP ? 0 : a_bytes));
+    const int wrow = SWAP ? m0 : n0;
     const uint32_t bar = full0 + 8u * (uint32_t)s;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(n * unit_bytes)) : "memory");
     int col = (u0 + i0) * p.block_k;
     for (int k = 0; k < n; ++k, sb += (uint32_t)unit_bytes, col += p.block_k)
       asm volatile(
           "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sb), "l"(reinterpret_cast<uint64_t>(&tmap_b)), "r"(bar), "r"(col), "r"(n0)
+          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sb), "l"(reinterpret_cast<uint64_t>(&tmap_b)), "r"(bar), "r"(col), "r"(wrow)
           : "memory");
   };
   if (warp == 0) {
@@ -225,8 +251,9 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else {
     const bool early = p.bias_static != 0;
     if (!early) pdl_wait();
-    for (int i = (int)threadIdx.x - 64; i < p.block_n; i += THREADS - 64) {
-      const int32_t b = (p.bias && n0 + i < p.oc) ? __ldg(p.bias + n0 + i) : 0;
+    const int ch0 = SWAP ? m0 : n0, channels = SWAP ? BLOCK_M : p.block_n;
+    for (int i = (int)threadIdx.x - 64; i < channels; i += THREADS - 64) {
+      const int32_t b = (p.bias && ch0 + i < p.oc) ? __ldg(p.bias + ch0 + i) : 0;
       // packed requantisation: (bias + rounding addend) pre-multiplied, see fast_requant()
       bias_s[i] = (p.fast_variant >= 0 && p.fast_variant < 8) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
     }
@@ -235,7 +262,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = (uint32_t)uniform((int)tmem_slot);
-  if (split > 1) cluster_arrive();   // this CTA's barriers exist (waited for before anything is sent to it)
+  if (SPLIT) cluster_arrive();   // this CTA's barriers exist (waited for before anything is sent to it)
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA
@@ -265,10 +292,12 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           "r"(base_w), "r"(base_h), "r"(img), "h"((uint16_t)(fx * p.dil_w)), "h"((uint16_t)(fy * p.dil_h))
           : "memory");
     };
+    const int xrow = SWAP ? n0 : m0;
+    const uint32_t xoff = SWAP ? (uint32_t)a_bytes : 0u;
     auto plain = [&](uint32_t sa, uint32_t bar) {
       asm volatile(
           "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc), "r"(m0)
+          " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa + xoff), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc), "r"(xrow)
           : "memory");
     };
     pdl_wait();
@@ -351,7 +380,22 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
   };
   if (warp >= 2) pdl_wait();
-  if (split == 1) {
+  if (!SPLIT && SWAP) {
+    if (warp >= 2) {
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar_acc, 0u, &abort_flag, 4));
+      tc_fence_after();
+      const int ch = m0 + row_in_tile;
+      for (int c = 0; ok && c < half_n; c += 16) {
+        int32_t v[16];
+        tmem_ld16(tbase + (uint32_t)c, v);
+        store_swapped(p, v, ch, n0 + c_first + c, bias_s[row_in_tile]);
+        store_swapped(p, v + 8, ch, n0 + c_first + c + 8, bias_s[row_in_tile]);
+      }
+      tmem_done();
+    } else if (warp == 1) {
+      tmem_free();
+    }
+  } else if (!SPLIT) {
     if (warp >= 2) {
       const int row = out_row(row_in_tile);
       const bool packed = p.fast_variant >= 0;
@@ -421,7 +465,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // other rank its run; `part` of the receiver holds one block of its rows from each of them.  16-byte
     // chunks of a row are XORed with the low bits of its number in the run (lanes hold different rows).
     // All index arithmetic (divisions among it) is done before the waits it would otherwise follow.
-    int rows = min(BLOCK_M, p.m_total - m0);
+    int rows = min(BLOCK_M, (SWAP ? p.oc : p.m_total) - m0);
     if (p.a_mode == 2) {
       const int images = p.images - cn;
       rows = images >= p.patch_n ? BLOCK_M : images << (p.patch_w_log2 + p.patch_h_log2);
@@ -439,12 +483,15 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       // this CTA's rows: eight columns a thread and turn
       const int t = (int)threadIdx.x - 64, per_row_log2 = 31 - __clz(p.block_n >> 3), per_row = 1 << per_row_log2;
       const int jobs = mine_rows << per_row_log2;
+      // (swapped operands: rows are output channels, so neighbouring threads take neighbouring rows)
       int job_rl = t >> per_row_log2, job_q = t & (per_row - 1);
+      if (SWAP && mine_rows > 0) { job_q = t / mine_rows; job_rl = t - job_q * mine_rows; }
       int row = -1;
       uint32_t res[2] = {0, 0};
       auto job_row = [&]() {
-        row = out_row(rank * rows_per + job_rl);
         const int col = n0 + job_q * 8;
+        if (SWAP) { row = m0 + rank * rows_per + job_rl; return; }
+        row = out_row(rank * rows_per + job_rl);
         if (col >= p.oc) row = -1;
         if (!with_res || row < 0) return;
         const uint2 q = *reinterpret_cast<const uint2*>(p.res + (size_t)row * p.oc + col);
@@ -489,6 +536,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         for (int k = t; k < jobs; k += THREADS - 64) {
           if (k != t) {
             job_rl = k >> per_row_log2; job_q = k & (per_row - 1);
+            if (SWAP) { job_q = k / mine_rows; job_rl = k - job_q * mine_rows; }
             job_row();
           }
           if (row < 0) continue;
@@ -504,7 +552,9 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
             v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
           }
-          if (p.fast_variant >= 0) {
+          if (SWAP) {
+            store_swapped(p, v, row, n0 + job_q * 8, bias_s[rank * rows_per + job_rl]);
+          } else if (p.fast_variant >= 0) {
             uint32_t w[2];
             requant<8>(p, v, bias_s + job_q * 8, res, w);
             *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.y) + (size_t)row * p.oc + n0 + job_q * 8) = make_uint2(w[0], w[1]);
@@ -533,13 +583,16 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }  // namespace
 
 int launch_conv_small(const CUtensorMap& a, const CUtensorMap& b, const SmallConvParams& p, int grid, int smem, cudaStream_t stream) {
+  static void (*const kernels[2])(CUtensorMap, CUtensorMap, SmallConvParams) = {conv_small_kernel<false>, conv_small_kernel<true>};
   static bool attr_of_device[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_of_device[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(conv_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_small_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (check_cuda(e, "cudaFuncSetAttribute(conv_small_kernel)")) return CVMK_ERR_CUDA;
+    for (auto k : kernels) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      if (check_cuda(e, "cudaFuncSetAttribute(conv_small_kernel)")) return CVMK_ERR_CUDA;
+    }
     attr_of_device[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -561,7 +614,7 @@ int launch_conv_small(const CUtensorMap& a, const CUtensorMap& b, const SmallCon
   }
   cfg.attrs = attr;
   cfg.numAttrs = (unsigned)n;
-  return check_cuda(cudaLaunchKernelEx(&cfg, conv_small_kernel, a, b, p), "conv_small_kernel launch");
+  return check_cuda(cudaLaunchKernelEx(&cfg, kernels[p.swap ? 1 : 0], a, b, p), "conv_small_kernel launch");
 }
 
 }  // namespace cvmk

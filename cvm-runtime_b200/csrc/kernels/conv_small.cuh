@@ -15,6 +15,7 @@ struct SmallConvParams {
   int patch_w, patch_h, patch_n, patch_w_log2, patch_h_log2, tiles_w, tiles_h;
   int block_k, block_n, stages;
   int group;                      // units that share a ring stage and its barrier
+  int swap;                       // dense: the weights are the 128-row operand, the activations the block_n-row one
   int num_n_tiles, images;
   int units;                      // (filter tap, channel block) pairs of the whole reduction
   int split, split_log2;          // CTAs of a cluster, each reducing units / split of them
@@ -32,7 +33,6 @@ struct SmallConvParams {
 };
 
 constexpr int SMALL_MAX_STAGES = 12;
-constexpr int SMALL_MAX_N = 64;   // tiles are 32 or 64 columns wide
 
 // Dynamic shared memory of a launch: the operand ring (which also holds the partial sums this CTA sends
 // when the reduction is cut) and, behind it, the ones it receives.

@@ -110,8 +110,6 @@ struct ConvParams {
   int bias_static;      // the bias vector is a parameter: it may be read before the previous kernel has finished
   const int8_t* w;      // the weight matrix [oc, kh * kw * c] and its size, for the L2 warm-up
   unsigned w_bytes;
-  int k_slices;         // > 1: `oc` counts k_slices x oc_real virtual columns; column block s reduces over
-  int oc_real;          //      K slice s (c bytes long) of the real columns and writes int32 partial sums
   DevChain chain;
 };
 
@@ -247,19 +245,12 @@ __device__ long long g_conv_trace[17 * 512];
 
 // Origin of a tile: first output channel, and either the first linear output row (modes 0, 1) or
 // the corner (w, h, n) of the spatial patch (mode 2).
-struct TileOrigin { int n0, m0, cw, ch, cn, nb, k0; };   // nb: first weight row, k0: first K byte (K slices)
+struct TileOrigin { int n0, m0, cw, ch, cn; };
 __device__ __forceinline__ TileOrigin tile_origin(const ConvParams& p, int tile) {
   TileOrigin t;
   const int mt = fdiv(tile, p.fd_n_tiles);
   t.n0 = (tile - mt * p.num_n_tiles) * p.block_n;
   t.m0 = mt * BLOCK_M;
-  t.nb = t.n0;
-  t.k0 = 0;
-  if (p.k_slices > 1) {
-    const int s = t.n0 / p.oc_real;
-    t.nb = t.n0 - s * p.oc_real;
-    t.k0 = s * p.c;
-  }
   t.cw = t.ch = t.cn = 0;
   if (p.a_mode >= 2) {
     const int r = fdiv(mt, p.fd_tiles_w);
@@ -553,12 +544,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               asm volatile(
                   "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                   " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar),
-                  "r"(cc + to.k0), "r"(m0)
+                  "r"(cc), "r"(m0)
                   : "memory");
             if (!b_resident) asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                 " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa + (uint32_t)a_bytes), "l"(reinterpret_cast<uint64_t>(&tmap_b)),
-                "r"(bar), "r"(kcol + to.k0), "r"(to.nb)
+                "r"(bar), "r"(kcol), "r"(to.n0)
                 : "memory");
           }
           if (mine) sa += (uint32_t)unit_bytes;
@@ -1020,6 +1011,13 @@ void* driver_entry(const char* name) {
   return fn;
 }
 
+int sm_count() {   // of the current device; without one, of the part this library is built for
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaGetLastError();
+  return sms;
+}
+
 CUtensorMapSwizzle swizzle_for(int row_bytes) {
   return row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                           : (row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
@@ -1109,26 +1107,42 @@ bool grouped_supported(const cvmk_conv_desc& d) {
 }
 
 // Which launches go to the small-launch kernel, and how it cuts them.
-struct SmallChoice { int split, block_n, stages, group; };   // split 0: the persistent kernel
+struct SmallChoice { int split, block_n, stages, group, swap; };   // split 0: the persistent kernel
 
 SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int patch_h, int patch_n) {
-  SmallChoice c = {0, 0, 0, 0};
+  SmallChoice c = {0, 0, 0, 0, 0};
   if (d.groups > 1 || dev_env("CVM_B200_NO_SMALL")) return c;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaGetLastError();
+  const int sms = sm_count();
   int64_t m_tiles = ((int64_t)d.N * d.OH * d.OW + BLOCK_M - 1) / BLOCK_M;
   if (a_mode >= 2) {
     if (a_mode == 3 && !pick_patch(d, &patch_w, &patch_h, &patch_n)) return c;
     m_tiles = (int64_t)((d.OW + patch_w - 1) / patch_w) * ((d.OH + patch_h - 1) / patch_h) * ((d.N + patch_n - 1) / patch_n);
   }
   const int bk = pick_block_k(d.C), units = d.KH * d.KW * (d.C / bk);
+  // Few rows over many weights: operands swapped, every CTA of two per SM streams its share of the weights.
+  if (is_pointwise(d) && d.OH == 1 && d.OW == 1 && d.N <= BLOCK_M && (int64_t)d.OC * d.C >= 1 << 19) {
+    bool plain = true;
+    for (int i = 0; i < d.ep.n; ++i)
+      plain &= d.ep.s[i].op != CVMK_EP_ADD_T && d.ep.s[i].op != CVMK_EP_SUB_T && d.ep.s[i].op != CVMK_EP_RSUB_T;
+    if (plain) {
+      const int mt = (d.OC + BLOCK_M - 1) / BLOCK_M;
+      c.swap = 1;
+      c.block_n = d.N <= 32 ? 32 : (d.N <= 64 ? 64 : 128);
+      c.split = 1;
+      while (c.split < 8 && units >= 4 * c.split && mt * 2 * c.split <= 2 * sms) c.split *= 2;
+      c.group = 1;
+      c.stages = std::min((units + c.split - 1) / c.split, SMALL_MAX_STAGES);
+      while (c.stages > 2 && small_smem_bytes(bk, c.block_n, c.stages, c.split) > 112 * 1024) --c.stages;
+      return c;
+    }
+  }
   // A tile's products take the same time whatever its width (the tensor core reads 128 rows of A for
   // them either way), its requantisation and its stores do not: narrow tiles while SMs are free.
   int bn = m_tiles * ((d.OC + 31) / 32) <= sms ? 32 : 64;
   if (const char* e = dev_env("CVM_B200_SMALL_N")) bn = atoi(e);
   const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
-  if (tiles > sms && !dev_env("CVM_B200_SMALL_FORCE")) return c;
+  const bool few_rows = is_pointwise(d) && (int64_t)d.N * d.OH * d.OW <= BLOCK_M;   // long reductions of one M tile
+  if (tiles > sms && !few_rows && !dev_env("CVM_B200_SMALL_FORCE")) return c;
   // Cutting the reduction costs an exchange of partial sums, about as much as ten 24 KB units take.
   int split = 1;
   const int unit_bytes = (BLOCK_M + bn) * bk, weight = units * unit_bytes / (24 * 1024);
@@ -1167,53 +1181,25 @@ extern "C" int cvmk_conv2d_tc_supported(const cvmk_conv_desc* d) {
   return 1;
 }
 
-// K slices for a pointwise layer of at most one M tile: 1 = not cut.  The slice count divides
-// the number of K blocks, leaves at least four blocks per slice, and is the smallest that makes
-// the best use of the SMs (tiles / (waves x SMs)).
-static int pick_k_slices(const cvmk_conv_desc& d, int bk, int bn) {
-  if (!is_pointwise(d) || d.groups > 1 || (int64_t)d.N * d.OH * d.OW > BLOCK_M || d.OC % bn != 0 || d.C % bk != 0) return 1;
-  if (dev_env("CVM_B200_NO_SPLIT_K")) return 1;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaGetLastError();
-  const int blocks = d.C / bk, nt = d.OC / bn;
-  if (blocks < 8 || 2 * nt >= sms) return 1;
+// Scratch for a pointwise layer of at most one M tile whose reduction is cut into slices (the count
+// divides the number of K blocks, leaves at least four per slice, and is the smallest that makes the best
+// use of the SMs).  Layers are cut over clusters now, which need no scratch: the answer is for
+// callers that size a buffer with it, and the buffer is not used.
+extern "C" int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d) {
+  if (!d || !cvmk_conv2d_tc_supported(d)) return 0;
+  const int bk = pick_block_k(d->C), bn = pick_block_n(d->OC);
+  if (!is_pointwise(*d) || d->groups > 1 || (int64_t)d->N * d->OH * d->OW > BLOCK_M || d->OC % bn != 0 || d->C % bk != 0) return 0;
+  const int sms = sm_count(), blocks = d->C / bk, nt = d->OC / bn;
+  if (blocks < 8 || 2 * nt >= sms) return 0;
   int best = 1;
   double best_eff = (double)nt / sms;
-  for (int s = 2; s * 4 <= blocks; ++s) {
+  for (int s = 2; s * 4 <= blocks && nt * s <= 4 * sms; ++s) {
     if (blocks % s) continue;
     const int tiles = nt * s;
-    if (tiles > 4 * sms) break;
     const double eff = (double)tiles / (double)(((tiles + sms - 1) / sms) * sms);
     if (eff > best_eff + 0.02) { best_eff = eff; best = s; }
   }
-  return best;
-}
-
-extern "C" int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d) {
-  if (!d || !cvmk_conv2d_tc_supported(d)) return 0;
-  if (is_pointwise(*d) && choose_small(*d, 0, 0, 0, 0).split > 0) return 0;   // cut over clusters instead
-  const int s = pick_k_slices(*d, pick_block_k(d->C), pick_block_n(d->OC));
-  return s > 1 ? (int64_t)d->N * d->OH * d->OW * s * d->OC * 4 : 0;
-}
-
-// Adds the k_slices partial sums of every output element and applies the chain.
-__global__ void __launch_bounds__(256) splitk_finish_kernel(const int32_t* __restrict__ part, void* y, int y_dtype, int m,
-                                                            int oc, int slices, const __grid_constant__ DevChain chain) {
-  const int quads = oc / 4;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m * quads) return;
-  const int row = i / quads, c0 = (i - row * quads) * 4;
-  const int4* src = reinterpret_cast<const int4*>(part + ((size_t)row * slices) * oc + c0);
-  int32_t v[4] = {0, 0, 0, 0};
-  for (int s = 0; s < slices; ++s) {
-    const int4 t = __ldg(src + (size_t)s * (oc / 4));
-    v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
-  }
-  const size_t lin = (size_t)row * oc + c0;
-  apply_chain<4>(chain, v, lin, c0, 1, nullptr, -1, 0);
-  if (y_dtype == CVMK_I8) *reinterpret_cast<uint32_t*>(reinterpret_cast<int8_t*>(y) + lin) = pack4(v[0], v[1], v[2], v[3]);
-  else *reinterpret_cast<int4*>(reinterpret_cast<int32_t*>(y) + lin) = make_int4(v[0], v[1], v[2], v[3]);
+  return best > 1 ? (int64_t)d->N * d->OH * d->OW * best * d->OC * 4 : 0;
 }
 
 extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* plan) {
@@ -1285,19 +1271,14 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     plan->block_n = bn;
   }
   plan->small_split = small.split;
+  plan->small_swap = small.swap;
   plan->reserved[0] = patch_w; plan->reserved[1] = patch_h; plan->reserved[2] = patch_n;
 
   // Output path: int8 tiles leave through shared memory and a TMA store; the first int8 tensor
   // operand of the chain (a residual join) comes in by TMA as well.
-  // Reductions cut along K write int32 partial sums into the caller's scratch with plain stores.
-  {
-    const int ks = pick_k_slices(*d, bk, bn);
-    const int64_t need = (int64_t)d->N * d->OH * d->OW * ks * d->OC * 4;
-    plan->k_slices = (!small.split && ks > 1 && d->workspace && d->workspace_bytes >= need && ((uintptr_t)d->workspace & 15) == 0) ? ks : 1;
-  }
-  plan->tma_out = !small.split && plan->k_slices == 1 && d->y_dtype == CVMK_I8 && d->OC % 32 == 0 && !dev_env("CVM_B200_NO_TMA_STORE");
+  plan->tma_out = !small.split && d->y_dtype == CVMK_I8 && d->OC % 32 == 0 && !dev_env("CVM_B200_NO_TMA_STORE");
   plan->res_step = -1;
-  if (plan->tma_out || (small.split && d->y_dtype == CVMK_I8 && d->OC % 32 == 0)) {
+  if (plan->tma_out || (small.split && !small.swap && d->y_dtype == CVMK_I8 && d->OC % 32 == 0)) {
     for (int i = 0; i < d->ep.n; ++i) {
       const cvmk_ep_step& s = d->ep.s[i];
       if ((s.op == CVMK_EP_ADD_T || s.op == CVMK_EP_SUB_T || s.op == CVMK_EP_RSUB_T) &&
@@ -1313,7 +1294,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // is still deep enough; short reductions (little work per output tile) may give up half of their
   // K block for it.
   const int group_bytes = plan->panels * BLOCK_M * plan->panel_bytes;
-  const int64_t k_all = (int64_t)d->KH * d->KW * cg / plan->k_slices;   // per tile
+  const int64_t k_all = (int64_t)d->KH * d->KW * cg;   // per tile
   const int budget = SMEM_DYNAMIC_MAX - 1024;
   plan->io_bufs = 1;
   // Weights resident in shared memory: one N tile, i.e. every tile of the launch multiplies the
@@ -1321,12 +1302,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // halo alone.
   const int halo_pad = ((10 * 18 * bk) + 1023) & ~1023;
   int resident = 0;
-  int sms_all = 148;
-  {
-    int dev0 = 0;
-    if (cudaGetDevice(&dev0) == cudaSuccess) cudaDeviceGetAttribute(&sms_all, cudaDevAttrMultiProcessorCount, dev0);
-    cudaGetLastError();
-  }
+  const int sms_all = sm_count();
   // (grouped: the grid is cut to a multiple of the N tiles below, so that every tile of a CTA
   //  covers the same groups and their 9 weight tiles each can stay as well)
   if (halo && (d->OC <= bn || (grouped && d->OC / bn <= sms_all)) && !dev_env("CVM_B200_NO_RESIDENT_WEIGHTS")) {
@@ -1361,9 +1337,8 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // (K x block_n bytes) in shared memory; the ring then carries activations only, a third or a
   // fifth of the bytes.  Taken when the weights leave room for a ring of at least four A blocks.
   plan->b_resident = 0;
-  if (!small.split && plan->a_im2col == 0 && plan->k_slices == 1 && !dev_env("CVM_B200_NO_RESIDENT_B")) {
-    int sms = 148, dev0 = 0;
-    if (cudaGetDevice(&dev0) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev0);
+  if (!small.split && plan->a_im2col == 0 && !dev_env("CVM_B200_NO_RESIDENT_B")) {
+    const int sms = sms_all;
     const int64_t m_tiles = ((int64_t)d->N * d->OH * d->OW + BLOCK_M - 1) / BLOCK_M;
     const int nt = (d->OC + bn - 1) / bn;
     const int64_t w_bytes = (int64_t)d->C * bn;
@@ -1423,10 +1398,10 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
                    (cuuint32_t)bk, (cuuint32_t)BLOCK_M, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    swizzle_for(bk), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   } else {
-    r = encode_rows(enc_tiled, ta, d->x, m_total, d->C, bk, BLOCK_M, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    r = encode_rows(enc_tiled, ta, d->x, m_total, d->C, bk, small.swap ? bn : BLOCK_M, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
   }
   if (r != CUDA_SUCCESS) { set_error("conv2d_tc_prepare: activation tensor map rejected (CUresult %d)", (int)r); return CVMK_ERR_CUDA; }
-  r = encode_rows(enc_tiled, tb, d->w, d->OC, k_total, grouped ? cg : bk, grouped ? cg : bn, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  r = encode_rows(enc_tiled, tb, d->w, d->OC, k_total, grouped ? cg : bk, grouped ? cg : (small.swap ? BLOCK_M : bn), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   if (r != CUDA_SUCCESS) { set_error("conv2d_tc_prepare: weight tensor map rejected (CUresult %d)", (int)r); return CVMK_ERR_CUDA; }
   if (plan->tma_out) {
     auto encode_out = [&](unsigned char* map, const void* base, CUtensorMapL2promotion promo) {
@@ -1448,10 +1423,9 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     num_m_tiles = (int64_t)((d->OW + patch_w - 1) / patch_w) * ((d->OH + patch_h - 1) / patch_h) *
                   ((d->N + patch_n - 1) / patch_n);
   const int64_t num_n_tiles = (d->OC + bn - 1) / bn;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t tiles = num_m_tiles * num_n_tiles * plan->k_slices;
+  const int sms = sms_all;
+  int64_t tiles = num_m_tiles * num_n_tiles;
+  if (small.swap) tiles = ((d->OC + BLOCK_M - 1) / BLOCK_M) * ((m_total + bn - 1) / bn);
   plan->grid = (int)(tiles < sms ? tiles : sms);
   if (small.split > 0) plan->grid = (int)(tiles * small.split);
   if (grouped && plan->a_im2col == 4) plan->grid = (int)(plan->grid / num_n_tiles * num_n_tiles);   // tile t + k * grid: same group as t
@@ -1504,19 +1478,6 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   p.w = d.w;
   p.w_bytes = (unsigned)std::min<int64_t>((int64_t)d.OC * d.KH * d.KW * p.c, (int64_t)1 << 30);
   p.tma_out = plan->tma_out; p.res_step = plan->res_step;
-  const int ks = plan->k_slices > 1 ? plan->k_slices : 1;
-  if (ks > 1) {   // virtual columns (slice, real column); int32 partial sums, no chain in this kernel
-    p.k_slices = ks;
-    p.oc_real = d.OC;
-    p.oc = ks * d.OC;
-    p.c = d.C / ks;
-    p.y = d.workspace;
-    p.y_dtype = CVMK_I32;
-    p.num_n_tiles *= ks;
-    p.num_units = d.C / ks / plan->block_k;
-    p.num_kb = (p.num_units + p.units - 1) / p.units;
-    p.fd_n_tiles = make_fastdiv(p.num_n_tiles);
-  }
   // Two issuing warps (and one producer) in the halo modes, where a tile takes one or two ring
   // stages and the ring has more: an issuer that waits for the first stage of its next tile is then
   // never more than one lap of that stage's barrier ahead of the producer, which is what a parity
@@ -1536,8 +1497,6 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   p.io_bufs = plan->io_bufs; p.ring_bytes = plan->ring_bytes;
   int rc = lower_chain(d.ep, &p.chain);
   if (rc != CVMK_OK) return rc;
-  DevChain finish_chain = p.chain;
-  if (ks > 1) p.chain.n = 0;
   // lower_chain() may merge steps: find the TMA-served operand again by its pointer.
   if (plan->res_step >= 0) {
     const void* want = d.ep.s[plan->res_step].ptr;
@@ -1558,7 +1517,7 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   // Packed requantisation: chain = [bias] rs_clamp [add_t|sub_t (the TMA-served operand) clip].
   p.fast_mode = 0;
   const bool small = plan->small_split > 0;
-  const bool packed_out = small ? (d.y_dtype == CVMK_I8 && d.OC % 32 == 0) : (p.tma_out && d.OC <= MAX_BIAS);
+  const bool packed_out = small ? (!plan->small_swap && d.y_dtype == CVMK_I8 && d.OC % 32 == 0) : (p.tma_out && d.OC <= MAX_BIAS);
   if (packed_out && d.acc_bound > 0 && !dev_env("CVM_B200_NO_FAST_REQUANT")) {
     const int i0 = p.first_step;
     const int left = p.chain.n - i0;
@@ -1614,6 +1573,11 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
     q.num_n_tiles = p.num_n_tiles; q.images = d.N; q.units = p.num_units; q.split = plan->small_split;
     while ((1 << q.split_log2) < q.split) ++q.split_log2;
     q.cblocks = p.c / p.block_k;
+    q.swap = plan->small_swap;
+    if (q.swap) {   // tile rows are output channels
+      q.num_n_tiles = (p.m_total + q.block_n - 1) / q.block_n;
+      p.fd_n_tiles = make_fastdiv(q.num_n_tiles);
+    }
     q.tmem_cols = 32;
     while (q.tmem_cols < q.block_n) q.tmem_cols *= 2;
     q.fd_n_tiles = p.fd_n_tiles; q.fd_tiles_w = p.fd_tiles_w; q.fd_tiles_h = p.fd_tiles_h; q.fd_ohow = p.fd_ohow; q.fd_ow = p.fd_ow;
@@ -1661,13 +1625,6 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   cfg.attrs = &attr;
   cfg.numAttrs = pdl ? 1 : 0;
   if (check_cuda(cudaLaunchKernelEx(&cfg, conv_tc_kernel, ta, tb, ty, tr, p), "conv_tc_kernel launch")) return CVMK_ERR_CUDA;
-  if (ks > 1) {
-    const int m = d.N * d.OH * d.OW;
-    const int work = m * (d.OC / 4);
-    splitk_finish_kernel<<<(work + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const int32_t*>(d.workspace), d.y, d.y_dtype, m, d.OC, ks, finish_chain);
-    return check_cuda(cudaGetLastError(), "splitk_finish_kernel launch");
-  }
   return CVMK_OK;
 }
 

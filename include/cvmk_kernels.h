@@ -139,11 +139,8 @@ typedef struct {
    * sub-pixels a - 1, a, a + 1, the outer ones from the neighbouring folded pixel at the edges. */
   int32_t group_fold;
   int32_t reserved1;
-  /* Optional scratch for reductions cut along K (dense layers of a few rows over a long K, whose
-   * few output tiles would leave most SMs idle): cvmk_conv2d_tc_workspace_bytes() says how much the
-   * shape wants (0: it is not cut).  With at least that much here, K slices run as separate tiles
-   * that write int32 partial sums, and a second small kernel adds them and applies the chain.
-   * Sums of integers: the result is the same bit for bit. */
+  /* Scratch that reductions cut along K once took (cvmk_conv2d_tc_workspace_bytes()).  They are cut
+   * over clusters of CTAs now, which exchange their partial sums on chip; not used. */
   void* workspace;
   int64_t workspace_bytes;
   cvmk_epilogue ep;
@@ -167,7 +164,7 @@ typedef struct __attribute__((aligned(64))) {
   int32_t io_bufs;    /* staging buffers per epilogue group: 1 or 2 */
   int32_t ring_bytes; /* bytes of the operand ring in shared memory */
   int32_t reserved[4];  /* [0..2] patch width / height / images (a_im2col = 2, 3), [3] (tap, channel block) units per ring stage */
-  int32_t k_slices;   /* > 1: the reduction is cut into this many slices (see cvmk_conv_desc.workspace) */
+  int32_t small_swap; /* small-launch kernel, dense: the weights are the 128-row operand */
   int32_t b_resident; /* 1: 1x1 layer, every CTA keeps its N tile of the weights in shared memory */
   int32_t small_split; /* > 0: the small-launch kernel, each tile's reduction cut over a cluster of so many CTAs */
   int32_t pad_[1];
