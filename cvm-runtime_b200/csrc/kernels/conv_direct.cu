@@ -29,6 +29,8 @@ __device__ __forceinline__ void store_one(void* y, int yd, int64_t i, int32_t v)
 // activation reads are warp-broadcast and weight reads are contiguous per thread.
 template <int XD>
 __global__ void __launch_bounds__(256) conv_direct_kernel(const __grid_constant__ DirectParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int icg = p.C / p.groups;
   const int ocg = p.OC / p.groups;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -78,6 +80,8 @@ __global__ void __launch_bounds__(256) conv_direct_kernel(const __grid_constant_
 // extraction of the packed words.
 template <int PX>
 __global__ void __launch_bounds__(128) depthwise_kernel(const __grid_constant__ DirectParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int cvec = p.C / 16;
   const int oxg = (p.OW + PX - 1) / PX;
   const int64_t total = (int64_t)p.N * p.OH * oxg * cvec;
@@ -145,6 +149,8 @@ __global__ void __launch_bounds__(128) depthwise_kernel(const __grid_constant__ 
 // it belongs to, so the inner loop is one multiply-add per product.
 template <int S>
 __global__ void __launch_bounds__(256) depthwise3x3_kernel(const __grid_constant__ DirectParams p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int PX = 4;
   constexpr int IN = (PX - 1) * S + 3;  // input pixels of a row that a strip touches
   const int cw = p.C / 4;
@@ -289,6 +295,8 @@ __device__ __forceinline__ void transpose4x4(uint32_t a, uint32_t b, uint32_t c,
 
 template <int S>
 __global__ void __launch_bounds__(256) dw3x3_tile_kernel(const __grid_constant__ Dw3Params p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) uint32_t tile[];
   constexpr int PX = 4;
   constexpr int IN = (PX - 1) * S + 3;
@@ -398,6 +406,8 @@ struct PackParams {
   int64_t total;  // rows * Kp / 16
 };
 __global__ void __launch_bounds__(256) im2col_pack_kernel(const __grid_constant__ PackParams p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int lut[];  // per k: (fy*dh) << 20 | (fx*dw) << 8 | c
   for (int k = threadIdx.x; k < p.K; k += blockDim.x) {
     const int fy = k / (p.KW * p.C), r = k - fy * (p.KW * p.C);
@@ -442,6 +452,8 @@ struct StemParams {
   int N, H, W, C, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw, Kp, K, clamp, wp;
 };
 __global__ void __launch_bounds__(512) stem_pack_kernel(const __grid_constant__ StemParams p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) int8_t srow[];  // [KH][C][wp], wp = W + 2 * pw
   const int n = blockIdx.x / p.OH, oy = blockIdx.x % p.OH;
   const int iy0 = oy * p.sh - p.ph;
@@ -579,8 +591,8 @@ int try_dw3x3_tile(const cvmk_conv_direct_desc* d, const DevChain& chain, cudaSt
       attr_set = true;
     }
   }
-  if (S == 1) dw3x3_tile_kernel<1><<<(unsigned)tiles, 256, smem, s>>>(p);
-  else dw3x3_tile_kernel<2><<<(unsigned)tiles, 256, smem, s>>>(p);
+  if (S == 1) launch_pdl(dw3x3_tile_kernel<1>, dim3((unsigned)tiles), dim3(256), smem, s, p);
+  else launch_pdl(dw3x3_tile_kernel<2>, dim3((unsigned)tiles), dim3(256), smem, s, p);
   return check_cuda(cudaGetLastError(), "dw3x3_tile_kernel launch");
 }
 
@@ -628,16 +640,16 @@ extern "C" int cvmk_conv2d_direct(const cvmk_conv_direct_desc* d, cvmk_stream_t 
       const int rc_tile = try_dw3x3_tile(d, p.chain, s);
       if (rc_tile >= 0) return rc_tile;
       const int64_t work3 = (int64_t)d->N * d->OH * (d->C / 4);
-      if (d->stride_h == 1) depthwise3x3_kernel<1><<<grid_sized(work3, 256), 256, 0, s>>>(p);
-      else depthwise3x3_kernel<2><<<grid_sized(work3, 256), 256, 0, s>>>(p);
+      if (d->stride_h == 1) launch_pdl(depthwise3x3_kernel<1>, dim3((unsigned)(grid_sized(work3, 256))), dim3(256), 0, s, p);
+      else launch_pdl(depthwise3x3_kernel<2>, dim3((unsigned)(grid_sized(work3, 256))), dim3(256), 0, s, p);
       return check_cuda(cudaGetLastError(), "depthwise3x3_kernel launch");
     }
     const int64_t work = (int64_t)d->N * d->OH * ((d->OW + 3) / 4) * (d->C / 16);
-    depthwise_kernel<4><<<grid_sized(work, 128), 128, 0, s>>>(p);
+    launch_pdl(depthwise_kernel<4>, dim3((unsigned)(grid_sized(work, 128))), dim3(128), 0, s, p);
     return check_cuda(cudaGetLastError(), "depthwise_kernel launch");
   }
-  if (d->x_dtype == CVMK_I8) conv_direct_kernel<CVMK_I8><<<grid_sized(p.total, 256), 256, 0, s>>>(p);
-  else conv_direct_kernel<CVMK_I32><<<grid_sized(p.total, 256), 256, 0, s>>>(p);
+  if (d->x_dtype == CVMK_I8) launch_pdl(conv_direct_kernel<CVMK_I8>, dim3((unsigned)(grid_sized(p.total, 256))), dim3(256), 0, s, p);
+  else launch_pdl(conv_direct_kernel<CVMK_I32>, dim3((unsigned)(grid_sized(p.total, 256))), dim3(256), 0, s, p);
   return check_cuda(cudaGetLastError(), "conv_direct_kernel launch");
 }
 
@@ -654,7 +666,7 @@ extern "C" int cvmk_im2col_pack(const cvmk_im2col_desc* d, cvmk_stream_t stream)
   p.sh = d->stride_h; p.sw = d->stride_w; p.ph = d->pad_h; p.pw = d->pad_w; p.dh = d->dil_h; p.dw = d->dil_w;
   p.Kp = d->Kp; p.K = d->KH * d->KW * d->C;
   p.total = (int64_t)d->N * d->OH * d->OW * (d->Kp / 16);
-  im2col_pack_kernel<<<grid_sized(p.total, 256), 256, p.K * sizeof(int), (cudaStream_t)stream>>>(p);
+  launch_pdl(im2col_pack_kernel, dim3((unsigned)(grid_sized(p.total, 256))), dim3(256), p.K * sizeof(int), (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "im2col_pack_kernel launch");
 }
 
@@ -686,6 +698,6 @@ extern "C" int cvmk_stem_pack(const cvmk_stem_pack_desc* d, cvmk_stream_t stream
   int threads = chunks * 32;             // a multiple of the chunk count, see the kernel
   while (threads > 512) threads -= chunks;
   if (chunks > 512) { set_error("stem_pack: Kp too large"); return CVMK_ERR_UNSUPPORTED; }
-  stem_pack_kernel<<<d->N * d->OH, threads, smem, (cudaStream_t)stream>>>(p);
+  launch_pdl(stem_pack_kernel, dim3((unsigned)(d->N * d->OH)), dim3(threads), smem, (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "stem_pack_kernel launch");
 }

@@ -299,6 +299,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();   // (after the TMEM allocation: see conv_small.cu)
   if (threadIdx.x == 0) { mbar_arrive(&out_free[0]); mbar_arrive(&out_free[1]); }  // both panels start free
   const uint32_t tmem_base = tmem_slot;
 

@@ -49,6 +49,8 @@ __device__ __forceinline__ int4 pack16(const int32_t* v) {
 template <int XD, int YD>
 __global__ void __launch_bounds__(256) elemwise_kernel(const void* __restrict__ x, void* __restrict__ y,
                                                        int64_t n, const __grid_constant__ DevChain chain) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t nvec = n / 16;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
@@ -117,6 +119,8 @@ __device__ __forceinline__ int32_t load_elem(const void* p, int dt, int64_t off)
 }
 
 __global__ void __launch_bounds__(256) strided_kernel(const __grid_constant__ StridedParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     int64_t ao = p.a_off, bo = p.b_off, yo = p.y_off;
@@ -209,6 +213,8 @@ __device__ __forceinline__ void strided_vec_body(const StridedVecParams& p, int6
   }
 }
 __global__ void __launch_bounds__(256) strided_vec_kernel(const __grid_constant__ StridedVecParams p) {
+  pdl_trigger();
+  pdl_wait();
   strided_vec_body(p, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 // Several element-wise copies in one launch, any strides and either element type on either side.
@@ -225,6 +231,8 @@ struct StridedCopyItem {
 constexpr int STRIDED_BATCH_MAX = 8;
 struct StridedCopyBatch { StridedCopyItem item[STRIDED_BATCH_MAX]; };
 __global__ void __launch_bounds__(256) strided_copy_batch_kernel(const __grid_constant__ StridedCopyBatch b) {
+  pdl_trigger();
+  pdl_wait();
   const StridedCopyItem& p = b.item[blockIdx.y];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
@@ -261,6 +269,8 @@ __global__ void __launch_bounds__(256) strided_copy_batch_kernel(const __grid_co
 // Several vector copies in one launch (the inputs of a concatenate): blockIdx.y picks the copy.
 struct StridedVecBatch { StridedVecParams item[STRIDED_BATCH_MAX]; };
 __global__ void __launch_bounds__(256) strided_vec_batch_kernel(const __grid_constant__ StridedVecBatch b) {
+  pdl_trigger();
+  pdl_wait();
   strided_vec_body(b.item[blockIdx.y], (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
@@ -273,6 +283,8 @@ struct ReduceParams {
   DevChain chain;
 };
 __global__ void __launch_bounds__(256) reduce_kernel(const __grid_constant__ ReduceParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     int64_t rem = i, base = 0;
@@ -304,57 +316,74 @@ __global__ void __launch_bounds__(256) reduce_kernel(const __grid_constant__ Red
   }
 }
 
-// max_pool2d, NHWC.  int8: one thread owns 16 channels of one output pixel (vmax4 on packed
-// bytes); int32: 4 channels.  Taps outside the image are skipped, which equals a max with INT_MIN
-// because the reference guarantees at least one tap inside (pad < pool size).
-// One thread per 16 neighbouring outputs (innermost kept extent, counted in groups of 16 here).
-__global__ void __launch_bounds__(128) reduce_vec16_kernel(const __grid_constant__ ReduceParams p) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
-    int64_t rem = i, base = 0;
-#pragma unroll
-    for (int k = 5; k >= 0; --k) {
-      if (k < p.n_keep) {
-        const int64_t c = rem % p.ke[k];
-        rem /= p.ke[k];
-        base += c * (k == p.n_keep - 1 ? 16 : p.ks[k]);
-      }
-    }
-    const int8_t* src = reinterpret_cast<const int8_t*>(p.x) + base;
+// Reduction of one run of elements at a constant stride over 16 neighbouring outputs at a time (the
+// innermost kept extent, counted in groups of 16 here): global pooling over channels-last tensors.  A
+// block takes 32 such groups and deals every run to 8 slices of 32 threads, which meet in shared
+// memory: a thread by itself had 49 dependent-latency loads to make (7 x 7 x 2048, one image: 10 us; with
+// a handful in flight at once 3 us).
+constexpr int RED_SLICES = 8;
+__global__ void __launch_bounds__(256) reduce_vec16_kernel(const __grid_constant__ ReduceParams p) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ int32_t part[RED_SLICES][32][17];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int32_t start = p.is_max && !p.init_zero ? INT32_MIN : 0;
+  for (int64_t g0 = (int64_t)blockIdx.x * 32; g0 < p.total; g0 += (int64_t)gridDim.x * 32) {
+    const int64_t i = g0 + lane;
     int32_t acc[16];
-    int64_t r0 = 0;
-    if (p.init_zero) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] = 0;
-    } else {
-      const int4 raw = __ldg(reinterpret_cast<const int4*>(src));
-      const int w[4] = {raw.x, raw.y, raw.z, raw.w};
+    for (int j = 0; j < 16; ++j) acc[j] = start;
+    if (i < p.total) {
+      int64_t rem = i, base = 0;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] = (int32_t)(int8_t)(w[j >> 2] >> ((j & 3) * 8));
-      r0 = 1;
-    }
-#pragma unroll 4
-    for (int64_t r = r0; r < p.red_total; ++r) {
-      const int4 raw = __ldg(reinterpret_cast<const int4*>(src + r * p.rs[0]));
-      const int w[4] = {raw.x, raw.y, raw.z, raw.w};
+      for (int k = 5; k >= 0; --k) {
+        if (k < p.n_keep) {
+          const int64_t q = rem / p.ke[k];
+          base += (rem - q * p.ke[k]) * (k == p.n_keep - 1 ? 16 : p.ks[k]);
+          rem = q;
+        }
+      }
+      const int8_t* src = reinterpret_cast<const int8_t*>(p.x) + base;
+      const int64_t step = p.rs[0];
+#pragma unroll 8
+      for (int r = slice; r < (int)p.red_total; r += RED_SLICES) {
+        const int4 raw = __ldg(reinterpret_cast<const int4*>(src + r * step));
+        const int w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int32_t val = (int32_t)(int8_t)(w[j >> 2] >> ((j & 3) * 8));
-        if (p.is_max) acc[j] = acc[j] < val ? val : acc[j];
-        else acc[j] = (int32_t)((uint32_t)acc[j] + (uint32_t)val);
+        for (int j = 0; j < 16; ++j) {
+          const int32_t val = (int32_t)(int8_t)(w[j >> 2] >> ((j & 3) * 8));
+          if (p.is_max) acc[j] = max(acc[j], val);
+          else acc[j] = (int32_t)((uint32_t)acc[j] + (uint32_t)val);
+        }
       }
     }
-    apply_chain<16>(p.chain, acc, (size_t)i * 16, 0, 0);
-    if (p.yd == CVMK_I8) {
-      reinterpret_cast<int4*>(p.y)[i] = pack16(acc);
-    } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        reinterpret_cast<int4*>(p.y)[i * 4 + q] = make_int4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+    for (int j = 0; j < 16; ++j) part[slice][lane][j] = acc[j];
+    __syncthreads();
+    // 32 x 16 results, two neighbouring ones a thread
+    const int v = threadIdx.x >> 3, j0 = (threadIdx.x & 7) * 2;
+    int32_t o[2] = {start, start};
+#pragma unroll
+    for (int s = 0; s < RED_SLICES; ++s)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int32_t val = part[s][v][j0 + j];
+        if (p.is_max) o[j] = max(o[j], val);
+        else o[j] = (int32_t)((uint32_t)o[j] + (uint32_t)val);
+      }
+    if (g0 + v < p.total) {
+      const int64_t out = (g0 + v) * 16 + j0;
+      apply_chain<2>(p.chain, o, (size_t)out, 0, 0);
+      if (p.yd == CVMK_I8) *reinterpret_cast<char2*>(reinterpret_cast<int8_t*>(p.y) + out) = make_char2((char)o[0], (char)o[1]);
+      else *reinterpret_cast<int2*>(reinterpret_cast<int32_t*>(p.y) + out) = make_int2(o[0], o[1]);
     }
+    __syncthreads();
   }
 }
 
+// max_pool2d, NHWC.  int8: one thread owns 16 channels of one output pixel (vmax4 on packed
+// bytes); int32: 4 channels.  Taps outside the image are skipped, which equals a max with INT_MIN
+// because the reference guarantees at least one tap inside (pad < pool size).
 struct PoolParams {
   const void* x; void* y;
   int N, H, W, C, OH, OW, KH, KW, sh, sw, ph, pw;
@@ -366,6 +395,8 @@ struct PoolParams {
 // 64-bit ones cost more instructions than the nine taps of a 3x3 window).
 template <int DT, bool IDX32>
 __global__ void __launch_bounds__(256) pool_vec_kernel(const __grid_constant__ PoolParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     int cv, ox, oy, n;
@@ -438,6 +469,8 @@ __global__ void __launch_bounds__(256) pool_vec_kernel(const __grid_constant__ P
 }
 // Any channel count: one thread per output element.
 __global__ void __launch_bounds__(256) pool_scalar_kernel(const __grid_constant__ PoolParams p, int dt) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t total = (int64_t)p.N * p.OH * p.OW * p.C;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -494,10 +527,10 @@ extern "C" int cvmk_elemwise(const void* x, int x_dtype, void* y, int y_dtype, i
   const int threads = 256;
   const int grid = grid_for((n + 15) / 16, threads);
   cudaStream_t s = (cudaStream_t)stream;
-  if (x_dtype == CVMK_I8 && y_dtype == CVMK_I8) elemwise_kernel<CVMK_I8, CVMK_I8><<<grid, threads, 0, s>>>(x, y, n, chain);
-  else if (x_dtype == CVMK_I8) elemwise_kernel<CVMK_I8, CVMK_I32><<<grid, threads, 0, s>>>(x, y, n, chain);
-  else if (y_dtype == CVMK_I8) elemwise_kernel<CVMK_I32, CVMK_I8><<<grid, threads, 0, s>>>(x, y, n, chain);
-  else elemwise_kernel<CVMK_I32, CVMK_I32><<<grid, threads, 0, s>>>(x, y, n, chain);
+  if (x_dtype == CVMK_I8 && y_dtype == CVMK_I8) launch_pdl(elemwise_kernel<CVMK_I8, CVMK_I8>, dim3((unsigned)(grid)), dim3(threads), 0, s, x, y, n, chain);
+  else if (x_dtype == CVMK_I8) launch_pdl(elemwise_kernel<CVMK_I8, CVMK_I32>, dim3((unsigned)(grid)), dim3(threads), 0, s, x, y, n, chain);
+  else if (y_dtype == CVMK_I8) launch_pdl(elemwise_kernel<CVMK_I32, CVMK_I8>, dim3((unsigned)(grid)), dim3(threads), 0, s, x, y, n, chain);
+  else launch_pdl(elemwise_kernel<CVMK_I32, CVMK_I32>, dim3((unsigned)(grid)), dim3(threads), 0, s, x, y, n, chain);
   return check_cuda(cudaGetLastError(), "elemwise_kernel launch");
 }
 
@@ -577,7 +610,7 @@ extern "C" int cvmk_strided_batch(const cvmk_strided_desc* d, int32_t n, cvmk_st
           it.a = e.a; it.y = e.y; it.ad = e.a_dtype; it.yd = e.y_dtype; it.a_off = e.a_off; it.y_off = e.y_off;
           largest = std::max(largest, it.total);
         }
-        strided_copy_batch_kernel<<<dim3((unsigned)grid_for(largest, 256), (unsigned)m), 256, 0, s>>>(b);
+        launch_pdl(strided_copy_batch_kernel, dim3((unsigned)grid_for(largest, 256), (unsigned)m), dim3(256), 0, s, b);
         if (check_cuda(cudaGetLastError(), "strided_copy_batch_kernel launch")) return CVMK_ERR_CUDA;
       }
       return CVMK_OK;
@@ -602,7 +635,7 @@ extern "C" int cvmk_strided_batch(const cvmk_strided_desc* d, int32_t n, cvmk_st
       }
       return CVMK_OK;
     }
-    strided_vec_batch_kernel<<<dim3((unsigned)grid_for(largest, 256), (unsigned)m), 256, 0, s>>>(b);
+    launch_pdl(strided_vec_batch_kernel, dim3((unsigned)grid_for(largest, 256), (unsigned)m), dim3(256), 0, s, b);
     if (check_cuda(cudaGetLastError(), "strided_vec_batch_kernel launch")) return CVMK_ERR_CUDA;
   }
   if (all) return CVMK_OK;
@@ -621,7 +654,7 @@ extern "C" int cvmk_strided(const cvmk_strided_desc* d, cvmk_stream_t stream) {
   {
     StridedVecParams p;
     if (strided_as_vectors(d, total, &p)) {
-      strided_vec_kernel<<<grid_for(p.total_vec, threads), threads, 0, s>>>(p);
+      launch_pdl(strided_vec_kernel, dim3((unsigned)(grid_for(p.total_vec, threads))), dim3(threads), 0, s, p);
       return check_cuda(cudaGetLastError(), "strided_vec_kernel launch");
     }
   }
@@ -639,7 +672,7 @@ extern "C" int cvmk_strided(const cvmk_strided_desc* d, cvmk_stream_t stream) {
   p.a_off = d->a_off; p.b_off = d->b_off; p.y_off = d->y_off;
   int rc = lower_chain(d->ep, &p.chain);
   if (rc != CVMK_OK) return rc;
-  strided_kernel<<<grid_for(total, threads), threads, 0, s>>>(p);
+  launch_pdl(strided_kernel, dim3((unsigned)(grid_for(total, threads))), dim3(threads), 0, s, p);
   return check_cuda(cudaGetLastError(), "strided_kernel launch");
 }
 
@@ -655,7 +688,7 @@ extern "C" int cvmk_reduce(const cvmk_reduce_desc* d, cvmk_stream_t stream) {
       re *= d->red_extent[k];
     }
     const int in = d->n_keep - 1;
-    bool ok = one_run && d->keep_stride[in] == 1 && d->keep_extent[in] % 16 == 0 && rs % 16 == 0 && aligned16(d->x) &&
+    bool ok = one_run && re < INT32_MAX && d->keep_stride[in] == 1 && d->keep_extent[in] % 16 == 0 && rs % 16 == 0 && aligned16(d->x) &&
               (d->y_dtype == CVMK_I32 ? aligned16(d->y) : aligned16(d->y));
     for (int k = 0; ok && k < in; ++k) ok = d->keep_stride[k] % 16 == 0;
     if (ok) {
@@ -670,7 +703,7 @@ extern "C" int cvmk_reduce(const cvmk_reduce_desc* d, cvmk_stream_t stream) {
       p.x = d->x; p.y = d->y; p.xd = d->x_dtype; p.yd = d->y_dtype;
       int rc = lower_chain(d->ep, &p.chain);
       if (rc != CVMK_OK) return rc;
-      reduce_vec16_kernel<<<grid_for(p.total, 128), 128, 0, (cudaStream_t)stream>>>(p);
+      launch_pdl(reduce_vec16_kernel, dim3((unsigned)grid_for(p.total, 32)), dim3(256), 0, (cudaStream_t)stream, p);
       return check_cuda(cudaGetLastError(), "reduce_vec16_kernel launch");
     }
   }
@@ -688,7 +721,7 @@ extern "C" int cvmk_reduce(const cvmk_reduce_desc* d, cvmk_stream_t stream) {
   int rc = lower_chain(d->ep, &p.chain);
   if (rc != CVMK_OK) return rc;
   const int threads = 256;
-  reduce_kernel<<<grid_for(p.total, threads), threads, 0, (cudaStream_t)stream>>>(p);
+  launch_pdl(reduce_kernel, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "reduce_kernel launch");
 }
 
@@ -700,6 +733,8 @@ extern "C" int cvmk_reduce(const cvmk_reduce_desc* d, cvmk_stream_t stream) {
 // values per instruction: a row of taps is one __vimax3_s16x2, the rows another.
 template <int K, bool IDX32>
 __global__ void __launch_bounds__(256) pool_window_kernel(const __grid_constant__ PoolParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     int cv, ox, oy, n;
@@ -785,23 +820,23 @@ extern "C" int cvmk_max_pool2d(const cvmk_pool_desc* d, cvmk_stream_t stream) {
     if (window) {
       const int grid = grid_for(p.total, threads);
       if (d->KH == 3) {
-        if (idx32) pool_window_kernel<3, true><<<grid, threads, 0, s>>>(p);
-        else pool_window_kernel<3, false><<<grid, threads, 0, s>>>(p);
+        if (idx32) launch_pdl(pool_window_kernel<3, true>, dim3((unsigned)(grid)), dim3(threads), 0, s, p);
+        else launch_pdl(pool_window_kernel<3, false>, dim3((unsigned)(grid)), dim3(threads), 0, s, p);
       } else {
-        if (idx32) pool_window_kernel<2, true><<<grid, threads, 0, s>>>(p);
-        else pool_window_kernel<2, false><<<grid, threads, 0, s>>>(p);
+        if (idx32) launch_pdl(pool_window_kernel<2, true>, dim3((unsigned)(grid)), dim3(threads), 0, s, p);
+        else launch_pdl(pool_window_kernel<2, false>, dim3((unsigned)(grid)), dim3(threads), 0, s, p);
       }
     } else if (d->dtype == CVMK_I8) {
-      if (idx32) pool_vec_kernel<CVMK_I8, true><<<grid_for(p.total, threads), threads, 0, s>>>(p);
-      else pool_vec_kernel<CVMK_I8, false><<<grid_for(p.total, threads), threads, 0, s>>>(p);
+      if (idx32) launch_pdl(pool_vec_kernel<CVMK_I8, true>, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, s, p);
+      else launch_pdl(pool_vec_kernel<CVMK_I8, false>, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, s, p);
     } else {
-      if (idx32) pool_vec_kernel<CVMK_I32, true><<<grid_for(p.total, threads), threads, 0, s>>>(p);
-      else pool_vec_kernel<CVMK_I32, false><<<grid_for(p.total, threads), threads, 0, s>>>(p);
+      if (idx32) launch_pdl(pool_vec_kernel<CVMK_I32, true>, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, s, p);
+      else launch_pdl(pool_vec_kernel<CVMK_I32, false>, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, s, p);
     }
   } else {
     p.cvec = 0;
     p.total = (int64_t)d->N * d->OH * d->OW * d->C;
-    pool_scalar_kernel<<<grid_for(p.total, threads), threads, 0, s>>>(p, d->dtype);
+    launch_pdl(pool_scalar_kernel, dim3((unsigned)(grid_for(p.total, threads))), dim3(threads), 0, s, p, d->dtype);
   }
   return check_cuda(cudaGetLastError(), "max_pool2d launch");
 }

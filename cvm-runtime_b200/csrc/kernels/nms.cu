@@ -105,6 +105,8 @@ template <bool CLAMP>
 __global__ void __launch_bounds__(THREADS, 1) gvc6_kernel(const int32_t* __restrict__ x, int32_t* __restrict__ y,
                                                           int32_t* __restrict__ valid_count, int N, int thr,
                                                           int chunk_rows, int clamp) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int ws[WARPS + 1];
   __shared__ int red[2][WARPS];
   const int b = blockIdx.y, c = blockIdx.x;
@@ -173,6 +175,8 @@ __global__ void __launch_bounds__(THREADS, 1) gvc6_kernel(const int32_t* __restr
 __global__ void __launch_bounds__(THREADS) gvc_kernel(const int32_t* __restrict__ x, int32_t* __restrict__ y,
                                                       int32_t* __restrict__ valid_count, int N, int K,
                                                       int thr, int clamp) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int ws[WARPS + 1];
   const int b = blockIdx.x;
   const int32_t* xb = x + (size_t)b * N * K;
@@ -277,6 +281,8 @@ __device__ __forceinline__ bool iou_ge_small(const int32_t* a, const int32_t* b,
 }
 
 __global__ void __launch_bounds__(THREADS) nms_kernel(const __grid_constant__ NmsParams p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   __shared__ int ws[WARPS + 1];
@@ -830,13 +836,11 @@ extern "C" int cvmk_get_valid_counts_clamped(const int32_t* x, int32_t* y, int32
     int chunk_rows = ((N + chunks - 1) / chunks + 3) & ~3;
     chunks = (N + chunk_rows - 1) / chunk_rows;
     if (clamp > 0)
-      gvc6_kernel<true><<<dim3((unsigned)chunks, (unsigned)B), THREADS, 0, (cudaStream_t)stream>>>(
-          x, y, valid_count, N, score_threshold, chunk_rows, clamp);
+      launch_pdl(gvc6_kernel<true>, dim3((unsigned)chunks, (unsigned)B), dim3(THREADS), 0, (cudaStream_t)stream, x, y, valid_count, N, score_threshold, chunk_rows, clamp);
     else
-      gvc6_kernel<false><<<dim3((unsigned)chunks, (unsigned)B), THREADS, 0, (cudaStream_t)stream>>>(
-          x, y, valid_count, N, score_threshold, chunk_rows, INT32_MAX);
+      launch_pdl(gvc6_kernel<false>, dim3((unsigned)chunks, (unsigned)B), dim3(THREADS), 0, (cudaStream_t)stream, x, y, valid_count, N, score_threshold, chunk_rows, INT32_MAX);
   } else
-    gvc_kernel<<<B, THREADS, 0, (cudaStream_t)stream>>>(x, y, valid_count, N, K, score_threshold,
+    launch_pdl(gvc_kernel, dim3((unsigned)(B)), dim3(THREADS), 0, (cudaStream_t)stream, x, y, valid_count, N, K, score_threshold,
                                                         clamp > 0 ? clamp : INT32_MAX);
   return check_cuda(cudaGetLastError(), "gvc_kernel launch");
 }
@@ -877,7 +881,7 @@ static int nms_launch(NmsParams& p, cudaStream_t stream, const char* what) {
     fillers = std::min(fillers, std::max(1, 4 * sms / p.B));
   }
   if (p.B > 65535) { set_error("non_max_suppression: batch %d too large", p.B); return CVMK_ERR_ARG; }
-  nms_kernel<<<dim3(1 + fillers, p.B), THREADS, smem, stream>>>(p);
+  launch_pdl(nms_kernel, dim3(1 + fillers, p.B), dim3(THREADS), smem, stream, p);
   return check_cuda(cudaGetLastError(), what);
 }
 

@@ -24,6 +24,8 @@ struct TakeParams {
 // y[o, m, n] = x[o, clamp(idx[m], 0, extent - 1), n]; one thread per output element, consecutive
 // threads along n (then m), so writes are coalesced and reads are coalesced runs of `inner`.
 __global__ void __launch_bounds__(256) take_kernel(const __grid_constant__ TakeParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     const int64_t n = i % p.inner, t = i / p.inner;
@@ -41,6 +43,8 @@ struct WhereParams {
 };
 
 __global__ void __launch_bounds__(256) where_kernel(const __grid_constant__ WhereParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += stride) {
     const int32_t c = load_any(p.c, p.cd, p.inner == 1 ? i : i / p.inner);
@@ -62,6 +66,8 @@ struct TransposeParams {
 };
 template <typename T, int TILE>
 __global__ void __launch_bounds__(256) transpose_kernel(const __grid_constant__ TransposeParams p) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ T tile[TILE][TILE + (sizeof(T) == 1 ? 4 : 1)];
   const T* x = reinterpret_cast<const T*>(p.x);
   T* y = reinterpret_cast<T*>(p.y);
@@ -142,7 +148,7 @@ extern "C" int cvmk_take(const cvmk_take_desc* d, cvmk_stream_t stream) {
   p.xd = d->x_dtype; p.id = d->idx_dtype; p.yd = d->y_dtype;
   p.count = d->count; p.inner = d->inner; p.extent = d->extent;
   p.total = d->outer * d->count * d->inner;
-  take_kernel<<<grid_for(p.total, 256), 256, 0, (cudaStream_t)stream>>>(p);
+  launch_pdl(take_kernel, dim3((unsigned)(grid_for(p.total, 256))), dim3(256), 0, (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "take_kernel launch");
 }
 
@@ -156,7 +162,7 @@ extern "C" int cvmk_where(const cvmk_where_desc* d, cvmk_stream_t stream) {
   p.c = d->cond; p.x = d->x; p.y = d->y; p.out = d->out;
   p.cd = d->cond_dtype; p.xd = d->x_dtype; p.yd = d->y_dtype; p.od = d->out_dtype;
   p.total = d->n; p.inner = d->inner;
-  where_kernel<<<grid_for(p.total, 256), 256, 0, (cudaStream_t)stream>>>(p);
+  launch_pdl(where_kernel, dim3((unsigned)(grid_for(p.total, 256))), dim3(256), 0, (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "where_kernel launch");
 }
 
@@ -175,8 +181,8 @@ extern "C" int cvmk_transpose_batched(const void* x, void* y, int32_t dtype, int
   p.total_tiles = batch * p.tiles_r * p.tiles_c;
   const int64_t cap = 148 * 8;
   const int grid = (int)(p.total_tiles < cap ? p.total_tiles : cap);
-  if (dtype == CVMK_I8) transpose_kernel<int8_t, 64><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
-  else transpose_kernel<int32_t, 32><<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+  if (dtype == CVMK_I8) launch_pdl(transpose_kernel<int8_t, 64>, dim3((unsigned)(grid)), dim3(256), 0, (cudaStream_t)stream, p);
+  else launch_pdl(transpose_kernel<int32_t, 32>, dim3((unsigned)(grid)), dim3(256), 0, (cudaStream_t)stream, p);
   return check_cuda(cudaGetLastError(), "transpose_kernel launch");
 }
 
