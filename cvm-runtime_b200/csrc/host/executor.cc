@@ -1619,6 +1619,8 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
   CUDA_OK(cudaMallocHost((void**)&status_host_, 256));
   pinned_.push_back(status_host_);
   *status_host_ = 0;
+  done_host_ = status_host_ + 32;
+  *done_host_ = 0;
   use_graph_ = dev_env("CVM_B200_NO_GRAPH") == nullptr;
   if (vmm().ok && !dev_env("CVM_B200_NO_PLANNER")) {
     const CUmemAllocationProp prop = device_prop(device_);
@@ -1647,9 +1649,13 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
       chunk_events_.resize(steps_[0].chunk.size());
       for (auto& e : chunk_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
-    auto capture_from = [&](size_t first, cudaGraphExec_t* exec) {
+    auto capture_from = [&](size_t first, cudaGraphExec_t* exec, bool staged = false) {
       cudaGraph_t graph = nullptr;
       CUDA_OK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+      if (staged) {
+        const cvmk_export_segment seg = {in_host_, in_dev_, 1, (int64_t)in_bytes_, (int64_t)in_bytes_};
+        KERNEL_OK(cvmk_export(&seg, 1, stream_));
+      }
       Enqueue(stream_, first);  // the chunked prefix is launched outside the graph
       CUDA_OK(cudaStreamEndCapture(stream_, &graph));
       CUDA_OK(cudaGraphInstantiate(exec, graph, 0));
@@ -1658,6 +1664,7 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
     capture_from(prefix_steps_, &graph_exec_);
     if (prefix_steps_pageable_ != prefix_steps_) capture_from(prefix_steps_pageable_, &graph_exec_pageable_);
     if (prefix_steps_ > 0) capture_from(0, &graph_exec_device_);
+    if (in_bytes_ <= kSmallInput) capture_from(0, &graph_exec_staged_, true);
   }
 }
 
@@ -1742,6 +1749,7 @@ Executor::~Executor() {
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   if (graph_exec_pageable_) cudaGraphExecDestroy(graph_exec_pageable_);
   if (graph_exec_device_) cudaGraphExecDestroy(graph_exec_device_);
+  if (graph_exec_staged_) cudaGraphExecDestroy(graph_exec_staged_);
   if (kernels_exec_) cudaGraphExecDestroy(kernels_exec_);
   for (auto e : piece_events_) cudaEventDestroy(e);
   for (auto e : chunk_events_) cudaEventDestroy(e);
@@ -1758,10 +1766,12 @@ Executor::~Executor() {
 
 // Where the bytes of an input come from.  Page-locked (or device) memory is read where it lies.  A
 // pageable input of up to 1 MiB is copied into the staging buffer by the calling thread (waking
-// helpers costs more than they save: 1 MiB takes about 50 us cold), a larger one by the pool.
+// helpers costs more than they save: 1 MiB takes about 50 us cold), a larger one by the pool.  A
+// page-locked input of up to 256 KiB is staged as well: the copy takes 4 us, and the inference
+// is then one graph that begins by fetching the staging buffer.
 Executor::Source Executor::SourceOf(const void* input) const {
-  if (IsDirect(input)) return Source::kDirect;
-  return in_bytes_ <= ((size_t)1 << 20) ? Source::kSmall : Source::kPool;
+  if (IsDirect(input)) return in_bytes_ <= kSmallDirect && graph_exec_staged_ && !IsDevice(input) ? Source::kSmall : Source::kDirect;
+  return in_bytes_ <= kSmallInput ? Source::kSmall : Source::kPool;
 }
 
 HostPool& Executor::pool() {
@@ -1865,6 +1875,23 @@ void Executor::Enqueue(cudaStream_t s, size_t first) {
     for (auto& h : heads_) CUDA_OK(cudaMemcpyAsync(h.host, h.dev, h.bytes, cudaMemcpyDeviceToHost, s));
   }
   KERNEL_OK(cvmk_export(seg, n, s));
+  if (download_ == Download::kKernel) KERNEL_OK(cvmk_signal(done_host_, s));
+}
+
+// Waits for the word that the last kernel writes after the heads: the host sees it some microseconds
+// before the stream reports its end.  The stream is asked now and then, so that an error ends the wait.
+void Executor::AwaitDone() {
+  volatile int32_t* done = done_host_;
+  for (uint32_t k = 1; *done == 0; ++k) {
+    if ((k & 1023) == 0) {
+      const cudaError_t e = cudaStreamQuery(stream_);
+      if (e == cudaErrorNotReady) continue;
+      CUDA_OK(e);
+      break;
+    }
+    HostPool::Relax();
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
 }
 
 // The part of an NMS head that is -1 whatever the data says, written while the GPU works.
@@ -1950,11 +1977,16 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
     guard.p = &pool();
     guard.p->Begin();
   }
+  const bool signal = download_ == Download::kKernel;
+  if (signal) *(volatile int32_t*)done_host_ = 0;
   BeginUpload(input, src);
   if (fill) StartFill(out);
   const bool pageable = graph_exec_pageable_ && src != Source::kDirect;
   const size_t prefix = on_device ? 0 : (pageable ? prefix_steps_pageable_ : prefix_steps_);
-  if (graph_exec_ && prefix > 0) {
+  if (src == Source::kSmall && graph_exec_staged_) {
+    memcpy(in_host_, input, in_bytes_);
+    CUDA_OK(cudaGraphLaunch(graph_exec_staged_, stream_));
+  } else if (graph_exec_ && prefix > 0) {
     // chunk c of the batch is uploaded on the copy stream while the leading steps run on chunk c - 1
     for (size_t c = 0; c < steps_[0].chunk.size(); ++c) {
       SendRange(input, src, c * chunk_bytes_, chunk_bytes_, copy_stream_);
@@ -1973,6 +2005,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
     else Enqueue(stream_);
   }
   if (pieces) DeliverPieces(out);
+  else if (signal) AwaitDone();
   else CUDA_OK(cudaStreamSynchronize(stream_));
   if (*status_host_ != 0) {
     const int code = *status_host_;

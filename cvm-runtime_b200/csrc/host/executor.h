@@ -119,6 +119,9 @@ class Executor {
   cudaStream_t copy_stream_ = nullptr;
   std::vector<cudaEvent_t> chunk_events_;
   cudaGraphExec_t graph_exec_device_ = nullptr;   // every step: the input is on the device already
+  cudaGraphExec_t graph_exec_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
+  int32_t* done_host_ = nullptr;    // pinned: the last kernel of an inference has delivered the heads
+  void AwaitDone();
   std::unique_ptr<HostPool> pool_;   // created by the first inference that has enough bytes to move
   HostPool& pool();
   // How the heads reach the host: small ones are written into page-locked memory by a kernel
@@ -164,6 +167,7 @@ class Executor {
   // Uploads: BeginUpload() starts the staging of a pageable input (the whole of it), SendRange()
   // queues the transfer of a part, Upload() does both for all of it.
   enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
+  static constexpr size_t kSmallInput = (size_t)1 << 20, kSmallDirect = (size_t)1 << 18;
   static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
   Source SourceOf(const void* input) const;
   void BeginUpload(const void* input, Source src);

@@ -8,15 +8,16 @@
 namespace cvm {
 
 namespace {
-inline void relax() {
+constexpr uint64_t kCount = 0xffffffffull;
+}  // namespace
+
+void HostPool::Relax() {
 #if defined(__x86_64__)
   _mm_pause();
 #else
   std::this_thread::yield();
 #endif
 }
-constexpr uint64_t kCount = 0xffffffffull;
-}  // namespace
 
 HostPool::HostPool(int helpers) {
   for (int i = 0; i < helpers; ++i) workers_.emplace_back([this] { Work(); });
@@ -89,20 +90,20 @@ void HostPool::Work() {
       cv_.wait(lk, [&] { return stop_ || active_; });
       if (stop_) return;
     }
-    if (!HelpOnce()) relax();
+    if (!HelpOnce()) Relax();
   }
 }
 
 void HostPool::WaitPiece(Slot slot, size_t k) {
   Job& j = jobs_[slot];
   while (!j.done[k].load(std::memory_order_acquire))
-    if (!RunPiece(j)) relax();
+    if (!RunPiece(j)) Relax();
 }
 
 void HostPool::Finish(Slot slot) {
   Job& j = jobs_[slot];
   while (j.completed.load(std::memory_order_acquire) < j.pieces)
-    if (!RunPiece(j)) relax();
+    if (!RunPiece(j)) Relax();
 }
 
 void stream_copy(char* dst, const char* src, size_t bytes) {

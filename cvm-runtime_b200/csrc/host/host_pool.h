@@ -38,6 +38,7 @@ class HostPool {
   void WaitPiece(Slot slot, size_t k);
   // Waits until the whole job has run.
   void Finish(Slot slot);
+  static void Relax();   // one turn of a spin
   // Runs one piece of any job, if one is free; false if there is none.
   bool HelpOnce();
 

@@ -211,8 +211,10 @@ CVMK_API int cvmk_strided_batch(const cvmk_strided_desc* d, int32_t n, cvmk_stre
 
 /* ------------------------------------------------------------------------------------------------
  * Copies up to CVMK_MAX_EXPORT_SEGMENTS row sets in one launch: rows * row_bytes bytes of each segment,
- * src rows src_pitch bytes apart, dst rows packed.  dst may be page-locked host memory: that is how
- * small results (and the status word) leave the GPU.
+ * src rows src_pitch bytes apart, dst rows packed.  Either side may be page-locked host memory: that is
+ * how small inputs enter and small results (and the status word) leave the GPU. 
+ * cvmk_signal() writes 1 to `flag` (an int32 in page-locked host memory) after everything before it in
+ * the stream is visible to the host.
  * ---------------------------------------------------------------------------------------------- */
 #define CVMK_MAX_EXPORT_SEGMENTS 8
 typedef struct {
@@ -220,6 +222,7 @@ typedef struct {
   int64_t rows, row_bytes, src_pitch;
 } cvmk_export_segment;
 CVMK_API int cvmk_export(const cvmk_export_segment* segments, int32_t n, cvmk_stream_t stream);
+CVMK_API int cvmk_signal(int32_t* flag, cvmk_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------
  * sum / max reduce (cpu/ops/reduce.cc:34-140).  Output point c (up to 6 kept extents, strides into
