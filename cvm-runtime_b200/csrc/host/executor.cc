@@ -208,19 +208,13 @@ struct Lowering {
   void add_step(const std::string& label, std::function<int(cudaStream_t)> fn) {
     ex.steps_.push_back({label, std::move(fn), {}});
   }
-  // Batch chunks for upload / compute overlap: four (CVM_B200_UPLOAD_CHUNKS) when the batch
-  // divides, else none.
-  static int upload_chunks() {
-    static const int k = [] {
-      const char* e = dev_env("CVM_B200_UPLOAD_CHUNKS");
-      const int v = e ? atoi(e) : 4;
-      return v >= 2 && v <= 16 ? v : 4;
-    }();
-    return k;
-  }
-  static int batch_chunks(int64_t n) {
-    const int k = upload_chunks();
-    return (n % k == 0 && n >= 2 * k && !dev_env("CVM_B200_NO_UPLOAD_OVERLAP")) ? k : 1;
+  // Parts of the batch for upload / compute overlap: an eighth, three quarters, an eighth.  Where the
+  // kernels take longer than the upload, what counts is how soon the first part is there; where the
+  // upload takes longer, how little is left to do when the last part has arrived.  Image numbers of
+  // the part boundaries; just {0, n} for batches under eight images.
+  static std::vector<int64_t> batch_parts(int64_t n) {
+    if (n < 8 || dev_env("CVM_B200_NO_UPLOAD_OVERLAP")) return {0, n};
+    return {0, (n + 4) / 8, (3 * n + 4) / 8, (5 * n + 4) / 8, (7 * n + 4) / 8, n};
   }
 
   // ------------------------------------------------------------------ analysis
@@ -705,40 +699,57 @@ struct Lowering {
       sd.status = ex.status_dev_;
       sd.acc_bound = probe.acc_bound;
       sd.ep = ch.ep;
+      if (W % 16 != 0) sd.x_pitch = (W + 15) / 16 * 16;   // TMA rows start on 16-byte boundaries: the rows are moved apart first
       if (cvmk_conv2d_stem_supported(&sd)) {
         std::vector<int8_t> ws((size_t)cvmk_conv2d_stem_weight_bytes(&sd), 0);
         KERNEL_OK(cvmk_conv2d_stem_pack_weights(&sd, wt.data.data(), ws.data()));
         int8_t* wsdev = (int8_t*)ex.dalloc(ws.size());
         CUDA_OK(cudaMemcpy(wsdev, ws.data(), ws.size(), cudaMemcpyHostToDevice));
         sd.w = wsdev;
-        // The batch is cut into chunks with a plan each, so that an inference can run the stem on
-        // the first images while the later ones are still being uploaded.
-        const int chunks = (uses[ex_] == 1 && !is_head[ex_]) ? batch_chunks(N) : 1;
-        const int per = N / chunks;
-        // plan 0 covers the whole batch (one launch when the input is already on the device);
-        // plans 1.. cover one chunk each
-        std::vector<cvmk_stem_conv_plan*> plans;
-        for (int c = -1; c < (chunks > 1 ? chunks : 0); ++c) {
+        // The batch is cut into parts with a plan each, so that an inference can run the stem on the
+        // first images while the later ones are still being uploaded.
+        const std::vector<int64_t> parts = (uses[ex_] == 1 && !is_head[ex_]) ? batch_parts(N) : std::vector<int64_t>{0, N};
+        const size_t count = parts.size() - 1;
+        const size_t image = (size_t)C * H * W;
+        int8_t* rows = nullptr;
+        const int pitch = sd.x_pitch;
+        if (pitch > 0) {
+          rows = (int8_t*)act_alloc((size_t)N * C * H * pitch);
+          sd.x = rows;
+          auto move = [this, rows, pitch, image, C, H, W](int64_t b0, int64_t b1) {
+            const char* from = (const char*)raw_in.ptr + (size_t)b0 * image;
+            char* to = (char*)rows + (size_t)b0 * C * H * pitch;
+            const int64_t n = (b1 - b0) * C * H;
+            return [from, to, n, W, pitch](cudaStream_t s) { return cvmk_repitch(from, to, n, W, pitch, s); };
+          };
+          bool aligned = true;
+          for (int64_t b : parts) aligned &= ((size_t)b * image) % 4 == 0;
+          add_step(label + "[rows]", move(0, N));
+          ex.steps_.back().from_input = true;
+          if (count > 1 && aligned)
+            for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(move(parts[c], parts[c + 1]));
+        }
+        auto plan_for = [&](int64_t b0, int64_t b1) {
           cvmk_stem_conv_desc cd = sd;
-          if (c >= 0) {
-            cd.N = per;
-            cd.x = sd.x + (size_t)c * per * C * H * W;
-            cd.y = (int8_t*)sd.y + (size_t)c * per * OH * OW * OC;
-          }
+          cd.N = (int)(b1 - b0);
+          cd.x = sd.x + (size_t)b0 * C * H * (pitch > 0 ? pitch : W);
+          cd.y = (int8_t*)sd.y + (size_t)b0 * OH * OW * OC;
           void* mem = nullptr;
           CHECK(posix_memalign(&mem, 64, sizeof(cvmk_stem_conv_plan)) == 0);
           ex.stem_plans_.emplace_back((cvmk_stem_conv_plan*)mem, plan_deleter);
-          KERNEL_OK(cvmk_conv2d_stem_prepare(&cd, ex.stem_plans_.back().get()));
-          plans.push_back(ex.stem_plans_.back().get());
-        }
-        cvmk_stem_conv_plan* whole = plans[0];
-        add_step(label + "[stem]", [whole](cudaStream_t s) { return cvmk_conv2d_stem_launch(whole, s); });
-        if (chunks > 1) {
-          ex.chunk_bytes_ = (size_t)per * C * H * W;
-          for (size_t c = 1; c < plans.size(); ++c) {
-            cvmk_stem_conv_plan* pl = plans[c];
-            ex.steps_.back().chunk.push_back([pl](cudaStream_t s) { return cvmk_conv2d_stem_launch(pl, s); });
-          }
+          cvmk_stem_conv_plan* pl = ex.stem_plans_.back().get();
+          KERNEL_OK(cvmk_conv2d_stem_prepare(&cd, pl));
+          return [pl](cudaStream_t s) { return cvmk_conv2d_stem_launch(pl, s); };
+        };
+        bool sliceable = count > 1;   // (parts start on 16-byte boundaries)
+        for (int64_t b : parts) sliceable &= ((size_t)b * C * H * (pitch > 0 ? pitch : W)) % 16 == 0;
+        add_step(label + "[stem]", plan_for(0, N));
+        ex.steps_.back().from_input = pitch == 0;
+        if (sliceable)
+          for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(plan_for(parts[c], parts[c + 1]));
+        if (count > 1) {
+          ex.part_end_.clear();
+          for (size_t c = 1; c <= count; ++c) ex.part_end_.push_back((size_t)parts[c] * image);
         }
         return;
       }
@@ -826,12 +837,16 @@ struct Lowering {
         d.ep.s[0].ptr = bfdev;
       }
       int fold = 1;
-      const int bchunks = batch_chunks(N);
+      const std::vector<int64_t> parts = batch_parts(N);
       if (!dense && !dw_tc && groups == 1 && KH == 1 && KW == 1 && sh == 1 && sw == 1 && ph == 0 && pw == 0 &&
           xin.nhwc && out.nhwc && (!use_bias || g.params.count(g.entry_id(n.inputs[2])) > 0) &&
           !dev_env("CVM_B200_NO_PIXEL_FOLD")) {
-        const int64_t per_chunk = (int64_t)(N / bchunks) * OH * OW;
-        while (fold < 4 && 2 * fold * C <= 128 && 2 * fold * OC <= 256 && per_chunk % (2 * fold) == 0) fold *= 2;
+        auto whole = [&](int f) {   // every part of the batch is a whole number of folded pixels
+          for (int64_t b : parts)
+            if (b * OH * OW % f != 0) return false;
+          return true;
+        };
+        while (fold < 4 && 2 * fold * C <= 128 && 2 * fold * OC <= 256 && whole(2 * fold)) fold *= 2;
       }
       if (fold > 1) {
         const int Cf = fold * C, OCf = fold * OC;
@@ -861,20 +876,20 @@ struct Lowering {
       cvmk_conv_plan* plan = ex.plans_.back().get();
       KERNEL_OK(cvmk_conv2d_tc_prepare(&d, plan));
       add_step(label + (dw_tc ? "[dw]" : "[tc]"), [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
-      // Quarter-batch plans (every operand is batch-major, so a chunk is a contiguous slice).
-      const int chunks = fold > 1 ? bchunks : batch_chunks(d.N);
-      if (chunks > 1 && xin.nhwc && out.nhwc) {
-        const int per = d.N / chunks;
-        const size_t out_elems = (size_t)per * d.OH * d.OW * d.OC;
-        for (int c = 0; c < chunks; ++c) {
+      // Plans for the parts of the batch (every operand is batch-major, so a part is a contiguous slice).
+      if (parts.size() > 2 && xin.nhwc && out.nhwc) {
+        const int64_t per_image = fold > 1 ? (int64_t)OH * OW : 1;   // (folded pixels: d.N counts fold-th parts of pixels)
+        for (size_t c = 0; c + 1 < parts.size(); ++c) {
+          const size_t first = (size_t)(parts[c] * per_image / fold);
           cvmk_conv_desc cd = d;
-          cd.N = per;
-          cd.x = d.x + (size_t)c * per * d.H * d.W * d.C;
-          cd.y = (char*)d.y + (size_t)c * out_elems * d.y_dtype;
+          cd.N = (int)((parts[c + 1] - parts[c]) * per_image / fold);
+          const size_t out_first = first * d.OH * d.OW * d.OC;
+          cd.x = d.x + first * d.H * d.W * d.C;
+          cd.y = (char*)d.y + out_first * d.y_dtype;
           for (int i = 0; i < cd.ep.n; ++i) {
             cvmk_ep_step& st = cd.ep.s[i];
             if ((st.op == CVMK_EP_ADD_T || st.op == CVMK_EP_SUB_T || st.op == CVMK_EP_RSUB_T) && st.ptr)
-              st.ptr = (const char*)st.ptr + (size_t)c * out_elems * st.ptr_dtype;
+              st.ptr = (const char*)st.ptr + out_first * st.ptr_dtype;
           }
           void* cmem = nullptr;
           CHECK(posix_memalign(&cmem, 64, sizeof(cvmk_conv_plan)) == 0);
@@ -896,21 +911,18 @@ struct Lowering {
       d.acc_bound = probe.acc_bound;
       d.ep = ch.ep;
       add_step(label + (depthwise ? "[dw]" : "[direct]"), [d](cudaStream_t s) { return cvmk_conv2d_direct(&d, s); });
-      // Quarter-batch forms (batch-major operands: a chunk is a contiguous slice), when no step of
+      // The parts of the batch (batch-major operands: a part is a contiguous slice), when no step of
       // the chain indexes another tensor.
-      const int chunks = batch_chunks(d.N);
-      bool sliceable = chunks > 1 && xin.nhwc && out.nhwc;
+      const std::vector<int64_t> parts = batch_parts(d.N);
+      bool sliceable = parts.size() > 2 && xin.nhwc && out.nhwc;
       for (int i = 0; i < d.ep.n; ++i)
         sliceable &= !(d.ep.s[i].op == CVMK_EP_ADD_T || d.ep.s[i].op == CVMK_EP_SUB_T || d.ep.s[i].op == CVMK_EP_RSUB_T);
-      if (sliceable) {
-        const int per = d.N / chunks;
-        for (int c = 0; c < chunks; ++c) {
-          cvmk_conv_direct_desc cd = d;
-          cd.N = per;
-          cd.x = (const char*)d.x + (size_t)c * per * d.H * d.W * d.C * d.x_dtype;
-          cd.y = (char*)d.y + (size_t)c * per * d.OH * d.OW * d.OC * d.y_dtype;
-          ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_conv2d_direct(&cd, s); });
-        }
+      for (size_t c = 0; sliceable && c + 1 < parts.size(); ++c) {
+        cvmk_conv_direct_desc cd = d;
+        cd.N = (int)(parts[c + 1] - parts[c]);
+        cd.x = (const char*)d.x + (size_t)parts[c] * d.H * d.W * d.C * d.x_dtype;
+        cd.y = (char*)d.y + (size_t)parts[c] * d.OH * d.OW * d.OC * d.y_dtype;
+        ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_conv2d_direct(&cd, s); });
       }
     }
   }
@@ -1000,16 +1012,13 @@ struct Lowering {
     d.stride_h = (int)n.attrs.t("strides")[0]; d.stride_w = (int)n.attrs.t("strides")[1];
     d.pad_h = (int)pad[0]; d.pad_w = (int)(pad.size() == 2 ? pad[1] : pad[0]);
     add_step("max_pool2d:" + n.name(), [d](cudaStream_t s) { return cvmk_max_pool2d(&d, s); });
-    const int chunks = batch_chunks(d.N);
-    if (chunks > 1 && x.nhwc && y.nhwc) {
-      const int per = d.N / chunks;
-      for (int c = 0; c < chunks; ++c) {
-        cvmk_pool_desc cd = d;
-        cd.N = per;
-        cd.x = (const char*)d.x + (size_t)c * per * d.H * d.W * d.C * d.dtype;
-        cd.y = (char*)d.y + (size_t)c * per * d.OH * d.OW * d.C * d.dtype;
-        ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_max_pool2d(&cd, s); });
-      }
+    const std::vector<int64_t> parts = batch_parts(d.N);
+    for (size_t c = 0; parts.size() > 2 && x.nhwc && y.nhwc && c + 1 < parts.size(); ++c) {
+      cvmk_pool_desc cd = d;
+      cd.N = (int)(parts[c + 1] - parts[c]);
+      cd.x = (const char*)d.x + (size_t)parts[c] * d.H * d.W * d.C * d.dtype;
+      cd.y = (char*)d.y + (size_t)parts[c] * d.OH * d.OW * d.C * d.dtype;
+      ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_max_pool2d(&cd, s); });
     }
   }
 
@@ -1569,20 +1578,16 @@ struct Lowering {
           step_pos.push_back((int)i);
         }
     }
-    // Upload / compute overlap: when the inference starts with the stem, the leading run of steps
-    // that can be cut along the batch (about as much work as the upload takes) is launched per
-    // chunk, outside the graph.
+    // Upload / compute overlap: when the inference starts with a step that takes the input part by
+    // part, the leading run of steps that can be cut along the batch may be launched per part.  How
+    // much of it is, is decided by measurement after the plan.  Everything the prefix touches is live
+    // for all of it (whole-batch buffers, filled part by part), so its length is also a memory
+    // decision: ten steps of ResNet-50 at batch 256 hold 1.3 GB, twenty 2.1 GB.
     {
-      const std::string tag = "[stem]";
-      const bool first = !ex.steps_.empty() && ex.steps_[0].chunk.size() > 1 && ex.steps_[0].label.size() >= tag.size() &&
-                         ex.steps_[0].label.compare(ex.steps_[0].label.size() - tag.size(), tag.size(), tag) == 0;
-      // The lengths actually used are chosen after the load-time measurements.  Everything the prefix
-      // touches is live for all of it (whole-batch buffers, filled chunk by chunk), so its length is
-      // also a memory decision: ten steps of ResNet-50 at batch 256 hold 1.3 GB, twenty 2.1 GB.
-      const size_t cap = 10;
+      const size_t cap = 14, parts = ex.part_end_.size();
       ex.prefix_max_ = 0;
-      if (first)
-        while (ex.prefix_max_ < ex.steps_.size() && ex.prefix_max_ < cap && ex.steps_[ex.prefix_max_].chunk.size() == ex.steps_[0].chunk.size())
+      if (parts > 1 && !ex.steps_.empty() && ex.steps_[0].from_input)
+        while (ex.prefix_max_ < ex.steps_.size() && ex.prefix_max_ < cap && ex.steps_[ex.prefix_max_].chunk.size() == parts)
           ++ex.prefix_max_;
     }
     plan_activations(order);
@@ -1640,32 +1645,50 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
   Upload(in_host_, stream_);
   Enqueue(stream_);
   CUDA_OK(cudaStreamSynchronize(stream_));
-  if (use_graph_) {
-    ChoosePrefixes();
-    CUDA_OK(cudaStreamSynchronize(stream_));
-    PlanForPrefix(std::max(prefix_steps_, prefix_steps_pageable_));   // memory for the prefix actually used
-    if (prefix_steps_ > 0 || prefix_steps_pageable_ > 0) {
-      CUDA_OK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
-      chunk_events_.resize(steps_[0].chunk.size());
-      for (auto& e : chunk_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    auto capture_from = [&](size_t first, cudaGraphExec_t* exec, bool staged = false) {
-      cudaGraph_t graph = nullptr;
-      CUDA_OK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-      if (staged) {
-        const cvmk_export_segment seg = {in_host_, in_dev_, 1, (int64_t)in_bytes_, (int64_t)in_bytes_};
-        KERNEL_OK(cvmk_export(&seg, 1, stream_));
-      }
-      Enqueue(stream_, first);  // the chunked prefix is launched outside the graph
-      CUDA_OK(cudaStreamEndCapture(stream_, &graph));
-      CUDA_OK(cudaGraphInstantiate(exec, graph, 0));
-      CUDA_OK(cudaGraphDestroy(graph));
-    };
-    capture_from(prefix_steps_, &graph_exec_);
-    if (prefix_steps_pageable_ != prefix_steps_) capture_from(prefix_steps_pageable_, &graph_exec_pageable_);
-    if (prefix_steps_ > 0) capture_from(0, &graph_exec_device_);
-    if (in_bytes_ <= kSmallInput) capture_from(0, &graph_exec_staged_, true);
+  if (!use_graph_) return;
+  if (prefix_max_ > 0) {
+    CUDA_OK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+    part_events_.resize(part_end_.size());
+    for (auto& e : part_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
+  graph_whole_ = Capture([this] { Enqueue(stream_); });
+  ChooseSchedules();
+  PlanForPrefix(std::max(from_pinned_.prefix, from_pageable_.prefix));   // memory for the prefix actually used
+  if (in_bytes_ <= kSmallInput)
+    graph_staged_ = Capture([this] {
+      const cvmk_export_segment seg = {in_host_, in_dev_, 1, (int64_t)in_bytes_, (int64_t)in_bytes_};
+      KERNEL_OK(cvmk_export(&seg, 1, stream_));
+      Enqueue(stream_);
+    });
+}
+
+cudaGraphExec_t Executor::Capture(const std::function<void()>& enqueue) {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  CUDA_OK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+  enqueue();
+  CUDA_OK(cudaStreamEndCapture(stream_, &graph));
+  const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+  cudaGraphDestroy(graph);
+  CUDA_OK(e);
+  return exec;
+}
+
+Executor::Schedule Executor::MakeSchedule(size_t prefix) {
+  Schedule s;
+  s.prefix = prefix;
+  for (size_t c = 0; prefix > 0 && c < part_end_.size(); ++c)
+    s.graphs.push_back(Capture([&] {
+      for (size_t k = 0; k < prefix; ++k) KERNEL_OK(steps_[k].chunk[c](stream_));
+      if (c + 1 == part_end_.size()) Enqueue(stream_, prefix);
+    }));
+  return s;
+}
+
+void Executor::DropSchedule(Schedule* s) {
+  for (auto g : s->graphs) cudaGraphExecDestroy(g);
+  s->graphs.clear();
+  s->prefix = 0;
 }
 
 bool Executor::IsDevice(const void* input) {
@@ -1683,76 +1706,66 @@ bool Executor::IsDirect(const void* input) {
   return false;
 }
 
-// How many leading steps to run chunk by chunk: the fewest whose device time, measured here step
-// by step on the whole batch and scaled by 1.3 (a quarter of the batch runs less efficiently than
-// the whole), reaches the time the upload takes -- measured here too, once for a page-locked source
-// and once through the staging path a pageable source takes.
-void Executor::ChoosePrefixes() {
-  prefix_steps_ = prefix_steps_pageable_ = 0;
-  if (prefix_max_ == 0 || dev_env("CVM_B200_NO_UPLOAD_OVERLAP")) { prefix_max_ = 0; return; }
-  if (const char* e = dev_env("CVM_B200_PREFIX_STEPS")) {
-    prefix_steps_ = prefix_steps_pageable_ = std::min(prefix_max_, (size_t)atoi(e));
-    return;
-  }
-  std::vector<cudaEvent_t> ev(prefix_max_ + 1);
-  for (auto& e : ev) CUDA_OK(cudaEventCreate(&e));
-  std::vector<double> step_ms(prefix_max_, 0.0);
-  for (int rep = 0; rep < 2; ++rep) {   // the second pass is the warm one
-    CUDA_OK(cudaEventRecord(ev[0], stream_));
-    for (size_t k = 0; k < prefix_max_; ++k) {
-      KERNEL_OK(steps_[k].launch(stream_));
-      CUDA_OK(cudaEventRecord(ev[k + 1], stream_));
-    }
-    CUDA_OK(cudaStreamSynchronize(stream_));
-  }
-  for (size_t k = 0; k < prefix_max_; ++k) {
-    float ms = 0;
-    CUDA_OK(cudaEventElapsedTime(&ms, ev[k], ev[k + 1]));
-    step_ms[k] = ms;
-  }
-  auto upload_ms = [&](const void* src) {
-    double best = 1e30;
-    for (int rep = 0; rep < 2; ++rep) {
-      CUDA_OK(cudaEventRecord(ev[0], stream_));
-      Upload(src, stream_);
-      CUDA_OK(cudaEventRecord(ev[1], stream_));
-      const auto t0 = std::chrono::steady_clock::now();
-      CUDA_OK(cudaStreamSynchronize(stream_));
-      float ms = 0;
-      CUDA_OK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-      // a pageable source is staged by host threads while the stream waits: wall time counts
-      const double wall = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-      best = std::min(best, std::max((double)ms, wall));
-    }
-    return best;
-  };
-  const double t_pinned = upload_ms(in_host_);
+// How many leading steps to run part by part: the count whose inference takes least, timed here (best of
+// three each) from page-locked and from pageable memory.  A few counts spread over the range, then
+// the neighbours of the best.  (Predicting it from step times and upload rates, as before, missed what
+// the launches of a part and the smaller grids cost: SSD-512 batch 8 ran at 712 instead of 661 us.)
+void Executor::ChooseSchedules() {
+  if (prefix_max_ == 0) return;
   std::vector<char> pageable(in_bytes_, 0);
-  const double t_pageable = upload_ms(pageable.data());
-  auto pick = [&](double t_upload) {
-    double sum = 0;
-    size_t n = 0;
-    while (n < prefix_max_ && 1.3 * sum < t_upload) sum += step_ms[n++];
-    return n;
+  auto best_for = [&](const void* input) {
+    const Source src = SourceOf(input);
+    auto time_of = [&](size_t prefix) {
+      Schedule s = MakeSchedule(prefix);
+      double best = 1e30;
+      for (int rep = 0; rep < 4; ++rep) {   // the first is a warm-up
+        if (src == Source::kPool) pool().Begin();
+        const auto t0 = std::chrono::steady_clock::now();
+        BeginUpload(input, src);
+        Launch(input, src, s);
+        CUDA_OK(cudaStreamSynchronize(stream_));
+        const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (src == Source::kPool) {
+          pool().Finish(HostPool::kUpload);
+          pool().End();
+        }
+        if (rep > 0) best = std::min(best, t);
+      }
+      DropSchedule(&s);
+      return best;
+    };
+    std::map<size_t, double> seen;
+    auto probe = [&](size_t p) { if (p <= prefix_max_ && !seen.count(p)) seen[p] = time_of(p); };
+    auto best = [&] {
+      auto at = seen.begin();
+      for (auto i = seen.begin(); i != seen.end(); ++i)
+        if (i->second < at->second) at = i;
+      return at->first;
+    };
+    for (size_t p : {(size_t)0, (size_t)2, (size_t)5, (size_t)9, prefix_max_}) probe(p);
+    for (size_t d : {(size_t)2, (size_t)1}) {
+      const size_t b = best();
+      probe(b + d);
+      if (b >= d) probe(b - d);
+    }
+    if (dev_env("CVM_B200_VERBOSE"))
+      for (auto& e : seen) fprintf(stderr, "%s prefix %zu: %.1f us\n", src == Source::kPool ? "pageable" : "page-locked", e.first, e.second * 1e6);
+    return best();
   };
-  prefix_steps_ = pick(t_pinned);
-  prefix_steps_pageable_ = std::max(prefix_steps_, pick(t_pageable));
-  if (dev_env("CVM_B200_VERBOSE"))
-    fprintf(stderr, "upload %.3f ms page-locked, %.3f ms pageable: %zu / %zu of %zu leading steps run per chunk\n", t_pinned,
-            t_pageable, prefix_steps_, prefix_steps_pageable_, prefix_max_);
-  for (auto& e : ev) cudaEventDestroy(e);
+  from_pinned_ = MakeSchedule(best_for(in_host_));
+  from_pageable_ = MakeSchedule(in_bytes_ <= kSmallInput ? 0 : best_for(pageable.data()));
 }
 
 Executor::~Executor() {
   cudaSetDevice(device_);
   if (stream_) cudaStreamSynchronize(stream_);
-  if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-  if (graph_exec_pageable_) cudaGraphExecDestroy(graph_exec_pageable_);
-  if (graph_exec_device_) cudaGraphExecDestroy(graph_exec_device_);
-  if (graph_exec_staged_) cudaGraphExecDestroy(graph_exec_staged_);
+  DropSchedule(&from_pinned_);
+  DropSchedule(&from_pageable_);
+  if (graph_whole_) cudaGraphExecDestroy(graph_whole_);
+  if (graph_staged_) cudaGraphExecDestroy(graph_staged_);
   if (kernels_exec_) cudaGraphExecDestroy(kernels_exec_);
   for (auto e : piece_events_) cudaEventDestroy(e);
-  for (auto e : chunk_events_) cudaEventDestroy(e);
+  for (auto e : part_events_) cudaEventDestroy(e);
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
   for (void* p : allocs_) cudaFree(p);
   for (auto& a : act_) {
@@ -1770,7 +1783,7 @@ Executor::~Executor() {
 // page-locked input of up to 256 KiB is staged as well: the copy takes 4 us, and the inference
 // is then one graph that begins by fetching the staging buffer.
 Executor::Source Executor::SourceOf(const void* input) const {
-  if (IsDirect(input)) return in_bytes_ <= kSmallDirect && graph_exec_staged_ && !IsDevice(input) ? Source::kSmall : Source::kDirect;
+  if (IsDirect(input)) return in_bytes_ <= kSmallDirect && graph_staged_ && !IsDevice(input) ? Source::kSmall : Source::kDirect;
   return in_bytes_ <= kSmallInput ? Source::kSmall : Source::kPool;
 }
 
@@ -1958,6 +1971,24 @@ void Executor::DeliverHead(char* out) {
   }
 }
 
+// Queues the upload and the kernels of one inference.
+void Executor::Launch(const void* input, Source src, const Schedule& how) {
+  if (how.prefix == 0) {
+    SendRange(input, src, 0, in_bytes_, stream_);
+    if (graph_whole_) CUDA_OK(cudaGraphLaunch(graph_whole_, stream_));
+    else Enqueue(stream_);
+    return;
+  }
+  size_t begin = 0;
+  for (size_t c = 0; c < how.graphs.size(); ++c) {
+    SendRange(input, src, begin, part_end_[c] - begin, copy_stream_);
+    CUDA_OK(cudaEventRecord(part_events_[c], copy_stream_));
+    CUDA_OK(cudaStreamWaitEvent(stream_, part_events_[c], 0));
+    CUDA_OK(cudaGraphLaunch(how.graphs[c], stream_));
+    begin = part_end_[c];
+  }
+}
+
 void Executor::Run(const void* input, size_t input_bytes, char* out) {
   CHECK(input_bytes == in_bytes_) << "input size " << input_bytes << " vs. " << in_bytes_;
   CUDA_OK(cudaSetDevice(device_));
@@ -1981,28 +2012,12 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
   if (signal) *(volatile int32_t*)done_host_ = 0;
   BeginUpload(input, src);
   if (fill) StartFill(out);
-  const bool pageable = graph_exec_pageable_ && src != Source::kDirect;
-  const size_t prefix = on_device ? 0 : (pageable ? prefix_steps_pageable_ : prefix_steps_);
-  if (src == Source::kSmall && graph_exec_staged_) {
+  if (src == Source::kSmall && graph_staged_) {
     memcpy(in_host_, input, in_bytes_);
-    CUDA_OK(cudaGraphLaunch(graph_exec_staged_, stream_));
-  } else if (graph_exec_ && prefix > 0) {
-    // chunk c of the batch is uploaded on the copy stream while the leading steps run on chunk c - 1
-    for (size_t c = 0; c < steps_[0].chunk.size(); ++c) {
-      SendRange(input, src, c * chunk_bytes_, chunk_bytes_, copy_stream_);
-      CUDA_OK(cudaEventRecord(chunk_events_[c], copy_stream_));
-      CUDA_OK(cudaStreamWaitEvent(stream_, chunk_events_[c], 0));
-      for (size_t k = 0; k < prefix; ++k) {
-        const int rc = steps_[k].chunk[c](stream_);
-        CHECK(rc == CVMK_OK) << "step " << steps_[k].label << " (chunk) failed (" << rc << "): " << cvmk_last_error();
-      }
-    }
-    CUDA_OK(cudaGraphLaunch(pageable ? graph_exec_pageable_ : graph_exec_, stream_));
+    CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
   } else {
-    SendRange(input, src, 0, in_bytes_, stream_);
-    cudaGraphExec_t whole = on_device && graph_exec_device_ ? graph_exec_device_ : graph_exec_;
-    if (whole) CUDA_OK(cudaGraphLaunch(whole, stream_));
-    else Enqueue(stream_);
+    static const Schedule whole;
+    Launch(input, src, on_device ? whole : (src == Source::kDirect ? from_pinned_ : from_pageable_));
   }
   if (pieces) DeliverPieces(out);
   else if (signal) AwaitDone();

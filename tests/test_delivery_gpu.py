@@ -51,3 +51,30 @@ def test_nms_head(anchors, top_k, mos, empty, gpu_run, wl, oracle):
     want = oracle.run_model(js, pb, x).view(np.int32).reshape(4, anchors, 6)
     last = 4 if empty is None else empty + 1
     assert np.array_equal(got[:last], want[:last])
+
+
+# stems over rows that do not start on 16-byte boundaries (moved apart first), widths beyond one TMA box, and
+# batches that are and are not cut into parts while they upload
+@pytest.mark.parametrize("width", [17, 31, 48, 100, 191, 224, 250, 301])
+@pytest.mark.parametrize("batch", [1, 8, 11])
+def test_image_stem(width, batch, rt, wl, oracle):
+    import torch
+    g = wl.GraphBuilder(width)
+    d = g.var("data", (batch, 3, 29, width), 8)
+    k = 7 if width % 2 else 3
+    y = g.conv(d, 32, k, 2, k // 2)
+    y = g.max_pool(y, 3, 2, 1)
+    y = g.conv(y, 64, 1, 1, 0)
+    y = g.conv(y, 64, 3, 1, 1)
+    js, pb = g.finish(y)
+    x = np.random.RandomState(width).randint(-128, 128, size=(batch, 3, 29, width)).astype(np.int8)
+    want = oracle.run_model(js, pb, x)
+    net = rt.CVMAPILoadModel(js, pb, 0)
+    try:
+        flat = torch.from_numpy(x.reshape(-1).view(np.uint8).copy())
+        for src in (flat, flat.pin_memory(), flat.cuda()):
+            out = torch.zeros(want.nbytes, dtype=torch.uint8)
+            rt.check_call(rt.lib().CVMAPIInference(net, ctypes.c_void_p(src.data_ptr()), flat.numel(), ctypes.c_void_p(out.data_ptr())))
+            assert np.array_equal(out.numpy(), want.view(np.uint8))
+    finally:
+        rt.CVMAPIFreeModel(net)
