@@ -605,13 +605,17 @@ struct Lowering {
     // the image: the CUDA-core form is bound by instruction issue at a fraction of the memory
     // rate (measured 15-25 % slower on such layers; faster for 32 and 64 channels, which stay there).
     const int dw_cg = 32;
+    // ... and when there are enough of them: a persistent CTA per SM with three tiles or fewer to its name
+    // spends most of the launch filling and draining (MobileNet, one image: 139 -> 100 us with every
+    // depthwise layer on the CUDA cores; 64 images: 328 against 353 us; the lines cross near 500 tiles).
+    const int64_t dw_tc_tiles = 512;
     bool dw_tc = false;
     if (depthwise && C % 128 == 0 && KH == 3 && KW == 3 && sh == 1 && sw == 1 && dh == 1 && dw == 1 &&
         out.dtype == CVMK_I8 && !dev_env("CVM_B200_NO_DW_TC") && !dev_env("CVM_B200_NO_TC")) {
       const int64_t linear = ((int64_t)N * OH * OW + 127) / 128;
       const int64_t tiles = (int64_t)((OW + 7) / 8) * ((OH + 15) / 16) * N;
       probe.groups = C / dw_cg;
-      dw_tc = tiles * 20 <= linear * 27 && cvmk_conv2d_tc_supported(&probe);
+      dw_tc = tiles * 20 <= linear * 27 && tiles * (C / 128) > dw_tc_tiles && cvmk_conv2d_tc_supported(&probe);
       if (!dw_tc) probe.groups = 0;
     }
     // 32 and 64 channels: 4 or 2 neighbouring pixels of a row are 128 contiguous bytes, so the layer
@@ -628,7 +632,7 @@ struct Lowering {
       cvmk_conv_desc fp = probe;
       fp.W = W / F; fp.OW = OW / F; fp.C = fp.OC = 128;
       fp.groups = 4; fp.group_fold = F;
-      if (tiles * 20 <= linear * 27 && cvmk_conv2d_tc_supported(&fp)) {
+      if (tiles * 20 <= linear * 27 && tiles > dw_tc_tiles && cvmk_conv2d_tc_supported(&fp)) {
         probe = fp;
         dw_tc = true;
         dw_fold = F;

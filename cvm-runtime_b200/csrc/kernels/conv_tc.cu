@@ -1142,7 +1142,13 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
   if (const char* e = dev_env("CVM_B200_SMALL_N")) bn = atoi(e);
   const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
   const bool few_rows = is_pointwise(d) && (int64_t)d.N * d.OH * d.OW <= BLOCK_M;   // long reductions of one M tile
-  if (tiles > sms && !few_rows && !dev_env("CVM_B200_SMALL_FORCE")) return c;
+  // More tiles than SMs are fine while the reduction is short: the persistent kernel's fixed costs then
+  // weigh more than the reuse of its 128 x 256 tiles.  Up to 3.5 tiles an SM for one 24 KB unit or two,
+  // 2.5 for up to four (13 images of ResNet-50: 386 -> 309 us); with eight units at 2.6 tiles an SM the
+  // persistent kernel is the faster one again (64 images: 722 against 745 us).
+  const int64_t unit24 = (int64_t)units * (BLOCK_M + bn) * bk / (24 * 1024);
+  const int halves = unit24 <= 2 ? 7 : (unit24 <= 4 ? 5 : 2);   // half tiles per SM
+  if (2 * tiles > (int64_t)halves * sms && !few_rows && !dev_env("CVM_B200_SMALL_FORCE")) return c;
   // Cutting the reduction costs an exchange of partial sums, about as much as ten 24 KB units take.
   int split = 1;
   const int unit_bytes = (BLOCK_M + bn) * bk, weight = units * unit_bytes / (24 * 1024);
@@ -1155,7 +1161,7 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
   const int per = (units + split - 1) / split;
   int group = per <= 3 ? per : (per == 4 ? 2 : 3);
   if (const char* e = dev_env("CVM_B200_SMALL_GROUP")) group = std::min(per, atoi(e));
-  int limit = 208 * 1024;
+  int limit = (tiles * split <= sms ? 208 : 112) * 1024;   // two CTAs an SM when there are more than SMs
   if (const char* e = dev_env("CVM_B200_SMALL_KB")) limit = atoi(e) * 1024;
   int stages = std::min((per + group - 1) / group, SMALL_MAX_STAGES);
   while (stages > 1 && small_smem_bytes(bk, bn, stages * group, split) > limit) --stages;
