@@ -1844,14 +1844,15 @@ void Executor::Upload(const void* input, cudaStream_t s) {
   }
 }
 
-// Heads of up to 1 MiB in all (8 MiB of an NMS head's rows: fetching its -1 tail too costs more) are
+// Heads of up to 1 MiB in all (256 KiB when they go out as they are: one thread's copy of the rest would
+// take longer than its download in pieces; 8 MiB of an NMS head's rows: fetching its -1 tail too costs more) are
 // written into page-locked memory by one kernel, with the status word: a copy node for each costs 3 us and more
 // and starts only after the kernel before it has drained.  A single larger head whose bytes are
 // the result leaves in pieces (DeliverPieces).
 void Executor::ChooseDownload() {
   size_t total = 0;
   for (const auto& h : heads_) total += h.live_bytes ? h.images * h.live_bytes : h.bytes;
-  const size_t small = (size_t)(plain_ && heads_[0].live_bytes ? 8 : 1) << 20;
+  const size_t small = plain_ ? (heads_[0].live_bytes ? (size_t)8 << 20 : (size_t)256 << 10) : (size_t)1 << 20;
   if (total <= small && heads_.size() + 2 <= CVMK_MAX_EXPORT_SEGMENTS) {
     download_ = Download::kKernel;
   } else {
@@ -1859,7 +1860,8 @@ void Executor::ChooseDownload() {
     download_ = plain_ ? Download::kPieces : Download::kCopies;
   }
   if (download_ == Download::kPieces) {
-    piece_events_.resize((heads_[0].bytes + kDownloadPiece - 1) / kDownloadPiece);
+    download_piece_ = heads_[0].bytes <= 4 * kDownloadPiece ? kDownloadPiece / 4 : kDownloadPiece;
+    piece_events_.resize((heads_[0].bytes + download_piece_ - 1) / download_piece_);
     for (auto& e : piece_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   if (download_ == Download::kKernel && heads_[0].live_bytes) {
@@ -1919,7 +1921,7 @@ void Executor::StartFill(char* out) {
   const size_t piece = (tail + per - 1) / per;
   pool().Start(HostPool::kFill, h.images * per, h.images * per, [=](size_t k) {
     const size_t b = k / per, off = std::min(tail, (k % per) * piece);
-    memset(out + b * image + live + off, 0xff, std::min(piece, tail - off));
+    stream_fill(out + b * image + live + off, 0xff, std::min(piece, tail - off));
   });
 }
 
@@ -1933,11 +1935,11 @@ void Executor::DeliverPieces(char* out) {
     return;
   }
   for (size_t k = 0; k < piece_events_.size(); ++k) {
-    const size_t off = k * kDownloadPiece;
-    CUDA_OK(cudaMemcpyAsync((char*)h.host + off, (const char*)h.dev + off, std::min(kDownloadPiece, h.bytes - off), cudaMemcpyDeviceToHost, stream_));
+    const size_t off = k * download_piece_;
+    CUDA_OK(cudaMemcpyAsync((char*)h.host + off, (const char*)h.dev + off, std::min(download_piece_, h.bytes - off), cudaMemcpyDeviceToHost, stream_));
     CUDA_OK(cudaEventRecord(piece_events_[k], stream_));
   }
-  const size_t unit = kStagePiece, units = (h.bytes + unit - 1) / unit, per = kDownloadPiece / unit;
+  const size_t unit = std::min(kStagePiece, download_piece_) / 2, units = (h.bytes + unit - 1) / unit, per = download_piece_ / unit;
   const char* from = (const char*)h.host;
   const size_t bytes = h.bytes;
   pool().Start(HostPool::kDownload, units, 0, [=](size_t k) { memcpy(out + k * unit, from + k * unit, std::min(unit, bytes - k * unit)); });

@@ -142,6 +142,7 @@ class Executor {
   Download download_ = Download::kCopies;
   bool plain_ = false;
   std::vector<cudaEvent_t> piece_events_;
+  size_t download_piece_ = 0;
   int32_t* valid_host_ = nullptr;    // pinned copy of HeadOut::valid_count
   void ChooseDownload();
   void StartFill(char* out);

@@ -1,5 +1,6 @@
 #include "host_pool.h"
 #include <algorithm>
+#include <chrono>
 #include <cstring>
 #if defined(__x86_64__)
 #include <emmintrin.h>
@@ -84,13 +85,28 @@ bool HostPool::HelpOnce() {
 }
 
 void HostPool::Work() {
+  auto last = std::chrono::steady_clock::now();   // the end of the last inference seen
+  bool was_active = false;
   for (;;) {
-    if (!active_.load(std::memory_order_acquire)) {
-      std::unique_lock<std::mutex> lk(mu_);
-      cv_.wait(lk, [&] { return stop_ || active_; });
-      if (stop_) return;
+    if (active_.load(std::memory_order_acquire)) {
+      was_active = true;
+      if (!HelpOnce()) Relax();
+      continue;
     }
-    if (!HelpOnce()) Relax();
+    // Inferences that follow one another closely find the helpers awake: a wake-up takes about as long
+    // as the first megabytes of an upload.
+    const auto now = std::chrono::steady_clock::now();
+    if (was_active) {
+      last = now;
+      was_active = false;
+    }
+    if (!stop_ && now - last < std::chrono::microseconds(kLingerUs)) {
+      Relax();
+      continue;
+    }
+    std::unique_lock<std::mutex> lk(mu_);
+    cv_.wait(lk, [&] { return stop_ || active_; });
+    if (stop_) return;
   }
 }
 
@@ -124,6 +140,26 @@ void stream_copy(char* dst, const char* src, size_t bytes) {
   memcpy(dst + vec, src + vec, bytes - vec);
 #else
   memcpy(dst, src, bytes);
+#endif
+}
+
+void stream_fill(char* dst, int byte, size_t bytes) {
+#if defined(__x86_64__)
+  const size_t head = std::min<size_t>(bytes, (16 - ((uintptr_t)dst & 15)) & 15);
+  memset(dst, byte, head);
+  dst += head; bytes -= head;
+  const size_t vec = bytes & ~(size_t)63;
+  const __m128i v = _mm_set1_epi8((char)byte);
+  for (size_t i = 0; i < vec; i += 64) {
+    _mm_stream_si128((__m128i*)(dst + i), v);
+    _mm_stream_si128((__m128i*)(dst + i + 16), v);
+    _mm_stream_si128((__m128i*)(dst + i + 32), v);
+    _mm_stream_si128((__m128i*)(dst + i + 48), v);
+  }
+  _mm_sfence();
+  memset(dst + vec, byte, bytes - vec);
+#else
+  memset(dst, byte, bytes);
 #endif
 }
 

@@ -2,7 +2,8 @@
 // buffer into the page-locked staging buffer, downloaded pieces into the caller's output buffer,
 // constant fills.  Each of these is a job cut into pieces; a piece is a call of the job's body.
 //
-// The helpers sleep between inferences.  Begin() wakes them once, and until End() they spin over
+// The helpers sleep between inferences that are more than a fifth of a millisecond apart.  Begin() wakes
+// them, and until End() they spin over
 // the jobs, lowest slot first, so that a job that starts while others run is picked up without a
 // wake-up (tens of microseconds, more than many of these jobs take).  The caller helps with every
 // job it waits for.
@@ -43,6 +44,7 @@ class HostPool {
   bool HelpOnce();
 
  private:
+  static constexpr int kLingerUs = 200;
   struct Job {
     // (generation << 32 | count): a claim is a compare-exchange of the whole word against `avail` of
     // the same generation, so a helper that looked at the slot's previous job cannot take a
@@ -67,5 +69,6 @@ class HostPool {
 // memcpy with stores that bypass the cache: for destinations the CPU does not read soon (the
 // staging buffer the copy engine reads, a large output).
 void stream_copy(char* dst, const char* src, size_t bytes);
+void stream_fill(char* dst, int byte, size_t bytes);   // memset the same way
 
 }  // namespace cvm
