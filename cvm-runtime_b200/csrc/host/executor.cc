@@ -1403,6 +1403,17 @@ struct Lowering {
     add_step(label, [x, y, vc, B, N, K, thr, clamp](cudaStream_t s) {
       return cvmk_get_valid_counts_clamped((const int32_t*)x.ptr, (int32_t*)y.ptr, (int32_t*)vc.ptr, B, N, K, thr, clamp, s);
     });
+    ex.steps_.back().from_input = from_raw;
+    const std::vector<int64_t> parts = batch_parts(B);
+    for (size_t c = 0; from_raw && parts.size() > 2 && c + 1 < parts.size(); ++c) {   // while later images upload
+      const int64_t b0 = parts[c], rows = b0 * N * K;
+      const int count = (int)(parts[c + 1] - b0);
+      ex.part_end_.resize(c + 1);
+      ex.part_end_[c] = (size_t)parts[c + 1] * N * K * 4;
+      ex.steps_.back().chunk.push_back([x, y, vc, b0, rows, count, N, K, thr, clamp](cudaStream_t s) {
+        return cvmk_get_valid_counts_clamped((const int32_t*)x.ptr + rows, (int32_t*)y.ptr + rows, (int32_t*)vc.ptr + b0, count, N, K, thr, clamp, s);
+      });
+    }
   }
 
   // Outputs of non_max_suppression that hold at most so many bytes of rows per image: images, bytes,
@@ -1446,6 +1457,11 @@ struct Lowering {
       if (bound < d.N) limited[g.entry_id(nid, 0)] = {(size_t)d.B, (size_t)bound * 24, d.valid_count};
     }
     add_step(label, [d](cudaStream_t s) { return cvmk_non_max_suppression(&d, s); });
+    const std::vector<int64_t> parts = batch_parts(d.B);
+    for (size_t c = 0; parts.size() > 2 && c + 1 < parts.size(); ++c) {
+      const int first = (int)parts[c], count = (int)(parts[c + 1] - parts[c]);
+      ex.steps_.back().chunk.push_back([d, first, count](cudaStream_t s) { return cvmk_non_max_suppression_part(&d, first, count, s); });
+    }
   }
 
   // Lifetimes of the activation buffers in schedule positions (one position per fused group, in

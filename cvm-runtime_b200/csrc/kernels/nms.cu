@@ -204,6 +204,7 @@ struct NmsParams {
   const int32_t* x; const int32_t* vc; int32_t* y;
   int32_t* xw;            // when set: rows outside the top_k best get -1 in the input as well
   int B, N;
+  int first, count;       // images of this launch
   int mos, thr, topk, force;
   uint32_t* scratch;      // per batch: keyA, keyB, idxA, idxB, removed, stop : 6 * npad words
   int64_t per_batch_words;
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(THREADS) nms_kernel(const __grid_constant__ Nm
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   __shared__ int ws[WARPS + 1];
-  const int b = blockIdx.y;
+  const int b = p.first + (int)blockIdx.y;
   const int N = p.N;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t* xb = p.x + (size_t)b * N * 6;
@@ -878,10 +879,10 @@ static int nms_launch(NmsParams& p, cudaStream_t stream, const char* what) {
   if (bound < p.N) {
     const long long tail_bytes = (long long)(p.N - bound) * 24;
     fillers = (int)std::min<long long>(8, std::max<long long>(1, tail_bytes / 65536));
-    fillers = std::min(fillers, std::max(1, 4 * sms / p.B));
+    fillers = std::min(fillers, std::max(1, 4 * sms / p.count));
   }
-  if (p.B > 65535) { set_error("non_max_suppression: batch %d too large", p.B); return CVMK_ERR_ARG; }
-  launch_pdl(nms_kernel, dim3(1 + fillers, p.B), dim3(THREADS), smem, stream, p);
+  if (p.count > 65535) { set_error("non_max_suppression: batch %d too large", p.B); return CVMK_ERR_ARG; }
+  launch_pdl(nms_kernel, dim3(1 + fillers, p.count), dim3(THREADS), smem, stream, p);
   return check_cuda(cudaGetLastError(), what);
 }
 
@@ -890,7 +891,11 @@ extern "C" int64_t cvmk_nms_scratch_bytes(int32_t B, int32_t N) {
 }
 
 extern "C" int cvmk_non_max_suppression(const cvmk_nms_desc* d, cvmk_stream_t stream) {
-  if (!d || !d->x || !d->valid_count || !d->y || !d->scratch || d->B < 1 || d->N < 1 || d->iou_threshold <= 0) {
+  return cvmk_non_max_suppression_part(d, 0, d ? d->B : 0, stream);
+}
+
+extern "C" int cvmk_non_max_suppression_part(const cvmk_nms_desc* d, int32_t first, int32_t count, cvmk_stream_t stream) {
+  if (!d || first < 0 || count < 1 || first + count > d->B || !d->x || !d->valid_count || !d->y || !d->scratch || d->B < 1 || d->N < 1 || d->iou_threshold <= 0) {
     set_error("non_max_suppression: bad argument");
     return CVMK_ERR_ARG;
   }
@@ -901,6 +906,7 @@ extern "C" int cvmk_non_max_suppression(const cvmk_nms_desc* d, cvmk_stream_t st
   NmsParams p;
   p.x = d->x; p.vc = d->valid_count; p.y = d->y; p.xw = d->x_writeback;
   p.B = d->B; p.N = d->N;
+  p.first = first; p.count = count;
   p.mos = d->max_output_size; p.thr = d->iou_threshold; p.topk = d->top_k; p.force = d->force_suppress;
   p.scratch = reinterpret_cast<uint32_t*>(d->scratch);
   p.npad = nms_npad(d->N);
@@ -950,6 +956,7 @@ extern "C" int cvmk_non_max_suppression_static(const int32_t* x, const int32_t* 
   NmsParams p;
   p.x = x; p.vc = valid_count; p.y = y; p.xw = nullptr;
   p.B = B; p.N = N;
+  p.first = 0; p.count = B;
   p.mos = max_output_size; p.thr = iou_threshold; p.topk = top_k; p.force = force_suppress;
   p.scratch = reinterpret_cast<uint32_t*>(scratch_of_device[dev]);
   p.npad = nms_npad(N);

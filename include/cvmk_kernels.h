@@ -416,6 +416,9 @@ typedef struct {
 } cvmk_nms_desc;
 CVMK_API int64_t cvmk_nms_scratch_bytes(int32_t B, int32_t N);
 CVMK_API int cvmk_non_max_suppression(const cvmk_nms_desc* d, cvmk_stream_t stream);
+/* The same for images [first, first + count) of the batch only, after a call for the ones before them (an
+ * image without valid boxes ends the operator's loop, so their valid counts are looked at). */
+CVMK_API int cvmk_non_max_suppression_part(const cvmk_nms_desc* d, int32_t first, int32_t count, cvmk_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------
  * non_max_suppression for callers that cannot allocate device memory.  No counterpart in the

@@ -41,15 +41,16 @@ def test_sizes_and_buffers(n, where, rt, wl, oracle):
 # rows past top_k / max_output_size are not downloaded; the operator's loop ends at an image without
 # valid boxes, whose successors keep what their memory held (zeros in a fresh handle)
 @pytest.mark.parametrize("empty", [None, 0, 1, 3])
+@pytest.mark.parametrize("batch", [4, 9])
 @pytest.mark.parametrize("anchors,top_k,mos", [(1001, 100, -1), (1000, 100, 37), (700, 800, 20), (5003, 1, -1)])
-def test_nms_head(anchors, top_k, mos, empty, gpu_run, wl, oracle):
-    js, pb, x = wl.ssd_tail(batch=4, anchors=anchors, top_k=top_k, max_output_size=mos)
+def test_nms_head(batch, anchors, top_k, mos, empty, gpu_run, wl, oracle):
+    js, pb, x = wl.ssd_tail(batch=batch, anchors=anchors, top_k=top_k, max_output_size=mos)
     if empty is not None:
         x = x.copy()
         x[empty, :, 1] = 3
-    got = gpu_run(js, pb, x).view(np.int32).reshape(4, anchors, 6)
-    want = oracle.run_model(js, pb, x).view(np.int32).reshape(4, anchors, 6)
-    last = 4 if empty is None else empty + 1
+    got = gpu_run(js, pb, x).view(np.int32).reshape(batch, anchors, 6)
+    want = oracle.run_model(js, pb, x).view(np.int32).reshape(batch, anchors, 6)
+    last = batch if empty is None else empty + 1
     assert np.array_equal(got[:last], want[:last])
 
 
