@@ -1484,14 +1484,17 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   p.w = d.w;
   p.w_bytes = (unsigned)std::min<int64_t>((int64_t)d.OC * d.KH * d.KW * p.c, (int64_t)1 << 30);
   p.tma_out = plan->tma_out; p.res_step = plan->res_step;
-  // Two issuing warps (and one producer) in the halo modes, where a tile takes one or two ring
-  // stages and the ring has more: an issuer that waits for the first stage of its next tile is then
-  // never more than one lap of that stage's barrier ahead of the producer, which is what a parity
-  // wait can tell apart.  (The same rule applied to the short 1x1 reductions of the other modes
-  // passed every single-kernel check and gained 12 % on 64 -> 64 and 256 -> 64 layers, but a
-  // bounded wait ran out in ResNet-50's end-to-end loop, where per-chunk kernels follow each other
-  // closely; it stays off until that is understood.)
-  p.two_issuers = (p.a_mode >= 3 && p.num_kb < p.stages && !dev_env("CVM_B200_ONE_ISSUER")) ? 1 : 0;
+  // Two issuing warps (and one producer) in the halo modes, where a tile takes one or two ring stages.
+  // The ring is cut to a whole number of tile pairs, so that a stage belongs to one issuer for good: it
+  // has itself consumed the stage's previous contents, which is what a parity wait relies on.  With a
+  // stage that changes hands, an issuer whose own loads came from L2 could reach the stage before the
+  // other's load, from DRAM, had landed there; the barrier was then a whole lap behind, where the
+  // parity reads "complete", and it multiplied what was in the stage.  (Now and then VGG-19 at batch 32
+  // ended with an expired wait.)  The short 1x1 reductions of the other modes run correctly this way
+  // too, and no faster: ResNet-50 batch 64 718.8 us against 720.4, batch 256 1948 against 1941.
+  const int pair = 2 * p.num_kb;
+  p.two_issuers = (p.a_mode >= 3 && pair <= p.stages && !dev_env("CVM_B200_ONE_ISSUER")) ? 1 : 0;
+  if (p.two_issuers) p.stages -= p.stages % pair;
 #ifdef CVMK_CONV_TIMING
   p.dbg = getenv("CVM_DBG") ? atoi(getenv("CVM_DBG")) : 0;
   if (getenv("CVM_HINT")) {
