@@ -35,9 +35,10 @@ struct SmallConvParams {
 constexpr int SMALL_MAX_STAGES = 12;
 
 // Dynamic shared memory of a launch: the operand ring (which also holds the partial sums this CTA sends
-// when the reduction is cut) and, behind it, the ones it receives.
+// when the reduction is cut, or else the tile's packed results on their way out: more than the ring where
+// that is a single unit of 32 channels) and, behind it, the partial sums it receives.
 __host__ __device__ inline int small_ring_bytes(int block_k, int block_n, int units, int split) {   // units in the ring
-  const int ring = units * (tc::BLOCK_M + block_n) * block_k, sums = split > 1 ? tc::BLOCK_M * block_n * 4 : 0;
+  const int ring = units * (tc::BLOCK_M + block_n) * block_k, sums = tc::BLOCK_M * block_n * (split > 1 ? 4 : 1);
   return ring > sums ? ring : sums;
 }
 inline int small_smem_bytes(int block_k, int block_n, int units, int split) {
