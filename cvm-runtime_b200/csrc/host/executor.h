@@ -15,6 +15,7 @@
 // There is no CPU fallback: every step is a CUDA kernel from this library.
 #pragma once
 #include <cuda_runtime.h>
+#include <chrono>
 #include <functional>
 #include <memory>
 #include <string>
@@ -90,6 +91,9 @@ class Executor {
   std::vector<Step> steps_;
   enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
   static constexpr size_t kSmallInput = (size_t)1 << 20, kSmallDirect = (size_t)1 << 18;
+  // A small input of at least kSmallShare is staged together with the pool's helpers if they are awake
+  // (547 KB 166 -> 150 us a call, 150 KB 224.4 -> 222.8); asleep, waking them costs more than that.
+  static constexpr size_t kSmallShare = (size_t)64 << 10, kSmallPiece = (size_t)32 << 10;
   static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
   // An inference: the first `prefix` steps part by part, one graph per part of the batch, each launched
   // when its part of the input is on the device; the last part's graph goes on with the rest of the
@@ -133,6 +137,7 @@ class Executor {
   std::vector<cudaEvent_t> part_events_;
   int32_t* done_host_ = nullptr;    // pinned: the last kernel of an inference has delivered the heads
   void AwaitDone();
+  std::chrono::steady_clock::time_point last_call_;   // the end of the last inference
   std::unique_ptr<HostPool> pool_;   // created by the first inference that has enough bytes to move
   HostPool& pool();
   // How the heads reach the host: small ones are written into page-locked memory by a kernel

@@ -105,7 +105,9 @@ void HostPool::Work() {
       continue;
     }
     std::unique_lock<std::mutex> lk(mu_);
+    ++asleep_;
     cv_.wait(lk, [&] { return stop_ || active_; });
+    --asleep_;
     if (stop_) return;
   }
 }

@@ -43,8 +43,10 @@ class HostPool {
   // Runs one piece of any job, if one is free; false if there is none.
   bool HelpOnce();
 
- private:
   static constexpr int kLingerUs = 200;
+  bool awake() const { return asleep_.load(std::memory_order_relaxed) == 0; }   // Begin() needs no wake-up
+
+ private:
   struct Job {
     // (generation << 32 | count): a claim is a compare-exchange of the whole word against `avail` of
     // the same generation, so a helper that looked at the slot's previous job cannot take a
@@ -64,6 +66,7 @@ class HostPool {
   std::mutex mu_;
   std::condition_variable cv_;
   std::atomic<bool> active_{false}, stop_{false};
+  std::atomic<int> asleep_{0};
 };
 
 // memcpy with stores that bypass the cache: for destinations the CPU does not read soon (the

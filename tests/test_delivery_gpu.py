@@ -18,7 +18,7 @@ def copy_case(wl, n):
 
 # one kernel writes heads of up to 1 MiB, larger ones leave in 1 MiB pieces; inputs above 1 MiB are
 # staged by the host threads in 256 KiB pieces
-@pytest.mark.parametrize("n", [1, 15, 4099, 1 << 20, (1 << 20) + 1, (3 << 20) + 77])
+@pytest.mark.parametrize("n", [1, 15, 4099, 300001, 1 << 20, (1 << 20) + 1, (3 << 20) + 77])
 @pytest.mark.parametrize("where", ["pageable", "pinned", "device"])
 def test_sizes_and_buffers(n, where, rt, wl, oracle):
     import torch
@@ -30,7 +30,7 @@ def test_sizes_and_buffers(n, where, rt, wl, oracle):
         src = {"pageable": flat, "pinned": flat.pin_memory(), "device": flat.cuda()}[where]
         out = torch.zeros(n, dtype=torch.uint8)
         for dst in (out, torch.zeros(n, dtype=torch.uint8).pin_memory()):
-            for _ in range(2):
+            for _ in range(4):   # (the helpers are awake from the third on)
                 dst.zero_()
                 rt.check_call(rt.lib().CVMAPIInference(net, ctypes.c_void_p(src.data_ptr()), n, ctypes.c_void_p(dst.data_ptr())))
                 assert np.array_equal(dst.numpy(), want.view(np.uint8))
