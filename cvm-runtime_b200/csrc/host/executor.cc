@@ -139,7 +139,7 @@ void Executor::PlanForPrefix(size_t prefix) {
     }
     phys_.clear();
   }
-  const int p = prefix > 0 ? step_pos_[prefix - 1] : -2;
+  const int p = prefix > 0 ? step_pos_[std::min(prefix, step_pos_.size()) - 1] : -2;   // (heads' steps have no position)
   for (auto& a : act_) {
     a.first = a.first0;
     a.last = a.last0;
@@ -344,10 +344,21 @@ struct Lowering {
       const int rows = (int)(src.nhwc ? hw : c), cols = (int)(src.nhwc ? c : hw);
       const int clamp = ep && ep->n == 1;
       const int lo = clamp ? ep->s[0].a : 0, hi = clamp ? ep->s[0].b : 0;
-      const DevBuf a = src, b = dst;
-      add_step(label, [a, b, batch, rows, cols, clamp, lo, hi](cudaStream_t s_) {
-        return cvmk_transpose_batched(a.ptr, b.ptr, a.dtype, batch, rows, cols, clamp, lo, hi, s_);
-      });
+      const int dtype = src.dtype;
+      const size_t image = (size_t)c * hw * dtype;
+      const char* from = (const char*)src.ptr;
+      char* to = (char*)dst.ptr;
+      auto range = [=](int64_t b0, int64_t b1) {
+        return [=](cudaStream_t s_) {
+          return cvmk_transpose_batched(from + b0 * image, to + b0 * image, dtype, b1 - b0, rows, cols, clamp, lo, hi, s_);
+        };
+      };
+      add_step(label, range(0, batch));
+      const std::vector<int64_t> parts = batch_parts(batch);
+      if (parts.size() > 2 && image % 16 == 0) {
+        for (size_t k = 0; k + 1 < parts.size(); ++k) ex.steps_.back().chunk.push_back(range(parts[k], parts[k + 1]));
+        ex.steps_.back().images = batch;
+      }
       return;
     }
     cvmk_strided_desc d;
@@ -732,6 +743,7 @@ struct Lowering {
           ex.steps_.back().from_input = true;
           if (count > 1 && aligned)
             for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(move(parts[c], parts[c + 1]));
+          ex.steps_.back().images = N;
         }
         auto plan_for = [&](int64_t b0, int64_t b1) {
           cvmk_stem_conv_desc cd = sd;
@@ -750,6 +762,7 @@ struct Lowering {
         add_step(label + "[stem]", plan_for(0, N));
         ex.steps_.back().from_input = pitch == 0;
         if (sliceable)
+          ex.steps_.back().images = N;
           for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(plan_for(parts[c], parts[c + 1]));
         if (count > 1) {
           ex.part_end_.clear();
@@ -882,6 +895,7 @@ struct Lowering {
       add_step(label + (dw_tc ? "[dw]" : "[tc]"), [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
       // Plans for the parts of the batch (every operand is batch-major, so a part is a contiguous slice).
       if (parts.size() > 2 && xin.nhwc && out.nhwc) {
+        ex.steps_.back().images = N;
         const int64_t per_image = fold > 1 ? (int64_t)OH * OW : 1;   // (folded pixels: d.N counts fold-th parts of pixels)
         for (size_t c = 0; c + 1 < parts.size(); ++c) {
           const size_t first = (size_t)(parts[c] * per_image / fold);
@@ -918,6 +932,7 @@ struct Lowering {
       // The parts of the batch (batch-major operands: a part is a contiguous slice), when no step of
       // the chain indexes another tensor.
       const std::vector<int64_t> parts = batch_parts(d.N);
+      ex.steps_.back().images = d.N;
       bool sliceable = parts.size() > 2 && xin.nhwc && out.nhwc;
       for (int i = 0; i < d.ep.n; ++i)
         sliceable &= !(d.ep.s[i].op == CVMK_EP_ADD_T || d.ep.s[i].op == CVMK_EP_SUB_T || d.ep.s[i].op == CVMK_EP_RSUB_T);
@@ -1404,6 +1419,7 @@ struct Lowering {
       return cvmk_get_valid_counts_clamped((const int32_t*)x.ptr, (int32_t*)y.ptr, (int32_t*)vc.ptr, B, N, K, thr, clamp, s);
     });
     ex.steps_.back().from_input = from_raw;
+    ex.steps_.back().images = B;
     const std::vector<int64_t> parts = batch_parts(B);
     for (size_t c = 0; from_raw && parts.size() > 2 && c + 1 < parts.size(); ++c) {   // while later images upload
       const int64_t b0 = parts[c], rows = b0 * N * K;
@@ -1457,6 +1473,7 @@ struct Lowering {
       if (bound < d.N) limited[g.entry_id(nid, 0)] = {(size_t)d.B, (size_t)bound * 24, d.valid_count};
     }
     add_step(label, [d](cudaStream_t s) { return cvmk_non_max_suppression(&d, s); });
+    ex.steps_.back().images = d.B;
     const std::vector<int64_t> parts = batch_parts(d.B);
     for (size_t c = 0; parts.size() > 2 && c + 1 < parts.size(); ++c) {
       const int first = (int)parts[c], count = (int)(parts[c + 1] - parts[c]);
@@ -1591,6 +1608,13 @@ struct Lowering {
         ep.s[0].a = -data_range;
         ep.s[0].b = data_range;
         emit_convert(raw_in, materialize(data_eid), "input:data", &ep);
+        Step& st = ex.steps_.back();
+        if (!st.chunk.empty()) {
+          st.from_input = true;
+          ex.part_end_.clear();
+          for (int64_t b : batch_parts(st.images))
+            if (b > 0) ex.part_end_.push_back(ex.in_bytes_ / st.images * b);
+        }
       }
       step_pos.assign(ex.steps_.size(), -1);
       for (size_t i = 0; i < order.size(); ++i)
@@ -1608,9 +1632,9 @@ struct Lowering {
       const size_t cap = 14, parts = ex.part_end_.size();
       ex.prefix_max_ = 0;
       if (parts > 1 && !ex.steps_.empty() && ex.steps_[0].from_input)
-        while (ex.prefix_max_ < ex.steps_.size() && ex.prefix_max_ < cap && ex.steps_[ex.prefix_max_].chunk.size() == parts)
-          ++ex.prefix_max_;
+        while (ex.prefix_max_ < ex.steps_.size() && ex.prefix_max_ < cap && cut_like_first(ex.steps_[ex.prefix_max_])) ++ex.prefix_max_;
     }
+    const size_t body = ex.steps_.size();
     plan_activations(order);
     // heads: row-major staging + pinned host mirrors
     for (const auto& e : g.outputs) {
@@ -1631,7 +1655,18 @@ struct Lowering {
       ex.pinned_.push_back(h.host);
       ex.heads_.push_back(h);
     }
+    // A short graph that can be cut as a whole: the parts of its head leave while later parts compute.
+    if (ex.prefix_max_ > 0 && ex.prefix_max_ == body && ex.heads_.size() == 1) {
+      if (ex.steps_.size() == body + 1 && cut_like_first(ex.steps_[body])) ++ex.prefix_max_;
+      const HeadOut& h = ex.heads_[0];
+      const int64_t images = ex.steps_[0].images;
+      if (ex.prefix_max_ == ex.steps_.size() && h.shape.size() > 1 && h.shape[0] == images)
+        for (int64_t b : batch_parts(images))
+          if (b > 0) ex.head_part_end_.push_back(h.bytes / images * b);
+    }
   }
+  // (the same number of images: a reshape between two steps may change what a part of the batch is)
+  bool cut_like_first(const Step& s) const { return s.chunk.size() == ex.part_end_.size() && s.images == ex.steps_[0].images; }
 };
 
 Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g), device_(device_id) {
@@ -1672,9 +1707,14 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
     part_events_.resize(part_end_.size());
     for (auto& e : part_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
+  if (!head_part_end_.empty()) {
+    CUDA_OK(cudaStreamCreateWithFlags(&down_stream_, cudaStreamNonBlocking));
+    part_done_.resize(part_end_.size());
+    for (auto& e : part_done_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
   graph_whole_ = Capture([this] { Enqueue(stream_); });
   ChooseSchedules();
-  PlanForPrefix(std::max(from_pinned_.prefix, from_pageable_.prefix));   // memory for the prefix actually used
+  PlanForPrefix(std::max({from_pinned_.prefix, from_pageable_.prefix, from_device_.prefix}));   // memory for the prefix actually used
   if (in_bytes_ <= kSmallInput)
     graph_staged_ = Capture([this] {
       // (whole 16-byte words whatever the size, see in_host_: 547 215 bytes one by one took 40 us)
@@ -1745,8 +1785,9 @@ void Executor::ChooseSchedules() {
         if (src == Source::kPool) pool().Begin();
         const auto t0 = std::chrono::steady_clock::now();
         BeginUpload(input, src);
-        Launch(input, src, s);
+        Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr);
         CUDA_OK(cudaStreamSynchronize(stream_));
+        if (down_stream_) CUDA_OK(cudaStreamSynchronize(down_stream_));
         const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (src == Source::kPool) {
           pool().Finish(HostPool::kUpload);
@@ -1765,6 +1806,11 @@ void Executor::ChooseSchedules() {
         if (i->second < at->second) at = i;
       return at->first;
     };
+    if (IsDevice(input)) {   // nothing to wait for: cut only where the head's parts can leave early
+      probe(0);
+      probe(prefix_max_);
+      return best();
+    }
     for (size_t p : {(size_t)0, (size_t)2, (size_t)5, (size_t)9, prefix_max_}) probe(p);
     for (size_t d : {(size_t)2, (size_t)1}) {
       const size_t b = best();
@@ -1775,6 +1821,14 @@ void Executor::ChooseSchedules() {
       for (auto& e : seen) fprintf(stderr, "%s prefix %zu: %.1f us\n", src == Source::kPool ? "pageable" : "page-locked", e.first, e.second * 1e6);
     return best();
   };
+  if (!head_part_end_.empty()) {
+    void* dev = nullptr;
+    CUDA_OK(cudaMalloc(&dev, in_bytes_));
+    CUDA_OK(cudaMemset(dev, 0, in_bytes_));
+    CUDA_OK(cudaDeviceSynchronize());
+    from_device_ = MakeSchedule(best_for(dev));
+    CUDA_OK(cudaFree(dev));
+  }
   from_pinned_ = MakeSchedule(best_for(in_host_));
   from_pageable_ = MakeSchedule(in_bytes_ <= kSmallInput ? 0 : best_for(pageable.data()));
 }
@@ -1784,12 +1838,15 @@ Executor::~Executor() {
   if (stream_) cudaStreamSynchronize(stream_);
   DropSchedule(&from_pinned_);
   DropSchedule(&from_pageable_);
+  DropSchedule(&from_device_);
   if (graph_whole_) cudaGraphExecDestroy(graph_whole_);
   if (graph_staged_) cudaGraphExecDestroy(graph_staged_);
   if (kernels_exec_) cudaGraphExecDestroy(kernels_exec_);
   for (auto e : piece_events_) cudaEventDestroy(e);
   for (auto e : part_events_) cudaEventDestroy(e);
+  for (auto e : part_done_) cudaEventDestroy(e);
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
+  if (down_stream_) cudaStreamDestroy(down_stream_);
   for (void* p : allocs_) cudaFree(p);
   for (auto& a : act_) {
     if (a.block >= 0) vmm().unmap(reinterpret_cast<CUdeviceptr>(a.va), a.va_size);
@@ -1849,6 +1906,7 @@ void Executor::SendRange(const void* input, Source src, size_t begin, size_t byt
       for (size_t k = off / kStagePiece; k * kStagePiece < end; ++k) pool().WaitPiece(HostPool::kUpload, k);
     CUDA_OK(cudaMemcpyAsync(dev + off, (char*)in_host_ + off, end - off, cudaMemcpyHostToDevice, s));
     off = end;
+    PollPieces();
   }
 }
 
@@ -1880,9 +1938,16 @@ void Executor::ChooseDownload() {
   }
   if (download_ == Download::kPieces) {
     download_piece_ = heads_[0].bytes <= 4 * kDownloadPiece ? kDownloadPiece / 4 : kDownloadPiece;
-    piece_events_.resize((heads_[0].bytes + download_piece_ - 1) / download_piece_);
+    if (prefix_max_ != steps_.size()) head_part_end_.clear();
+    size_t at = 0;
+    for (size_t end : head_part_end_.empty() ? std::vector<size_t>{heads_[0].bytes} : head_part_end_) {
+      for (; at < end; at = piece_end_.back()) piece_end_.push_back(std::min(end, at + download_piece_));
+      part_pieces_.push_back(piece_end_.size());
+    }
+    piece_events_.resize(piece_end_.size());
     for (auto& e : piece_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
+  if (download_ != Download::kPieces) head_part_end_.clear();
   if (download_ == Download::kKernel && heads_[0].live_bytes) {
     CUDA_OK(cudaMallocHost((void**)&valid_host_, heads_[0].images * 4));
     pinned_.push_back(valid_host_);
@@ -1946,32 +2011,47 @@ void Executor::StartFill(char* out) {
 
 // One large head: the copy engine brings it in pieces, the pool copies every piece that has arrived
 // into the caller's buffer.  A page-locked buffer takes the pieces directly.
-void Executor::DeliverPieces(char* out) {
-  const HeadOut& h = heads_[0];
-  if (IsDirect(out)) {
-    CUDA_OK(cudaMemcpyAsync(out, h.dev, h.bytes, cudaMemcpyDefault, stream_));
-    CUDA_OK(cudaStreamSynchronize(stream_));
+void Executor::StartDelivery(char* out) {
+  queued_pieces_ = arrived_pieces_ = 0;
+  deliver_units_ = 0;
+  if (IsDirect(out)) return;
+  const size_t unit = DeliverUnit(), bytes = heads_[0].bytes;
+  const char* from = (const char*)heads_[0].host;
+  deliver_units_ = (bytes + unit - 1) / unit;
+  pool().Start(HostPool::kDownload, deliver_units_, 0, [=](size_t k) { memcpy(out + k * unit, from + k * unit, std::min(unit, bytes - k * unit)); });
+}
+
+// Queues the pieces up to number `end` (exclusive) that are not queued yet.
+void Executor::QueuePieces(char* head, size_t end, cudaStream_t s) {
+  for (; queued_pieces_ < end; ++queued_pieces_) {
+    const size_t at = queued_pieces_ ? piece_end_[queued_pieces_ - 1] : 0;
+    CUDA_OK(cudaMemcpyAsync(head + at, (const char*)heads_[0].dev + at, piece_end_[queued_pieces_] - at, cudaMemcpyDefault, s));
+    CUDA_OK(cudaEventRecord(piece_events_[queued_pieces_], s));
+  }
+}
+
+// Hands the pieces that have arrived to the pool.
+void Executor::PollPieces() {
+  if (!deliver_units_) return;
+  const size_t before = arrived_pieces_;
+  for (; arrived_pieces_ < queued_pieces_; ++arrived_pieces_) {
+    const cudaError_t e = cudaEventQuery(piece_events_[arrived_pieces_]);
+    if (e == cudaErrorNotReady) break;
+    CUDA_OK(e);
+  }
+  if (arrived_pieces_ == before) return;
+  const bool all = arrived_pieces_ == piece_end_.size();
+  pool().Release(HostPool::kDownload, all ? deliver_units_ : piece_end_[arrived_pieces_ - 1] / DeliverUnit());
+}
+
+void Executor::DeliverPieces() {
+  if (!deliver_units_) {
+    CUDA_OK(cudaEventSynchronize(piece_events_.back()));
     return;
   }
-  for (size_t k = 0; k < piece_events_.size(); ++k) {
-    const size_t off = k * download_piece_;
-    CUDA_OK(cudaMemcpyAsync((char*)h.host + off, (const char*)h.dev + off, std::min(download_piece_, h.bytes - off), cudaMemcpyDeviceToHost, stream_));
-    CUDA_OK(cudaEventRecord(piece_events_[k], stream_));
-  }
-  const size_t unit = std::min(kStagePiece, download_piece_) / 2, units = (h.bytes + unit - 1) / unit, per = download_piece_ / unit;
-  const char* from = (const char*)h.host;
-  const size_t bytes = h.bytes;
-  pool().Start(HostPool::kDownload, units, 0, [=](size_t k) { memcpy(out + k * unit, from + k * unit, std::min(unit, bytes - k * unit)); });
-  for (size_t k = 0; k < piece_events_.size(); ++k) {
-    cudaError_t e;
-    while ((e = cudaEventQuery(piece_events_[k])) == cudaErrorNotReady) pool().HelpOnce();
-    if (e != cudaSuccess) {   // nothing more will arrive: let the job end before reporting
-      pool().Release(HostPool::kDownload, units);
-      CUDA_OK(e);
-    }
-    pool().Release(HostPool::kDownload, std::min(units, (k + 1) * per));
-  }
+  for (PollPieces(); arrived_pieces_ < piece_end_.size(); PollPieces()) pool().HelpOnce();
   pool().Finish(HostPool::kDownload);
+  deliver_units_ = 0;
 }
 
 // The head is in page-locked memory (and the GPU idle): into the caller's buffer.
@@ -1996,22 +2076,36 @@ void Executor::DeliverHead(char* out) {
   }
 }
 
-// Queues the upload and the kernels of one inference.
-void Executor::Launch(const void* input, Source src, const Schedule& how) {
+// Queues the upload and the kernels of one inference, and the download of its head to `head` when that
+// leaves in pieces (null otherwise).  When all of the graph runs part by part, the head's part follows each on a
+// stream of its own: both directions of the link and the kernels then work at the same time (64 images of
+// 64 -> 64 channels at 56 x 56, 12.8 MB each way: 607 -> 465 us from page-locked memory, 374 -> 346 from the
+// device's own).
+void Executor::Launch(const void* input, Source src, const Schedule& how, char* head) {
+  queued_pieces_ = arrived_pieces_ = 0;
   if (how.prefix == 0) {
     SendRange(input, src, 0, in_bytes_, stream_);
     if (graph_whole_) CUDA_OK(cudaGraphLaunch(graph_whole_, stream_));
     else Enqueue(stream_);
+    if (head) QueuePieces(head, piece_end_.size(), stream_);
     return;
   }
+  const bool parts_leave = head && how.prefix == steps_.size() && !head_part_end_.empty();
   size_t begin = 0;
   for (size_t c = 0; c < how.graphs.size(); ++c) {
     SendRange(input, src, begin, part_end_[c] - begin, copy_stream_);
     CUDA_OK(cudaEventRecord(part_events_[c], copy_stream_));
     CUDA_OK(cudaStreamWaitEvent(stream_, part_events_[c], 0));
     CUDA_OK(cudaGraphLaunch(how.graphs[c], stream_));
+    if (parts_leave) {
+      CUDA_OK(cudaEventRecord(part_done_[c], stream_));
+      CUDA_OK(cudaStreamWaitEvent(down_stream_, part_done_[c], 0));
+      QueuePieces(head, part_pieces_[c], down_stream_);
+      PollPieces();
+    }
     begin = part_end_[c];
   }
+  if (head && !parts_leave) QueuePieces(head, piece_end_.size(), stream_);
 }
 
 void Executor::Run(const void* input, size_t input_bytes, char* out) {
@@ -2026,6 +2120,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
     HostPool* p = nullptr;
     ~PoolGuard() {
       if (!p) return;
+      p->ReleaseAll(HostPool::kDownload);   // (when an error ends this early)
       for (int k = 0; k < HostPool::kSlots; ++k) p->Finish((HostPool::Slot)k);
       p->End();
     }
@@ -2038,6 +2133,8 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
   if (signal) *(volatile int32_t*)done_host_ = 0;
   BeginUpload(input, src);
   if (fill) StartFill(out);
+  if (pieces) StartDelivery(out);
+  char* const head = !pieces ? nullptr : (deliver_units_ ? (char*)heads_[0].host : out);   // where the copy engine writes
   if (src == Source::kSmall && graph_staged_) {
     const bool share = in_bytes_ >= kSmallShare;
     if (share && pool_ && pool_->awake()) {
@@ -2055,16 +2152,16 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
       memcpy(in_host_, input, in_bytes_);
     }
     CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
+    if (head) QueuePieces(head, piece_end_.size(), stream_);
     // calls that follow one another closely: the helpers wake up for the next one while the GPU works
     if (share && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) {
       guard.p = &pool();
       guard.p->Begin();
     }
   } else {
-    static const Schedule whole;
-    Launch(input, src, on_device ? whole : (src == Source::kDirect ? from_pinned_ : from_pageable_));
+    Launch(input, src, on_device ? from_device_ : (src == Source::kDirect ? from_pinned_ : from_pageable_), head);
   }
-  if (pieces) DeliverPieces(out);
+  if (pieces) DeliverPieces();
   else if (signal) AwaitDone();
   else CUDA_OK(cudaStreamSynchronize(stream_));
   if (*status_host_ != 0) {

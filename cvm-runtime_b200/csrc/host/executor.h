@@ -40,6 +40,7 @@ struct Step {
   // The same operator on one part of the batch each (empty when the step cannot be cut along the
   // batch): the leading steps of an inference run part by part while later parts upload.
   std::vector<std::function<int(cudaStream_t)>> chunk;
+  int64_t images = 0;        // of the batch that `chunk` cuts
   bool from_input = false;   // reads the uploaded bytes and nothing else of the batch
 };
 
@@ -107,6 +108,7 @@ class Executor {
   // pageable memory (staged by host threads first).  prefix_max_ bounds it (the memory planner keeps
   // everything those steps touch live together).
   Schedule from_pinned_, from_pageable_;
+  Schedule from_device_;   // an input in device memory: the whole graph, unless the head's parts can leave early
   cudaGraphExec_t graph_whole_ = nullptr;    // every step: the input is on the device already
   cudaGraphExec_t graph_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
   size_t prefix_max_ = 0;
@@ -114,10 +116,11 @@ class Executor {
   static void DropSchedule(Schedule* s);
   cudaGraphExec_t Capture(const std::function<void()>& enqueue);
   void ChooseSchedules();
-  void Launch(const void* input, Source src, const Schedule& how);
+  void Launch(const void* input, Source src, const Schedule& how, char* head);
   static bool IsDirect(const void* input);
   static bool IsDevice(const void* input);
   std::vector<size_t> part_end_;   // input bytes up to the end of each part of the batch
+  std::vector<size_t> head_part_end_;   // the same of the only head, where its parts may leave one by one
   std::vector<HeadOut> heads_;
   std::vector<void*> allocs_;
   std::vector<void*> pinned_;
@@ -135,6 +138,8 @@ class Executor {
   // upload / compute overlap: the copy stream and one event per part of the batch
   cudaStream_t copy_stream_ = nullptr;
   std::vector<cudaEvent_t> part_events_;
+  cudaStream_t down_stream_ = nullptr;   // the parts of a head, each behind its part_done_ event
+  std::vector<cudaEvent_t> part_done_;
   int32_t* done_host_ = nullptr;    // pinned: the last kernel of an inference has delivered the heads
   void AwaitDone();
   std::chrono::steady_clock::time_point last_call_;   // the end of the last inference
@@ -148,10 +153,16 @@ class Executor {
   bool plain_ = false;
   std::vector<cudaEvent_t> piece_events_;
   size_t download_piece_ = 0;
+  std::vector<size_t> piece_end_, part_pieces_;   // head bytes up to each piece's end; pieces up to each part's end
+  size_t queued_pieces_ = 0, arrived_pieces_ = 0, deliver_units_ = 0;   // of the inference that runs
+  size_t DeliverUnit() const { return std::min(kStagePiece, download_piece_) / 2; }
   int32_t* valid_host_ = nullptr;    // pinned copy of HeadOut::valid_count
   void ChooseDownload();
   void StartFill(char* out);
-  void DeliverPieces(char* out);
+  void StartDelivery(char* out);
+  void QueuePieces(char* head, size_t end, cudaStream_t s);
+  void PollPieces();
+  void DeliverPieces();
   void DeliverHead(char* out);
 
   void* dalloc(size_t bytes);

@@ -35,6 +35,7 @@ class HostPool {
   // `available` pieces may run at once, the others when Release() says so.
   void Start(Slot slot, size_t pieces, size_t available, std::function<void(size_t)> body);
   void Release(Slot slot, size_t available);
+  void ReleaseAll(Slot slot) { Release(slot, jobs_[slot].pieces); }
   // Waits until piece k has run, running pieces of this job meanwhile.
   void WaitPiece(Slot slot, size_t k);
   // Waits until the whole job has run.

@@ -79,3 +79,23 @@ def test_image_stem(width, batch, rt, wl, oracle):
             assert np.array_equal(out.numpy(), want.view(np.uint8))
     finally:
         rt.CVMAPIFreeModel(net)
+
+
+# graphs that are cut along the batch as a whole: the parts of the head leave while later parts compute;
+# widths whose images are and are not whole 16-byte words, a head below and some above the size that leaves in pieces
+@pytest.mark.parametrize("batch,channels,size", [(8, 32, 14), (9, 64, 33), (31, 32, 37), (40, 64, 56), (3, 128, 61)])
+def test_head_in_parts(batch, channels, size, rt, wl, oracle):
+    import torch
+    js, pb, x = wl.conv_chain(batch=batch, channels=channels, size=size)
+    net = rt.CVMAPILoadModel(js, pb, 0)
+    try:
+        for turn in range(2):
+            x = np.roll(x, 1, axis=0)
+            want = oracle.run_model(js, pb, x).view(np.uint8).reshape(-1)
+            flat = torch.from_numpy(x.reshape(-1).view(np.uint8).copy())
+            for src in (flat, flat.pin_memory(), flat.cuda()):
+                for dst in (torch.zeros(want.size, dtype=torch.uint8), torch.zeros(want.size, dtype=torch.uint8).pin_memory()):
+                    rt.check_call(rt.lib().CVMAPIInference(net, ctypes.c_void_p(src.data_ptr()), flat.numel(), ctypes.c_void_p(dst.data_ptr())))
+                    assert np.array_equal(dst.numpy(), want)
+    finally:
+        rt.CVMAPIFreeModel(net)
