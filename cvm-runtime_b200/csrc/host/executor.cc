@@ -1031,6 +1031,7 @@ struct Lowering {
     d.stride_h = (int)n.attrs.t("strides")[0]; d.stride_w = (int)n.attrs.t("strides")[1];
     d.pad_h = (int)pad[0]; d.pad_w = (int)(pad.size() == 2 ? pad[1] : pad[0]);
     add_step("max_pool2d:" + n.name(), [d](cudaStream_t s) { return cvmk_max_pool2d(&d, s); });
+    ex.steps_.back().images = d.N;
     const std::vector<int64_t> parts = batch_parts(d.N);
     for (size_t c = 0; parts.size() > 2 && x.nhwc && y.nhwc && c + 1 < parts.size(); ++c) {
       cvmk_pool_desc cd = d;
