@@ -189,6 +189,15 @@ void Executor::MapActivations() {
   }
 }
 
+// How a batch may be cut for upload / compute overlap: five parts (an eighth, three quarters, an eighth), four
+// (1/8, 1/4, 5/16, 5/16) or two (3/8, 5/8), as indices into Lowering::batch_ranges().  Where the kernels take
+// longer than the upload, what counts is how soon the first part is there and how few launches each step takes;
+// where the upload takes longer, how little is left to do when the last part has arrived.  Measured at load
+// (ChooseSchedules); against five parts always: ResNet-50, 256 images 2389 -> 2321 us (four parts), VGG-19, 32
+// images 865 -> 835 (two).
+const std::vector<int> kCuts[] = {{0, 1, 2, 3, 4}, {0, 1, 5, 6}, {7, 8}};
+constexpr size_t kMaxParts = 5;
+
 struct Lowering {
   Executor& ex;
   const Graph& g;
@@ -205,18 +214,25 @@ struct Lowering {
 
   Lowering(Executor& e, const Graph& gr) : ex(e), g(gr) {}
 
+  // The parts of the batch that steps are prepared for, as ranges of images in the order of kCuts (none for
+  // batches under eight images).
+  struct Range { int64_t begin, end; };
+  static std::vector<Range> batch_ranges(int64_t n) {
+    if (n < 8 || dev_env("CVM_B200_NO_UPLOAD_OVERLAP")) return {};
+    const int at[][2] = {{0, 2}, {2, 6}, {6, 10}, {10, 14}, {14, 16}, {6, 11}, {11, 16}, {0, 6}, {6, 16}};   // sixteenths
+    std::vector<Range> r;
+    for (const auto& a : at) r.push_back({(n * a[0] + 8) / 16, (n * a[1] + 8) / 16});
+    return r;
+  }
+  void input_ranges(const std::vector<Range>& parts, size_t image_bytes) {
+    if (parts.empty()) return;
+    ex.range_end_.clear();
+    for (const Range& r : parts) ex.range_end_.push_back((size_t)r.end * image_bytes);
+  }
+
   void add_step(const std::string& label, std::function<int(cudaStream_t)> fn) {
     ex.steps_.push_back({label, std::move(fn), {}});
   }
-  // Parts of the batch for upload / compute overlap: an eighth, three quarters, an eighth.  Where the
-  // kernels take longer than the upload, what counts is how soon the first part is there; where the
-  // upload takes longer, how little is left to do when the last part has arrived.  Image numbers of
-  // the part boundaries; just {0, n} for batches under eight images.
-  static std::vector<int64_t> batch_parts(int64_t n) {
-    if (n < 8 || dev_env("CVM_B200_NO_UPLOAD_OVERLAP")) return {0, n};
-    return {0, (n + 4) / 8, (3 * n + 4) / 8, (5 * n + 4) / 8, (7 * n + 4) / 8, n};
-  }
-
   // ------------------------------------------------------------------ analysis
   void analyse() {
     const uint32_t ne = g.num_entries;
@@ -354,11 +370,9 @@ struct Lowering {
         };
       };
       add_step(label, range(0, batch));
-      const std::vector<int64_t> parts = batch_parts(batch);
-      if (parts.size() > 2 && image % 16 == 0) {
-        for (size_t k = 0; k + 1 < parts.size(); ++k) ex.steps_.back().chunk.push_back(range(parts[k], parts[k + 1]));
-        ex.steps_.back().images = batch;
-      }
+      if (image % 16 == 0)
+        for (const Range& r : batch_ranges(batch)) ex.steps_.back().chunk.push_back(range(r.begin, r.end));
+      ex.steps_.back().images = batch;
       return;
     }
     cvmk_strided_desc d;
@@ -723,8 +737,7 @@ struct Lowering {
         sd.w = wsdev;
         // The batch is cut into parts with a plan each, so that an inference can run the stem on the
         // first images while the later ones are still being uploaded.
-        const std::vector<int64_t> parts = (uses[ex_] == 1 && !is_head[ex_]) ? batch_parts(N) : std::vector<int64_t>{0, N};
-        const size_t count = parts.size() - 1;
+        const std::vector<Range> parts = (uses[ex_] == 1 && !is_head[ex_]) ? batch_ranges(N) : std::vector<Range>();
         const size_t image = (size_t)C * H * W;
         int8_t* rows = nullptr;
         const int pitch = sd.x_pitch;
@@ -738,11 +751,11 @@ struct Lowering {
             return [from, to, n, W, pitch](cudaStream_t s) { return cvmk_repitch(from, to, n, W, pitch, s); };
           };
           bool aligned = true;
-          for (int64_t b : parts) aligned &= ((size_t)b * image) % 4 == 0;
+          for (const Range& r : parts) aligned &= ((size_t)r.begin * image) % 4 == 0;
           add_step(label + "[rows]", move(0, N));
           ex.steps_.back().from_input = true;
-          if (count > 1 && aligned)
-            for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(move(parts[c], parts[c + 1]));
+          for (const Range& r : parts)
+            if (aligned) ex.steps_.back().chunk.push_back(move(r.begin, r.end));
           ex.steps_.back().images = N;
         }
         auto plan_for = [&](int64_t b0, int64_t b1) {
@@ -757,17 +770,11 @@ struct Lowering {
           KERNEL_OK(cvmk_conv2d_stem_prepare(&cd, pl));
           return [pl](cudaStream_t s) { return cvmk_conv2d_stem_launch(pl, s); };
         };
-        bool sliceable = count > 1;   // (parts start on 16-byte boundaries)
-        for (int64_t b : parts) sliceable &= ((size_t)b * C * H * (pitch > 0 ? pitch : W)) % 16 == 0;
         add_step(label + "[stem]", plan_for(0, N));
         ex.steps_.back().from_input = pitch == 0;
-        if (sliceable)
-          ex.steps_.back().images = N;
-          for (size_t c = 0; c < count; ++c) ex.steps_.back().chunk.push_back(plan_for(parts[c], parts[c + 1]));
-        if (count > 1) {
-          ex.part_end_.clear();
-          for (size_t c = 1; c <= count; ++c) ex.part_end_.push_back((size_t)parts[c] * image);
-        }
+        ex.steps_.back().images = N;
+        for (const Range& r : parts) ex.steps_.back().chunk.push_back(plan_for(r.begin, r.end));   // (whole rows of 16 bytes)
+        input_ranges(parts, image);
         return;
       }
     }
@@ -854,14 +861,14 @@ struct Lowering {
         d.ep.s[0].ptr = bfdev;
       }
       int fold = 1;
-      const std::vector<int64_t> parts = batch_parts(N);
+      const std::vector<Range> parts = batch_ranges(N);
       if (!dense && !dw_tc && groups == 1 && KH == 1 && KW == 1 && sh == 1 && sw == 1 && ph == 0 && pw == 0 &&
           xin.nhwc && out.nhwc && (!use_bias || g.params.count(g.entry_id(n.inputs[2])) > 0) &&
           !dev_env("CVM_B200_NO_PIXEL_FOLD")) {
         auto whole = [&](int f) {   // every part of the batch is a whole number of folded pixels
-          for (int64_t b : parts)
-            if (b * OH * OW % f != 0) return false;
-          return true;
+          for (const Range& r : parts)
+            if (r.begin * OH * OW % f != 0) return false;
+          return (int64_t)N * OH * OW % f == 0;
         };
         while (fold < 4 && 2 * fold * C <= 128 && 2 * fold * OC <= 256 && whole(2 * fold)) fold *= 2;
       }
@@ -894,13 +901,13 @@ struct Lowering {
       KERNEL_OK(cvmk_conv2d_tc_prepare(&d, plan));
       add_step(label + (dw_tc ? "[dw]" : "[tc]"), [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
       // Plans for the parts of the batch (every operand is batch-major, so a part is a contiguous slice).
-      if (parts.size() > 2 && xin.nhwc && out.nhwc) {
+      if (xin.nhwc && out.nhwc) {
         ex.steps_.back().images = N;
         const int64_t per_image = fold > 1 ? (int64_t)OH * OW : 1;   // (folded pixels: d.N counts fold-th parts of pixels)
-        for (size_t c = 0; c + 1 < parts.size(); ++c) {
-          const size_t first = (size_t)(parts[c] * per_image / fold);
+        for (const Range& r : parts) {
+          const size_t first = (size_t)(r.begin * per_image / fold);
           cvmk_conv_desc cd = d;
-          cd.N = (int)((parts[c + 1] - parts[c]) * per_image / fold);
+          cd.N = (int)((r.end - r.begin) * per_image / fold);
           const size_t out_first = first * d.OH * d.OW * d.OC;
           cd.x = d.x + first * d.H * d.W * d.C;
           cd.y = (char*)d.y + out_first * d.y_dtype;
@@ -931,16 +938,15 @@ struct Lowering {
       add_step(label + (depthwise ? "[dw]" : "[direct]"), [d](cudaStream_t s) { return cvmk_conv2d_direct(&d, s); });
       // The parts of the batch (batch-major operands: a part is a contiguous slice), when no step of
       // the chain indexes another tensor.
-      const std::vector<int64_t> parts = batch_parts(d.N);
       ex.steps_.back().images = d.N;
-      bool sliceable = parts.size() > 2 && xin.nhwc && out.nhwc;
+      bool sliceable = xin.nhwc && out.nhwc;
       for (int i = 0; i < d.ep.n; ++i)
         sliceable &= !(d.ep.s[i].op == CVMK_EP_ADD_T || d.ep.s[i].op == CVMK_EP_SUB_T || d.ep.s[i].op == CVMK_EP_RSUB_T);
-      for (size_t c = 0; sliceable && c + 1 < parts.size(); ++c) {
+      for (const Range& r : sliceable ? batch_ranges(d.N) : std::vector<Range>()) {
         cvmk_conv_direct_desc cd = d;
-        cd.N = (int)(parts[c + 1] - parts[c]);
-        cd.x = (const char*)d.x + (size_t)parts[c] * d.H * d.W * d.C * d.x_dtype;
-        cd.y = (char*)d.y + (size_t)parts[c] * d.OH * d.OW * d.OC * d.y_dtype;
+        cd.N = (int)(r.end - r.begin);
+        cd.x = (const char*)d.x + (size_t)r.begin * d.H * d.W * d.C * d.x_dtype;
+        cd.y = (char*)d.y + (size_t)r.begin * d.OH * d.OW * d.OC * d.y_dtype;
         ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_conv2d_direct(&cd, s); });
       }
     }
@@ -1032,12 +1038,11 @@ struct Lowering {
     d.pad_h = (int)pad[0]; d.pad_w = (int)(pad.size() == 2 ? pad[1] : pad[0]);
     add_step("max_pool2d:" + n.name(), [d](cudaStream_t s) { return cvmk_max_pool2d(&d, s); });
     ex.steps_.back().images = d.N;
-    const std::vector<int64_t> parts = batch_parts(d.N);
-    for (size_t c = 0; parts.size() > 2 && x.nhwc && y.nhwc && c + 1 < parts.size(); ++c) {
+    for (const Range& r : x.nhwc && y.nhwc ? batch_ranges(d.N) : std::vector<Range>()) {
       cvmk_pool_desc cd = d;
-      cd.N = (int)(parts[c + 1] - parts[c]);
-      cd.x = (const char*)d.x + (size_t)parts[c] * d.H * d.W * d.C * d.dtype;
-      cd.y = (char*)d.y + (size_t)parts[c] * d.OH * d.OW * d.C * d.dtype;
+      cd.N = (int)(r.end - r.begin);
+      cd.x = (const char*)d.x + (size_t)r.begin * d.H * d.W * d.C * d.dtype;
+      cd.y = (char*)d.y + (size_t)r.begin * d.OH * d.OW * d.C * d.dtype;
       ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_max_pool2d(&cd, s); });
     }
   }
@@ -1421,12 +1426,11 @@ struct Lowering {
     });
     ex.steps_.back().from_input = from_raw;
     ex.steps_.back().images = B;
-    const std::vector<int64_t> parts = batch_parts(B);
-    for (size_t c = 0; from_raw && parts.size() > 2 && c + 1 < parts.size(); ++c) {   // while later images upload
-      const int64_t b0 = parts[c], rows = b0 * N * K;
-      const int count = (int)(parts[c + 1] - b0);
-      ex.part_end_.resize(c + 1);
-      ex.part_end_[c] = (size_t)parts[c + 1] * N * K * 4;
+    const std::vector<Range> parts = from_raw ? batch_ranges(B) : std::vector<Range>();
+    input_ranges(parts, (size_t)N * K * 4);
+    for (const Range& r : parts) {   // while later images upload
+      const int64_t b0 = r.begin, rows = b0 * N * K;
+      const int count = (int)(r.end - b0);
       ex.steps_.back().chunk.push_back([x, y, vc, b0, rows, count, N, K, thr, clamp](cudaStream_t s) {
         return cvmk_get_valid_counts_clamped((const int32_t*)x.ptr + rows, (int32_t*)y.ptr + rows, (int32_t*)vc.ptr + b0, count, N, K, thr, clamp, s);
       });
@@ -1475,9 +1479,8 @@ struct Lowering {
     }
     add_step(label, [d](cudaStream_t s) { return cvmk_non_max_suppression(&d, s); });
     ex.steps_.back().images = d.B;
-    const std::vector<int64_t> parts = batch_parts(d.B);
-    for (size_t c = 0; parts.size() > 2 && c + 1 < parts.size(); ++c) {
-      const int first = (int)parts[c], count = (int)(parts[c + 1] - parts[c]);
+    for (const Range& r : batch_ranges(d.B)) {
+      const int first = (int)r.begin, count = (int)(r.end - r.begin);
       ex.steps_.back().chunk.push_back([d, first, count](cudaStream_t s) { return cvmk_non_max_suppression_part(&d, first, count, s); });
     }
   }
@@ -1612,9 +1615,7 @@ struct Lowering {
         Step& st = ex.steps_.back();
         if (!st.chunk.empty()) {
           st.from_input = true;
-          ex.part_end_.clear();
-          for (int64_t b : batch_parts(st.images))
-            if (b > 0) ex.part_end_.push_back(ex.in_bytes_ / st.images * b);
+          input_ranges(batch_ranges(st.images), ex.in_bytes_ / st.images);
         }
       }
       step_pos.assign(ex.steps_.size(), -1);
@@ -1630,9 +1631,9 @@ struct Lowering {
     // for all of it (whole-batch buffers, filled part by part), so its length is also a memory
     // decision: ten steps of ResNet-50 at batch 256 hold 1.3 GB, twenty 2.1 GB.
     {
-      const size_t cap = 14, parts = ex.part_end_.size();
+      const size_t cap = 14;
       ex.prefix_max_ = 0;
-      if (parts > 1 && !ex.steps_.empty() && ex.steps_[0].from_input)
+      if (!ex.range_end_.empty() && !ex.steps_.empty() && ex.steps_[0].from_input)
         while (ex.prefix_max_ < ex.steps_.size() && ex.prefix_max_ < cap && cut_like_first(ex.steps_[ex.prefix_max_])) ++ex.prefix_max_;
     }
     const size_t body = ex.steps_.size();
@@ -1662,12 +1663,11 @@ struct Lowering {
       const HeadOut& h = ex.heads_[0];
       const int64_t images = ex.steps_[0].images;
       if (ex.prefix_max_ == ex.steps_.size() && h.shape.size() > 1 && h.shape[0] == images)
-        for (int64_t b : batch_parts(images))
-          if (b > 0) ex.head_part_end_.push_back(h.bytes / images * b);
+        for (const Range& r : batch_ranges(images)) ex.head_range_end_.push_back(h.bytes / images * r.end);
     }
   }
   // (the same number of images: a reshape between two steps may change what a part of the batch is)
-  bool cut_like_first(const Step& s) const { return s.chunk.size() == ex.part_end_.size() && s.images == ex.steps_[0].images; }
+  bool cut_like_first(const Step& s) const { return s.chunk.size() == ex.range_end_.size() && s.images == ex.steps_[0].images; }
 };
 
 Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g), device_(device_id) {
@@ -1705,12 +1705,12 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
   if (!use_graph_) return;
   if (prefix_max_ > 0) {
     CUDA_OK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
-    part_events_.resize(part_end_.size());
+    part_events_.resize(kMaxParts);
     for (auto& e : part_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  if (!head_part_end_.empty()) {
+  if (!head_range_end_.empty()) {
     CUDA_OK(cudaStreamCreateWithFlags(&down_stream_, cudaStreamNonBlocking));
-    part_done_.resize(part_end_.size());
+    part_done_.resize(kMaxParts);
     for (auto& e : part_done_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   graph_whole_ = Capture([this] { Enqueue(stream_); });
@@ -1738,13 +1738,15 @@ cudaGraphExec_t Executor::Capture(const std::function<void()>& enqueue) {
   return exec;
 }
 
-Executor::Schedule Executor::MakeSchedule(size_t prefix) {
+Executor::Schedule Executor::MakeSchedule(size_t prefix, int cut) {
   Schedule s;
   s.prefix = prefix;
-  for (size_t c = 0; prefix > 0 && c < part_end_.size(); ++c)
+  s.cut = cut;
+  if (prefix == 0) return s;
+  for (int r : kCuts[cut])
     s.graphs.push_back(Capture([&] {
-      for (size_t k = 0; k < prefix; ++k) KERNEL_OK(steps_[k].chunk[c](stream_));
-      if (c + 1 == part_end_.size()) Enqueue(stream_, prefix);
+      for (size_t k = 0; k < prefix; ++k) KERNEL_OK(steps_[k].chunk[r](stream_));
+      if (r == kCuts[cut].back()) Enqueue(stream_, prefix);
     }));
   return s;
 }
@@ -1770,17 +1772,17 @@ bool Executor::IsDirect(const void* input) {
   return false;
 }
 
-// How many leading steps to run part by part: the count whose inference takes least, timed here (best of
-// three each) from page-locked and from pageable memory.  A few counts spread over the range, then
-// the neighbours of the best.  (Predicting it from step times and upload rates, as before, missed what
+// How many leading steps to run part by part, and in which parts: the choice whose inference takes least, timed
+// here (best of three each) from page-locked and from pageable memory.  A few counts spread over the range,
+// then the neighbours of the best.  (Predicting it from step times and upload rates, as before, missed what
 // the launches of a part and the smaller grids cost: SSD-512 batch 8 ran at 712 instead of 661 us.)
 void Executor::ChooseSchedules() {
   if (prefix_max_ == 0) return;
   std::vector<char> pageable(in_bytes_, 0);
   auto best_for = [&](const void* input) {
     const Source src = SourceOf(input);
-    auto time_of = [&](size_t prefix) {
-      Schedule s = MakeSchedule(prefix);
+    auto time_of = [&](size_t prefix, int cut) {
+      Schedule s = MakeSchedule(prefix, cut);
       double best = 1e30;
       for (int rep = 0; rep < 4; ++rep) {   // the first is a warm-up
         if (src == Source::kPool) pool().Begin();
@@ -1799,39 +1801,53 @@ void Executor::ChooseSchedules() {
       DropSchedule(&s);
       return best;
     };
-    std::map<size_t, double> seen;
-    auto probe = [&](size_t p) { if (p <= prefix_max_ && !seen.count(p)) seen[p] = time_of(p); };
+    std::map<std::pair<size_t, int>, double> seen;
+    auto probe = [&](size_t p, int cut) {
+      if (p == 0) cut = 0;
+      if (p <= prefix_max_ && !seen.count({p, cut})) seen[{p, cut}] = time_of(p, cut);
+    };
     auto best = [&] {
       auto at = seen.begin();
+      // (five parts unless others are better by more than a hundredth: the data here are zeros, with
+      //  which detection steps take less than they will)
+      auto cost = [](const std::pair<const std::pair<size_t, int>, double>& e) { return e.second * (e.first.second ? 1.01 : 1.0); };
       for (auto i = seen.begin(); i != seen.end(); ++i)
-        if (i->second < at->second) at = i;
+        if (cost(*i) < cost(*at)) at = i;
       return at->first;
     };
     if (IsDevice(input)) {   // nothing to wait for: cut only where the head's parts can leave early
-      probe(0);
-      probe(prefix_max_);
+      probe(0, 0);
+      for (int cut : {0, 1, 2}) probe(prefix_max_, cut);
       return best();
     }
-    for (size_t p : {(size_t)0, (size_t)2, (size_t)5, (size_t)9, prefix_max_}) probe(p);
+    for (size_t p : {(size_t)0, (size_t)2, (size_t)5, (size_t)9, prefix_max_}) probe(p, 0);
+    for (size_t p : {(size_t)2, (size_t)5, (size_t)9, prefix_max_})
+      for (int cut : {1, 2}) probe(p, cut);
     for (size_t d : {(size_t)2, (size_t)1}) {
-      const size_t b = best();
-      probe(b + d);
-      if (b >= d) probe(b - d);
+      const auto b = best();
+      probe(b.first + d, b.second);
+      if (b.first >= d) probe(b.first - d, b.second);
     }
     if (dev_env("CVM_B200_VERBOSE"))
-      for (auto& e : seen) fprintf(stderr, "%s prefix %zu: %.1f us\n", src == Source::kPool ? "pageable" : "page-locked", e.first, e.second * 1e6);
+      for (auto& e : seen)
+        fprintf(stderr, "%s prefix %zu in %zu parts: %.1f us\n", src == Source::kPool ? "pageable" : "page-locked", e.first.first,
+                kCuts[e.first.second].size(), e.second * 1e6);
     return best();
   };
-  if (!head_part_end_.empty()) {
+  auto choose = [&](const void* input) {
+    const auto b = best_for(input);
+    return MakeSchedule(b.first, b.second);
+  };
+  if (!head_range_end_.empty()) {
     void* dev = nullptr;
     CUDA_OK(cudaMalloc(&dev, in_bytes_));
     CUDA_OK(cudaMemset(dev, 0, in_bytes_));
     CUDA_OK(cudaDeviceSynchronize());
-    from_device_ = MakeSchedule(best_for(dev));
+    from_device_ = choose(dev);
     CUDA_OK(cudaFree(dev));
   }
-  from_pinned_ = MakeSchedule(best_for(in_host_));
-  from_pageable_ = MakeSchedule(in_bytes_ <= kSmallInput ? 0 : best_for(pageable.data()));
+  from_pinned_ = choose(in_host_);
+  if (in_bytes_ > kSmallInput) from_pageable_ = choose(pageable.data());
 }
 
 Executor::~Executor() {
@@ -1939,16 +1955,17 @@ void Executor::ChooseDownload() {
   }
   if (download_ == Download::kPieces) {
     download_piece_ = heads_[0].bytes <= 4 * kDownloadPiece ? kDownloadPiece / 4 : kDownloadPiece;
-    if (prefix_max_ != steps_.size()) head_part_end_.clear();
+    if (prefix_max_ != steps_.size()) head_range_end_.clear();
+    std::vector<size_t> ends = head_range_end_;   // (no piece crosses the end of a part)
+    ends.push_back(heads_[0].bytes);
+    std::sort(ends.begin(), ends.end());
     size_t at = 0;
-    for (size_t end : head_part_end_.empty() ? std::vector<size_t>{heads_[0].bytes} : head_part_end_) {
+    for (size_t end : ends)
       for (; at < end; at = piece_end_.back()) piece_end_.push_back(std::min(end, at + download_piece_));
-      part_pieces_.push_back(piece_end_.size());
-    }
     piece_events_.resize(piece_end_.size());
     for (auto& e : piece_events_) CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  if (download_ != Download::kPieces) head_part_end_.clear();
+  if (download_ != Download::kPieces) head_range_end_.clear();
   if (download_ == Download::kKernel && heads_[0].live_bytes) {
     CUDA_OK(cudaMallocHost((void**)&valid_host_, heads_[0].images * 4));
     pinned_.push_back(valid_host_);
@@ -2022,9 +2039,9 @@ void Executor::StartDelivery(char* out) {
   pool().Start(HostPool::kDownload, deliver_units_, 0, [=](size_t k) { memcpy(out + k * unit, from + k * unit, std::min(unit, bytes - k * unit)); });
 }
 
-// Queues the pieces up to number `end` (exclusive) that are not queued yet.
-void Executor::QueuePieces(char* head, size_t end, cudaStream_t s) {
-  for (; queued_pieces_ < end; ++queued_pieces_) {
+// Queues the pieces of the head's first `bytes` that are not queued yet.
+void Executor::QueuePieces(char* head, size_t bytes, cudaStream_t s) {
+  for (; queued_pieces_ < piece_end_.size() && piece_end_[queued_pieces_] <= bytes; ++queued_pieces_) {
     const size_t at = queued_pieces_ ? piece_end_[queued_pieces_ - 1] : 0;
     CUDA_OK(cudaMemcpyAsync(head + at, (const char*)heads_[0].dev + at, piece_end_[queued_pieces_] - at, cudaMemcpyDefault, s));
     CUDA_OK(cudaEventRecord(piece_events_[queued_pieces_], s));
@@ -2088,25 +2105,26 @@ void Executor::Launch(const void* input, Source src, const Schedule& how, char* 
     SendRange(input, src, 0, in_bytes_, stream_);
     if (graph_whole_) CUDA_OK(cudaGraphLaunch(graph_whole_, stream_));
     else Enqueue(stream_);
-    if (head) QueuePieces(head, piece_end_.size(), stream_);
+    if (head) QueuePieces(head, heads_[0].bytes, stream_);
     return;
   }
-  const bool parts_leave = head && how.prefix == steps_.size() && !head_part_end_.empty();
+  const bool parts_leave = head && how.prefix == steps_.size() && !head_range_end_.empty();
   size_t begin = 0;
   for (size_t c = 0; c < how.graphs.size(); ++c) {
-    SendRange(input, src, begin, part_end_[c] - begin, copy_stream_);
+    const int r = kCuts[how.cut][c];
+    SendRange(input, src, begin, range_end_[r] - begin, copy_stream_);
     CUDA_OK(cudaEventRecord(part_events_[c], copy_stream_));
     CUDA_OK(cudaStreamWaitEvent(stream_, part_events_[c], 0));
     CUDA_OK(cudaGraphLaunch(how.graphs[c], stream_));
     if (parts_leave) {
       CUDA_OK(cudaEventRecord(part_done_[c], stream_));
       CUDA_OK(cudaStreamWaitEvent(down_stream_, part_done_[c], 0));
-      QueuePieces(head, part_pieces_[c], down_stream_);
+      QueuePieces(head, head_range_end_[r], down_stream_);
       PollPieces();
     }
-    begin = part_end_[c];
+    begin = range_end_[r];
   }
-  if (head && !parts_leave) QueuePieces(head, piece_end_.size(), stream_);
+  if (head && !parts_leave) QueuePieces(head, heads_[0].bytes, stream_);
 }
 
 void Executor::Run(const void* input, size_t input_bytes, char* out) {
@@ -2153,7 +2171,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
       memcpy(in_host_, input, in_bytes_);
     }
     CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
-    if (head) QueuePieces(head, piece_end_.size(), stream_);
+    if (head) QueuePieces(head, heads_[0].bytes, stream_);
     // calls that follow one another closely: the helpers wake up for the next one while the GPU works
     if (share && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) {
       guard.p = &pool();

@@ -101,6 +101,7 @@ class Executor {
   // steps and the delivery of the heads.  Without a prefix: one graph.
   struct Schedule {
     size_t prefix = 0;
+    int cut = 0;                            // which parts (kCuts)
     std::vector<cudaGraphExec_t> graphs;
   };
   // How long the prefix should be depends on how fast the input arrives: chosen at load by timing
@@ -112,15 +113,15 @@ class Executor {
   cudaGraphExec_t graph_whole_ = nullptr;    // every step: the input is on the device already
   cudaGraphExec_t graph_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
   size_t prefix_max_ = 0;
-  Schedule MakeSchedule(size_t prefix);
+  Schedule MakeSchedule(size_t prefix, int cut);
   static void DropSchedule(Schedule* s);
   cudaGraphExec_t Capture(const std::function<void()>& enqueue);
   void ChooseSchedules();
   void Launch(const void* input, Source src, const Schedule& how, char* head);
   static bool IsDirect(const void* input);
   static bool IsDevice(const void* input);
-  std::vector<size_t> part_end_;   // input bytes up to the end of each part of the batch
-  std::vector<size_t> head_part_end_;   // the same of the only head, where its parts may leave one by one
+  std::vector<size_t> range_end_;   // input bytes up to the end of each range of images that steps are prepared for
+  std::vector<size_t> head_range_end_;   // the same of the only head, where its parts may leave one by one
   std::vector<HeadOut> heads_;
   std::vector<void*> allocs_;
   std::vector<void*> pinned_;
@@ -153,14 +154,14 @@ class Executor {
   bool plain_ = false;
   std::vector<cudaEvent_t> piece_events_;
   size_t download_piece_ = 0;
-  std::vector<size_t> piece_end_, part_pieces_;   // head bytes up to each piece's end; pieces up to each part's end
+  std::vector<size_t> piece_end_;   // head bytes up to each piece's end
   size_t queued_pieces_ = 0, arrived_pieces_ = 0, deliver_units_ = 0;   // of the inference that runs
   size_t DeliverUnit() const { return std::min(kStagePiece, download_piece_) / 2; }
   int32_t* valid_host_ = nullptr;    // pinned copy of HeadOut::valid_count
   void ChooseDownload();
   void StartFill(char* out);
   void StartDelivery(char* out);
-  void QueuePieces(char* head, size_t end, cudaStream_t s);
+  void QueuePieces(char* head, size_t bytes, cudaStream_t s);
   void PollPieces();
   void DeliverPieces();
   void DeliverHead(char* out);
