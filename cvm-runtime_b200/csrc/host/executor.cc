@@ -904,7 +904,17 @@ struct Lowering {
       if (xin.nhwc && out.nhwc) {
         ex.steps_.back().images = N;
         const int64_t per_image = fold > 1 ? (int64_t)OH * OW : 1;   // (folded pixels: d.N counts fold-th parts of pixels)
+        // (every part's operands start on 16 bytes: odd images of 8 or 24 channels do not)
+        bool aligned = true;
         for (const Range& r : parts) {
+          const size_t out_first = (size_t)(r.begin * per_image / fold) * d.OH * d.OW * d.OC;
+          aligned &= out_first * d.y_dtype % 16 == 0;
+          for (int i = 0; i < d.ep.n; ++i) {
+            const cvmk_ep_step& st = d.ep.s[i];
+            if ((st.op == CVMK_EP_ADD_T || st.op == CVMK_EP_SUB_T || st.op == CVMK_EP_RSUB_T) && st.ptr) aligned &= out_first * st.ptr_dtype % 16 == 0;
+          }
+        }
+        for (const Range& r : aligned ? parts : std::vector<Range>()) {
           const size_t first = (size_t)(r.begin * per_image / fold);
           cvmk_conv_desc cd = d;
           cd.N = (int)((r.end - r.begin) * per_image / fold);

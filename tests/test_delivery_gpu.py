@@ -99,3 +99,17 @@ def test_head_in_parts(batch, channels, size, rt, wl, oracle):
                     assert np.array_equal(dst.numpy(), want)
     finally:
         rt.CVMAPIFreeModel(net)
+
+
+# layers whose parts of the batch would not start on 16 bytes (odd images of 8 or 24 channels) are not cut
+@pytest.mark.parametrize("oc", [8, 24, 40])
+@pytest.mark.parametrize("batch", [8, 9, 15])
+def test_parts_that_do_not_align(oc, batch, gpu_run, wl, oracle):
+    g = wl.GraphBuilder(oc)
+    d = g.var("data", (batch, 3, 37, 37), 8)
+    y = g.conv(d, 32, 3, 2, 1)
+    y = g.conv(y, oc, 3, 1, 1)
+    y = g.max_pool(y, 3, 2, 1)
+    js, pb = g.finish(g.conv(y, oc, 1, 1, 0, relu=False))
+    x = np.random.RandomState(batch).randint(-128, 128, size=(batch, 3, 37, 37)).astype(np.int8)
+    assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
