@@ -2083,10 +2083,20 @@ void Executor::DeliverPieces() {
 }
 
 // The head is in page-locked memory (and the GPU idle): into the caller's buffer.
-void Executor::DeliverHead(char* out) {
+void Executor::DeliverHead(char* out, HostPool* awake) {
   const HeadOut& h = heads_[0];
   if (!h.live_bytes) {
-    memcpy(out, h.host, h.bytes);
+    if (!awake || h.bytes < kSmallShare) {
+      memcpy(out, h.host, h.bytes);
+      return;
+    }
+    const char* src = (const char*)h.host;
+    const size_t bytes = h.bytes, pieces = (bytes + kSmallPiece - 1) / kSmallPiece;
+    awake->Start(HostPool::kDownload, pieces, pieces, [=](size_t k) {
+      const size_t off = k * kSmallPiece;
+      memcpy(out + off, src + off, std::min(kSmallPiece, bytes - off));
+    });
+    awake->Finish(HostPool::kDownload);
     return;
   }
   const size_t image = h.bytes / h.images, live = h.live_bytes;
@@ -2182,13 +2192,15 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
     }
     CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
     if (head) QueuePieces(head, heads_[0].bytes, stream_);
-    // calls that follow one another closely: the helpers wake up for the next one while the GPU works
-    if (share && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) {
-      guard.p = &pool();
-      guard.p->Begin();
-    }
   } else {
     Launch(input, src, on_device ? from_device_ : (src == Source::kDirect ? from_pinned_ : from_pageable_), head);
+  }
+  // calls that follow one another closely: the helpers wake up while the GPU works, for the head and for
+  // the next call's input
+  const bool worth = (src == Source::kSmall && in_bytes_ >= kSmallShare) || (signal && plain_ && heads_[0].bytes >= kSmallShare);
+  if (worth && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) {
+    guard.p = &pool();
+    guard.p->Begin();
   }
   if (pieces) DeliverPieces();
   else if (signal) AwaitDone();
@@ -2200,7 +2212,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
     cudaStreamSynchronize(stream_);
     FATAL() << "a device-side wait ran out (status word 0x" << std::hex << code << ")";
   }
-  if (plain_ && !pieces) DeliverHead(out);
+  if (plain_ && !pieces) DeliverHead(out, guard.p);
   last_call_ = std::chrono::steady_clock::now();
 }
 

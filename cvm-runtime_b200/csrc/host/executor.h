@@ -92,8 +92,8 @@ class Executor {
   std::vector<Step> steps_;
   enum class Source { kDirect, kSmall, kPool };   // read where it lies; staged by the caller; staged by the pool
   static constexpr size_t kSmallInput = (size_t)1 << 20, kSmallDirect = (size_t)1 << 18;
-  // A small input of at least kSmallShare is staged together with the pool's helpers if they are awake
-  // (547 KB 166 -> 150 us a call, 150 KB 224.4 -> 222.8); asleep, waking them costs more than that.
+  // A small input (or head) of at least kSmallShare is copied together with the pool's helpers if they are
+  // awake (547 KB 166 -> 150 us a call, 150 KB 224.4 -> 222.8); asleep, waking them costs more than that.
   static constexpr size_t kSmallShare = (size_t)64 << 10, kSmallPiece = (size_t)32 << 10;
   static constexpr size_t kStagePiece = (size_t)256 << 10, kDownloadPiece = (size_t)1 << 20;
   // An inference: the first `prefix` steps part by part, one graph per part of the batch, each launched
@@ -164,7 +164,7 @@ class Executor {
   void QueuePieces(char* head, size_t bytes, cudaStream_t s);
   void PollPieces();
   void DeliverPieces();
-  void DeliverHead(char* out);
+  void DeliverHead(char* out, HostPool* awake);
 
   void* dalloc(size_t bytes);
   // Activation memory.  Every activation buffer gets a virtual address range of its own when the
