@@ -1795,17 +1795,14 @@ void Executor::ChooseSchedules() {
       Schedule s = MakeSchedule(prefix, cut);
       double best = 1e30;
       for (int rep = 0; rep < 4; ++rep) {   // the first is a warm-up
-        if (src == Source::kPool) pool().Begin();
+        HostPool::Use helpers;
+        if (src == Source::kPool) helpers.Begin(pool());
         const auto t0 = std::chrono::steady_clock::now();
         BeginUpload(input, src);
         Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr);
         CUDA_OK(cudaStreamSynchronize(stream_));
         if (down_stream_) CUDA_OK(cudaStreamSynchronize(down_stream_));
         const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-        if (src == Source::kPool) {
-          pool().Finish(HostPool::kUpload);
-          pool().End();
-        }
         if (rep > 0) best = std::min(best, t);
       }
       DropSchedule(&s);
@@ -1906,6 +1903,15 @@ HostPool& Executor::pool() {
   return *pool_;
 }
 
+// After an error: waits for what is queued, so that no copy engine or kernel reads or writes the caller's
+// buffers (or the staging buffers of the next call) once the error has been reported.
+void Executor::Settle() {
+  for (cudaStream_t s : {copy_stream_, stream_, down_stream_})
+    if (s) cudaStreamSynchronize(s);
+  cudaGetLastError();
+  queued_pieces_ = arrived_pieces_ = deliver_units_ = 0;
+}
+
 void Executor::BeginUpload(const void* input, Source src) {
   if (src != Source::kPool) return;
   const char* from = (const char*)input;
@@ -1939,13 +1945,10 @@ void Executor::SendRange(const void* input, Source src, size_t begin, size_t byt
 
 void Executor::Upload(const void* input, cudaStream_t s) {
   const Source src = SourceOf(input);
-  if (src == Source::kPool) pool().Begin();
+  HostPool::Use helpers;
+  if (src == Source::kPool) helpers.Begin(pool());
   BeginUpload(input, src);
   SendRange(input, src, 0, in_bytes_, s);
-  if (src == Source::kPool) {
-    pool().Finish(HostPool::kUpload);
-    pool().End();
-  }
 }
 
 // Heads of up to 1 MiB in all (256 KiB when they go out as they are: one thread's copy of the rest would
@@ -2150,24 +2153,21 @@ void Executor::Launch(const void* input, Source src, const Schedule& how, char* 
 void Executor::Run(const void* input, size_t input_bytes, char* out) {
   CHECK(input_bytes == in_bytes_) << "input size " << input_bytes << " vs. " << in_bytes_;
   CUDA_OK(cudaSetDevice(device_));
+  try {
+    RunOnce(input, out);
+  } catch (...) {
+    Settle();
+    throw;
+  }
+}
+
+void Executor::RunOnce(const void* input, char* out) {
   const auto called = std::chrono::steady_clock::now();
   const Source src = SourceOf(input);
   const bool on_device = src == Source::kDirect && IsDevice(input);
   const bool fill = plain_ && heads_[0].live_bytes > 0, pieces = plain_ && download_ == Download::kPieces;
-  // Whatever way this ends, no helper touches the caller's buffers afterwards.
-  struct PoolGuard {
-    HostPool* p = nullptr;
-    ~PoolGuard() {
-      if (!p) return;
-      p->ReleaseAll(HostPool::kDownload);   // (when an error ends this early)
-      for (int k = 0; k < HostPool::kSlots; ++k) p->Finish((HostPool::Slot)k);
-      p->End();
-    }
-  } guard;
-  if (src == Source::kPool || fill || pieces) {
-    guard.p = &pool();
-    guard.p->Begin();
-  }
+  HostPool::Use guard;
+  if (src == Source::kPool || fill || pieces) guard.Begin(pool());
   const bool signal = download_ == Download::kKernel;
   if (signal) *(volatile int32_t*)done_host_ = 0;
   BeginUpload(input, src);
@@ -2177,8 +2177,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
   if (src == Source::kSmall && graph_staged_) {
     const bool share = in_bytes_ >= kSmallShare;
     if (share && pool_ && pool_->awake()) {
-      guard.p = pool_.get();
-      guard.p->Begin();
+      guard.Begin(*pool_);
       const char* from = (const char*)input;
       char* to = (char*)in_host_;
       const size_t bytes = in_bytes_, pieces = (bytes + kSmallPiece - 1) / kSmallPiece;
@@ -2198,10 +2197,7 @@ void Executor::Run(const void* input, size_t input_bytes, char* out) {
   // calls that follow one another closely: the helpers wake up while the GPU works, for the head and for
   // the next call's input
   const bool worth = (src == Source::kSmall && in_bytes_ >= kSmallShare) || (signal && plain_ && heads_[0].bytes >= kSmallShare);
-  if (worth && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) {
-    guard.p = &pool();
-    guard.p->Begin();
-  }
+  if (worth && !guard.p && called - last_call_ < std::chrono::microseconds(HostPool::kLingerUs)) guard.Begin(pool());
   if (pieces) DeliverPieces();
   else if (signal) AwaitDone();
   else CUDA_OK(cudaStreamSynchronize(stream_));
@@ -2257,13 +2253,18 @@ std::vector<std::pair<std::string, float>> Executor::ProfileOnce(const void* inp
   std::vector<std::pair<std::string, float>> out;
   std::vector<cudaEvent_t> ev(steps_.size() + 1);
   for (auto& e : ev) CUDA_OK(cudaEventCreate(&e));
-  Upload(input, stream_);
-  CUDA_OK(cudaEventRecord(ev[0], stream_));
-  for (size_t i = 0; i < steps_.size(); ++i) {
-    KERNEL_OK(steps_[i].launch(stream_));
-    CUDA_OK(cudaEventRecord(ev[i + 1], stream_));
+  try {
+    Upload(input, stream_);
+    CUDA_OK(cudaEventRecord(ev[0], stream_));
+    for (size_t i = 0; i < steps_.size(); ++i) {
+      KERNEL_OK(steps_[i].launch(stream_));
+      CUDA_OK(cudaEventRecord(ev[i + 1], stream_));
+    }
+    CUDA_OK(cudaStreamSynchronize(stream_));
+  } catch (...) {
+    Settle();
+    throw;
   }
-  CUDA_OK(cudaStreamSynchronize(stream_));
   for (size_t i = 0; i < steps_.size(); ++i) {
     float ms = 0;
     CUDA_OK(cudaEventElapsedTime(&ms, ev[i], ev[i + 1]));

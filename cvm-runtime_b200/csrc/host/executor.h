@@ -143,6 +143,8 @@ class Executor {
   std::vector<cudaEvent_t> part_done_;
   int32_t* done_host_ = nullptr;    // pinned: the last kernel of an inference has delivered the heads
   void AwaitDone();
+  void RunOnce(const void* input, char* out);
+  void Settle();
   std::chrono::steady_clock::time_point last_call_;   // the end of the last inference
   std::unique_ptr<HostPool> pool_;   // created by the first inference that has enough bytes to move
   HostPool& pool();

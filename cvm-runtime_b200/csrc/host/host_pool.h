@@ -44,6 +44,27 @@ class HostPool {
   // Runs one piece of any job, if one is free; false if there is none.
   bool HelpOnce();
 
+  // Helpers at work, until it goes out of scope: whatever way that comes about, all jobs have run by then
+  // and none touches the buffers of their bodies afterwards.
+  struct Use {
+    HostPool* p = nullptr;
+    Use() = default;
+    Use(const Use&) = delete;
+    Use& operator=(const Use&) = delete;
+    void Begin(HostPool& pool) {
+      p = &pool;
+      p->Begin();
+    }
+    ~Use() {
+      if (!p) return;
+      for (int k = 0; k < kSlots; ++k) {
+        p->ReleaseAll((Slot)k);   // (pieces that an error kept back)
+        p->Finish((Slot)k);
+      }
+      p->End();
+    }
+  };
+
   static constexpr int kLingerUs = 200;
   bool awake() const { return asleep_.load(std::memory_order_relaxed) == 0; }   // Begin() needs no wake-up
 

@@ -1,0 +1,73 @@
+/* Drives the C-ABI of the host runtime over the fake device.
+ *   executor_host fail_run  early|late in out   every call of an inference that can fail does, one at a time
+ * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
+ * params.bin and input.bin of the working directory, writes the bytes of the last good inference to
+ * output.bin and prints "@name=value" lines.
+ */
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <fstream>
+#include <iterator>
+#include <string>
+#include <vector>
+#include "cvm/c_api.h"
+#include "cvm/c_api_ext.h"
+#include "fake_device.h"
+
+static std::string slurp(const char* path) {
+  std::ifstream f(path, std::ios::binary);
+  return std::string(std::istreambuf_iterator<char>(f), std::istreambuf_iterator<char>());
+}
+static char* buffer(const std::string& kind, size_t n) {
+  void* p = nullptr;
+  if (kind == "pinned") cudaMallocHost(&p, n);
+  else p = malloc(n);
+  return (char*)p;
+}
+
+int main(int argc, char** argv) {
+  if (argc < 5) return 2;
+  const std::string mode = argv[1], graph = slurp("graph.json"), params = slurp("params.bin"), input = slurp("input.bin");
+  fake::late = std::string(argv[2]) == "late";
+  auto load = [&](void** net) { return CVMAPILoadModel(graph.data(), (int)graph.size(), params.data(), (int)params.size(), net, 1, 0); };
+  void* net = nullptr;
+  if (load(&net) != 0) return 3;
+  unsigned long long bytes = 0;
+  CVMAPIGetOutputLength(net, &bytes);
+  char* in = buffer(argv[3], input.size());
+  char* out = buffer(argv[4], bytes);
+  memcpy(in, input.data(), input.size());
+  auto infer = [&] { return CVMAPIInference(net, in, (int)input.size(), out); };
+
+  if (mode == "fail_run") {
+    long failed = 0, in_flight = 0, wrong_after = 0;
+    for (long n = 1;; ++n) {
+      fake::reset_calls(n);
+      const int status = infer();
+      const bool reached = fake::calls >= n;
+      const size_t pending = fake::pending();
+      fake::reset_calls(0);
+      if (!reached) { printf("@last_status=%d\n", status); break; }
+      failed += status == 2;
+      in_flight += status != 0 && pending > 0;
+      memset(out, 0x55, bytes);
+      if (infer() != 0 || (bytes == input.size() && memcmp(out, input.data(), bytes))) ++wrong_after;
+    }
+    // the same through the per-step profile, which uploads the caller's input too
+    for (long n = 1;; ++n) {
+      static char text[1 << 16];
+      fake::reset_calls(n);
+      const int status = CVMXProfileSteps(net, in, (int)input.size(), text, sizeof(text));
+      const bool reached = fake::calls >= n;
+      in_flight += status != 0 && fake::pending() > 0;
+      fake::reset_calls(0);
+      if (!reached) break;
+    }
+    printf("@failed=%ld @in_flight=%ld @wrong_after=%ld\n", failed, in_flight, wrong_after);
+  }
+  std::ofstream("output.bin", std::ios::binary).write(out, (std::streamsize)bytes);
+  CVMAPIFreeModel(net);
+  return 0;
+}

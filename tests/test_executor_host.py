@@ -1,0 +1,73 @@
+"""The executor's host logic on a device made of host memory (tests/executor_host/fake_device.cc): what
+happens to the caller's buffers, to queued transfers and to memory when a call fails on the way.
+
+The host sources of the library are compiled against the fake with the address sanitizer, so that a helper
+or a queued copy that touches memory that is gone ends the program.
+"""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+SRC = os.path.join(HERE, "executor_host")
+OUT = os.path.join(SRC, "build")
+BIN = os.path.join(OUT, "executor_host")
+HOST = os.path.join(ROOT, "cvm-runtime_b200", "csrc", "host")
+CUDA = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    if shutil.which("g++") is None or not os.path.exists(os.path.join(CUDA, "cuda_runtime.h")):
+        pytest.skip("no host compiler or CUDA headers")
+    srcs = [os.path.join(HOST, f) for f in ("ops.cc", "graph.cc", "host_pool.cc", "executor.cc", "c_api.cc")]
+    srcs += [os.path.join(SRC, f) for f in ("fake_device.cc", "main.cc")]
+    inc = os.path.join(ROOT, "include")
+    headers = [os.path.join(d, f) for d in (HOST, SRC, inc, os.path.join(inc, "cvm")) for f in os.listdir(d) if f.endswith(".h")]
+    newest = max(os.path.getmtime(h) for h in headers)
+    os.makedirs(OUT, exist_ok=True)
+    objs, procs = [], []
+    flags = ["-std=c++17", "-O0", "-g1", "-fsanitize=address", "-pthread", "-I" + CUDA, "-I" + inc, "-I" + HOST]
+    for s in srcs:
+        o = os.path.join(OUT, os.path.basename(s) + ".o")
+        objs.append(o)
+        if not os.path.exists(o) or os.path.getmtime(o) < max(os.path.getmtime(s), newest):
+            procs.append(subprocess.Popen(["g++"] + flags + ["-c", s, "-o", o]))
+    assert all(p.wait() == 0 for p in procs)
+    if procs or not os.path.exists(BIN):
+        subprocess.check_call(["g++", "-fsanitize=address", "-pthread"] + objs + ["-o", BIN])
+
+    def run(work, *args):
+        env = dict(os.environ, ASAN_OPTIONS="detect_leaks=0:alloc_dealloc_mismatch=0")
+        p = subprocess.run([BIN] + [str(a) for a in args], cwd=work, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True,
+                           env=env, timeout=300)
+        assert p.returncode == 0, p.stderr[-4000:]
+        return dict(tok[1:].split("=", 1) for tok in p.stdout.split() if tok.startswith("@"))
+    return run
+
+
+def put(path, js, pb, x):
+    for name, data in (("graph.json", js.encode() if isinstance(js, str) else js), ("params.bin", pb), ("input.bin", x.tobytes())):
+        with open(os.path.join(path, name), "wb") as f:
+            f.write(data)
+
+
+def chain(wl, batch):   # on the fake device the result is the input; 2 MiB at batch 8: staged, cut into parts, leaves in pieces
+    return wl.conv_chain(batch=batch, channels=64, size=64)
+
+
+@pytest.mark.parametrize("when", ["late", "early"])
+@pytest.mark.parametrize("src,dst", [("pageable", "pageable"), ("pinned", "pinned"), ("pageable", "pinned"), ("pinned", "pageable")])
+@pytest.mark.parametrize("batch", [1, 8])
+def test_a_failing_call_leaves_no_transfer_behind(when, src, dst, batch, host, wl, tmp_path):
+    js, pb, x = chain(wl, batch)
+    put(tmp_path, js, pb, x)
+    f = host(tmp_path, "fail_run", when, src, dst)
+    assert int(f["failed"]) > 0 and f["last_status"] == "0"
+    assert f["in_flight"] == "0"      # nothing queued that reads the input or writes the output
+    assert f["wrong_after"] == "0"    # the handle answers the next call
+    assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int8), x.reshape(-1))
