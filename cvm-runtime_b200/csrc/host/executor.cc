@@ -1799,7 +1799,7 @@ void Executor::ChooseSchedules() {
         if (src == Source::kPool) helpers.Begin(pool());
         const auto t0 = std::chrono::steady_clock::now();
         BeginUpload(input, src);
-        Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr);
+        Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr, true);
         CUDA_OK(cudaStreamSynchronize(stream_));
         if (down_stream_) CUDA_OK(cudaStreamSynchronize(down_stream_));
         const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -2121,8 +2121,8 @@ void Executor::DeliverHead(char* out, HostPool* awake) {
 // leaves in pieces (null otherwise).  When all of the graph runs part by part, the head's part follows each on a
 // stream of its own: both directions of the link and the kernels then work at the same time (64 images of
 // 64 -> 64 channels at 56 x 56, 12.8 MB each way: 607 -> 465 us from page-locked memory, 374 -> 346 from the
-// device's own).
-void Executor::Launch(const void* input, Source src, const Schedule& how, char* head) {
+// device's own).  Without `early` the head leaves after all of the input has been read.
+void Executor::Launch(const void* input, Source src, const Schedule& how, char* head, bool early) {
   queued_pieces_ = arrived_pieces_ = 0;
   if (how.prefix == 0) {
     SendRange(input, src, 0, in_bytes_, stream_);
@@ -2131,7 +2131,7 @@ void Executor::Launch(const void* input, Source src, const Schedule& how, char* 
     if (head) QueuePieces(head, heads_[0].bytes, stream_);
     return;
   }
-  const bool parts_leave = head && how.prefix == steps_.size() && !head_range_end_.empty();
+  const bool parts_leave = early && head && how.prefix == steps_.size() && !head_range_end_.empty();
   size_t begin = 0;
   for (size_t c = 0; c < how.graphs.size(); ++c) {
     const int r = kCuts[how.cut][c];
@@ -2171,7 +2171,10 @@ void Executor::RunOnce(const void* input, char* out) {
   const bool signal = download_ == Download::kKernel;
   if (signal) *(volatile int32_t*)done_host_ = 0;
   BeginUpload(input, src);
-  if (fill) StartFill(out);
+  // a caller may have its result where its input is: then nothing is written before all of that is read
+  const uintptr_t in_at = (uintptr_t)input, out_at = (uintptr_t)out;
+  const bool apart = in_at + in_bytes_ <= out_at || (plain_ && out_at + heads_[0].bytes <= in_at);
+  if (fill && apart) StartFill(out);
   if (pieces) StartDelivery(out);
   char* const head = !pieces ? nullptr : (deliver_units_ ? (char*)heads_[0].host : out);   // where the copy engine writes
   if (src == Source::kSmall && graph_staged_) {
@@ -2192,7 +2195,7 @@ void Executor::RunOnce(const void* input, char* out) {
     CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
     if (head) QueuePieces(head, heads_[0].bytes, stream_);
   } else {
-    Launch(input, src, on_device ? from_device_ : (src == Source::kDirect ? from_pinned_ : from_pageable_), head);
+    Launch(input, src, on_device ? from_device_ : (src == Source::kDirect ? from_pinned_ : from_pageable_), head, apart);
   }
   // calls that follow one another closely: the helpers wake up while the GPU works, for the head and for
   // the next call's input
@@ -2208,6 +2211,7 @@ void Executor::RunOnce(const void* input, char* out) {
     cudaStreamSynchronize(stream_);
     FATAL() << "a device-side wait ran out (status word 0x" << std::hex << code << ")";
   }
+  if (fill && !apart) StartFill(out);
   if (plain_ && !pieces) DeliverHead(out, guard.p);
   last_call_ = std::chrono::steady_clock::now();
 }

@@ -117,7 +117,7 @@ class Executor {
   static void DropSchedule(Schedule* s);
   cudaGraphExec_t Capture(const std::function<void()>& enqueue);
   void ChooseSchedules();
-  void Launch(const void* input, Source src, const Schedule& how, char* head);
+  void Launch(const void* input, Source src, const Schedule& how, char* head, bool early);
   static bool IsDirect(const void* input);
   static bool IsDevice(const void* input);
   std::vector<size_t> range_end_;   // input bytes up to the end of each range of images that steps are prepared for

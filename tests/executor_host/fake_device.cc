@@ -1,13 +1,14 @@
 /* A device made of host memory, for tests of the executor's host logic: the CUDA runtime calls and the
  * kernel launchers it uses, with streams, events and graphs whose work runs when the host waits for it
  * (or at once), and any call made to fail on demand.  "Kernels" only move bytes: a convolution of as
- * many outputs as inputs copies them, get_valid_counts keeps every row, non_max_suppression the first ones.
+ * many outputs as inputs copies them, get_valid_counts keeps every row, non_max_suppression the last ones.
  */
 #include "fake_device.h"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
@@ -15,6 +16,7 @@
 #include <map>
 #include <mutex>
 #include <set>
+#include <thread>
 #include <vector>
 #include "cvmk_kernels.h"
 
@@ -23,6 +25,7 @@ namespace fake {
 bool late = true;
 long fail_at = 0, calls = 0, conv_plans = 0;
 size_t memory_limit = 0, device_bytes = 0;
+int slow_images = 0;
 
 namespace {
 
@@ -88,6 +91,9 @@ int launch(cvmk_stream_t s, std::function<void()> f) {
   if (fails()) return CVMK_ERR_CUDA;
   work(s, std::move(f));
   return CVMK_OK;
+}
+void images(int64_t n) {
+  if (slow_images && n >= slow_images) std::this_thread::sleep_for(std::chrono::milliseconds(2));
 }
 int nothing(cvmk_stream_t s) { return launch(s, [] {}); }
 
@@ -255,7 +261,10 @@ int cvmk_elemwise(const void* x, int xd, void* y, int yd, int64_t n, const cvmk_
 }
 int cvmk_transpose_batched(const void* x, void* y, int32_t dtype, int64_t batch, int32_t rows, int32_t cols, int32_t, int32_t, int32_t,
                            cvmk_stream_t s) {
-  return launch(s, [=] { memcpy(y, x, (size_t)dtype * batch * rows * cols); });
+  return launch(s, [=] {
+    memcpy(y, x, (size_t)dtype * batch * rows * cols);
+    images(batch);
+  });
 }
 int cvmk_export(const cvmk_export_segment* seg, int32_t n, cvmk_stream_t s) {
   const std::vector<cvmk_export_segment> v(seg, seg + n);
@@ -276,7 +285,10 @@ int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* plan) {
 int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s) {
   const cvmk_conv_desc d = plan->d;
   const size_t in = (size_t)d.N * d.H * d.W * d.C, out = (size_t)d.N * d.OH * d.OW * d.OC * d.y_dtype;
-  return launch(s, [=] { if (in == out) memcpy(d.y, d.x, out); });
+  return launch(s, [=] {
+    if (in == out) memcpy(d.y, d.x, out);
+    images(d.N);
+  });
 }
 int cvmk_conv2d_direct(const cvmk_conv_direct_desc*, cvmk_stream_t s) { return nothing(s); }
 int cvmk_conv2d_stem_supported(const cvmk_stem_conv_desc*) { return 1; }
@@ -310,7 +322,7 @@ int cvmk_non_max_suppression_part(const cvmk_nms_desc* p, int32_t first, int32_t
     for (int32_t b = first; b < first + n; ++b) {
       const size_t at = (size_t)b * d.N * 6;
       memset(d.y + at, 0xff, (size_t)d.N * 24);
-      memcpy(d.y + at, d.x + at, rows * 24);
+      memcpy(d.y + at, d.x + at + (d.N - rows) * 6, rows * 24);
     }
   });
 }

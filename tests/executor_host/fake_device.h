@@ -13,6 +13,10 @@ extern long fail_at, calls;
 extern size_t memory_limit;
 extern size_t device_bytes;
 
+// A convolution or change of layout over at least so many images takes milliseconds (0: none), so that the timing
+// at load prefers to run a batch of that size in parts.
+extern int slow_images;
+
 void reset_calls(long fail);
 size_t pending();         // operations queued and not yet run, over all streams
 size_t live_objects();    // allocations, streams, events and graphs that exist

@@ -1,10 +1,12 @@
 /* Drives the C-ABI of the host runtime over the fake device.
  *   executor_host fail_run  early|late in out   every call of an inference that can fail does, one at a time
+ *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
  * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
- * params.bin and input.bin of the working directory, writes the bytes of the last good inference to
+ * params.bin and input.bin of the working directory, fake::slow_images of the environment (SLOW_IMAGES), writes the bytes of the last good inference to
  * output.bin and prints "@name=value" lines.
  */
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -32,6 +34,7 @@ int main(int argc, char** argv) {
   const std::string mode = argv[1], graph = slurp("graph.json"), params = slurp("params.bin"), input = slurp("input.bin");
   fake::late = std::string(argv[2]) == "late";
   auto load = [&](void** net) { return CVMAPILoadModel(graph.data(), (int)graph.size(), params.data(), (int)params.size(), net, 1, 0); };
+  if (const char* n = getenv("SLOW_IMAGES")) fake::slow_images = atoi(n);
   void* net = nullptr;
   if (load(&net) != 0) return 3;
   unsigned long long bytes = 0;
@@ -41,6 +44,14 @@ int main(int argc, char** argv) {
   memcpy(in, input.data(), input.size());
   auto infer = [&] { return CVMAPIInference(net, in, (int)input.size(), out); };
 
+  if (mode == "in_place") {
+    free(out);
+    const size_t ahead = (size_t)atoll(argv[4]);
+    in = buffer(argv[3], std::max<size_t>(input.size(), ahead + bytes));
+    memcpy(in, input.data(), input.size());
+    out = in + ahead;
+    printf("@status=%d\n", infer());
+  }
   if (mode == "fail_run") {
     long failed = 0, in_flight = 0, wrong_after = 0;
     for (long n = 1;; ++n) {

@@ -41,8 +41,8 @@ def host(tmp_path_factory):
     if procs or not os.path.exists(BIN):
         subprocess.check_call(["g++", "-fsanitize=address", "-pthread"] + objs + ["-o", BIN])
 
-    def run(work, *args):
-        env = dict(os.environ, ASAN_OPTIONS="detect_leaks=0:alloc_dealloc_mismatch=0")
+    def run(work, *args, slow_images=0):
+        env = dict(os.environ, SLOW_IMAGES=str(slow_images), ASAN_OPTIONS="detect_leaks=0:alloc_dealloc_mismatch=0")
         p = subprocess.run([BIN] + [str(a) for a in args], cwd=work, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True,
                            env=env, timeout=300)
         assert p.returncode == 0, p.stderr[-4000:]
@@ -66,8 +66,26 @@ def chain(wl, batch):   # on the fake device the result is the input; 2 MiB at b
 def test_a_failing_call_leaves_no_transfer_behind(when, src, dst, batch, host, wl, tmp_path):
     js, pb, x = chain(wl, batch)
     put(tmp_path, js, pb, x)
-    f = host(tmp_path, "fail_run", when, src, dst)
+    f = host(tmp_path, "fail_run", when, src, dst, slow_images=8)   # (batch 8: runs in parts)
     assert int(f["failed"]) > 0 and f["last_status"] == "0"
     assert f["in_flight"] == "0"      # nothing queued that reads the input or writes the output
     assert f["wrong_after"] == "0"    # the handle answers the next call
     assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int8), x.reshape(-1))
+
+
+# The caller's input and output may overlap, as with the reference, which copies the input before it computes:
+# nothing is written there before the whole input is on the device.
+@pytest.mark.parametrize("when", ["late", "early"])
+@pytest.mark.parametrize("src", ["pageable", "pinned"])
+@pytest.mark.parametrize("ahead", [0, 300000])
+def test_output_over_the_input(when, src, ahead, host, wl, tmp_path):
+    js, pb, x = chain(wl, 9)
+    put(tmp_path, js, pb, x)
+    assert host(tmp_path, "in_place", when, src, ahead, slow_images=9)["status"] == "0"
+    assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int8), x.reshape(-1))
+    js, pb, x = wl.ssd_tail(batch=9, anchors=1500, top_k=100)
+    put(tmp_path, js, pb, x)
+    assert host(tmp_path, "in_place", when, src, ahead)["status"] == "0"
+    want = np.full(x.shape, -1, np.int32)
+    want[:, :100] = x[:, -100:]   # (what the fake device's operators do)
+    assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int32), want.reshape(-1))
