@@ -1680,10 +1680,20 @@ struct Lowering {
   bool cut_like_first(const Step& s) const { return s.chunk.size() == ex.range_end_.size() && s.images == ex.steps_[0].images; }
 };
 
+// (a constructor that throws has no destructor: what it had made by then is given back here)
 Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g), device_(device_id) {
+  try {
+    Load(plain_elem_bytes);
+  } catch (...) {
+    Release();
+    throw;
+  }
+}
+
+void Executor::Load(int plain_elem_bytes) {
   int count = 0;
   CUDA_OK(cudaGetDeviceCount(&count));
-  CHECK(device_id >= 0 && device_id < count) << "device_id " << device_id << " out of range (" << count << " GPUs)";
+  CHECK(device_ >= 0 && device_ < count) << "device_id " << device_ << " out of range (" << count << " GPUs)";
   CUDA_OK(cudaSetDevice(device_));
   CUDA_OK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   status_dev_ = (int32_t*)dalloc(256);
@@ -1702,7 +1712,7 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
       vmm_gran_ = gran;
     }
   }
-  Lowering low(*this, g);
+  Lowering low(*this, g_);
   low.run();
   plain_ = heads_.size() == 1 && heads_[0].dtype == plain_elem_bytes;
   if (!plain_)
@@ -1736,16 +1746,22 @@ Executor::Executor(const Graph& g, int device_id, int plain_elem_bytes) : g_(g),
     });
 }
 
-cudaGraphExec_t Executor::Capture(const std::function<void()>& enqueue) {
+Executor::GraphExec Executor::Capture(const std::function<void()>& enqueue) {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   CUDA_OK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  enqueue();
+  try {
+    enqueue();
+  } catch (...) {
+    if (cudaStreamEndCapture(stream_, &graph) == cudaSuccess) cudaGraphDestroy(graph);
+    cudaGetLastError();
+    throw;
+  }
   CUDA_OK(cudaStreamEndCapture(stream_, &graph));
   const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   CUDA_OK(e);
-  return exec;
+  return GraphExec(exec);
 }
 
 Executor::Schedule Executor::MakeSchedule(size_t prefix, int cut) {
@@ -1759,12 +1775,6 @@ Executor::Schedule Executor::MakeSchedule(size_t prefix, int cut) {
       if (r == kCuts[cut].back()) Enqueue(stream_, prefix);
     }));
   return s;
-}
-
-void Executor::DropSchedule(Schedule* s) {
-  for (auto g : s->graphs) cudaGraphExecDestroy(g);
-  s->graphs.clear();
-  s->prefix = 0;
 }
 
 bool Executor::IsDevice(const void* input) {
@@ -1794,18 +1804,22 @@ void Executor::ChooseSchedules() {
     auto time_of = [&](size_t prefix, int cut) {
       Schedule s = MakeSchedule(prefix, cut);
       double best = 1e30;
-      for (int rep = 0; rep < 4; ++rep) {   // the first is a warm-up
-        HostPool::Use helpers;
-        if (src == Source::kPool) helpers.Begin(pool());
-        const auto t0 = std::chrono::steady_clock::now();
-        BeginUpload(input, src);
-        Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr, true);
-        CUDA_OK(cudaStreamSynchronize(stream_));
-        if (down_stream_) CUDA_OK(cudaStreamSynchronize(down_stream_));
-        const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-        if (rep > 0) best = std::min(best, t);
+      try {
+        for (int rep = 0; rep < 4; ++rep) {   // the first is a warm-up
+          HostPool::Use helpers;
+          if (src == Source::kPool) helpers.Begin(pool());
+          const auto t0 = std::chrono::steady_clock::now();
+          BeginUpload(input, src);
+          Launch(input, src, s, download_ == Download::kPieces ? (char*)heads_[0].host : nullptr, true);
+          CUDA_OK(cudaStreamSynchronize(stream_));
+          if (down_stream_) CUDA_OK(cudaStreamSynchronize(down_stream_));
+          const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+          if (rep > 0) best = std::min(best, t);
+        }
+      } catch (...) {
+        Settle();   // (the input of these timings is about to go)
+        throw;
       }
-      DropSchedule(&s);
       return best;
     };
     std::map<std::pair<size_t, int>, double> seen;
@@ -1846,29 +1860,33 @@ void Executor::ChooseSchedules() {
     return MakeSchedule(b.first, b.second);
   };
   if (!head_range_end_.empty()) {
+    // (an input to time with; where there is no room for it, such inputs go through the whole graph)
     void* dev = nullptr;
-    CUDA_OK(cudaMalloc(&dev, in_bytes_));
-    CUDA_OK(cudaMemset(dev, 0, in_bytes_));
-    CUDA_OK(cudaDeviceSynchronize());
-    from_device_ = choose(dev);
-    CUDA_OK(cudaFree(dev));
+    if (cudaMalloc(&dev, in_bytes_) == cudaSuccess) {
+      const std::unique_ptr<void, cudaError_t (*)(void*)> hold(dev, cudaFree);
+      CUDA_OK(cudaMemset(dev, 0, in_bytes_));
+      CUDA_OK(cudaDeviceSynchronize());
+      from_device_ = choose(dev);
+    } else {
+      cudaGetLastError();
+    }
   }
   from_pinned_ = choose(in_host_);
   if (in_bytes_ > kSmallInput) from_pageable_ = choose(pageable.data());
 }
 
-Executor::~Executor() {
+Executor::~Executor() { Release(); }
+
+void Executor::Release() {
   cudaSetDevice(device_);
-  if (stream_) cudaStreamSynchronize(stream_);
-  DropSchedule(&from_pinned_);
-  DropSchedule(&from_pageable_);
-  DropSchedule(&from_device_);
-  if (graph_whole_) cudaGraphExecDestroy(graph_whole_);
-  if (graph_staged_) cudaGraphExecDestroy(graph_staged_);
-  if (kernels_exec_) cudaGraphExecDestroy(kernels_exec_);
-  for (auto e : piece_events_) cudaEventDestroy(e);
-  for (auto e : part_events_) cudaEventDestroy(e);
-  for (auto e : part_done_) cudaEventDestroy(e);
+  Settle();
+  for (Schedule* s : {&from_pinned_, &from_pageable_, &from_device_}) s->graphs.clear();
+  graph_whole_.reset();
+  graph_staged_.reset();
+  kernels_exec_.reset();
+  for (auto* events : {&piece_events_, &part_events_, &part_done_})
+    for (auto e : *events)
+      if (e) cudaEventDestroy(e);
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
   if (down_stream_) cudaStreamDestroy(down_stream_);
   for (void* p : allocs_) cudaFree(p);
@@ -1879,6 +1897,7 @@ Executor::~Executor() {
   for (auto& b : phys_) vmm().release((CUmemGenericAllocationHandle)b.handle);
   for (void* p : pinned_) cudaFreeHost(p);
   if (stream_) cudaStreamDestroy(stream_);
+  cudaGetLastError();
 }
 
 // Where the bytes of an input come from.  Page-locked (or device) memory is read where it lies.  A
@@ -2126,7 +2145,7 @@ void Executor::Launch(const void* input, Source src, const Schedule& how, char* 
   queued_pieces_ = arrived_pieces_ = 0;
   if (how.prefix == 0) {
     SendRange(input, src, 0, in_bytes_, stream_);
-    if (graph_whole_) CUDA_OK(cudaGraphLaunch(graph_whole_, stream_));
+    if (graph_whole_) CUDA_OK(cudaGraphLaunch(graph_whole_.get(), stream_));
     else Enqueue(stream_);
     if (head) QueuePieces(head, heads_[0].bytes, stream_);
     return;
@@ -2138,7 +2157,7 @@ void Executor::Launch(const void* input, Source src, const Schedule& how, char* 
     SendRange(input, src, begin, range_end_[r] - begin, copy_stream_);
     CUDA_OK(cudaEventRecord(part_events_[c], copy_stream_));
     CUDA_OK(cudaStreamWaitEvent(stream_, part_events_[c], 0));
-    CUDA_OK(cudaGraphLaunch(how.graphs[c], stream_));
+    CUDA_OK(cudaGraphLaunch(how.graphs[c].get(), stream_));
     if (parts_leave) {
       CUDA_OK(cudaEventRecord(part_done_[c], stream_));
       CUDA_OK(cudaStreamWaitEvent(down_stream_, part_done_[c], 0));
@@ -2192,7 +2211,7 @@ void Executor::RunOnce(const void* input, char* out) {
     } else {
       memcpy(in_host_, input, in_bytes_);
     }
-    CUDA_OK(cudaGraphLaunch(graph_staged_, stream_));
+    CUDA_OK(cudaGraphLaunch(graph_staged_.get(), stream_));
     if (head) QueuePieces(head, heads_[0].bytes, stream_);
   } else {
     Launch(input, src, on_device ? from_device_ : (src == Source::kDirect ? from_pinned_ : from_pageable_), head, apart);
@@ -2223,31 +2242,40 @@ void Executor::SetStatusWord(int code) {
   CUDA_OK(cudaStreamSynchronize(stream_));
 }
 
+namespace {
+class TimingEvents {
+ public:
+  explicit TimingEvents(size_t n) {
+    for (size_t k = 0; k < n; ++k) {
+      cudaEvent_t e = nullptr;
+      CUDA_OK(cudaEventCreate(&e));
+      e_.emplace_back(e, cudaEventDestroy);
+    }
+  }
+  cudaEvent_t operator[](size_t k) const { return e_[k].get(); }
+
+ private:
+  std::vector<std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)>> e_;
+};
+}  // namespace
+
 float Executor::ReplayDevice(int iters) {
   CHECK(iters > 0);
   CUDA_OK(cudaSetDevice(device_));
-  if (use_graph_ && !kernels_exec_) {
-    cudaGraph_t graph = nullptr;
-    CUDA_OK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    for (auto& st : steps_) KERNEL_OK(st.launch(stream_));
-    CUDA_OK(cudaStreamEndCapture(stream_, &graph));
-    CUDA_OK(cudaGraphInstantiate(&kernels_exec_, graph, 0));
-    CUDA_OK(cudaGraphDestroy(graph));
-  }
-  cudaEvent_t e0, e1;
-  CUDA_OK(cudaEventCreate(&e0));
-  CUDA_OK(cudaEventCreate(&e1));
-  CUDA_OK(cudaEventRecord(e0, stream_));
+  if (use_graph_ && !kernels_exec_)
+    kernels_exec_ = Capture([this] {
+      for (auto& st : steps_) KERNEL_OK(st.launch(stream_));
+    });
+  TimingEvents ev(2);
+  CUDA_OK(cudaEventRecord(ev[0], stream_));
   for (int i = 0; i < iters; ++i) {
-    if (kernels_exec_) CUDA_OK(cudaGraphLaunch(kernels_exec_, stream_));
+    if (kernels_exec_) CUDA_OK(cudaGraphLaunch(kernels_exec_.get(), stream_));
     else for (auto& st : steps_) KERNEL_OK(st.launch(stream_));
   }
-  CUDA_OK(cudaEventRecord(e1, stream_));
-  CUDA_OK(cudaEventSynchronize(e1));
+  CUDA_OK(cudaEventRecord(ev[1], stream_));
+  CUDA_OK(cudaEventSynchronize(ev[1]));
   float ms = 0;
-  CUDA_OK(cudaEventElapsedTime(&ms, e0, e1));
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  CUDA_OK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
   return ms;
 }
 
@@ -2255,8 +2283,7 @@ std::vector<std::pair<std::string, float>> Executor::ProfileOnce(const void* inp
   CHECK(input_bytes == in_bytes_);
   CUDA_OK(cudaSetDevice(device_));
   std::vector<std::pair<std::string, float>> out;
-  std::vector<cudaEvent_t> ev(steps_.size() + 1);
-  for (auto& e : ev) CUDA_OK(cudaEventCreate(&e));
+  TimingEvents ev(steps_.size() + 1);
   try {
     Upload(input, stream_);
     CUDA_OK(cudaEventRecord(ev[0], stream_));
@@ -2274,7 +2301,6 @@ std::vector<std::pair<std::string, float>> Executor::ProfileOnce(const void* inp
     CUDA_OK(cudaEventElapsedTime(&ms, ev[i], ev[i + 1]));
     out.emplace_back(steps_[i].label, ms);
   }
-  for (auto& e : ev) cudaEventDestroy(e);
   return out;
 }
 

@@ -99,10 +99,14 @@ class Executor {
   // An inference: the first `prefix` steps part by part, one graph per part of the batch, each launched
   // when its part of the input is on the device; the last part's graph goes on with the rest of the
   // steps and the delivery of the heads.  Without a prefix: one graph.
+  struct DropGraph {
+    void operator()(cudaGraphExec_t g) const { cudaGraphExecDestroy(g); }
+  };
+  using GraphExec = std::unique_ptr<CUgraphExec_st, DropGraph>;
   struct Schedule {
     size_t prefix = 0;
     int cut = 0;                            // which parts (kCuts)
-    std::vector<cudaGraphExec_t> graphs;
+    std::vector<GraphExec> graphs;
   };
   // How long the prefix should be depends on how fast the input arrives: chosen at load by timing
   // inferences, once from page-locked memory (read by the copy engine where it lies) and once from
@@ -110,12 +114,13 @@ class Executor {
   // everything those steps touch live together).
   Schedule from_pinned_, from_pageable_;
   Schedule from_device_;   // an input in device memory: the whole graph, unless the head's parts can leave early
-  cudaGraphExec_t graph_whole_ = nullptr;    // every step: the input is on the device already
-  cudaGraphExec_t graph_staged_ = nullptr;   // the same behind a kernel that fetches the staging buffer (small inputs)
+  GraphExec graph_whole_;    // every step: the input is on the device already
+  GraphExec graph_staged_;   // the same behind a kernel that fetches the staging buffer (small inputs)
   size_t prefix_max_ = 0;
   Schedule MakeSchedule(size_t prefix, int cut);
-  static void DropSchedule(Schedule* s);
-  cudaGraphExec_t Capture(const std::function<void()>& enqueue);
+  void Load(int plain_elem_bytes);
+  void Release();
+  GraphExec Capture(const std::function<void()>& enqueue);
   void ChooseSchedules();
   void Launch(const void* input, Source src, const Schedule& how, char* head, bool early);
   static bool IsDirect(const void* input);
@@ -134,7 +139,7 @@ class Executor {
   size_t in_bytes_ = 0;
   int32_t* status_dev_ = nullptr;
   int32_t* status_host_ = nullptr;
-  cudaGraphExec_t kernels_exec_ = nullptr;
+  GraphExec kernels_exec_;
   bool use_graph_ = true;
   // upload / compute overlap: the copy stream and one event per part of the batch
   cudaStream_t copy_stream_ = nullptr;

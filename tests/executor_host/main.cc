@@ -1,6 +1,7 @@
 /* Drives the C-ABI of the host runtime over the fake device.
  *   executor_host fail_run  early|late in out   every call of an inference that can fail does, one at a time
  *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
+ *   executor_host fail_load early|late - -     calls that can fail while a model is loaded do, one at a time
  * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
  * params.bin and input.bin of the working directory, fake::slow_images of the environment (SLOW_IMAGES), writes the bytes of the last good inference to
  * output.bin and prints "@name=value" lines.
@@ -36,6 +37,26 @@ int main(int argc, char** argv) {
   auto load = [&](void** net) { return CVMAPILoadModel(graph.data(), (int)graph.size(), params.data(), (int)params.size(), net, 1, 0); };
   if (const char* n = getenv("SLOW_IMAGES")) fake::slow_images = atoi(n);
   void* net = nullptr;
+  if (mode == "fail_load") {
+    long failed = 0, left = 0, odd = 0;
+    for (long n = 1;; n += 1 + n / 25) {
+      fake::reset_calls(n);
+      const int status = load(&net);
+      if (status == 0) CVMAPIFreeModel(net);
+      left += fake::live_objects() != 0 || fake::device_bytes != 0;
+      odd += status != 0 && status != 2;
+      failed += status != 0;
+      if (fake::calls < n) break;
+    }
+    // the memory a loaded model holds is enough to load it
+    load(&net);
+    fake::memory_limit = fake::device_bytes;
+    CVMAPIFreeModel(net);
+    const int tight = load(&net);
+    if (tight == 0) CVMAPIFreeModel(net);
+    printf("@failed=%ld @left=%ld @odd=%ld @tight=%d\n", failed, left, odd, tight);
+    return 0;
+  }
   if (load(&net) != 0) return 3;
   unsigned long long bytes = 0;
   CVMAPIGetOutputLength(net, &bytes);

@@ -89,3 +89,12 @@ def test_output_over_the_input(when, src, ahead, host, wl, tmp_path):
     want = np.full(x.shape, -1, np.int32)
     want[:, :100] = x[:, -100:]   # (what the fake device's operators do)
     assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int32), want.reshape(-1))
+
+
+@pytest.mark.parametrize("when", ["late", "early"])
+def test_a_failing_load_gives_everything_back(when, host, wl, tmp_path):
+    put(tmp_path, *wl.conv_chain(batch=8, channels=64, size=48))   # (1.2 MB: timed from pageable memory too)
+    f = host(tmp_path, "fail_load", when, "-", "-")
+    assert int(f["failed"]) > 100
+    assert f["left"] == "0" and f["odd"] == "0"
+    assert f["tight"] == "0"   # the memory that a loaded model holds is enough to load it
