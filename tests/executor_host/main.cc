@@ -48,7 +48,7 @@ int main(int argc, char** argv) {
       failed += status != 0;
       if (fake::calls < n) break;
     }
-    // the memory a loaded model holds is enough to load it
+    fake::reset_calls(0);   // the memory a loaded model holds is enough to load it
     load(&net);
     fake::memory_limit = fake::device_bytes;
     CVMAPIFreeModel(net);
