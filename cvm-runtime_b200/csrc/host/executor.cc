@@ -130,15 +130,7 @@ void* Executor::dalloc_activation(size_t bytes, uint32_t root) {
 // virtual range of a buffer is -- so nothing is lost to fragmentation.
 void Executor::PlanForPrefix(size_t prefix) {
   if (!vmm_ || act_.empty()) return;
-  if (!phys_.empty()) {
-    for (auto& a : act_)
-      if (a.block >= 0) { vmm().unmap(reinterpret_cast<CUdeviceptr>(a.va), a.va_size); a.block = -1; }
-    for (auto& b : phys_) {
-      vmm().release((CUmemGenericAllocationHandle)b.handle);
-      device_bytes_ -= b.size;
-    }
-    phys_.clear();
-  }
+  UnmapActivations();
   const int p = prefix > 0 ? step_pos_[std::min(prefix, step_pos_.size()) - 1] : -2;   // (heads' steps have no position)
   for (auto& a : act_) {
     a.first = a.first0;
@@ -146,6 +138,18 @@ void Executor::PlanForPrefix(size_t prefix) {
     if (a.first <= p) { a.first = -1; a.last = std::max(a.last, p); }
   }
   MapActivations();
+}
+
+void Executor::UnmapActivations() {
+  for (auto& a : act_) {
+    if (a.mapped) vmm().unmap(reinterpret_cast<CUdeviceptr>(a.va), a.mapped);
+    a.mapped = 0;
+  }
+  for (auto& b : phys_) {
+    vmm().release((CUmemGenericAllocationHandle)b.handle);
+    device_bytes_ -= b.size;
+  }
+  phys_.clear();
 }
 
 void Executor::MapActivations() {
@@ -182,10 +186,10 @@ void Executor::MapActivations() {
       phys_[mine[k]].free_at = a.last + 1;
       const CUresult r = vmm().map(va + k * vmm_gran_, vmm_gran_, 0, (CUmemGenericAllocationHandle)phys_[mine[k]].handle, 0);
       CHECK(r == CUDA_SUCCESS) << "cuMemMap failed (" << (int)r << ")";
+      a.mapped += vmm_gran_;
     }
     const CUresult r = vmm().set_access(va, a.va_size, &access, 1);
     CHECK(r == CUDA_SUCCESS) << "cuMemSetAccess failed (" << (int)r << ")";
-    a.block = mine.empty() ? -1 : mine[0];
   }
 }
 
@@ -1534,8 +1538,15 @@ struct Lowering {
         if (Executor::ActBuf* a = of_entry[g.entry_id(e)]) a->last = std::max(a->last, group_pos(nid));
     for (auto& a : act) { a.first0 = a.first; a.last0 = a.last; }
     ex.step_pos_ = step_pos;
-    // first with the longest prefix that may be chosen; the constructor plans again once it is known
-    ex.PlanForPrefix(ex.prefix_max_);
+    // first with the longest prefix that may be chosen; Load() plans again once it is known.  Where the device has
+    // no room for that many buffers at once, inferences run without a prefix.
+    try {
+      ex.PlanForPrefix(ex.prefix_max_);
+    } catch (const std::exception&) {
+      if (ex.prefix_max_ == 0) throw;
+      ex.prefix_max_ = 0;
+      ex.PlanForPrefix(0);
+    }
   }
 
   void lower_node(uint32_t nid) {
@@ -1890,11 +1901,8 @@ void Executor::Release() {
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
   if (down_stream_) cudaStreamDestroy(down_stream_);
   for (void* p : allocs_) cudaFree(p);
-  for (auto& a : act_) {
-    if (a.block >= 0) vmm().unmap(reinterpret_cast<CUdeviceptr>(a.va), a.va_size);
-    vmm().address_free(reinterpret_cast<CUdeviceptr>(a.va), a.va_size);
-  }
-  for (auto& b : phys_) vmm().release((CUmemGenericAllocationHandle)b.handle);
+  UnmapActivations();
+  for (auto& a : act_) vmm().address_free(reinterpret_cast<CUdeviceptr>(a.va), a.va_size);
   for (void* p : pinned_) cudaFreeHost(p);
   if (stream_) cudaStreamDestroy(stream_);
   cudaGetLastError();

@@ -187,11 +187,12 @@ class Executor {
     uint32_t root = UINT32_MAX;   // node whose lowering made the allocation
     int first = 0, last = 0;      // schedule positions of the first write and the last read
     int first0 = 0, last0 = 0;    // the same before the chunked prefix stretched them
-    int block = -1;               // physical block backing it
+    size_t mapped = 0;            // bytes of it that have physical memory
   };
   struct PhysBlock { unsigned long long handle = 0; size_t size = 0; int free_at = 0; };
   void* dalloc_activation(size_t bytes, uint32_t root);
   void MapActivations();
+  void UnmapActivations();
   // Lifetimes for a chunked prefix of `prefix` steps (everything those steps touch lives across
   // all of them), then the physical backing; whatever was mapped before is released first.
   void PlanForPrefix(size_t prefix);

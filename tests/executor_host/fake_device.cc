@@ -16,6 +16,7 @@
 #include <map>
 #include <mutex>
 #include <set>
+#include <string>
 #include <thread>
 #include <vector>
 #include "cvmk_kernels.h"
@@ -95,6 +96,51 @@ int launch(cvmk_stream_t s, std::function<void()> f) {
 void images(int64_t n) {
   if (slow_images && n >= slow_images) std::this_thread::sleep_for(std::chrono::milliseconds(2));
 }
+
+// virtual memory: a reserved range is ordinary memory from the start, mapping it is bookkeeping
+constexpr size_t kGranule = (size_t)64 << 10;
+std::map<CUdeviceptr, size_t> reserved;
+std::set<CUdeviceptr> mapped;   // granules
+size_t chunks = 0;
+CUresult granularity(size_t* g, const CUmemAllocationProp*, CUmemAllocationGranularity_flags) { *g = kGranule; return CUDA_SUCCESS; }
+CUresult reserve(CUdeviceptr* p, size_t n, size_t, CUdeviceptr, unsigned long long) {
+  if (fails()) return CUDA_ERROR_OUT_OF_MEMORY;
+  *p = (CUdeviceptr)aligned_alloc(kGranule, n);
+  memset((void*)*p, 0, n);
+  reserved[*p] = n;
+  return CUDA_SUCCESS;
+}
+CUresult address_free(CUdeviceptr p, size_t n) {
+  for (size_t at = 0; at < n; at += kGranule)
+    if (mapped.count(p + at)) return CUDA_ERROR_INVALID_VALUE;
+  if (reserved[p] != n) abort();
+  reserved.erase(p);
+  free((void*)p);
+  return CUDA_SUCCESS;
+}
+CUresult create(CUmemGenericAllocationHandle* h, size_t n, const CUmemAllocationProp*, unsigned long long) {
+  if (fails() || (memory_limit && device_bytes + n > memory_limit)) return CUDA_ERROR_OUT_OF_MEMORY;
+  device_bytes += n;
+  *h = ++chunks;
+  return CUDA_SUCCESS;
+}
+CUresult release(CUmemGenericAllocationHandle) {
+  --chunks;
+  device_bytes -= kGranule;
+  return CUDA_SUCCESS;
+}
+CUresult map(CUdeviceptr p, size_t, size_t, CUmemGenericAllocationHandle, unsigned long long) {
+  if (fails()) return CUDA_ERROR_UNKNOWN;
+  if (!mapped.insert(p).second) abort();
+  return CUDA_SUCCESS;
+}
+CUresult unmap(CUdeviceptr p, size_t n) {
+  for (size_t at = 0; at < n; at += kGranule)
+    if (!mapped.erase(p + at)) return CUDA_ERROR_INVALID_VALUE;
+  return CUDA_SUCCESS;
+}
+CUresult set_access(CUdeviceptr, size_t, const CUmemAccessDesc*, size_t) { return fails() ? CUDA_ERROR_UNKNOWN : CUDA_SUCCESS; }
+
 int nothing(cvmk_stream_t s) { return launch(s, [] {}); }
 
 }  // namespace
@@ -105,7 +151,7 @@ size_t pending() {
   for (Stream* s : streams) n += s->queue.size();
   return n;
 }
-size_t live_objects() { return streams.size() + events.size() + graphs.size() + memory.size(); }
+size_t live_objects() { return streams.size() + events.size() + graphs.size() + memory.size() + reserved.size() + mapped.size() + chunks; }
 
 }  // namespace fake
 
@@ -117,9 +163,14 @@ cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "made to fail"; }
-cudaError_t cudaGetDriverEntryPoint(const char*, void** fn, unsigned long long, cudaDriverEntryPointQueryResult* q) {
-  *fn = nullptr;
-  if (q) *q = cudaDriverEntryPointSymbolNotFound;
+cudaError_t cudaGetDriverEntryPoint(const char* name, void** fn, unsigned long long, cudaDriverEntryPointQueryResult* q) {
+  static const std::map<std::string, void*> known = {
+      {"cuMemGetAllocationGranularity", (void*)granularity}, {"cuMemAddressReserve", (void*)reserve},
+      {"cuMemAddressFree", (void*)address_free}, {"cuMemCreate", (void*)create}, {"cuMemRelease", (void*)release},
+      {"cuMemMap", (void*)map}, {"cuMemUnmap", (void*)unmap}, {"cuMemSetAccess", (void*)set_access}};
+  auto it = known.find(name);
+  *fn = it == known.end() ? nullptr : it->second;
+  *q = *fn ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
   return cudaSuccess;
 }
 cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n, cudaMemoryTypeDevice); }

@@ -2,6 +2,7 @@
  *   executor_host fail_run  early|late in out   every call of an inference that can fail does, one at a time
  *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
  *   executor_host fail_load early|late - -     calls that can fail while a model is loaded do, one at a time
+ *   executor_host tight     early|late - -     loads with no more device memory than the last one held, as long as that shrinks
  * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
  * params.bin and input.bin of the working directory, fake::slow_images of the environment (SLOW_IMAGES), writes the bytes of the last good inference to
  * output.bin and prints "@name=value" lines.
@@ -48,13 +49,21 @@ int main(int argc, char** argv) {
       failed += status != 0;
       if (fake::calls < n) break;
     }
-    fake::reset_calls(0);   // the memory a loaded model holds is enough to load it
+    printf("@failed=%ld @left=%ld @odd=%ld\n", failed, left, odd);
+    return 0;
+  }
+  if (mode == "tight") {
+    long sizes = 0, refused = 0;
+    size_t least = 0;
     load(&net);
-    fake::memory_limit = fake::device_bytes;
-    CVMAPIFreeModel(net);
-    const int tight = load(&net);
-    if (tight == 0) CVMAPIFreeModel(net);
-    printf("@failed=%ld @left=%ld @odd=%ld @tight=%d\n", failed, left, odd, tight);
+    for (size_t held = fake::device_bytes; ; held = fake::device_bytes) {
+      CVMAPIFreeModel(net);
+      if (held == least) break;
+      ++sizes;
+      least = fake::memory_limit = held;
+      if (load(&net) != 0) { ++refused; break; }
+    }
+    printf("@sizes=%ld @refused=%ld @left=%d\n", sizes, refused, fake::live_objects() != 0);
     return 0;
   }
   if (load(&net) != 0) return 3;

@@ -97,4 +97,9 @@ def test_a_failing_load_gives_everything_back(when, host, wl, tmp_path):
     f = host(tmp_path, "fail_load", when, "-", "-")
     assert int(f["failed"]) > 100
     assert f["left"] == "0" and f["odd"] == "0"
-    assert f["tight"] == "0"   # the memory that a loaded model holds is enough to load it
+
+
+def test_the_memory_a_model_holds_is_enough_to_load_it(host, wl, tmp_path):
+    put(tmp_path, *wl.mobilenet_v1(batch=16, size=96))
+    f = host(tmp_path, "tight", "early", "-", "-")
+    assert int(f["sizes"]) > 0 and f["refused"] == "0" and f["left"] == "0"
