@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <thread>
 
 namespace cvm {
 
@@ -1925,7 +1926,7 @@ HostPool& Executor::pool() {
     cudaGetDeviceCount(&gpus);
     // five helpers beside the calling thread, fewer when the host has few cores per GPU: one core
     // copies 14 GB/s here, four just reach the link's 55 GB/s, six leave room for a fill beside it
-    pool_.reset(new HostPool(hw ? std::max(1, std::min(5, (int)hw / std::max(1, gpus) - 1)) : 1));
+    pool_.reset(new HostPool(device_, hw ? std::max(1, std::min(5, (int)hw / std::max(1, gpus) - 1)) : 1));
   }
   return *pool_;
 }

@@ -2,21 +2,21 @@
 // buffer into the page-locked staging buffer, downloaded pieces into the caller's output buffer,
 // constant fills.  Each of these is a job cut into pieces; a piece is a call of the job's body.
 //
+// A HostPool is what one handle has of them: its jobs.  The threads belong to a crew that all handles of a
+// device share, started with the first of them and ended with the last: three handles on one GPU keep
+// five helpers busy, not fifteen.
+//
 // The helpers sleep between inferences that are more than a fifth of a millisecond apart.  Begin() wakes
-// them, and until End() they spin over
-// the jobs, lowest slot first, so that a job that starts while others run is picked up without a
-// wake-up (tens of microseconds, more than many of these jobs take).  The caller helps with every
-// job it waits for.
+// them, and until End() they spin over the jobs, lowest slot first, so that a job that starts while others
+// run is picked up without a wake-up (tens of microseconds, more than many of these jobs take); after some
+// twenty microseconds without a piece they offer their core to other threads between two looks.  The caller
+// helps with every job it waits for.
 #pragma once
 #include <atomic>
-#include <condition_variable>
 #include <cstddef>
 #include <cstdint>
 #include <functional>
 #include <memory>
-#include <mutex>
-#include <thread>
-#include <vector>
 
 namespace cvm {
 
@@ -24,7 +24,9 @@ class HostPool {
  public:
   enum Slot { kUpload = 0, kDownload = 1, kFill = 2, kSlots = 3 };   // in order of urgency
 
-  explicit HostPool(int helpers);
+  // `device` names the crew; `helpers` is how many threads it has if it does not exist yet (fewer where the
+  // system gives no more, none is fine).
+  HostPool(int device, int helpers);
   ~HostPool();
   HostPool(const HostPool&) = delete;
   HostPool& operator=(const HostPool&) = delete;
@@ -35,7 +37,7 @@ class HostPool {
   // `available` pieces may run at once, the others when Release() says so.
   void Start(Slot slot, size_t pieces, size_t available, std::function<void(size_t)> body);
   void Release(Slot slot, size_t available);
-  void ReleaseAll(Slot slot) { Release(slot, jobs_[slot].pieces); }
+  void ReleaseAll(Slot slot) { Release(slot, desk_->jobs[slot].pieces); }
   // Waits until piece k has run, running pieces of this job meanwhile.
   void WaitPiece(Slot slot, size_t k);
   // Waits until the whole job has run.
@@ -52,6 +54,7 @@ class HostPool {
     Use(const Use&) = delete;
     Use& operator=(const Use&) = delete;
     void Begin(HostPool& pool) {
+      if (p) return;   // (at work already)
       p = &pool;
       p->Begin();
     }
@@ -66,7 +69,7 @@ class HostPool {
   };
 
   static constexpr int kLingerUs = 200;
-  bool awake() const { return asleep_.load(std::memory_order_relaxed) == 0; }   // Begin() needs no wake-up
+  bool awake() const;   // Begin() needs no wake-up
 
  private:
   struct Job {
@@ -80,15 +83,20 @@ class HostPool {
     size_t done_cap = 0;
     std::atomic<size_t> completed{0};
   };
-  bool RunPiece(Job& j);
-  void Work();
+  // The jobs of one pool.  The crew never frees a desk while its threads run, so that they may look at any at
+  // any time; a desk whose pool is gone has no pieces to claim and goes to the next pool.
+  struct Desk {
+    Job jobs[kSlots];
+    std::atomic<bool> active{false};
+    bool taken = false;
+    Desk* next = nullptr;
+  };
+  struct Crew;
+  static std::shared_ptr<Crew> crew_of(int device, int helpers);
+  static bool RunPiece(Job& j);
 
-  Job jobs_[kSlots];
-  std::vector<std::thread> workers_;
-  std::mutex mu_;
-  std::condition_variable cv_;
-  std::atomic<bool> active_{false}, stop_{false};
-  std::atomic<int> asleep_{0};
+  std::shared_ptr<Crew> crew_;
+  Desk* desk_;
 };
 
 // memcpy with stores that bypass the cache: for destinations the CPU does not read soon (the

@@ -41,10 +41,14 @@ def host(tmp_path_factory):
     if procs or not os.path.exists(BIN):
         subprocess.check_call(["g++", "-fsanitize=address", "-pthread"] + objs + ["-o", BIN])
 
-    def run(work, *args, slow_images=0):
+    pool = os.path.join(OUT, "pool")
+    if procs or not os.path.exists(pool) or os.path.getmtime(pool) < os.path.getmtime(os.path.join(SRC, "pool.cc")):
+        subprocess.check_call(["g++"] + flags + [os.path.join(SRC, "pool.cc"), os.path.join(OUT, "host_pool.cc.o"), "-o", pool, "-ldl"])
+
+    def run(work, *args, slow_images=0, binary=BIN):
         env = dict(os.environ, SLOW_IMAGES=str(slow_images), ASAN_OPTIONS="detect_leaks=0:alloc_dealloc_mismatch=0")
-        p = subprocess.run([BIN] + [str(a) for a in args], cwd=work, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True,
-                           env=env, timeout=300)
+        p = subprocess.run([os.path.join(OUT, binary)] + [str(a) for a in args], cwd=work, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True,
+                           env=env, timeout=60)
         assert p.returncode == 0, p.stderr[-4000:]
         return dict(tok[1:].split("=", 1) for tok in p.stdout.split() if tok.startswith("@"))
     return run
@@ -103,3 +107,17 @@ def test_the_memory_a_model_holds_is_enough_to_load_it(host, wl, tmp_path):
     put(tmp_path, *wl.mobilenet_v1(batch=16, size=96))
     f = host(tmp_path, "tight", "early", "-", "-")
     assert int(f["sizes"]) > 0 and f["refused"] == "0" and f["left"] == "0"
+
+
+# handles of one GPU share its helpers; one handle starts and ends them each time, several come and go beside one
+# that stays
+@pytest.mark.parametrize("handles", [1, 2, 5])
+def test_handles_share_the_helpers_of_a_device(handles, host, tmp_path):
+    f = host(tmp_path, "share", handles, binary="pool")
+    assert f["wrong"] == "0" and f["left"] == "0"
+    assert 1 <= int(f["helpers"]) <= 5
+
+
+def test_callers_do_without_helpers(host, tmp_path):
+    f = host(tmp_path, "none", binary="pool")
+    assert f["wrong"] == "0" and f["threads"] == "1"
