@@ -238,6 +238,26 @@ struct Lowering {
   void add_step(const std::string& label, std::function<int(cudaStream_t)> fn) {
     ex.steps_.push_back({label, std::move(fn), {}});
   }
+  // The launch of a convolution on one part of the batch.  Its plan (tensor maps and more) is prepared when a
+  // schedule first captures the part: most steps of a network are never run in parts.
+  template <typename Plan, typename Desc>
+  static std::function<int(cudaStream_t)> part_launch(const Desc& desc, int (*prepare)(const Desc*, Plan*),
+                                                      int (*launch)(const Plan*, cvmk_stream_t)) {
+    std::shared_ptr<Plan> plan;
+    return [=](cudaStream_t s) mutable {
+      if (!plan) {
+        void* mem = nullptr;
+        CHECK(posix_memalign(&mem, 64, sizeof(Plan)) == 0);
+        plan.reset((Plan*)mem, plan_deleter);
+        const int rc = prepare(&desc, plan.get());
+        if (rc != CVMK_OK) {
+          plan.reset();
+          return rc;
+        }
+      }
+      return launch(plan.get(), s);
+    };
+  }
   // ------------------------------------------------------------------ analysis
   void analyse() {
     const uint32_t ne = g.num_entries;
@@ -763,22 +783,24 @@ struct Lowering {
             if (aligned) ex.steps_.back().chunk.push_back(move(r.begin, r.end));
           ex.steps_.back().images = N;
         }
-        auto plan_for = [&](int64_t b0, int64_t b1) {
-          cvmk_stem_conv_desc cd = sd;
-          cd.N = (int)(b1 - b0);
-          cd.x = sd.x + (size_t)b0 * C * H * (pitch > 0 ? pitch : W);
-          cd.y = (int8_t*)sd.y + (size_t)b0 * OH * OW * OC;
+        cvmk_stem_conv_plan* plan = nullptr;
+        {
           void* mem = nullptr;
           CHECK(posix_memalign(&mem, 64, sizeof(cvmk_stem_conv_plan)) == 0);
           ex.stem_plans_.emplace_back((cvmk_stem_conv_plan*)mem, plan_deleter);
-          cvmk_stem_conv_plan* pl = ex.stem_plans_.back().get();
-          KERNEL_OK(cvmk_conv2d_stem_prepare(&cd, pl));
-          return [pl](cudaStream_t s) { return cvmk_conv2d_stem_launch(pl, s); };
-        };
-        add_step(label + "[stem]", plan_for(0, N));
+          plan = ex.stem_plans_.back().get();
+          KERNEL_OK(cvmk_conv2d_stem_prepare(&sd, plan));
+        }
+        add_step(label + "[stem]", [plan](cudaStream_t s) { return cvmk_conv2d_stem_launch(plan, s); });
         ex.steps_.back().from_input = pitch == 0;
         ex.steps_.back().images = N;
-        for (const Range& r : parts) ex.steps_.back().chunk.push_back(plan_for(r.begin, r.end));   // (whole rows of 16 bytes)
+        for (const Range& r : parts) {   // (whole rows of 16 bytes)
+          cvmk_stem_conv_desc cd = sd;
+          cd.N = (int)(r.end - r.begin);
+          cd.x = sd.x + (size_t)r.begin * C * H * (pitch > 0 ? pitch : W);
+          cd.y = (int8_t*)sd.y + (size_t)r.begin * OH * OW * OC;
+          ex.steps_.back().chunk.push_back(part_launch(cd, cvmk_conv2d_stem_prepare, cvmk_conv2d_stem_launch));
+        }
         input_ranges(parts, image);
         return;
       }
@@ -905,7 +927,7 @@ struct Lowering {
       cvmk_conv_plan* plan = ex.plans_.back().get();
       KERNEL_OK(cvmk_conv2d_tc_prepare(&d, plan));
       add_step(label + (dw_tc ? "[dw]" : "[tc]"), [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
-      // Plans for the parts of the batch (every operand is batch-major, so a part is a contiguous slice).
+      // The parts of the batch (every operand is batch-major, so a part is a contiguous slice).
       if (xin.nhwc && out.nhwc) {
         ex.steps_.back().images = N;
         const int64_t per_image = fold > 1 ? (int64_t)OH * OW : 1;   // (folded pixels: d.N counts fold-th parts of pixels)
@@ -931,12 +953,7 @@ struct Lowering {
             if ((st.op == CVMK_EP_ADD_T || st.op == CVMK_EP_SUB_T || st.op == CVMK_EP_RSUB_T) && st.ptr)
               st.ptr = (const char*)st.ptr + out_first * st.ptr_dtype;
           }
-          void* cmem = nullptr;
-          CHECK(posix_memalign(&cmem, 64, sizeof(cvmk_conv_plan)) == 0);
-          ex.plans_.emplace_back((cvmk_conv_plan*)cmem, plan_deleter);
-          cvmk_conv_plan* cp = ex.plans_.back().get();
-          KERNEL_OK(cvmk_conv2d_tc_prepare(&cd, cp));
-          ex.steps_.back().chunk.push_back([cp](cudaStream_t s) { return cvmk_conv2d_tc_launch(cp, s); });
+          ex.steps_.back().chunk.push_back(part_launch(cd, cvmk_conv2d_tc_prepare, cvmk_conv2d_tc_launch));
         }
       }
     } else {

@@ -3,6 +3,7 @@
  *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
  *   executor_host fail_load early|late - -     calls that can fail while a model is loaded do, one at a time
  *   executor_host tight     early|late - -     loads with no more device memory than the last one held, as long as that shrinks
+ *   executor_host plans     early|late - -     how many convolution plans a load prepares
  * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
  * params.bin and input.bin of the working directory, fake::slow_images of the environment (SLOW_IMAGES), writes the bytes of the last good inference to
  * output.bin and prints "@name=value" lines.
@@ -50,6 +51,12 @@ int main(int argc, char** argv) {
       if (fake::calls < n) break;
     }
     printf("@failed=%ld @left=%ld @odd=%ld\n", failed, left, odd);
+    return 0;
+  }
+  if (mode == "plans") {
+    const int status = load(&net);
+    printf("@status=%d @plans=%ld\n", status, fake::conv_plans);
+    if (status == 0) CVMAPIFreeModel(net);
     return 0;
   }
   if (mode == "tight") {

@@ -109,6 +109,14 @@ def test_the_memory_a_model_holds_is_enough_to_load_it(host, wl, tmp_path):
     assert int(f["sizes"]) > 0 and f["refused"] == "0" and f["left"] == "0"
 
 
+# plans for the parts of the batch are made for the (at most fourteen) leading steps that run in parts, not for every
+# layer of the network: 53 convolutions, and nine parts of no more than thirteen of them
+def test_parts_are_prepared_for_the_steps_that_run_in_parts(host, wl, tmp_path):
+    put(tmp_path, *wl.resnet50(batch=8, size=64))
+    f = host(tmp_path, "plans", "early", "-", "-")
+    assert f["status"] == "0" and 53 <= int(f["plans"]) <= 53 + 13 * 9
+
+
 # handles of one GPU share its helpers; one handle starts and ends them each time, several come and go beside one
 # that stays
 @pytest.mark.parametrize("handles", [1, 2, 5])
