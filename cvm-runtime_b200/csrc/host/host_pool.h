@@ -72,7 +72,8 @@ class HostPool {
   bool awake() const;   // Begin() needs no wake-up
 
  private:
-  struct Job {
+  // (a cache line or more to itself: helpers poll all of them)
+  struct alignas(64) Job {
     // (generation << 32 | count): a claim is a compare-exchange of the whole word against `avail` of
     // the same generation, so a helper that looked at the slot's previous job cannot take a
     // piece the present one does not have.
@@ -87,7 +88,7 @@ class HostPool {
   // any time; a desk whose pool is gone has no pieces to claim and goes to the next pool.
   struct Desk {
     Job jobs[kSlots];
-    std::atomic<bool> active{false};
+    alignas(64) std::atomic<bool> active{false};
     bool taken = false;
     Desk* next = nullptr;
   };
