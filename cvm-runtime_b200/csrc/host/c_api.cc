@@ -342,6 +342,15 @@ int CVMXProfileSteps(void* net, const char* input_data, int input_len, char* tex
   API_END();
 }
 
+int CVMXSchedules(void* net, char* text, int text_len) {
+  API_BEGIN();
+  CHECK(net != nullptr); CHECK(text != nullptr); CHECK(text_len > 0);
+  const std::string out = static_cast<Model*>(net)->executor().DescribeSchedules();
+  CHECK((int)out.size() < text_len) << "the text needs " << out.size() + 1 << " bytes";
+  memcpy(text, out.c_str(), out.size() + 1);
+  API_END();
+}
+
 int CVMXSetStatusWord(void* net, int code) {
   API_BEGIN();
   CHECK(net != nullptr);

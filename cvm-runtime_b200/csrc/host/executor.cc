@@ -2261,6 +2261,13 @@ void Executor::RunOnce(const void* input, char* out) {
   last_call_ = std::chrono::steady_clock::now();
 }
 
+std::string Executor::DescribeSchedules() const {
+  std::ostringstream os;
+  const std::pair<const char*, const Schedule*> all[] = {{"pinned", &from_pinned_}, {"pageable", &from_pageable_}, {"device", &from_device_}};
+  for (const auto& s : all) os << s.first << "\t" << s.second->prefix << "\t" << std::max<size_t>(1, s.second->graphs.size()) << "\n";
+  return os.str();
+}
+
 void Executor::SetStatusWord(int code) {
   CUDA_OK(cudaSetDevice(device_));
   const int32_t v = code;

@@ -81,6 +81,8 @@ class Executor {
   // Replays only the kernels (input already in device memory, no upload / download) `iters`
   // times and returns the device time in milliseconds measured with CUDA events on the stream.
   float ReplayDevice(int iters);
+  // The schedules chosen at load (CVMXSchedules).
+  std::string DescribeSchedules() const;
   // Writes `code` into the device status word the kernels report their expired waits in.
   void SetStatusWord(int code);
 

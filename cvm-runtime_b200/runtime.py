@@ -264,3 +264,11 @@ def profile_steps(net, input_data):
         label, ms = line.rsplit("\t", 1)
         rows.append((label, float(ms)))
     return rows
+
+
+def schedules(net):
+    """{"pinned" | "pageable" | "device": (leading steps run part by part, parts of the batch)}, as chosen at load."""
+    buf = ctypes.create_string_buffer(256)
+    check_call(lib().CVMXSchedules(net, buf, ctypes.c_int(len(buf))), "CVMXSchedules")
+    rows = [line.split("\t") for line in buf.value.decode().splitlines()]
+    return {kind: (int(steps), int(parts)) for kind, steps, parts in rows}

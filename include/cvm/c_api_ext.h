@@ -35,6 +35,10 @@ CVM_DLL int CVMXReplayDevice(void* net, int iters, float* total_ms);
  * "<operator label>\t<milliseconds>\n" per launch into `text` (NUL-terminated). */
 CVM_DLL int CVMXProfileSteps(void* net, const char* input_data, int input_len, char* text,
                              int text_len);
+/* What the timing at load chose for the three places an input can lie in, one line
+ * "<pinned|pageable|device>\t<leading steps run part by part>\t<parts of the batch>\n" each, into `text`
+ * (NUL-terminated); 0 steps in 1 part: the whole graph at once. */
+CVM_DLL int CVMXSchedules(void* net, char* text, int text_len);
 
 /* Writes `code` into the model's device status word: the word every tensor-core kernel ORs a
  * non-zero value into when one of its bounded waits runs out.  The next CVMAPIInference on the

@@ -3,7 +3,7 @@
  *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
  *   executor_host fail_load early|late - -     calls that can fail while a model is loaded do, one at a time
  *   executor_host tight     early|late - -     loads with no more device memory than the last one held, as long as that shrinks
- *   executor_host plans     early|late - -     how many convolution plans a load prepares
+ *   executor_host plans     early|late - -     how many convolution plans a load prepares, and its schedules
  * `in` and `out` say which memory the caller's buffers are: pageable or pinned.  Reads graph.json,
  * params.bin and input.bin of the working directory, fake::slow_images of the environment (SLOW_IMAGES), writes the bytes of the last good inference to
  * output.bin and prints "@name=value" lines.
@@ -56,6 +56,12 @@ int main(int argc, char** argv) {
   if (mode == "plans") {
     const int status = load(&net);
     printf("@status=%d @plans=%ld\n", status, fake::conv_plans);
+    char text[256] = "";
+    if (status == 0 && CVMXSchedules(net, text, sizeof(text)) == 0) {
+      for (char* c = text; *c; ++c) *c = *c == '\t' ? ':' : *c;
+      for (char* line = strtok(text, "\n"); line; line = strtok(nullptr, "\n")) printf("@%.*s=%s\n", (int)strcspn(line, ":"), line, strchr(line, ':') + 1);
+    }
+    printf("@short=%d\n", status == 0 ? CVMXSchedules(net, text, 4) : -1);
     if (status == 0) CVMAPIFreeModel(net);
     return 0;
   }

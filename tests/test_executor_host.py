@@ -113,8 +113,12 @@ def test_the_memory_a_model_holds_is_enough_to_load_it(host, wl, tmp_path):
 # layer of the network: 53 convolutions, and nine parts of no more than thirteen of them
 def test_parts_are_prepared_for_the_steps_that_run_in_parts(host, wl, tmp_path):
     put(tmp_path, *wl.resnet50(batch=8, size=64))
-    f = host(tmp_path, "plans", "early", "-", "-")
+    f = host(tmp_path, "plans", "early", "-", "-", slow_images=8)
     assert f["status"] == "0" and 53 <= int(f["plans"]) <= 53 + 13 * 9
+    # ... and the handle says what it chose: steps and parts for each place an input can lie in
+    steps, parts = map(int, f["pinned"].split(":"))
+    assert 0 < steps <= 14 and parts in (2, 4, 5)
+    assert f["device"] == "0:1" and f["short"] == "2"
 
 
 # handles of one GPU share its helpers; one handle starts and ends them each time, several come and go beside one
