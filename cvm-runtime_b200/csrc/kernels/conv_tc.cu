@@ -1119,7 +1119,11 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
     m_tiles = (int64_t)((d.OW + patch_w - 1) / patch_w) * ((d.OH + patch_h - 1) / patch_h) * ((d.N + patch_n - 1) / patch_n);
   }
   const int bk = pick_block_k(d.C), units = d.KH * d.KW * (d.C / bk);
-  // Few rows over many weights: operands swapped, every CTA of two per SM streams its share of the weights.
+  // Few rows over many weights: operands swapped, every CTA streams its share of the weights.  Two CTAs an SM of
+  // 112 KB each, except for more than 64 rows: the partial sums they then exchange take up to 120 KB, so one CTA an
+  // SM fits, and the reduction is cut so that all are resident, with the ring in the rest of the memory (128 rows,
+  // cut and sized for two an SM: 4096 -> 4096 24.9 us, 25088 -> 4096 44.7, two rounds of CTAs with a ring of two
+  // units; for one an SM 10.3 and 31.9.  64 rows: two an SM 8.2 and 22.1, one 8.2 and 27.4).
   if (is_pointwise(d) && d.OH == 1 && d.OW == 1 && d.N <= BLOCK_M && (int64_t)d.OC * d.C >= 1 << 19) {
     bool plain = true;
     for (int i = 0; i < d.ep.n; ++i)
@@ -1129,10 +1133,11 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
       c.swap = 1;
       c.block_n = d.N <= 32 ? 32 : (d.N <= 64 ? 64 : 128);
       c.split = 1;
-      while (c.split < 8 && units >= 4 * c.split && mt * 2 * c.split <= 2 * sms) c.split *= 2;
+      const int per_sm = c.block_n == 128 ? 1 : 2, limit = (per_sm == 1 ? 208 : 112) * 1024;
+      while (c.split < 8 && units >= 4 * c.split && mt * 2 * c.split <= per_sm * sms) c.split *= 2;
       c.group = 1;
       c.stages = std::min((units + c.split - 1) / c.split, SMALL_MAX_STAGES);
-      while (c.stages > 2 && small_smem_bytes(bk, c.block_n, c.stages, c.split) > 112 * 1024) --c.stages;
+      while (c.stages > 2 && small_smem_bytes(bk, c.block_n, c.stages, c.split) > limit) --c.stages;
       return c;
     }
   }

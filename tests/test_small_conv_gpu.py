@@ -24,7 +24,7 @@ def test_convolution(n, c, h, w, oc, k, stride, gpu_run, oracle, wl):
 
 # the weights as the 128-row operand: rows around the widths of the narrow one, channels that end inside a tile
 @pytest.mark.parametrize("rows", [1, 31, 33, 64, 65, 128, 129])
-@pytest.mark.parametrize("k,units", [(1024, 1000), (4096, 136)])
+@pytest.mark.parametrize("k,units", [(1024, 1000), (4096, 136), (16384, 1024)])   # (the last: rings that turn, cut over eight CTAs)
 def test_dense(rows, k, units, gpu_run, oracle, wl):
     g = wl.GraphBuilder(rows)
     y = g.dense(g.var("data", (rows, k), 8), units, shift=0 if rows % 2 else None)
