@@ -1192,26 +1192,8 @@ extern "C" int cvmk_conv2d_tc_supported(const cvmk_conv_desc* d) {
   return 1;
 }
 
-// Scratch for a pointwise layer of at most one M tile whose reduction is cut into slices (the count
-// divides the number of K blocks, leaves at least four per slice, and is the smallest that makes the best
-// use of the SMs).  Layers are cut over clusters now, which need no scratch: the answer is for
-// callers that size a buffer with it, and the buffer is not used.
-extern "C" int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d) {
-  if (!d || !cvmk_conv2d_tc_supported(d)) return 0;
-  const int bk = pick_block_k(d->C), bn = pick_block_n(d->OC);
-  if (!is_pointwise(*d) || d->groups > 1 || (int64_t)d->N * d->OH * d->OW > BLOCK_M || d->OC % bn != 0 || d->C % bk != 0) return 0;
-  const int sms = sm_count(), blocks = d->C / bk, nt = d->OC / bn;
-  if (blocks < 8 || 2 * nt >= sms) return 0;
-  int best = 1;
-  double best_eff = (double)nt / sms;
-  for (int s = 2; s * 4 <= blocks && nt * s <= 4 * sms; ++s) {
-    if (blocks % s) continue;
-    const int tiles = nt * s;
-    const double eff = (double)tiles / (double)(((tiles + sms - 1) / sms) * sms);
-    if (eff > best_eff + 0.02) { best_eff = eff; best = s; }
-  }
-  return best > 1 ? (int64_t)d->N * d->OH * d->OW * best * d->OC * 4 : 0;
-}
+// (no launch takes scratch: reductions are cut over clusters, which exchange their sums on chip)
+extern "C" int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc*) { return 0; }
 
 extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* plan) {
   if (!d || !plan) { set_error("conv2d_tc_prepare: null argument"); return CVMK_ERR_ARG; }

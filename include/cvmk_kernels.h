@@ -139,8 +139,8 @@ typedef struct {
    * sub-pixels a - 1, a, a + 1, the outer ones from the neighbouring folded pixel at the edges. */
   int32_t group_fold;
   int32_t reserved1;
-  /* Scratch that reductions cut along K once took (cvmk_conv2d_tc_workspace_bytes()).  They are cut
-   * over clusters of CTAs now, which exchange their partial sums on chip; not used. */
+  /* Scratch of cvmk_conv2d_tc_workspace_bytes() bytes, i.e. none: reductions are cut over clusters of
+   * CTAs, which exchange their partial sums on chip.  Not used. */
   void* workspace;
   int64_t workspace_bytes;
   cvmk_epilogue ep;
@@ -171,7 +171,7 @@ typedef struct __attribute__((aligned(64))) {
 } cvmk_conv_plan;
 
 CVMK_API int cvmk_conv2d_tc_supported(const cvmk_conv_desc* d);
-CVMK_API int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d);
+CVMK_API int64_t cvmk_conv2d_tc_workspace_bytes(const cvmk_conv_desc* d);   /* 0 for every layer */
 CVMK_API int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* plan);
 CVMK_API int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t stream);
 

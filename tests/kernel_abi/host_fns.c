@@ -1,5 +1,5 @@
 /* Host-side functions of the kernel C-ABI that need no device: the shapes the tensor-core
- * convolution cuts along K and the scratch they want, and the operand order the stem convolution
+ * convolution takes and the scratch they want (none), and the operand order the stem convolution
  * packs its filter into.  Compiled as plain C against include/cvmk_kernels.h (which is therefore
  * checked to be a C header) and linked with the runtime library; the test reads the lines printed
  * here and the packed bytes written to the file named on the command line.
