@@ -10,8 +10,13 @@
 //     producing kernel (conv2d / dense / reduce / element-wise), so their int32 intermediates are
 //     never written;
 //   - pre-packed int8 weights (OIHW -> OHWI) and TMA tensor maps for the tensor-core convolutions;
-//   - a CUDA graph of the whole step list and the output download; the input upload is queued
-//     in front of it (straight from page-locked caller memory, staged in chunks otherwise).
+//   - CUDA graphs: one of every step and the way of the heads to the host, behind a kernel that fetches
+//     the staging buffer where the input is small; and, for batches that upload while they compute,
+//     one per part of the batch over the leading steps, launched when the part is on the device
+//     (Schedule).  Where the cut lies is timed at load, for inputs in page-locked, pageable and
+//     device memory separately.
+// The result is written into page-locked memory by a kernel (small heads), or leaves in pieces that host
+// threads (HostPool) move on, part by part of the batch where the whole graph runs that way.
 // There is no CPU fallback: every step is a CUDA kernel from this library.
 #pragma once
 #include <cuda_runtime.h>

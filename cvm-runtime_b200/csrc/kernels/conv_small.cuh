@@ -24,8 +24,7 @@ struct SmallConvParams {
   int* status;
   const int32_t* bias;
   int bias_static, first_step;
-  const int8_t* res;              // int8 operand of a fused tensor add / subtract (step res_step), or nullptr
-  int res_step;
+  const int8_t* res;              // int8 operand of a fused tensor add / subtract, or nullptr
   int fast_variant;               // -1: the chain step by step; else as in conv_tc.cu (+ 8: wide)
   int f_mul, f_add, f_pre_lo, f_pre_hi;
   tc::FastQ fq;

@@ -1580,7 +1580,6 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
     q.fd_cblocks = make_fastdiv(p.c / p.block_k);
     q.fd_kw = make_fastdiv(p.kw);
     q.status = p.status; q.bias = p.bias; q.bias_static = p.bias_static; q.first_step = p.first_step;
-    q.res_step = p.res_step;
     q.res = p.res_step >= 0 ? reinterpret_cast<const int8_t*>(p.chain.s[p.res_step].ptr) : nullptr;
     q.fast_variant = p.fast_mode ? p.fast_variant + 8 * p.fast_wide : -1;
     if (p.fast_mode == 1) q.res = nullptr;
