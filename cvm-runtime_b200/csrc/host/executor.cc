@@ -1813,12 +1813,17 @@ bool Executor::IsDevice(const void* input) {
   return false;
 }
 
-bool Executor::IsDirect(const void* input) {
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, input) == cudaSuccess)
-    return at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
-  cudaGetLastError();
-  return false;
+// Memory that the copy engine can be given, all of it: a range that is page-locked only in part is not.
+bool Executor::IsDirect(const void* p, size_t bytes) {
+  auto type_of = [](const void* q) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, q) == cudaSuccess) return at.type;
+    cudaGetLastError();
+    return cudaMemoryTypeUnregistered;
+  };
+  const cudaMemoryType first = type_of(p);
+  if (first == cudaMemoryTypeHost) return bytes < 2 || type_of((const char*)p + bytes - 1) == cudaMemoryTypeHost;
+  return first == cudaMemoryTypeDevice || first == cudaMemoryTypeManaged;
 }
 
 // How many leading steps to run part by part, and in which parts: the choice whose inference takes least, timed
@@ -1932,7 +1937,7 @@ void Executor::Release() {
 // page-locked input of up to 256 KiB is staged as well: the copy takes 4 us, and the inference
 // is then one graph that begins by fetching the staging buffer.
 Executor::Source Executor::SourceOf(const void* input) const {
-  if (IsDirect(input)) return in_bytes_ <= kSmallDirect && graph_staged_ && !IsDevice(input) ? Source::kSmall : Source::kDirect;
+  if (IsDirect(input, in_bytes_)) return in_bytes_ <= kSmallDirect && graph_staged_ && !IsDevice(input) ? Source::kSmall : Source::kDirect;
   return in_bytes_ <= kSmallInput ? Source::kSmall : Source::kPool;
 }
 
@@ -2090,7 +2095,7 @@ void Executor::StartFill(char* out) {
 void Executor::StartDelivery(char* out) {
   queued_pieces_ = arrived_pieces_ = 0;
   deliver_units_ = 0;
-  if (IsDirect(out)) return;
+  if (IsDirect(out, heads_[0].bytes)) return;
   const size_t unit = DeliverUnit(), bytes = heads_[0].bytes;
   const char* from = (const char*)heads_[0].host;
   deliver_units_ = (bytes + unit - 1) / unit;
@@ -2157,8 +2162,10 @@ void Executor::DeliverHead(char* out, HostPool* awake) {
   size_t b = 0;
   while (b < h.images && valid_host_[b] > 0) ++b;
   if (b + 1 < h.images) {
-    CUDA_OK(cudaMemcpyAsync(out + (b + 1) * image, (const char*)h.dev + (b + 1) * image, h.bytes - (b + 1) * image, cudaMemcpyDeviceToHost, stream_));
+    const size_t at = (b + 1) * image;
+    CUDA_OK(cudaMemcpyAsync((char*)h.host + at, (const char*)h.dev + at, h.bytes - at, cudaMemcpyDeviceToHost, stream_));
     CUDA_OK(cudaStreamSynchronize(stream_));
+    memcpy(out + at, (const char*)h.host + at, h.bytes - at);
   }
 }
 

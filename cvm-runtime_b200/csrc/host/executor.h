@@ -130,7 +130,7 @@ class Executor {
   GraphExec Capture(const std::function<void()>& enqueue);
   void ChooseSchedules();
   void Launch(const void* input, Source src, const Schedule& how, char* head, bool early);
-  static bool IsDirect(const void* input);
+  static bool IsDirect(const void* p, size_t bytes);
   static bool IsDevice(const void* input);
   std::vector<size_t> range_end_;   // input bytes up to the end of each range of images that steps are prepared for
   std::vector<size_t> head_range_end_;   // the same of the only head, where its parts may leave one by one

@@ -68,6 +68,16 @@ void work(void* s, std::function<void()> f) {
   op.run = std::move(f);
   push((Stream*)s, std::move(op));
 }
+const std::pair<char* const, std::pair<size_t, cudaMemoryType>>* known(const void* p) {
+  auto it = memory.upper_bound((char*)p);
+  if (it == memory.begin()) return nullptr;
+  --it;
+  return it->first + it->second.first > (char*)p ? &*it : nullptr;
+}
+bool leaves_its_range(const void* p, size_t n) {
+  auto* m = known(p);
+  return m && (char*)p + n > m->first + m->second.first;
+}
 cudaError_t take(void** p, size_t n, cudaMemoryType kind) {
   if (fails()) return cudaErrorMemoryAllocation;
   if (kind == cudaMemoryTypeDevice) {
@@ -151,6 +161,8 @@ size_t pending() {
   for (Stream* s : streams) n += s->queue.size();
   return n;
 }
+void host_register(void* p, size_t n) { memory[(char*)p] = {n, cudaMemoryTypeHost}; }
+void host_unregister(void* p) { memory.erase((char*)p); }
 size_t live_objects() { return streams.size() + events.size() + graphs.size() + memory.size() + reserved.size() + mapped.size() + chunks; }
 
 }  // namespace fake
@@ -180,8 +192,7 @@ cudaError_t cudaFreeHost(void* p) { return give(p); }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* at, const void* p) {
   memset(at, 0, sizeof(*at));
   at->type = cudaMemoryTypeUnregistered;
-  auto it = memory.upper_bound((char*)p);
-  if (it != memory.begin() && (--it)->first + it->second.first > (char*)p) at->type = it->second.second;
+  if (auto* m = known(p)) at->type = m->second.second;
   return cudaSuccess;
 }
 cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return ok_or_fail(); }
@@ -193,6 +204,7 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
   if (fails()) return cudaErrorUnknown;
+  if (leaves_its_range(d, n) || leaves_its_range(s, n)) return cudaErrorInvalidValue;
   work(st, [=] { memmove(d, s, n); });
   return cudaSuccess;
 }

@@ -20,6 +20,8 @@ extern int slow_images;
 void reset_calls(long fail);
 size_t pending();         // operations queued and not yet run, over all streams
 size_t live_objects();    // allocations, streams, events and graphs that exist
+void host_register(void* p, size_t n);     // as cudaHostRegister() does; a copy that leaves the range fails
+void host_unregister(void* p);
 extern long conv_plans;   // cvmk_conv2d_tc_prepare() calls
 
 }  // namespace fake

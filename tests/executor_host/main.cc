@@ -1,6 +1,7 @@
 /* Drives the C-ABI of the host runtime over the fake device.
  *   executor_host fail_run  early|late in out   every call of an inference that can fail does, one at a time
  *   executor_host in_place  early|late in N    one inference whose output begins N bytes into the input
+ *   executor_host half      early|late in out  buffers whose first half only is page-locked, where `in` or `out` is "half"
  *   executor_host fail_load early|late - -     calls that can fail while a model is loaded do, one at a time
  *   executor_host tight     early|late - -     loads with no more device memory than the last one held, as long as that shrinks
  *   executor_host plans     early|late - -     how many convolution plans a load prepares, and its schedules
@@ -29,6 +30,7 @@ static char* buffer(const std::string& kind, size_t n) {
   void* p = nullptr;
   if (kind == "pinned") cudaMallocHost(&p, n);
   else p = malloc(n);
+  if (kind == "half") fake::host_register(p, n / 2);
   return (char*)p;
 }
 
@@ -95,6 +97,7 @@ int main(int argc, char** argv) {
     out = in + ahead;
     printf("@status=%d\n", infer());
   }
+  if (mode == "half") printf("@status=%d\n", infer());
   if (mode == "fail_run") {
     long failed = 0, in_flight = 0, wrong_after = 0;
     for (long n = 1;; ++n) {

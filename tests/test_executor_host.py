@@ -95,6 +95,16 @@ def test_output_over_the_input(when, src, ahead, host, wl, tmp_path):
     assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int32), want.reshape(-1))
 
 
+# a copy between the device and memory that is page-locked in part is refused by the driver; such buffers go the way
+# of pageable ones
+@pytest.mark.parametrize("src,dst", [("half", "pageable"), ("pageable", "half"), ("half", "half")])
+def test_buffers_that_are_page_locked_in_part(src, dst, host, wl, tmp_path):
+    js, pb, x = chain(wl, 9)
+    put(tmp_path, js, pb, x)
+    assert host(tmp_path, "half", "early", src, dst, slow_images=9)["status"] == "0"
+    assert np.array_equal(np.fromfile(tmp_path / "output.bin", np.int8), x.reshape(-1))
+
+
 @pytest.mark.parametrize("when", ["late", "early"])
 def test_a_failing_load_gives_everything_back(when, host, wl, tmp_path):
     put(tmp_path, *wl.conv_chain(batch=8, channels=64, size=48))   # (1.2 MB: timed from pageable memory too)
