@@ -25,6 +25,7 @@ struct SmallConvParams {
   const int32_t* bias;
   int bias_static, first_step;
   const int8_t* res;              // int8 operand of a fused tensor add / subtract, or nullptr
+  int pad_;                       // what follows lies better this way (without it 57 launches of ResNet-50, 13 images: 313.0 -> 314.1 us)
   int fast_variant;               // -1: the chain step by step; else as in conv_tc.cu (+ 8: wide)
   int f_mul, f_add, f_pre_lo, f_pre_hi;
   tc::FastQ fq;
