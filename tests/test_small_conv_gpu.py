@@ -11,11 +11,13 @@ pytestmark = pytest.mark.gpu
 # (n, c, h, w, oc, k, stride): one unit of 32 channels (a ring smaller than the tile it stages on the way
 # out), 64- and 32-column tiles, channels that end inside a tile, ragged last tiles, two to four units behind one
 # barrier, rings that turn, reductions cut over two to eight CTAs with rows the cut does not divide,
-# strided filters (im2col loads), patches of several images
+# strided filters (im2col loads), patches of several images; two and three CTAs an SM whose rings turn, one unit
+# behind each of eight barriers
 @pytest.mark.parametrize("n,c,h,w,oc,k,stride", [
     (5, 32, 85, 85, 64, 1, 1), (3, 32, 85, 85, 64, 3, 2), (5, 32, 85, 85, 40, 1, 1), (1, 32, 9, 9, 8, 1, 1), (2, 64, 61, 61, 72, 1, 1),
     (1, 128, 57, 57, 128, 1, 1), (1, 256, 29, 31, 64, 1, 1), (1, 512, 14, 14, 32, 1, 1), (1, 1024, 14, 14, 256, 1, 1),
-    (1, 512, 7, 7, 512, 3, 1), (3, 256, 7, 7, 128, 3, 1), (1, 512, 13, 13, 512, 3, 2), (1, 2048, 7, 7, 512, 1, 1), (1, 128, 11, 5, 136, 3, 1)])
+    (1, 512, 7, 7, 512, 3, 1), (3, 256, 7, 7, 128, 3, 1), (1, 512, 13, 13, 512, 3, 2), (1, 2048, 7, 7, 512, 1, 1), (1, 128, 11, 5, 136, 3, 1),
+    (11, 512, 29, 29, 192, 1, 1), (13, 512, 41, 43, 128, 1, 1), (5, 256, 27, 27, 264, 3, 1), (10, 1024, 14, 14, 520, 1, 1)])
 def test_convolution(n, c, h, w, oc, k, stride, gpu_run, oracle, wl):
     for shift, relu in ((wl.GraphBuilder.default_shift(c * k * k), True), (None, False)):   # packed and step by step
         js, pb, x = cases.conv_case(c + oc, n, c, h, w, oc, k, stride, k // 2, shift=shift, relu=relu)
