@@ -43,17 +43,6 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // A value that is the same for the whole warp, out of a shuffle: the compiler then keeps it (and what is
 // computed from it) in uniform registers, where TMA and tensor instructions take their operands.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// The address, in the cluster's shared window, of `addr` in the CTA of rank `rank`.
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-  uint32_t d;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
-  return d;
-}
 // Copies `bytes` of this CTA's shared memory to `dst` (an address of the cluster window) and reports them
 // to the mbarrier `bar` of the receiving CTA.
 __device__ __forceinline__ void bulk_to_rank(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {

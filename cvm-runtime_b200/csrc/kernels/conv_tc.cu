@@ -3,18 +3,18 @@
 //
 //   D[pixel, oc] = sum_{kh,kw,c} X[n, oh*s-p+kh*d, ow*s-p+kw*d, c] * Wt[oc, kh, kw, c]
 //
-// One CTA owns a 128-pixel x BLOCK_N-channel tile of the output and walks K = KH*KW*C in slabs of
-// BLOCK_K bytes.  TMA brings each slab of activations (im2col-mode tensor map: 128 consecutive
-// output pixels of one filter tap, zero-filled outside the image; a plain 2-D map when the conv
-// is a 1x1 / dense) and of weights into a swizzled shared-memory ring; one thread issues
-// tcgen05.mma kind::i8 (int8 x int8 -> int32) into a TMEM accumulator; four warps drain the
-// accumulator with tcgen05.ld, run the fused element chain (bias, relu, round-shift, clip,
-// residual add ...) and store int8 / int32 NHWC.  Two accumulators alternate (four, when a tile is
-// at most 128 columns wide) so the drain of tile i overlaps the MMAs of the tiles after it.  The
-// int32 sum never reaches HBM.  Stride-1 3 x 3 filters over at most 128 channels (and every
-// grouped layer) stage the input halo of a spatial patch once and let every filter tap multiply a
-// window of it; in those modes the second producer warp issues the instructions of every second
-// tile instead of loading.
+// A pair of CTAs owns a 256-pixel x BLOCK_N-channel tile of the output, 128 pixels each, and walks
+// K = KH*KW*C in slabs of BLOCK_K bytes.  TMA brings each slab of activations (im2col-mode tensor
+// map: 128 consecutive output pixels of one filter tap, zero-filled outside the image; a plain 2-D
+// map when the conv is a 1x1 / dense) and of weights (half of the rows to each CTA) into a swizzled
+// shared-memory ring; one thread of the pair issues tcgen05.mma kind::i8 (int8 x int8 -> int32) into
+// TMEM accumulators; four warps of each CTA drain its accumulator with tcgen05.ld, run the fused
+// element chain (bias, relu, round-shift, clip, residual add ...) and store int8 / int32 NHWC.  Two
+// accumulators alternate (four, when a tile is at most 128 columns wide) so the drain of tile i
+// overlaps the MMAs of the tiles after it.  The int32 sum never reaches HBM.  Stride-1 3 x 3 filters
+// over at most 128 channels (and every grouped layer) stage the input halo of a spatial patch once and
+// let every filter tap multiply a window of it; in those modes the second producer warp issues the
+// instructions of every second tile instead of loading.
 //
 // int8 outputs leave through shared memory: eight epilogue warps write their packed results into
 // a swizzled staging panel (128 rows x up to 128 bytes) that one thread hands to a TMA store, and
@@ -186,24 +186,38 @@ __device__ __forceinline__ void fast_chunk(const ConvParams& p, const FastQ& fq,
   *q1 = b;
 }
 
+// Arrival at a barrier of this CTA or of the other one of its pair (an address of the cluster's shared window).
+__device__ __forceinline__ void arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // `acc_free`: the barrier that hands the accumulator back to the MMA warp.  The warp arrives at it
 // as soon as its last columns are in registers (the loads have completed: tcgen05.wait::ld), not
 // after the arithmetic on them: the MMA warp's way back to a full accumulator (it notices, issues,
 // the instructions run, this group notices) then overlaps the last quarter of this tile's work
 // instead of following it.  Used when the tile is so wide that TMEM holds only two accumulators
-// (nullptr otherwise: with four, the MMA warp is tiles ahead anyway).
+// (0 otherwise: with four, the MMA warp is tiles ahead anyway).
 template <int RELU1, int KIND, int WIDE>
 __device__ __forceinline__ void fast_row(const ConvParams& p, uint32_t tbase, int chunks, const int32_t* bias_row,
-                                         uint8_t* io_base, int panel_size, int row_in_tile, int pw, uint64_t* acc_free) {
+                                         uint8_t* io_base, int panel_size, int row_in_tile, int pw, uint32_t acc_free) {
   const FastQ fq = {p.f_lo1, p.f_hi1, p.f_lo2, p.f_hi2};
   const uint32_t row_off = (uint32_t)row_in_tile * (uint32_t)pw;
   const uint32_t sw = (row_off >> 7) & (((uint32_t)pw - 1u) >> 4);  // swizzle key of this row, as in panel_offset()
   auto release = [&]() {
-    if (acc_free == nullptr) return;
+    if (acc_free == 0) return;
     tc_fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(acc_free);
+    if ((threadIdx.x & 31) == 0) arrive_at(acc_free);
   };
+  if (KIND == 0) {   // (without an operand a chunk is so little code that half of it in the SM's caches is worth more than a round trip)
+    for (int ci = 0; ci < chunks; ++ci) {
+      int32_t v[32];
+      tmem_ld32(tbase + (uint32_t)(ci * 32), v);
+      if (ci + 1 == chunks) release();
+      fast_chunk<RELU1, KIND, WIDE>(p, fq, v, ci, bias_row, io_base, panel_size, row_off, sw);
+    }
+    return;
+  }
   int ci = 0;
   for (; ci + 2 <= chunks; ci += 2) {  // two chunks per TMEM round trip
     int32_t v0[32], v1[32];
@@ -243,13 +257,33 @@ __device__ long long g_conv_trace[17 * 512];
 #define TFLUSH(slot) do {} while (0)
 #endif
 
+// TMA loads into this CTA's shared memory that report to `bar`, a barrier of the pair's first CTA.
+__device__ __forceinline__ void load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::
+                   "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];" ::
+                   "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ void load_im2col(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c, int w, int h, int n, uint16_t off_w,
+                                            uint16_t off_h) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::
+                   "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h) : "memory");
+}
+
 // Origin of a tile: first output channel, and either the first linear output row (modes 0, 1) or
 // the corner (w, h, n) of the spatial patch (mode 2).
-struct TileOrigin { int n0, m0, cw, ch, cn; };
-__device__ __forceinline__ TileOrigin tile_origin(const ConvParams& p, int tile) {
+// `tile` is two neighbouring M tiles, one for each CTA of the pair; the last one may lack its second half, whose CTA
+// then loads the tile before it once more (live is false) and stores nothing.
+struct TileOrigin { int n0, m0, cw, ch, cn; bool live; };
+__device__ __forceinline__ TileOrigin tile_origin(const ConvParams& p, int tile, int rank) {
   TileOrigin t;
-  const int mt = fdiv(tile, p.fd_n_tiles);
+  int mt = fdiv(tile, p.fd_n_tiles);
   t.n0 = (tile - mt * p.num_n_tiles) * p.block_n;
+  mt = 2 * mt + rank;
+  t.live = mt < p.num_m_tiles;
+  if (!t.live) mt = p.num_m_tiles - 1;
   t.m0 = mt * BLOCK_M;
   t.cw = t.ch = t.cn = 0;
   if (p.a_mode >= 2) {
@@ -262,6 +296,15 @@ __device__ __forceinline__ TileOrigin tile_origin(const ConvParams& p, int tile)
   return t;
 }
 
+// The two CTAs of a cluster multiply a 256-row tile together (tcgen05 cta_group::2).  Each loads its own 128 rows of
+// A and HALF of B's rows, the first CTA's MMA warp issues the instructions for both, and each CTA drains and stores
+// its own 128 rows.  An SM then takes 32 KB from L2 for what costs a CTA of its own 48 KB (128 x 256 tiles, 128
+// channels), and that port (64 bytes a clock) is what bounds long reductions; resident weights take half the room.  The
+// ring stages of the two CTAs are one: the second CTA's loads report to the first one's barrier, a commit frees the
+// stage in both.  Against single CTAs, in a chain of such layers: 3 x 3 over 512 channels at 28 x 28, 32 images
+// 44.2 -> 39.2 us; 3 x 3 over 256 at 14 x 14, 256 images 25.6 -> 22.4; 512 -> 512 at 14 x 14, 256 images 19.6 -> 15.6;
+// 3 x 3 over 512 at 7 x 7, 64 images (tiles of 128 channels) 17.2 -> 12.2.  There is no form for single CTAs beside it:
+// a launch of another kernel than the one before it takes two microseconds more (its code is not in the caches).
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_r,
@@ -289,14 +332,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) TRACE(16, 0);
+  constexpr int CG = 2;   // CTAs of a pair
+  const int rank = __shfl_sync(0xffffffffu, (int)cluster_rank(), 0);
+  const int first_own = (int)blockIdx.x >> 1, tile_step = (int)gridDim.x >> 1;
   const int a_bytes = BLOCK_M * p.block_k;
   // (grouped: an N tile is gpt = block_n / c groups of c channels whose activations lie side by side
   //  in one halo of block_k = block_n bytes per pixel; a weight tile is the c x c block of one group)
   const int gpt = p.grouped ? p.block_n / p.c : 1;
-  const int b_bytes = p.grouped ? p.c * p.c : p.block_n * p.block_k;
-  // b_resident: a 1x1 layer whose N tiles divide the grid, so that every tile of a CTA has the same
-  // first output channel: the K blocks of that N tile are loaded once and stay in front of the
-  // ring, which then carries activations only.
+  const int b_bytes = (p.grouped ? p.c * p.c : p.block_n * p.block_k) / CG;   // (this CTA's half of the rows)
+  // b_resident: a 1x1 layer whose N tiles divide the pairs, so that every tile of a CTA has the same
+  // first output channel: its half of the K blocks of that N tile is loaded once and stays in front of
+  // the ring, which then carries activations only.
   const bool b_resident = p.b_resident != 0;
   const int unit_bytes = a_bytes + (b_resident ? 0 : b_bytes);   // one A tile and the B tile that goes with it
   const int num_units = p.num_units;
@@ -319,7 +365,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   uint8_t* const ring = smem + resident_bytes;
   const int stage_bytes = w_resident ? halo_pad : (halo ? halo_pad + taps * b_bytes : p.units * unit_bytes);
   const int num_kb = p.num_kb;  // ring stages consumed per tile
-  const int num_tiles = p.num_m_tiles * p.num_n_tiles;
+  const int num_tiles = ((p.num_m_tiles + 1) >> 1) * p.num_n_tiles;   // of the pair
   const bool bias_in_smem = (p.bias != nullptr || p.fast_mode) && p.oc <= MAX_BIAS;
 
   if (threadIdx.x == 0) {
@@ -329,7 +375,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
     for (int a = 0; a < 4; ++a) {
       mbar_init(&bar_acc_full[a], 1);
-      mbar_init(&bar_acc_empty[a], NUM_EPI_WARPS / 2);
+      mbar_init(&bar_acc_empty[a], NUM_EPI_WARPS / 2 * CG);
     }
     for (int a = 0; a < 2; ++a) {
       for (int b = 0; b < 2; ++b) {
@@ -341,7 +387,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);   // before this CTA lets the next kernel start
+  if (warp == 1) tmem_alloc<CG>(&tmem_slot, (uint32_t)p.tmem_cols);   // before this CTA lets the next kernel start
   // Programmatic dependent launch: the next kernel of the stream may start its own prologue on SMs
   // this grid has left.  Until griddepcontrol.wait returns, the previous kernel of the stream may
   // still be running, so only memory that no kernel writes is touched before it: the tensor maps
@@ -377,6 +423,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     asm volatile("bar.arrive 1, %0;" ::"r"(setup_threads) : "memory");
   }
   if (is_producer && !two_issuers) asm volatile("bar.sync 2, 64;" ::: "memory");
+  // (neither CTA signals the other's barriers or writes its TMEM before both have them)
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   auto stage_bias = [&]() {
     const int padded = min(MAX_BIAS, (p.oc + 31) & ~31);
     for (int i = (int)threadIdx.x - 32; i < padded; i += NUM_THREADS - 64) {   // warps 1..10
@@ -399,6 +448,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     tc_fence_after();
     tmem_base = tmem_slot;
   }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (threadIdx.x == 0) TRACE(16, 2);
 
   if (is_producer) {
@@ -420,53 +471,31 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // loads: the filter taps are walked with nested counters (no divisions), and everything
       // that is constant for a tile is computed once per tile.
       const uint32_t smem_base = smem_u32(ring);
-      const uint32_t full0 = smem_u32(&bar_full[0]);
-      const TileOrigin to_first = tile_origin(p, (int)blockIdx.x);
-      if (w_resident && which == 0) {  // the weight rows of this CTA's N tile, once (every tile of a CTA has the same n0)
-        const uint32_t wb = smem_u32(&bar_weights);
-        if (leader) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wb), "r"((uint32_t)resident_bytes) : "memory");
+      // (everything reports to the first CTA, which announces the bytes of both)
+      const uint32_t full0 = map_rank(smem_u32(&bar_full[0]), 0), weights0 = map_rank(smem_u32(&bar_weights), 0);
+      const bool announces = leader && rank == 0;
+      const int b_row = rank * ((p.grouped ? p.c : p.block_n) / CG);
+      const TileOrigin to_first = tile_origin(p, first_own, rank);
+      if ((w_resident || b_resident) && which == 0) {   // this CTA's half of the weights of its N tile, once (every tile has the same n0)
+        if (announces) mbar_expect_tx(&bar_weights, (uint32_t)(CG * resident_bytes));
         uint32_t dst = smem_u32(smem);
-        for (int cb = 0; cb < (p.grouped ? gpt : p.num_kb); ++cb) {
-          int kcol = p.grouped ? 0 : cb * p.block_k;
-          const int wrow = p.grouped ? to_first.n0 + cb * p.c : to_first.n0;
-          for (int t = 0; t < taps; ++t) {
-            if (leader) asm volatile(
-                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(&tmap_b)), "r"(wb),
-                "r"(kcol), "r"(wrow)
-                : "memory");
-            dst += (uint32_t)b_bytes;
-            kcol += p.c;
+        if (w_resident) {
+          for (int cb = 0; cb < (p.grouped ? gpt : p.num_kb); ++cb) {
+            int kcol = p.grouped ? 0 : cb * p.block_k;
+            const int wrow = to_first.n0 + b_row + (p.grouped ? cb * p.c : 0);
+            for (int t = 0; t < taps; ++t, dst += (uint32_t)b_bytes, kcol += p.c)
+              if (leader) load_2d(dst, &tmap_b, weights0, kcol, wrow);
           }
+        } else {
+          for (int u = 0; u < p.num_units; ++u, dst += (uint32_t)b_bytes)
+            if (leader) load_2d(dst, &tmap_b, weights0, u * p.block_k, to_first.n0 + b_row);
         }
-      }
-      if (b_resident && which == 0) {   // this CTA's N tile of the weights, once
-        const uint32_t wb = smem_u32(&bar_weights);
-        if (leader) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wb), "r"((uint32_t)resident_bytes) : "memory");
-        uint32_t dst = smem_u32(smem);
-        for (int u = 0; u < p.num_units; ++u, dst += (uint32_t)b_bytes)
-          if (leader) asm volatile(
-              "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(&tmap_b)), "r"(wb),
-              "r"(u * p.block_k), "r"(to_first.n0)
-              : "memory");
       }
       asm volatile("griddepcontrol.wait;" ::: "memory");
       if (which == 0 && leader) TRACE(16, 1);
-      for (int tile = blockIdx.x; live && tile < num_tiles; tile += gridDim.x) {
-        const TileOrigin to = tile == (int)blockIdx.x ? to_first : tile_origin(p, tile);
-        const int m0 = to.m0;
-        if (which == 0 && tile == (int)blockIdx.x && leader) TRACE(16, 7);
-        int img = 0, base_w = 0, base_h = 0;
-        if (p.a_mode == 1) {
-          img = fdiv(m0, p.fd_ohow);
-          const int rem = m0 - img * (p.oh * p.ow);
-          const int oy = fdiv(rem, p.fd_ow);
-          const int ox = rem - oy * p.ow;
-          base_w = ox * p.stride_w - p.pad_w;
-          base_h = oy * p.stride_h - p.pad_h;
-        }
-        if (halo) {
+      if (halo) {
+        for (int tile = first_own; live && tile < num_tiles; tile += tile_step) {
+          const TileOrigin to = tile == first_own ? to_first : tile_origin(p, tile, rank);
           for (int cb = 0; cb < num_kb; ++cb) {
             const bool my_stage = two_issuers || turn == 0;   // (a single producer takes every stage)
             turn ^= 1;
@@ -477,23 +506,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (leader) TRACE(which * 2, pseq);
             const uint32_t sa = smem_base + (uint32_t)(stage * stage_bytes);
             const uint32_t bar = full0 + 8u * (uint32_t)stage;
-            if (leader) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                         "r"((uint32_t)(halo_bytes + (w_resident ? 0 : taps * b_bytes))) : "memory");
+            if (announces) mbar_expect_tx(&bar_full[stage], (uint32_t)(CG * (halo_bytes + (w_resident ? 0 : taps * b_bytes))));
             const int cc = cb * p.block_k;
             const int ca = p.grouped ? cc + to.n0 : cc;   // a group reads its own input channels
-            if (leader) asm volatile(
-                "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)),
-                "r"(bar), "r"(ca), "r"(to.cw - p.pad_w), "r"(to.ch - p.pad_h), "r"(to.cn)
-                : "memory");
+            if (leader) load_4d(sa, &tmap_a, bar, ca, to.cw - p.pad_w, to.ch - p.pad_h, to.cn);
             uint32_t sb = sa + (uint32_t)halo_pad;
             int kcol = cc;
             for (int t = 0; t < (w_resident ? 0 : taps); ++t) {   // (grouped convolutions always keep their weights)
-              if (leader) asm volatile(
-                  "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%3, %4}], [%2];" ::"r"(sb), "l"(reinterpret_cast<uint64_t>(&tmap_b)),
-                  "r"(bar), "r"(kcol), "r"(to.n0)
-                  : "memory");
+              if (leader) load_2d(sb, &tmap_b, bar, kcol, to.n0 + b_row);
               sb += (uint32_t)b_bytes;
               kcol += p.c;
             }
@@ -502,68 +522,86 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             stage += two_issuers ? 1 : 2;
             if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
           }
-          continue;
         }
-        // Units (filter tap x channel block) in weight-matrix order; p.units of them share a stage.
-        int kcol = 0, fy = 0, fx = 0, cc = 0, slot = 0;
-        bool mine = false;
-        uint32_t sa = 0, bar = 0;
-        for (int unit = 0; unit < num_units; ++unit) {
-          if (slot == 0) {
-            mine = two_issuers || turn == 0;
+      } else if (p.a_mode == 0) {
+        for (int tile = first_own; live && tile < num_tiles; tile += tile_step) {
+          const TileOrigin to = tile == first_own ? to_first : tile_origin(p, tile, rank);
+          for (int unit = 0, kcol = 0; unit < num_units;) {
+            const int in_stage = min(p.units, num_units - unit);
+            unit += in_stage;
+            const bool mine = turn == 0;
             turn ^= 1;
-            if (mine) {
-              if (which == 0 && pseq == 0 && leader) TRACE(16, 8);
-              TSTART(tw);
-              if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) { live = false; break; }
-              TADD(0, tw);
-              if (leader) TRACE(which * 2, pseq);
-              sa = smem_base + (uint32_t)(stage * stage_bytes);
-              bar = full0 + 8u * (uint32_t)stage;
-              const int in_stage = min(p.units, num_units - unit);
-              if (leader) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                           "r"((uint32_t)(in_stage * unit_bytes)) : "memory");
+            if (!mine) { kcol += in_stage * p.block_k; continue; }
+            if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) { live = false; break; }
+            if (leader) TRACE(which * 2, pseq);
+            uint32_t sa = smem_base + (uint32_t)(stage * stage_bytes);
+            const uint32_t bar = full0 + 8u * (uint32_t)stage;
+            if (announces) mbar_expect_tx(&bar_full[stage], (uint32_t)(CG * in_stage * unit_bytes));
+            for (int u = 0; u < in_stage; ++u, sa += (uint32_t)unit_bytes, kcol += p.block_k) {
+              if (leader) load_2d(sa, &tmap_a, bar, kcol, to.m0);
+              if (leader && !b_resident) load_2d(sa + (uint32_t)a_bytes, &tmap_b, bar, kcol, to.n0 + b_row);
             }
+            if (leader) TRACE(which * 2 + 1, pseq);
+            ++pseq;
+            stage += 2;
+            if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
           }
-          if (mine && leader) {
-            const int off_w = fx * p.dil_w, off_h = fy * p.dil_h;
-            if (p.a_mode == 2)  // the patch of this tile, shifted by the filter tap; zero fill outside the image
-              asm volatile(
-                  "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)),
-                  "r"(bar), "r"(cc), "r"(to.cw + off_w - p.pad_w), "r"(to.ch + off_h - p.pad_h), "r"(to.cn)
-                  : "memory");
-            else if (p.a_mode == 1)
-              asm volatile(
-                  "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(sa),
-                  "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar), "r"(cc), "r"(base_w), "r"(base_h), "r"(img),
-                  "h"((uint16_t)off_w), "h"((uint16_t)off_h)
-                  : "memory");
-            else
-              asm volatile(
-                  "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                  " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&tmap_a)), "r"(bar),
-                  "r"(cc), "r"(m0)
-                  : "memory");
-            if (!b_resident) asm volatile(
-                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                " [%0], [%1, {%3, %4}], [%2];" ::"r"(sa + (uint32_t)a_bytes), "l"(reinterpret_cast<uint64_t>(&tmap_b)),
-                "r"(bar), "r"(kcol), "r"(to.n0)
-                : "memory");
+        }
+      } else {
+        for (int tile = first_own; live && tile < num_tiles; tile += tile_step) {
+          const TileOrigin to = tile == first_own ? to_first : tile_origin(p, tile, rank);
+          const int m0 = to.m0;
+          if (which == 0 && tile == first_own && leader) TRACE(16, 7);
+          int img = 0, base_w = 0, base_h = 0;
+          if (p.a_mode == 1) {
+            img = fdiv(m0, p.fd_ohow);
+            const int rem = m0 - img * (p.oh * p.ow);
+            const int oy = fdiv(rem, p.fd_ow);
+            const int ox = rem - oy * p.ow;
+            base_w = ox * p.stride_w - p.pad_w;
+            base_h = oy * p.stride_h - p.pad_h;
           }
-          if (mine) sa += (uint32_t)unit_bytes;
-          // next unit
-          kcol += p.block_k;
-          cc += p.block_k;
-          if (cc >= p.c) { cc = 0; if (++fx == p.kw) { fx = 0; ++fy; } }
-          if (++slot == p.units || unit + 1 == num_units) {
-            slot = 0;
-            if (mine) {
-              if (leader) TRACE(which * 2 + 1, pseq);
-              ++pseq;
-              stage += two_issuers ? 1 : 2;
-              if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
+          // Units (filter tap x channel block) in weight-matrix order; p.units of them share a stage.
+          int kcol = 0, fy = 0, fx = 0, cc = 0, slot = 0;
+          bool mine = false;
+          uint32_t sa = 0, bar = 0;
+          for (int unit = 0; unit < num_units; ++unit) {
+            if (slot == 0) {
+              mine = turn == 0;
+              turn ^= 1;
+              if (mine) {
+                if (which == 0 && pseq == 0 && leader) TRACE(16, 8);
+                TSTART(tw);
+                if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) { live = false; break; }
+                TADD(0, tw);
+                if (leader) TRACE(which * 2, pseq);
+                sa = smem_base + (uint32_t)(stage * stage_bytes);
+                bar = full0 + 8u * (uint32_t)stage;
+                const int in_stage = min(p.units, num_units - unit);
+                if (announces) mbar_expect_tx(&bar_full[stage], (uint32_t)(CG * in_stage * unit_bytes));
+              }
+            }
+            if (mine && leader) {
+              const int off_w = fx * p.dil_w, off_h = fy * p.dil_h;
+              if (p.a_mode == 2)   // the patch of this tile, shifted by the filter tap; zero fill outside the image
+                load_4d(sa, &tmap_a, bar, cc, to.cw + off_w - p.pad_w, to.ch + off_h - p.pad_h, to.cn);
+              else
+                load_im2col(sa, &tmap_a, bar, cc, base_w, base_h, img, (uint16_t)off_w, (uint16_t)off_h);
+              load_2d(sa + (uint32_t)a_bytes, &tmap_b, bar, kcol, to.n0 + b_row);
+            }
+            if (mine) sa += (uint32_t)unit_bytes;
+            // next unit
+            kcol += p.block_k;
+            cc += p.block_k;
+            if (cc >= p.c) { cc = 0; if (++fx == p.kw) { fx = 0; ++fy; } }
+            if (++slot == p.units || unit + 1 == num_units) {
+              slot = 0;
+              if (mine) {
+                if (leader) TRACE(which * 2 + 1, pseq);
+                ++pseq;
+                stage += 2;
+                if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
+              }
             }
           }
         }
@@ -582,7 +620,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const int issuers = two_issuers ? 2 : 1;
       const int me = warp == 1 ? 0 : 1;
       const bool leader = elect_one();
-      const uint32_t idesc = umma_idesc_i8(p.grouped ? p.c : p.block_n);
+      const uint32_t idesc = umma_idesc_i8(p.grouped ? p.c : p.block_n, CG * BLOCK_M);
       const uint64_t desc_a0 = umma_desc(smem_u32(ring), p.block_k);
       const uint64_t desc_w0 = umma_desc(smem_u32(smem), p.grouped ? p.c : p.block_k);  // resident weights (a_mode 4)
       const uint32_t w_lo0 = (uint32_t)desc_w0, w_hi = (uint32_t)(desc_w0 >> 32);
@@ -597,28 +635,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const uint32_t a_q = (uint32_t)a_bytes >> 4, b_q = (uint32_t)b_bytes >> 4;
       const uint32_t halo_pad_q = (uint32_t)halo_pad >> 4, halo_row_q = (uint32_t)(halo_w * p.block_k) >> 4;
       const uint32_t pix_q = (uint32_t)p.block_k >> 4;   // grouped: one pixel of the halo row
-      // grouped: where filter column t of group g starts inside a halo row (16-byte units).  Without
-      // folding that is halo pixel t, the group's own 32 channels.  With F sub-pixels per pixel the
-      // group of sub-pixel a reads sub-pixel a + t - 1: the same halo pixel (1) for most, the last
-      // sub-pixel of pixel 0 / the first of pixel 2 at the ends.
-      uint32_t g_off[4][3];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const int fold = p.group_fold > 1 ? p.group_fold : 1;
-        const int cs = p.block_n / fold;          // channels per sub-pixel
-        const int gps = cs >> 5;                  // 32-channel groups per sub-pixel
-        const int a = p.group_fold > 1 ? g / gps : 0, h = p.group_fold > 1 ? g - a * gps : g;
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-          int px = t, b = 0;
-          if (p.group_fold > 1) {
-            const int bp = a + t - 1;
-            px = bp < 0 ? 0 : (bp >= fold ? 2 : 1);
-            b = bp - (px - 1) * fold;
-          }
-          g_off[g][t] = (uint32_t)px * pix_q + (uint32_t)((b * cs + h * 32) >> 4);
-        }
-      }
       // this issuer's first tile is the CTA's tile number `me`: me * num_kb stages and me accumulators in
       int stage = (me * num_kb) % p.stages;
       uint32_t phase = (uint32_t)((me * num_kb) / p.stages) & 1u;
@@ -638,8 +654,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       int owed_stage = -1, owed_acc = -1;
       auto flush = [&]() {
         if (leader) {
-          if (owed_acc >= 0) mma_commit(&bar_acc_full[owed_acc]);
-          if (owed_stage >= 0) mma_commit(&bar_empty[owed_stage]);
+          if (owed_acc >= 0) mma_commit<CG>(&bar_acc_full[owed_acc]);
+          if (owed_stage >= 0) mma_commit<CG>(&bar_empty[owed_stage]);
         }
         owed_acc = owed_stage = -1;
       };
@@ -652,24 +668,81 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       TDECL;
       TSTART(tl);
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      if ((w_resident || b_resident) && blockIdx.x < num_tiles && !mbar_wait(&bar_weights, 0u, &abort_flag, 7)) live = false;
-      for (int tile = blockIdx.x + me * (int)gridDim.x; live && tile < num_tiles; tile += issuers * (int)gridDim.x) {
-        TSTART(tw);
-        if (!ensure(&bar_acc_empty[acc], acc_phase ^ 1, 2)) { live = false; break; }
-        TADD(1, tw);
-        if (leader) TRACE(6, tseq);
-        ++tseq;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.block_n);
-        int unit = 0;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!ensure(&bar_full[stage], phase, 3)) { live = false; break; }
-          TADD(2, tw);
-          if (leader) TRACE(4, mseq);
+      if (rank != 0) live = false;   // the first CTA issues for both
+      if (live && (w_resident || b_resident) && first_own < num_tiles && !mbar_wait(&bar_weights, 0u, &abort_flag, 7)) live = false;
+      // (two loops, each with little code: what a loop's other branch holds costs its instructions' way to the SM)
+      if (!halo) {
+        for (int tile = first_own; live && tile < num_tiles; tile += tile_step) {
+          if (!mbar_wait(&bar_acc_empty[acc], acc_phase ^ 1, &abort_flag, 2)) { live = false; break; }
+          if (leader) TRACE(6, tseq);
+          ++tseq;
           tc_fence_after();
-          const uint32_t st = a_lo0 + stage_q * (uint32_t)stage;
-          if (halo) {
-            TSTART(ti);
+          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.block_n);
+          for (int unit = 0; unit < num_units;) {
+            if (!mbar_wait(&bar_full[stage], phase, &abort_flag, 3)) { live = false; break; }
+            if (leader) TRACE(4, mseq);
+            tc_fence_after();
+            const int in_stage = min(p.units, num_units - unit);
+            uint32_t al = a_lo0 + stage_q * (uint32_t)stage;
+            // B next to A in the stage, or K block `unit` of the resident weights
+            uint32_t bl = b_resident ? w_lo0 + (uint32_t)unit * b_q : al + a_q;
+            const uint32_t b_step = b_resident ? b_q : unit_q;
+            // (a stage of these modes is one to four instructions groups: its commit follows at once --
+            //  deferring it would only take a stage out of a ring that is three deep)
+            if (leader) {
+              if (nk == 4) {
+                for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<4, CG>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
+              } else if (nk == 2) {
+                for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<2, CG>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
+              } else {
+                for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<1, CG>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
+              }
+              mma_commit<CG>(&bar_empty[stage]);
+              TRACE(5, mseq);
+            }
+            unit += in_stage;
+            ++mseq;
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          }
+          if (!live) break;
+          if (leader) mma_commit<CG>(&bar_acc_full[acc]);
+          if (++acc == p.acc_bufs) { acc = 0; acc_phase ^= 1; }
+        }
+      } else {
+        // grouped: where filter column t of group g starts inside a halo row (16-byte units).  Without
+        // folding that is halo pixel t, the group's own 32 channels.  With F sub-pixels per pixel the
+        // group of sub-pixel a reads sub-pixel a + t - 1: the same halo pixel (1) for most, the last
+        // sub-pixel of pixel 0 / the first of pixel 2 at the ends.
+        uint32_t g_off[4][3] = {};
+        if (p.grouped)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int fold = p.group_fold > 1 ? p.group_fold : 1;
+          const int cs = p.block_n / fold;          // channels per sub-pixel
+          const int gps = cs >> 5;                  // 32-channel groups per sub-pixel
+          const int a = p.group_fold > 1 ? g / gps : 0, h = p.group_fold > 1 ? g - a * gps : g;
+#pragma unroll
+          for (int t = 0; t < 3; ++t) {
+            int px = t, b = 0;
+            if (p.group_fold > 1) {
+              const int bp = a + t - 1;
+              px = bp < 0 ? 0 : (bp >= fold ? 2 : 1);
+              b = bp - (px - 1) * fold;
+            }
+            g_off[g][t] = (uint32_t)px * pix_q + (uint32_t)((b * cs + h * 32) >> 4);
+          }
+        }
+        for (int tile = first_own + me * tile_step; live && tile < num_tiles; tile += issuers * tile_step) {
+          if (!ensure(&bar_acc_empty[acc], acc_phase ^ 1, 2)) { live = false; break; }
+          if (leader) TRACE(6, tseq);
+          ++tseq;
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.block_n);
+          for (int kb = 0; kb < num_kb; ++kb) {
+            if (!ensure(&bar_full[stage], phase, 3)) { live = false; break; }
+            if (leader) TRACE(4, mseq);
+            tc_fence_after();
+            const uint32_t st = a_lo0 + stage_q * (uint32_t)stage;
             if (p.grouped) {
               // every group of the N tile: its own columns of the halo rows, its own 9 weight tiles,
               // its own accumulator columns (the first tap overwrites them)
@@ -683,7 +756,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     const uint32_t al = st + (uint32_t)fy * halo_row_q;
 #pragma unroll
                     for (int fx = 0; fx < 3; ++fx) {
-                      if (leader) mma_i8_k<1>(d_blk, al + g_off[g][fx], halo_hi, bl, w_hi, idesc, (uint32_t)(fy | fx));
+                      if (leader) mma_i8_k<1, CG>(d_blk, al + g_off[g][fx], halo_hi, bl, w_hi, idesc, (uint32_t)(fy | fx));
                       bl += b_q;
                     }
                     if (fy == 0 && g == 0) flush();
@@ -699,52 +772,26 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 uint32_t al = st + (uint32_t)fy * halo_row_q;
 #pragma unroll
                 for (int fx = 0; fx < 3; ++fx) {
-                  if (leader) mma_i8_k<2>(d_tmem, al, halo_hi, bl, a_hi, idesc, (uint32_t)(kb | fy | fx));
+                  if (leader) mma_i8_k<2, CG>(d_tmem, al, halo_hi, bl, a_hi, idesc, (uint32_t)(kb | fy | fx));
                   al += 4u;   // one pixel of 64 channels
                   bl += b_q;
                 }
                 if (fy == 0) flush();
               }
             }
-            TADD(13, ti);
             owed_stage = stage;
             if (leader) TRACE(5, mseq);
             ++mseq;
-            TADD(14, ti);
-            TSET(tw);
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
-            continue;
           }
-          const int in_stage = min(p.units, num_units - unit);
-          uint32_t al = st;
-          // B next to A in the stage, or K block `unit` of the resident weights
-          uint32_t bl = b_resident ? w_lo0 + (uint32_t)unit * b_q : st + a_q;
-          const uint32_t b_step = b_resident ? b_q : unit_q;
-          // (a stage of these modes is one to four instructions groups: its commit follows at once --
-          //  deferring it would only take a stage out of a ring that is three deep)
-          if (leader) {
-            if (nk == 4) {
-              for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<4>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
-            } else if (nk == 2) {
-              for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<2>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
-            } else {
-              for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<1>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
-            }
-            mma_commit(&bar_empty[stage]);
-            TRACE(5, mseq);
-          }
-          unit += in_stage;
-          ++mseq;
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          if (!live) break;
+          owed_acc = acc;
+          // on to this issuer's next tile: past the other issuer's stages and accumulator
+          for (int k = 0; k < issuers; ++k)
+            if (++acc == p.acc_bufs) { acc = 0; acc_phase ^= 1; }
+          for (int k = 0; k < (issuers - 1) * num_kb; ++k)
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-        if (!live) break;
-        owed_acc = acc;
-        if (!halo) flush();
-        // on to this issuer's next tile: past the other issuer's stages and accumulator
-        for (int k = 0; k < issuers; ++k)
-          if (++acc == p.acc_bufs) { acc = 0; acc_phase ^= 1; }
-        for (int k = 0; k < (issuers - 1) * num_kb; ++k)
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
       if (live) flush();
       TADD(3, tl);
@@ -770,8 +817,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint8_t* group_base = smem + p.ring_bytes + (size_t)group * p.io_bufs * buf_bytes;
     const bool vec_ok = (p.y_dtype == CVMK_I8) ? (p.oc % 16 == 0) : (p.oc % 4 == 0);
     const bool four_acc = p.acc_bufs == 4;
-    const int stride_tiles = 2 * gridDim.x;
-    const int first_tile = blockIdx.x + group * gridDim.x;
+    const int stride_tiles = 2 * tile_step;
+    const int first_tile = first_own + group * tile_step;
+    const uint32_t acc_empty0 = map_rank(smem_u32(&bar_acc_empty[0]), 0);   // with the issuer
     // patch mode: this thread's pixel inside the patch
     int pr_w = 0, pr_h = 0, pr_n = 0;
     if (p.a_mode >= 2) {
@@ -785,34 +833,35 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     (void)leader;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int tile = first_tile; tile < num_tiles; tile += stride_tiles, ++k) {
-      const TileOrigin to = tile_origin(p, tile);
+      const TileOrigin to = tile_origin(p, tile, rank);
       const int n0 = to.n0;
       int row = to.m0 + row_in_tile;  // linear output row; m_total marks a row outside the tensor
       if (p.a_mode >= 2) {
         const int ow = to.cw + pr_w, oh = to.ch + pr_h, on = to.cn + pr_n;
         row = (ow < p.ow && oh < p.oh && on * p.oh * p.ow < p.m_total) ? (on * p.oh + oh) * p.ow + ow : p.m_total;
       }
+      if (!to.live) row = p.m_total;
       const int buf = p.io_bufs == 2 ? (k & 1) : 0;
       const uint32_t use = (uint32_t)(p.io_bufs == 2 ? (k >> 1) : k);  // how often this buffer was used before
       uint8_t* io_base = group_base + (size_t)buf * buf_bytes;
       TSTART(tw);
       // this group's k-th tile: accumulator g, or g and g + 2 in turn
       const int acc = four_acc ? group + 2 * (k & 1) : group;
-      bool ok = mbar_wait(&bar_acc_full[acc], (uint32_t)((four_acc ? k >> 1 : k) & 1), &abort_flag, 4);
+      // the staging buffer is ours: its previous store has been read, or the operand tile landed
+      bool ok = !p.tma_out || mbar_wait(&bar_res[group][buf], use & 1u, &abort_flag, 5);
+      TADD(5 + 4 * group, tw);
+      if (leader) TRACE(8 + 3 * group, k);
+      ok = ok && mbar_wait(&bar_acc_full[acc], (uint32_t)((four_acc ? k >> 1 : k) & 1), &abort_flag, 4);
       TADD(4 + 4 * group, tw);
       if (leader) TRACE(7 + 3 * group, k);
       tc_fence_after();
-      // the staging buffer is ours: its previous store has been read, or the operand tile landed
-      if (ok && p.tma_out) ok = mbar_wait(&bar_res[group][buf], use & 1u, &abort_flag, 5);
-      TADD(5 + 4 * group, tw);
-      if (leader) TRACE(8 + 3 * group, k);
       if (!ok) break;
       if (ok) {
         const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * p.block_n);
         if (p.fast_mode) {
           const int chunks = min(p.block_n, p.oc - n0) >> 5;  // OC is a multiple of 32 on this path
           const int32_t* brow = bias_s + n0;
-          uint64_t* early_free = four_acc ? nullptr : &bar_acc_empty[acc];
+          const uint32_t early_free = four_acc ? 0u : acc_empty0 + 8u * (uint32_t)acc;
           switch (p.fast_variant + 8 * p.fast_wide) {
             case 0: fast_row<0, 0, 0>(p, tbase, chunks, brow, io_base, panel_size, row_in_tile, pw, early_free); break;
             case 1: fast_row<1, 0, 0>(p, tbase, chunks, brow, io_base, panel_size, row_in_tile, pw, early_free); break;
@@ -900,7 +949,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       if (p.tma_out) fence_async_smem();  // make the staged bytes visible to the TMA engine
       __syncwarp();
       if (lane == 0) {
-        if (!p.fast_mode || four_acc) mbar_arrive(&bar_acc_empty[acc]);   // (else fast_row has handed it back already)
+        if (!p.fast_mode || four_acc) arrive_at(acc_empty0 + 8u * (uint32_t)acc);   // (else fast_row has handed it back already)
         if (p.tma_out) mbar_arrive(&bar_staged[group][buf]);
       }
       TADD(6 + 4 * group, tw);
@@ -920,11 +969,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const int panel_size = BLOCK_M * p.panel_bytes;
     const int buf_bytes = p.panels * panel_size;
     uint8_t* io_all = smem + p.ring_bytes;
+    // (it touches nothing of the other CTA: the arrival the teardown waits for)
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     auto buffer_of = [&](int g, int b) { return io_all + (size_t)(g * p.io_bufs + b) * buf_bytes; };
     auto hand_back = [&](int g, int b, int next_tile) {
       if (next_tile >= num_tiles) return;
       if (!has_res) { if (leader) mbar_arrive(&bar_res[g][b]); return; }
-      const TileOrigin to = tile_origin(p, next_tile);
+      const TileOrigin to = tile_origin(p, next_tile, rank);
       uint8_t* dst = buffer_of(g, b);
       if (leader) {
         mbar_expect_tx(&bar_res[g][b], (uint32_t)buf_bytes);
@@ -939,17 +991,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // every buffer starts free (or with the operand of its first tile on the way)
     for (int g = 0; g < 2; ++g)
-      for (int b = 0; b < p.io_bufs; ++b) hand_back(g, b, (int)blockIdx.x + (2 * b + g) * (int)gridDim.x);
+      for (int b = 0; b < p.io_bufs; ++b) hand_back(g, b, first_own + (2 * b + g) * tile_step);
     int i = 0;  // position in this CTA's tile sequence
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++i) {
+    for (int tile = first_own; tile < num_tiles; tile += tile_step, ++i) {
       const int g = i & 1, k = i >> 1;
       const int b = p.io_bufs == 2 ? (k & 1) : 0;
       const uint32_t use = (uint32_t)(p.io_bufs == 2 ? (k >> 1) : k);
       if (!mbar_wait(&bar_staged[g][b], use & 1u, &abort_flag, 6)) break;
       if (leader) TRACE(13, i);
-      const TileOrigin to = tile_origin(p, tile);
+      const TileOrigin to = tile_origin(p, tile, rank);
       const uint8_t* src = buffer_of(g, b);
-      if (leader) {
+      if (leader && to.live) {
         for (int q = 0; q < p.panels; ++q) {
           if (to.n0 + q * 128 >= p.oc) break;
           if (p.a_mode >= 2) tma_store_4d(&tmap_y, src + (size_t)q * panel_size, to.n0 + q * 128, to.cw, to.ch, to.cn);
@@ -960,7 +1012,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         TRACE(14, i);
       }
       __syncwarp();
-      hand_back(g, b, tile + 2 * p.io_bufs * (int)gridDim.x);
+      hand_back(g, b, tile + 2 * p.io_bufs * tile_step);
       if (leader) TRACE(15, i);
     }
     // Every store has been read out of shared memory (wait_group.read above); the writes
@@ -969,20 +1021,21 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   }
 
   // ------------------------------------------------------------------ teardown
+  // Every warp leaves on its own.  The TMEM columns of both CTAs go back, and the CTAs with them, once every warp that
+  // reads them, reads the other's operands or reports to its barriers has arrived here.
   __syncwarp();
   if (threadIdx.x == 0) TRACE(16, 3);
-  tc_fence_before();
-  __syncthreads();
-  if (threadIdx.x == 0) TRACE(16, 4);
   if (abort_flag) {
-    // Give copies that may still be in flight time to land before shared memory is released.
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    if (threadIdx.x == 0 && p.status) atomicOr(p.status, 0x100 | abort_flag);
-    __syncthreads();
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);   // copies that may still be in flight land before shared memory is released
+    if (lane == 0 && p.status) atomicOr(p.status, 0x100 | abort_flag);
+    __syncwarp();
   }
+  tc_fence_before();
+  if (warp != IO_WARP || !p.tma_out) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   if (warp == 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_after();
-    tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+    tmem_dealloc<CG>(tmem_base, (uint32_t)p.tmem_cols);
     if (lane == 0) TRACE(16, 5);
   }
 }
@@ -1106,16 +1159,25 @@ bool grouped_supported(const cvmk_conv_desc& d) {
   return halo_tiles_fit(d);
 }
 
-// About how long the persistent kernel takes over a layer, in microseconds (see choose_small): what a launch costs
-// whatever it holds, and the tiles of the CTA with most of them, each the longer of its operands at 180 KB a
-// microsecond and its requantisation.  Halo tiles are bound by their instructions.
-double tc_launch_us(const cvmk_conv_desc& d, int a_mode, int64_t m_tiles, int sms) {
+// Output channels per tile of the persistent kernel: 128 where 256 would leave half of the SMs without a tile of a long
+// reduction (3 x 3 over 512 channels at 7 x 7, 64 images: 15.5 against 12.2 us).
+int tc_block_n(const cvmk_conv_desc& d, int64_t m_tiles, int sms) {
   const int bn = pick_block_n(d.OC);
+  const bool idle = (m_tiles + 1) / 2 * ((d.OC + 255) / 256) * 4 <= sms && (int64_t)d.KH * d.KW * d.C >= 1024;
+  return bn == 256 && idle ? 128 : bn;
+}
+
+// About how long the persistent kernel takes over a layer, in microseconds (see choose_small): what a launch costs
+// whatever it holds (5.0 measured; 0.8 more because among small launches it is a change of kernels and back, which
+// a chain of equal layers does not show: ResNet-50, 13 images of 197 x 197 318 -> 310 us on the device with it), and
+// the tiles of the pair with most of them, each the longer of its operands at 130 KB a microsecond and its
+// requantisation.  Halo tiles are bound by their instructions.
+double tc_launch_us(const cvmk_conv_desc& d, int a_mode, int64_t m_tiles, int sms) {
   if (a_mode == 3) m_tiles = (int64_t)((d.OW + 7) / 8) * ((d.OH + 15) / 16) * d.N;
-  const int64_t tiles = m_tiles * ((d.OC + bn - 1) / bn), rounds = (tiles + sms - 1) / sms;
-  if (a_mode == 3) return 4.6 + rounds * (0.45 + 1.0 * d.C * bn / (128 * 128));
-  const double kb = (double)d.KH * d.KW * d.C * (BLOCK_M + bn) / 1024;
-  return 6.1 - 1.1 * bn / 256 + rounds * std::max(kb / 180, 1.55 * bn / 256) + tiles * kb / 36000;
+  const int bn = tc_block_n(d, m_tiles, sms), pairs = sms / 2;
+  const int64_t rounds = ((m_tiles + 1) / 2 * ((d.OC + bn - 1) / bn) + pairs - 1) / pairs;
+  if (a_mode == 3) return 5.4 + rounds * (0.45 + 1.0 * d.C * bn / (128 * 128));
+  return 5.8 + rounds * std::max((double)d.KH * d.KW * d.C * (BLOCK_M + bn / 2) / 1024 / 130, 1.0 * bn / 256);
 }
 
 // Which launches go to the small-launch kernel, and how it cuts them.
@@ -1310,6 +1372,12 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
       }
     }
   }
+  if (!small.split && !halo) {
+    const int64_t m_tiles = plan->a_im2col == 2 ? (int64_t)((d->OW + patch_w - 1) / patch_w) * ((d->OH + patch_h - 1) / patch_h) * ((d->N + patch_n - 1) / patch_n)
+                                                : ((int64_t)d->N * d->OH * d->OW + BLOCK_M - 1) / BLOCK_M;
+    plan->block_n = bn = tc_block_n(*d, m_tiles, sm_count());
+  }
+  const int b_rows = bn / 2;   // rows of B that a CTA of the pair loads
   plan->panels = bn == 256 ? 2 : 1;
   plan->panel_bytes = bn < 128 ? bn : 128;
   // Staging: each epilogue group owns one buffer, or two when they fit beside an operand ring that
@@ -1324,12 +1392,12 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // halo alone.
   const int halo_pad = ((10 * 18 * bk) + 1023) & ~1023;
   int resident = 0;
-  const int sms_all = sm_count();
+  const int sms_all = sm_count(), pairs = sms_all / 2;
   // (grouped: the grid is cut to a multiple of the N tiles below, so that every tile of a CTA
   //  covers the same groups and their 9 weight tiles each can stay as well)
-  if (halo && (d->OC <= bn || (grouped && d->OC / bn <= sms_all)) && !dev_env("CVM_B200_NO_RESIDENT_WEIGHTS")) {
+  if (halo && (d->OC <= bn || (grouped && d->OC / bn <= pairs)) && !dev_env("CVM_B200_NO_RESIDENT_WEIGHTS")) {
     // all channel blocks (one or two) stay, if three halo stages and one staging buffer per group still fit
-    const int all = grouped ? d->KH * d->KW * bn * cg : (cg / bk) * d->KH * d->KW * bn * bk;
+    const int all = (grouped ? d->KH * d->KW * bn * cg : (cg / bk) * d->KH * d->KW * bn * bk) / 2;   // a CTA's half
     if (budget - all - 2 * group_bytes >= 3 * halo_pad) {
       resident = all;
       plan->a_im2col = 4;
@@ -1339,16 +1407,20 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     set_error("conv2d_tc_prepare: the weights of a grouped convolution's N tile must fit shared memory");
     return CVMK_ERR_UNSUPPORTED;
   }
-  const int halo_stage = halo ? (resident ? halo_pad : halo_pad + d->KH * d->KW * bn * bk) : 0;
+  const int halo_stage = halo ? (resident ? halo_pad : halo_pad + d->KH * d->KW * b_rows * bk) : 0;
   if (halo) {
     if (plan->tma_out && (budget - resident - 4 * group_bytes) / halo_stage >= 3) plan->io_bufs = 2;
   } else if (plan->tma_out && !dev_env("CVM_B200_SINGLE_STAGING")) {
-    auto ring_depth = [&](int k) { return (budget - 4 * group_bytes) / ((BLOCK_M + bn) * k); };
+    auto ring_depth = [&](int k) { return (budget - 4 * group_bytes) / ((BLOCK_M + b_rows) * k); };
     // Long reductions want the shared memory for operands in flight (three 128-byte K blocks
     // cover the load latency, three 64-byte ones do not), short ones for the second staging buffer
     // (their tiles are bound by the epilogue).
-    const bool deep_ring_first = bk == 128 && k_all >= 256 && ring_depth(128) < 3 &&
-                                 (budget - 2 * group_bytes) / ((BLOCK_M + bn) * 128) >= 3 && !dev_env("CVM_B200_DOUBLE_STAGING");
+    // A residual join of three tiles and more a CTA wants the second buffer even more: with one, the operand of a group's
+    // next tile is requested only when its last tile has left (256 -> 1024 at 14 x 14, 256 images 33.3 -> 27.2 us).
+    const int64_t rows = (int64_t)d->N * d->OH * d->OW;
+    const bool joins = plan->res_step >= 0 && k_all <= 256 && (rows + BLOCK_M - 1) / BLOCK_M * ((d->OC + bn - 1) / bn) > 2LL * sms_all;
+    const bool deep_ring_first = bk == 128 && !joins && k_all >= 256 && ring_depth(128) < 3 &&
+                                 (budget - 2 * group_bytes) / ((BLOCK_M + b_rows) * 128) >= 3 && !dev_env("CVM_B200_DOUBLE_STAGING");
     if (deep_ring_first) plan->io_bufs = 1;
     else if (ring_depth(bk) >= 3) plan->io_bufs = 2;
     else if (bk == 128 && k_all <= 512 && ring_depth(64) >= 3) { plan->io_bufs = 2; bk = 64; }
@@ -1363,9 +1435,9 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     const int sms = sms_all;
     const int64_t m_tiles = ((int64_t)d->N * d->OH * d->OW + BLOCK_M - 1) / BLOCK_M;
     const int nt = (d->OC + bn - 1) / bn;
-    const int64_t w_bytes = (int64_t)d->C * bn;
+    const int64_t w_bytes = (int64_t)d->C * b_rows;
     const int io1 = plan->tma_out ? 2 * plan->io_bufs * group_bytes : 0;
-    if (m_tiles * nt >= 2LL * sms && sms % nt == 0 && d->OC % bn == 0 &&
+    if (m_tiles * nt >= 2LL * sms && pairs % nt == 0 && d->OC % bn == 0 &&
         budget - io1 - w_bytes >= 4LL * BLOCK_M * bk) {
       plan->b_resident = 1;
       resident = (int)w_bytes;
@@ -1375,7 +1447,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   // Every hand-over of a ring stage (TMA completion -> MMA thread -> commit -> producer) costs a
   // fixed latency of several hundred cycles whatever the stage holds, so small (tap, channel block)
   // units are grouped: up to four per stage, about 48 KB, while the ring stays three deep.
-  const int unit_bytes = (BLOCK_M + (plan->b_resident ? 0 : bn)) * bk;
+  const int unit_bytes = (BLOCK_M + (plan->b_resident ? 0 : b_rows)) * bk;
   const int num_units = (int)(k_all / bk);
   int units = 48 * 1024 / unit_bytes;
   if (units > 4) units = 4;
@@ -1392,6 +1464,9 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
   plan->stages = stages;
   plan->ring_bytes = resident + stages * stage_bytes;  // resident weights (a_im2col 4) sit in front of the ring
   plan->smem_bytes = plan->ring_bytes + io_bytes + 1024;
+  // A pair takes its TMEM columns on two SMs.  No other kernel's clusters may hold columns beside it and wait for
+  // CTAs that wait for its own: it leaves them no shared memory (conv_small's take 25 KB and more).
+  plan->smem_bytes = std::max(plan->smem_bytes, 206 * 1024);
   if (small.split > 0) {
     plan->stages = small.stages;
     plan->smem_bytes = small_smem_bytes(bk, bn, small.stages * small.group, small.split);
@@ -1423,7 +1498,7 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     r = encode_rows(enc_tiled, ta, d->x, m_total, d->C, bk, small.swap ? bn : BLOCK_M, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
   }
   if (r != CUDA_SUCCESS) { set_error("conv2d_tc_prepare: activation tensor map rejected (CUresult %d)", (int)r); return CVMK_ERR_CUDA; }
-  r = encode_rows(enc_tiled, tb, d->w, d->OC, k_total, grouped ? cg : bk, grouped ? cg : (small.swap ? BLOCK_M : bn), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  r = encode_rows(enc_tiled, tb, d->w, d->OC, k_total, grouped ? cg : bk, small.split ? (small.swap ? BLOCK_M : bn) : (grouped ? cg / 2 : b_rows), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   if (r != CUDA_SUCCESS) { set_error("conv2d_tc_prepare: weight tensor map rejected (CUresult %d)", (int)r); return CVMK_ERR_CUDA; }
   if (plan->tma_out) {
     auto encode_out = [&](unsigned char* map, const void* base, CUtensorMapL2promotion promo) {
@@ -1445,12 +1520,15 @@ extern "C" int cvmk_conv2d_tc_prepare(const cvmk_conv_desc* d, cvmk_conv_plan* p
     num_m_tiles = (int64_t)((d->OW + patch_w - 1) / patch_w) * ((d->OH + patch_h - 1) / patch_h) *
                   ((d->N + patch_n - 1) / patch_n);
   const int64_t num_n_tiles = (d->OC + bn - 1) / bn;
-  const int sms = sms_all;
   int64_t tiles = num_m_tiles * num_n_tiles;
   if (small.swap) tiles = ((d->OC + BLOCK_M - 1) / BLOCK_M) * ((m_total + bn - 1) / bn);
-  plan->grid = (int)(tiles < sms ? tiles : sms);
-  if (small.split > 0) plan->grid = (int)(tiles * small.split);
-  if (grouped && plan->a_im2col == 4) plan->grid = (int)(plan->grid / num_n_tiles * num_n_tiles);   // tile t + k * grid: same group as t
+  if (small.split > 0) {
+    plan->grid = (int)(tiles * small.split);
+  } else {
+    int64_t walkers = std::min<int64_t>((num_m_tiles + 1) / 2 * num_n_tiles, pairs);
+    if (grouped) walkers = walkers / num_n_tiles * num_n_tiles;   // tile t + k * walkers: same group as t
+    plan->grid = 2 * (int)walkers;
+  }
   return CVMK_OK;
 }
 
@@ -1491,10 +1569,7 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   p.fd_ohow = make_fastdiv(d.OH * d.OW);
   p.fd_ow = make_fastdiv(d.OW);
   p.acc_bufs = (plan->block_n <= 128 && !dev_env("CVM_B200_TWO_ACCUMULATORS")) ? 4 : 2;
-  int cols = p.acc_bufs * plan->block_n;
-  int pow2 = 32;
-  while (pow2 < cols) pow2 *= 2;
-  p.tmem_cols = pow2;
+  p.tmem_cols = 512;   // (all of it whatever the tile takes: the columns then have the same addresses in both CTAs)
   p.status = d.status;
   p.bias_static = d.bias_static;
   p.w = d.w;
@@ -1626,9 +1701,9 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   cudaGetDevice(&dev);
   bool& attr_set = attr_set_dev[dev & 63];
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_DYNAMIC_MAX);
-    if (check_cuda(e, "cudaFuncSetAttribute(conv_tc_kernel)")) return CVMK_ERR_CUDA;
+    if (check_cuda(cudaFuncSetAttribute(conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYNAMIC_MAX),
+                   "cudaFuncSetAttribute(conv_tc_kernel)"))
+      return CVMK_ERR_CUDA;
     attr_set = true;
   }
   CUtensorMap ta, tb, ty, tr;
@@ -1642,12 +1717,15 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = (size_t)plan->smem_bytes;
   cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   static const bool pdl = dev_env("CVM_B200_NO_PDL") == nullptr;
-  cfg.attrs = &attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
   if (check_cuda(cudaLaunchKernelEx(&cfg, conv_tc_kernel, ta, tb, ty, tr, p), "conv_tc_kernel launch")) return CVMK_ERR_CUDA;
   return CVMK_OK;
 }

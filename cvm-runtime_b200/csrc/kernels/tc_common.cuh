@@ -15,6 +15,18 @@ constexpr uint32_t SPIN_LIMIT = 1u << 19;  // x 2 us per hardware wait
 __device__ uint32_t g_wait_hint = 2000u;  // development builds: suspend-time hint of the waits, settable
 #endif
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The address, in the cluster's shared window, of `addr` in the CTA of rank `rank`.
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+  return d;
+}
+
 // Division of a non-negative 31-bit number by a divisor fixed at launch: q = umulhi(n, mul) >> shr
 // (mul = ceil(2^(31 + ceil(log2 d)) / d)); d = 1 is flagged by mul = 0.  Every thread that walks
 // tiles divides several times per tile, and a hardware-emulated 32-bit division is a dependent
@@ -151,16 +163,21 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
+// (CG: CTAs that multiply together, 1, or 2 for the two of a pair, which both allocate and free)
+template <int CG = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(slot)),
-               "r"(cols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (CG == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 }
+template <int CG = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols)
-               : "memory");
+  if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                        uint32_t idesc, uint32_t accumulate) {
@@ -178,40 +195,38 @@ __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_
 // changes from instruction to instruction, so the issuing thread spends one 32-bit add per
 // operand and instruction.  That matters: the issuing warp shares its scheduler with epilogue
 // warps, and every instruction of its loop waits its turn.
-template <int NK>
+// CG = 2: one instruction of both CTAs of a pair, M = 256: rows 0..127 of A and of the result lie with the first
+// CTA, the others with the second, at the same shared-memory offsets and TMEM addresses; half of B's rows with each.
+#define CVMK_MMA_I8(CG)                                               \
+  "{\n"                                                               \
+  ".reg .pred p;\n"                                                   \
+  ".reg .b64 da, db;\n"                                               \
+  "setp.ne.b32 p, %6, 0;\n"                                           \
+  "mov.b64 da, {%1, %2};\n"                                           \
+  "mov.b64 db, {%3, %4};\n"                                           \
+  "tcgen05.mma.cta_group::" CG ".kind::i8 [%0], da, db, %5, p;\n"     \
+  "}\n"
+template <int NK, int CG = 1>
 __device__ __forceinline__ void mma_i8_k(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                          uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      ".reg .b64 da, db;\n"
-      "setp.ne.b32 p, %6, 0;\n"
-      "mov.b64 da, {%1, %2};\n"
-      "mov.b64 db, {%3, %4};\n"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
 #pragma unroll
-  for (int j = 1; j < NK; ++j) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        ".reg .b64 da, db;\n"
-        "setp.eq.b32 p, 0, 0;\n"
-        "mov.b64 da, {%1, %2};\n"
-        "mov.b64 db, {%3, %4};\n"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n"
-        "}\n" ::"r"(d_tmem),
-        "r"(a_lo + 2u * (uint32_t)j), "r"(a_hi), "r"(b_lo + 2u * (uint32_t)j), "r"(b_hi), "r"(idesc)
-        : "memory");
+  for (int j = 0; j < NK; ++j) {
+    const uint32_t al = a_lo + 2u * (uint32_t)j, bl = b_lo + 2u * (uint32_t)j, acc = j == 0 ? accumulate : 1u;
+    if (CG == 2) asm volatile(CVMK_MMA_I8("2")::"r"(d_tmem), "r"(al), "r"(a_hi), "r"(bl), "r"(b_hi), "r"(idesc), "r"(acc) : "memory");
+    else asm volatile(CVMK_MMA_I8("1")::"r"(d_tmem), "r"(al), "r"(a_hi), "r"(bl), "r"(b_hi), "r"(idesc), "r"(acc) : "memory");
   }
 }
-// Arrive on `bar` once every tcgen05.mma issued so far by this thread has finished.
+#undef CVMK_MMA_I8
+// Arrive on `bar` once every tcgen05.mma issued so far by this thread has finished; CG = 2: on the
+// barriers at this place in both CTAs of the pair.
+template <int CG = 1>
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
+  if (CG == 2)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int32_t (&v)[32]) {
   asm volatile(
@@ -226,6 +241,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int32_t (&v)[32]) {
       : "r"(taddr)
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The same in two steps: 32 columns set out, and are there.  The registers hold nothing before the wait, which
+// therefore names them.
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, int32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32_wait(int32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])::"memory");
 }
 
 // Two adjacent 32-column chunks with one wait: both loads are in flight together, so a row of the
@@ -253,10 +281,10 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, int row_bytes) {
   d |= layout << 61;
   return d;
 }
-// Instruction descriptor: s8 x s8 -> s32, both operands K-major, M = 128, N = block_n.
-__device__ __forceinline__ uint32_t umma_idesc_i8(int n) {
+// Instruction descriptor: s8 x s8 -> s32, both operands K-major, M = 128 (256 for a pair of CTAs), N = block_n.
+__device__ __forceinline__ uint32_t umma_idesc_i8(int n, int m = BLOCK_M) {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(BLOCK_M >> 4) << 24);
+         ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int c0, int c1) {
