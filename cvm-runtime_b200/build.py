@@ -13,7 +13,7 @@ ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libcvm_runtime.so")
 MEASURE_LIB = os.path.join(HERE, "libcvm_measure.so")
 
-KERNEL_SRCS = ["common.cu", "conv_tc.cu", "conv_small.cu", "conv_stem.cu", "conv_direct.cu", "elemwise.cu", "transform.cu", "nms.cu"]
+KERNEL_SRCS = ["common.cu", "conv_tc.cu", "conv_small.cu", "conv_stem.cu", "conv_direct.cu", "conv_dw.cu", "elemwise.cu", "transform.cu", "nms.cu"]
 HOST_SRCS = ["ops.cc", "graph.cc", "host_pool.cc", "executor.cc", "c_api.cc"]
 MEASURE_SRCS = ["measure.cu"]
 

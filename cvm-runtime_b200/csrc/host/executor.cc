@@ -650,46 +650,7 @@ struct Lowering {
       probe.bias_static = (!use_bias || g.params.count(g.entry_id(n.inputs[2])) > 0) ? 1 : 0;
     }
     const bool depthwise = !dense && groups == C && OC == C && C % 16 == 0 && safe8[ex_];
-    // Depthwise 3x3 stride-1 layers over a multiple of 128 channels run on the tensor cores as
-    // groups of 32 channels with block-diagonal weights when the kernel's 8 x 16 pixel tiles fit
-    // the image: the CUDA-core form is bound by instruction issue at a fraction of the memory
-    // rate (measured 15-25 % slower on such layers; faster for 32 and 64 channels, which stay there).
-    const int dw_cg = 32;
-    // ... and when there are enough of them: a persistent CTA per SM with three tiles or fewer to its name
-    // spends most of the launch filling and draining (MobileNet, one image: 139 -> 100 us with every
-    // depthwise layer on the CUDA cores; 64 images: 328 against 353 us; the lines cross near 500 tiles).
-    const int64_t dw_tc_tiles = 512;
-    bool dw_tc = false;
-    if (depthwise && C % 128 == 0 && KH == 3 && KW == 3 && sh == 1 && sw == 1 && dh == 1 && dw == 1 &&
-        out.dtype == CVMK_I8 && !dev_env("CVM_B200_NO_DW_TC") && !dev_env("CVM_B200_NO_TC")) {
-      const int64_t linear = ((int64_t)N * OH * OW + 127) / 128;
-      const int64_t tiles = (int64_t)((OW + 7) / 8) * ((OH + 15) / 16) * N;
-      probe.groups = C / dw_cg;
-      dw_tc = tiles * 20 <= linear * 27 && tiles * (C / 128) > dw_tc_tiles && cvmk_conv2d_tc_supported(&probe);
-      if (!dw_tc) probe.groups = 0;
-    }
-    // 32 and 64 channels: 4 or 2 neighbouring pixels of a row are 128 contiguous bytes, so the layer
-    // is given to the same kernel as a 128-channel one over a quarter / half of the width, whose
-    // filter moves in steps of one real pixel (cvmk_conv_desc.group_fold).
-    int dw_fold = 1;
-    if (depthwise && !dw_tc && (C == 32 || C == 64) && KH == 3 && KW == 3 && sh == 1 && sw == 1 && dh == 1 && dw == 1 &&
-        pw == 1 && OW == W && W % (128 / C) == 0 && out.dtype == CVMK_I8 &&
-        (!use_bias || g.params.count(g.entry_id(n.inputs[2])) > 0) && !dev_env("CVM_B200_NO_DW_TC") &&
-        !dev_env("CVM_B200_NO_DW_FOLD") && !dev_env("CVM_B200_NO_TC")) {
-      const int F = 128 / C;
-      const int64_t linear = ((int64_t)N * OH * (OW / F) + 127) / 128;
-      const int64_t tiles = (int64_t)((OW / F + 7) / 8) * ((OH + 15) / 16) * N;
-      cvmk_conv_desc fp = probe;
-      fp.W = W / F; fp.OW = OW / F; fp.C = fp.OC = 128;
-      fp.groups = 4; fp.group_fold = F;
-      if (tiles * 20 <= linear * 27 && tiles > dw_tc_tiles && cvmk_conv2d_tc_supported(&fp)) {
-        probe = fp;
-        dw_tc = true;
-        dw_fold = F;
-      }
-    }
-    const bool tc = (dw_tc || groups == 1) && cvmk_conv2d_tc_supported(&probe) && !dev_env("CVM_B200_NO_TC");
-    const int wcg = dw_tc ? dw_cg : icg;   // input channels per weight row as the kernels take them
+    const bool tc = groups == 1 && cvmk_conv2d_tc_supported(&probe) && !dev_env("CVM_B200_NO_TC");
     // Few-channel convolutions (image stems): gather patches into a [M, Kp] matrix, then run the
     // tensor-core kernel on it as a 1x1 convolution.
     const int kflat = KH * KW * icg, kp = kflat > 64 ? (kflat + 63) / 64 * 64 : (kflat + 31) / 32 * 32;
@@ -717,14 +678,8 @@ struct Lowering {
       tc_pad = cvmk_conv2d_tc_supported(&pp) && plain_chain && bias_param && safe8[ex_] && out.shape.size() == 4;
     }
     // weights: OIHW int32 -> int8, [OC, KH, KW, C/groups] (depthwise: [KH, KW, C])
-    std::vector<int8_t> w8((size_t)(tc_pad ? OCp : OC) * dw_fold * KH * KW * wcg, 0);
-    if (dw_tc) {   // [OC, KH, KW, 32]: row o holds its filter in column o % 32 of every tap
-      for (int o = 0; o < OC * dw_fold; ++o) {   // (folded: the C filters once per sub-pixel)
-        const int c = o % OC;
-        for (int k = 0; k < KH * KW; ++k)
-          w8[((size_t)o * KH * KW + k) * wcg + (c % wcg)] = (int8_t)wt.data[(size_t)c * KH * KW + k];
-      }
-    } else if (depthwise && !tc) {
+    std::vector<int8_t> w8((size_t)(tc_pad ? OCp : OC) * KH * KW * icg, 0);
+    if (depthwise && !tc) {
       for (int c = 0; c < C; ++c)
         for (int k = 0; k < KH * KW; ++k) w8[(size_t)k * C + c] = (int8_t)wt.data[(size_t)c * KH * KW + k];
     } else {
@@ -878,18 +833,9 @@ struct Lowering {
       // block-diagonal weights [f * OC, f * C] -> [M / f, f * OC], byte for byte the same output:
       // f times the multiplies (zeros), 1 / f of the tiles.  32 -> 64 channels at 112 x 112, batch
       // 256: 0.116 -> 0.058 ms with f = 4; 64 -> 64 at 56 x 56: 0.032 -> 0.022 ms with f = 2.
-      if (dw_fold > 1 && use_bias) {   // the bias once per sub-pixel
-        const auto& bv = g.params.find(g.entry_id(n.inputs[2]))->second.data;
-        std::vector<int32_t> bf(128, 0);
-        for (int j = 0; j < dw_fold; ++j)
-          for (int o = 0; o < OC; ++o) bf[(size_t)j * OC + o] = bv[o];
-        int32_t* bfdev = (int32_t*)ex.dalloc(bf.size() * 4);
-        CUDA_OK(cudaMemcpy(bfdev, bf.data(), bf.size() * 4, cudaMemcpyHostToDevice));
-        d.ep.s[0].ptr = bfdev;
-      }
       int fold = 1;
       const std::vector<Range> parts = batch_ranges(N);
-      if (!dense && !dw_tc && groups == 1 && KH == 1 && KW == 1 && sh == 1 && sw == 1 && ph == 0 && pw == 0 &&
+      if (!dense && groups == 1 && KH == 1 && KW == 1 && sh == 1 && sw == 1 && ph == 0 && pw == 0 &&
           xin.nhwc && out.nhwc && (!use_bias || g.params.count(g.entry_id(n.inputs[2])) > 0) &&
           !dev_env("CVM_B200_NO_PIXEL_FOLD")) {
         auto whole = [&](int f) {   // every part of the batch is a whole number of folded pixels
@@ -926,7 +872,7 @@ struct Lowering {
       ex.plans_.emplace_back((cvmk_conv_plan*)mem, plan_deleter);
       cvmk_conv_plan* plan = ex.plans_.back().get();
       KERNEL_OK(cvmk_conv2d_tc_prepare(&d, plan));
-      add_step(label + (dw_tc ? "[dw]" : "[tc]"), [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
+      add_step(label + "[tc]", [plan](cudaStream_t s) { return cvmk_conv2d_tc_launch(plan, s); });
       // The parts of the batch (every operand is batch-major, so a part is a contiguous slice).
       if (xin.nhwc && out.nhwc) {
         ex.steps_.back().images = N;
@@ -966,6 +912,8 @@ struct Lowering {
       d.stride_h = sh; d.stride_w = sw; d.pad_h = ph; d.pad_w = pw; d.dil_h = dh; d.dil_w = dw;
       d.depthwise = depthwise;
       d.acc_bound = probe.acc_bound;
+      d.bias_static = probe.bias_static;
+      d.status = ex.status_dev_;
       d.ep = ch.ep;
       add_step(label + (depthwise ? "[dw]" : "[direct]"), [d](cudaStream_t s) { return cvmk_conv2d_direct(&d, s); });
       // The parts of the batch (batch-major operands: a part is a contiguous slice), when no step of
