@@ -40,10 +40,11 @@ namespace {
 
 using namespace tc;
 
-constexpr int STEM_THREADS = 320;   // warps 0-3 load + fold, 4 MMA, 5-8 epilogue, 9 output stores
+constexpr int STEM_THREADS = 448;   // warps 0-3 load + fold, 4 MMA, 5-12 epilogue, 13 output stores
 constexpr int FOLDERS = 128;
 constexpr int MMA_WARP = 4;
-constexpr int STORE_WARP = 9;
+constexpr int STORE_WARP = 13;
+constexpr int MAX_ACCS = 8, MAX_PANELS = 4;
 constexpr int PIX = 16;             // bytes per staged pixel
 constexpr int MAX_OC = 128;
 constexpr int STEM_SMEM_MAX = 110 * 1024;   // two CTAs per SM
@@ -63,6 +64,10 @@ struct StemConvParams {
   int fold_words;       // 1: rows are folded four staged pixels at a time on 32-bit words
   int planar_bytes, staged_bytes, w_bytes;
   int tmem_cols;
+  int accs, panels;     // accumulators (all of half of TMEM, eight at most) and output panels, powers of two
+  int accs_log2, panels_log2;
+  int planar_bufs;
+  FastDiv fd_quads;     // by xw / 4
   int off_planar, off_staged, off_out, off_bias;  // byte offsets of the shared-memory regions after the weights
   int* status;
   const int32_t* bias;
@@ -111,8 +116,9 @@ __device__ __forceinline__ uint32_t desc_hi_plain(uint32_t sbo) {
   return (sbo >> 4) | (1u << 14);   // bit 46 of the descriptor: version (sm_100)
 }
 
-// One staged pixel: the S x S input pixels of all C channels, byte (a * S + b) * C + c = channel c of
-// the pixel at sub-row a, sub-column b; clamped to +-clamp; zero where the image ends.
+// One staged pixel: the S x S input pixels of all C channels, byte (a * C + c) * S + b = channel c of
+// the pixel at sub-row a, sub-column b (so that what one row of one channel gives a pixel stays together);
+// clamped to +-clamp; zero where the image ends.
 template <int C, int S>
 __device__ __forceinline__ uint4 fold_pixel(const StemConvParams& p, const uint8_t* planar, int R, int X) {
   uint32_t o[4] = {0u, 0u, 0u, 0u};
@@ -131,7 +137,7 @@ __device__ __forceinline__ uint4 fold_pixel(const StemConvParams& p, const uint8
       for (int c = 0; c < C; ++c) {
         int v = (int)(int8_t)src[(size_t)c * p.in_rows * p.wbox];
         v = inside ? max(min(v, p.clamp), -p.clamp) : 0;
-        const int i = (a * S + b) * C + c;
+        const int i = (a * C + c) * S + b;
         o[i >> 2] |= (uint32_t)(v & 0xff) << (8 * (i & 3));
       }
     }
@@ -142,20 +148,18 @@ __device__ __forceinline__ uint4 fold_pixel(const StemConvParams& p, const uint8
 // The same on words, four staged pixels (X0 .. X0 + 3, X0 a multiple of 4) per call, for a single
 // box that carries zero columns left and right of the image (so that no column needs a test) and a
 // clamp to +-127 (only -128 moves).  Per sub-row and channel the 4 * S input bytes the pixels
-// take come out of two or three aligned words and a funnel shift; one byte permute moves each
-// byte into place.
+// take come out of two or three aligned words and a funnel shift.  The integer pipe is what the CTAs of an SM
+// run out of, so the bytes move two (stride 2) or, as a 4 x 4 transpose, four at a time: 12 or 8 permutes for four
+// pixels of 12 or 3 bytes, where one for each byte took 48 or 12.
 __device__ __forceinline__ uint32_t clamp127(uint32_t x) {
-  const uint32_t z = x ^ 0x80808080u;
-  const uint32_t m = ~(((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z) & 0x80808080u;   // 0x80 in every byte that is -128
-  return x + (m >> 7);
+  const uint32_t t = (x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu;    // top bits: the lower seven are not all zero
+  return x + ((x & ~t & 0x80808080u) >> 7);              // -128 and nothing else goes up by one
 }
 template <int C, int S>
 __device__ __forceinline__ void fold_four(const StemConvParams& p, const uint8_t* planar, uint8_t* dst, int R, int X0) {
-  uint32_t o[4][4];
+  uint32_t s[2 * 4][2];   // [a * C + c]: pixel j, sub-column b at byte j * S + b
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[j][q] = 0u;
+  for (int i = 0; i < 8; ++i) s[i][0] = s[i][1] = 0u;
   const int first = X0 * S - p.pw + p.lpad;          // first input column of the four pixels, inside the box
   const uint32_t sh = (uint32_t)(first & 3) * 8u;
 #pragma unroll
@@ -163,24 +167,29 @@ __device__ __forceinline__ void fold_four(const StemConvParams& p, const uint8_t
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       const uint32_t* w = reinterpret_cast<const uint32_t*>(planar + ((size_t)c * p.in_rows + (R * S + a)) * p.wbox + (first & ~3));
-      uint32_t s[S];   // the 4 * S bytes: pixel j, sub-column b at byte j * S + b
       const uint32_t w0 = w[0], w1 = w[1];
-      s[0] = clamp127(__funnelshift_r(w0, w1, sh));
-      if (S == 2) s[S - 1] = clamp127(__funnelshift_r(w1, w[2], sh));
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int b = 0; b < S; ++b) {
-          const int from = j * S + b;                 // byte of s[]
-          const int to = (a * S + b) * C + c;         // byte of the staged pixel
-          const uint32_t sel = (0x3210u & ~(0xFu << (4 * (to & 3)))) | ((uint32_t)(4 + (from & 3)) << (4 * (to & 3)));
-          o[j][to >> 2] = __byte_perm(o[j][to >> 2], s[from >> 2], sel);
-        }
+      s[a * C + c][0] = clamp127(__funnelshift_r(w0, w1, sh));
+      if (S == 2) s[a * C + c][1] = clamp127(__funnelshift_r(w1, w[2], sh));
     }
   }
+  uint4* out = reinterpret_cast<uint4*>(dst + (size_t)X0 * PIX);
+  if (S == 2) {   // halves of words: sub-columns 0 and 1 of one row and channel
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    *reinterpret_cast<uint4*>(dst + (size_t)(X0 + j) * PIX) = make_uint4(o[j][0], o[j][1], o[j][2], o[j][3]);
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;
+      uint32_t o[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = 2 * q < S * C ? __byte_perm(s[2 * q][j >> 1], s[2 * q + 1][j >> 1], sel) : 0u;
+      out[j] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  } else {        // bytes: channel c of pixel j is byte j of s[c]
+    const uint32_t l01 = __byte_perm(s[0][0], s[1][0], 0x5140), h01 = __byte_perm(s[0][0], s[1][0], 0x7362);
+    const uint32_t l23 = __byte_perm(s[2][0], s[3][0], 0x5140), h23 = __byte_perm(s[2][0], s[3][0], 0x7362);
+    out[0] = make_uint4(__byte_perm(l01, l23, 0x5410), 0u, 0u, 0u);
+    out[1] = make_uint4(__byte_perm(l01, l23, 0x7632), 0u, 0u, 0u);
+    out[2] = make_uint4(__byte_perm(h01, h23, 0x5410), 0u, 0u, 0u);
+    out[3] = make_uint4(__byte_perm(h01, h23, 0x7632), 0u, 0u, 0u);
+  }
 }
 
 template <int C, int S>
@@ -188,7 +197,7 @@ __device__ __forceinline__ void fold_block(const StemConvParams& p, const uint8_
   if (p.fold_words) {
     const int quads = p.xw >> 2;   // xw is a multiple of 4 on this path
     for (int i = t; i < p.srows * quads; i += FOLDERS) {
-      const int R = i / quads, X0 = (i - R * quads) * 4;
+      const int R = fdiv(i, p.fd_quads), X0 = (i - R * quads) * 4;
       fold_four<C, S>(p, planar, staged + (size_t)R * p.pitch, R, X0);
     }
     return;
@@ -198,8 +207,7 @@ __device__ __forceinline__ void fold_block(const StemConvParams& p, const uint8_
       *reinterpret_cast<uint4*>(staged + (size_t)R * p.pitch + X * PIX) = fold_pixel<C, S>(p, planar, R, X);
 }
 
-// Packed requantisation of one thread's row (see fast_requant): straight-line per 32 columns, two
-// chunks per TMEM round trip.
+// Packed requantisation of one thread's row (see fast_requant): straight-line per 32 columns.
 template <int RELU1>
 __device__ __forceinline__ void stem_fast_chunk(const FastQ& fq, int mul, int32_t (&v)[32], int ci, const int32_t* bias_s,
                                                 uint8_t* panel, uint32_t sw_key) {
@@ -222,14 +230,7 @@ __device__ __forceinline__ void stem_fast_chunk(const FastQ& fq, int mul, int32_
 template <int RELU1>
 __device__ __forceinline__ void stem_fast_row(const FastQ& fq, int mul, uint32_t tbase, int chunks, const int32_t* bias_s,
                                               uint8_t* panel, uint32_t sw_key) {
-  int ci = 0;
-  for (; ci + 2 <= chunks; ci += 2) {
-    int32_t v0[32], v1[32];
-    tmem_ld64(tbase + (uint32_t)(ci * 32), v0, v1);
-    stem_fast_chunk<RELU1>(fq, mul, v0, ci, bias_s, panel, sw_key);
-    stem_fast_chunk<RELU1>(fq, mul, v1, ci + 1, bias_s, panel, sw_key);
-  }
-  if (ci < chunks) {
+  for (int ci = 0; ci < chunks; ++ci) {
     int32_t v[32];
     tmem_ld32(tbase + (uint32_t)(ci * 32), v);
     stem_fast_chunk<RELU1>(fq, mul, v, ci, bias_s, panel, sw_key);
@@ -254,12 +255,37 @@ __device__ long long g_stem_timing[296 * 16];
 #define STFLUSH(slot) do {} while (0)
 #endif
 
+// The weights of a tap, packed as byte (a * 2 + b) * C + c, in the order of the staged pixels, (a * C + c) * 2 + b
+// (of one channel the two are the same, and with stride 1).
+template <int C>
+__device__ __forceinline__ uint4 staged_order(const uint4& v) {
+  const uint32_t in[4] = {v.x, v.y, v.z, v.w};
+  uint32_t o[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int t = 0; t < 4 * C; ++t) {
+    const int ac = t >> 1, from = (2 * (ac / C) + (t & 1)) * C + ac % C;
+    o[t >> 2] |= ((in[from >> 2] >> (8 * (from & 3))) & 0xffu) << (8 * (t & 3));
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// The products of one tile.  The lane is chosen at each instruction: conv_tc.cu says why.
+template <int KH, int NJ>
+__device__ __forceinline__ void stem_products(bool leader, uint32_t d_tmem, uint32_t al, uint32_t row_step, uint32_t a_hi, uint32_t bl,
+                                              uint32_t b_step, uint32_t b_hi, uint32_t idesc) {
+#pragma unroll
+  for (int ky = 0; ky < KH; ++ky, al += row_step)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j, bl += b_step)
+      if (leader) mma_i8_k<1>(d_tmem, al + 2u * (uint32_t)j, a_hi, bl, b_hi, idesc, (uint32_t)(ky | j));
+}
+
 __global__ void __launch_bounds__(STEM_THREADS, 2)
 conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
                  const __grid_constant__ StemConvParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t planar_full[2], staged_full[2], staged_empty[2];
-  __shared__ uint64_t acc_full[2], acc_empty[2], out_free[2], out_full[2];
+  __shared__ uint64_t acc_full[MAX_ACCS], acc_empty[MAX_ACCS], out_free[MAX_PANELS], out_full[MAX_PANELS];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
 
@@ -279,28 +305,31 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       mbar_init(&planar_full[b], 1);
       mbar_init(&staged_full[b], FOLDERS / 32);
       mbar_init(&staged_empty[b], 1);
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 4);
-      mbar_init(&out_free[b], 1);
-      mbar_init(&out_full[b], 4);
     }
+    for (int b = 0; b < p.accs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+    for (int b = 0; b < p.panels; ++b) { mbar_init(&out_free[b], 1); mbar_init(&out_full[b], 4); }
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // weights -> shared memory, same byte order as in global memory
-  for (int i = threadIdx.x; i < p.w_bytes / 16; i += STEM_THREADS)
-    reinterpret_cast<uint4*>(wq)[i] = __ldg(reinterpret_cast<const uint4*>(p.w) + i);
+  // weights -> shared memory, the 16 bytes of a tap in the order of the staged pixels
+  for (int i = threadIdx.x; i < p.w_bytes / 16; i += STEM_THREADS) {
+    uint4 v = __ldg(reinterpret_cast<const uint4*>(p.w) + i);
+    if (p.S == 2) v = p.C == 1 ? v : (p.C == 2 ? staged_order<2>(v) : (p.C == 3 ? staged_order<3>(v) : staged_order<4>(v)));
+    reinterpret_cast<uint4*>(wq)[i] = v;
+  }
+  fence_async_smem();
+  if (warp == MMA_WARP) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
+  pdl_wait();      // (so far only parameters were read)
   for (int i = threadIdx.x; i < p.OC; i += STEM_THREADS) {
     const int32_t b = p.bias ? __ldg(p.bias + i) : 0;
     bias_s[i] = p.fast_mode ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
   }
-  fence_async_smem();
-  if (warp == MMA_WARP) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   pdl_trigger();   // (after the TMEM allocation: see conv_small.cu)
-  if (threadIdx.x == 0) { mbar_arrive(&out_free[0]); mbar_arrive(&out_free[1]); }  // both panels start free
+  if (threadIdx.x == 0)
+    for (int b = 0; b < p.panels; ++b) mbar_arrive(&out_free[b]);   // all panels start free
   const uint32_t tmem_base = tmem_slot;
 
   if (warp < MMA_WARP) {
@@ -319,7 +348,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (issuer) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_x)) : "memory");
       if ((int)blockIdx.x < p.num_blocks) load_block(blockIdx.x, 0);
-      if ((int)(blockIdx.x + gridDim.x) < p.num_blocks) load_block(blockIdx.x + gridDim.x, 1);
+      if (p.planar_bufs == 2 && (int)(blockIdx.x + gridDim.x) < p.num_blocks) load_block(blockIdx.x + gridDim.x, 1);
     }
     uint32_t bi = 0;
     STDECL;
@@ -328,12 +357,13 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       const int buf = (int)(bi & 1u);
       const uint32_t par = (bi >> 1) & 1u;
       STSTART(tw);
-      bool ok = mbar_wait(&planar_full[buf], par, &abort_flag, 2);
+      const int pbuf = p.planar_bufs == 2 ? buf : 0;
+      bool ok = mbar_wait(&planar_full[pbuf], p.planar_bufs == 2 ? par : bi & 1u, &abort_flag, 2);
       STADD(0, tw);
       ok = ok && mbar_wait(&staged_empty[buf], par ^ 1u, &abort_flag, 3);
       STADD(1, tw);
       if (ok) {
-        const uint8_t* src = planar + (size_t)buf * p.planar_bytes;
+        const uint8_t* src = planar + (size_t)pbuf * p.planar_bytes;
         uint8_t* dst = staged + (size_t)buf * p.staged_bytes;
         switch (p.C * 2 + p.S - 3) {   // (C, S) -> 2 * (C - 1) + (S - 1)
           case 0: fold_block<1, 1>(p, src, dst, t); break;
@@ -349,7 +379,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       fence_async_smem();   // the staged rows are read by the tensor core, the planar rows rewritten by TMA
       // every folder is done with the planar rows; if a wait ran out for anyone, all leave together
       if (bar_any(1, FOLDERS, !ok)) break;
-      if (issuer && blk + 2 * (int)gridDim.x < p.num_blocks) load_block(blk + 2 * (int)gridDim.x, buf);
+      if (issuer && blk + p.planar_bufs * (int)gridDim.x < p.num_blocks) load_block(blk + p.planar_bufs * (int)gridDim.x, pbuf);
       __syncwarp();
       if (lane == 0) mbar_arrive(&staged_full[buf]);
       STADD(2, tw);
@@ -381,23 +411,25 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const uint32_t a_blk = desc_lo_plain(smem_u32(staged + (size_t)sbuf * p.staged_bytes), PIX);
         for (int rr = 0; live && rr < p.rows_per_block && oy0 + rr < p.OH; ++rr) {
           for (int sg = 0; sg < p.segs; ++sg, ++tile) {
-            const int buf = (int)(tile & 1u);
-            if (!mbar_wait(&acc_empty[buf], ((tile >> 1) & 1u) ^ 1u, &abort_flag, 5)) { live = false; break; }
+            const int buf = (int)(tile & (uint32_t)(p.accs - 1));
+            if (!mbar_wait(&acc_empty[buf], ((tile >> p.accs_log2) & 1u) ^ 1u, &abort_flag, 5)) { live = false; break; }
             STADD(3, tw);
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(buf * p.OC);
             // tap (ky', 2j) of output pixel m of this segment: staged row rr + ky', staged pixel sg * seg_w + m + 2j
-            uint32_t al_row = a_blk + (uint32_t)rr * row_step + (uint32_t)(sg * p.seg_w);
-            uint32_t bl = b_lo0;
-            if (leader) {
-              uint32_t acc = 0;
-              for (int ky = 0; ky < p.khp; ++ky, al_row += row_step) {
-                uint32_t al = al_row;
-                for (int j = 0; j < p.nj; ++j, al += 2u, bl += b_step, acc = 1u)
-                  mma_i8_k<1>(d_tmem, al, a_hi, bl, b_hi, idesc, acc);
+            const uint32_t al = a_blk + (uint32_t)rr * row_step + (uint32_t)(sg * p.seg_w);
+            switch (p.khp * 4 + p.nj) {   // the filters that image stems have, straight line
+              case 18: stem_products<4, 2>(leader, d_tmem, al, row_step, a_hi, b_lo0, b_step, b_hi, idesc); break;   // 7 x 7 / 8 x 8, stride 2
+              case 14: stem_products<3, 2>(leader, d_tmem, al, row_step, a_hi, b_lo0, b_step, b_hi, idesc); break;   // 3 x 3; 5 x 5, stride 2
+              case 9: stem_products<2, 1>(leader, d_tmem, al, row_step, a_hi, b_lo0, b_step, b_hi, idesc); break;    // 3 x 3, stride 2
+              default: {
+                uint32_t bl = b_lo0;
+                for (int ky = 0; ky < p.khp; ++ky)
+                  for (int j = 0; j < p.nj; ++j, bl += b_step)
+                    if (leader) mma_i8_k<1>(d_tmem, al + (uint32_t)ky * row_step + 2u * (uint32_t)j, a_hi, bl, b_hi, idesc, (uint32_t)(ky | j));
               }
-              mma_commit(&acc_full[buf]);
             }
+            if (leader) mma_commit(&acc_full[buf]);
             STADD(5, tw);
           }
         }
@@ -410,6 +442,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   } else if (warp < STORE_WARP) {
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;
+    const int group = (warp - MMA_WARP - 1) >> 2;   // two groups of four warps take the tiles in turn
     const int row_in_tile = quarter * 32 + lane;
     const bool leader = warp == MMA_WARP + 1 && lane == 0;
     (void)leader;
@@ -428,15 +461,15 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       for (int rr = 0; live && rr < p.rows_per_block && oy0 + rr < p.OH; ++rr) {
         const int oy = oy0 + rr;
         for (int sg = 0; sg < p.segs; ++sg, ++tile) {
-          const int buf = (int)(tile & 1u);
-          const uint32_t par = (tile >> 1) & 1u;
+          if ((int)(tile & 1u) != group) continue;
+          const int buf = (int)(tile & (uint32_t)(p.accs - 1)), pan = (int)(tile & (uint32_t)(p.panels - 1));
           STSTART(tw);
-          if (!mbar_wait(&acc_full[buf], par, &abort_flag, 6)) { live = false; break; }
+          if (!mbar_wait(&acc_full[buf], (tile >> p.accs_log2) & 1u, &abort_flag, 6)) { live = false; break; }
           STADD(6, tw);
           tc_fence_after();
-          if (!mbar_wait(&out_free[buf], par, &abort_flag, 7)) { live = false; break; }
+          if (!mbar_wait(&out_free[pan], (tile >> p.panels_log2) & 1u, &abort_flag, 7)) { live = false; break; }
           STADD(7, tw);
-          uint8_t* panel = out_panels + (size_t)buf * panel_bytes + row_off;
+          uint8_t* panel = out_panels + (size_t)pan * panel_bytes + row_off;
           const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * p.OC);
           const int ox = sg * p.seg_w + row_in_tile;
           const bool valid = row_in_tile < p.seg_w && ox < p.OW;
@@ -474,7 +507,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           __syncwarp();
           if (lane == 0) {
             mbar_arrive(&acc_empty[buf]);
-            mbar_arrive(&out_full[buf]);
+            mbar_arrive(&out_full[pan]);
           }
           STADD(8, tw);
           if (abort_flag) { live = false; break; }
@@ -497,8 +530,8 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       const int oy0 = (blk - n * p.blocks_per_image) * p.rows_per_block;
       for (int rr = 0; live && rr < p.rows_per_block && oy0 + rr < p.OH; ++rr) {
         for (int sg = 0; sg < p.segs; ++sg, ++tile) {
-          const int buf = (int)(tile & 1u);
-          if (!mbar_wait(&out_full[buf], (tile >> 1) & 1u, &abort_flag, 8)) { live = false; break; }
+          const int buf = (int)(tile & (uint32_t)(p.panels - 1));
+          if (!mbar_wait(&out_full[buf], (tile >> p.panels_log2) & 1u, &abort_flag, 8)) { live = false; break; }
           if (leader) {
             tma_store_3d(&tmap_y, out_panels + (size_t)buf * panel_bytes, 0, sg * p.seg_w, n * p.OH + oy0 + rr);
             tma_store_commit();
@@ -535,6 +568,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 struct StemLayout {
   int S, khp, kwp, nj, rows_per_block, segs, seg_w, srows, xw, pitch, in_rows, wbox, nwb, box_stride, lpad, fold_words;
   int planar_bytes, staged_bytes, w_bytes, off_planar, off_staged, off_out, off_bias, smem_bytes;
+  int panels, planar_bufs;
 };
 
 bool stem_layout(const cvmk_stem_conv_desc& d, StemLayout* L) {
@@ -569,28 +603,42 @@ bool stem_layout(const cvmk_stem_conv_desc& d, StemLayout* L) {
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaGetLastError();
-  // Blocks of 8 output rows re-fold few rows (KH' - 1 per block); smaller blocks when the batch is
-  // too small to give every CTA slot one, or when shared memory is short.
-  for (int rpb = 8; rpb >= 1; rpb /= 2) {
-    L->rows_per_block = std::min(rpb, (int)d.OH);
-    const int64_t blocks = (int64_t)d.N * ((d.OH + L->rows_per_block - 1) / L->rows_per_block);
-    L->srows = L->rows_per_block + L->khp - 1;
-    L->in_rows = L->srows * S;
-    L->box_stride = (d.C * L->in_rows * L->wbox + 127) / 128 * 128;   // (one box, or nwb boxes of wbox columns)
-    L->planar_bytes = L->nwb * L->box_stride;
-    L->staged_bytes = (L->srows * L->pitch + 127) / 128 * 128;
-    L->off_planar = (L->w_bytes + 1023) / 1024 * 1024;
-    L->off_staged = L->off_planar + 2 * L->planar_bytes;
-    // rows of a tile past the segment's width read on past the staged row they start in: whatever
-    // follows (the next rows, the panels) is inside this CTA's shared memory
-    L->off_out = (L->off_staged + 2 * L->staged_bytes + 1023) / 1024 * 1024;
-    L->off_bias = L->off_out + 2 * BLOCK_M * d.OC;
-    L->smem_bytes = L->off_bias + d.OC * 4 + 1024;
-    const bool fits = L->smem_bytes <= STEM_SMEM_MAX && L->in_rows <= 256;
-    if (fits && (blocks >= 2 * sms || rpb <= 2)) return true;
-    if (rpb == 1) return fits;
+  // Rows of a block.  A round of blocks (two CTAs an SM) takes as long as its output rows, a fifth of a row for each
+  // staged row that the block before has folded too, and two fifths to hand buffers over; the last round counts like
+  // the others.  (3 x 3 on 32 images of 224 x 224: 8 rows a block 68.6 us, 4 rows 63.2; 7 x 7, stride 2, on 256: 125.0 and 131.4.)
+  bool found = false;
+  double best = 0;
+  for (int rpb = std::min(8, (int)d.OH); rpb >= 1; --rpb) {
+    StemLayout l = *L;
+    l.rows_per_block = rpb;
+    l.srows = l.rows_per_block + l.khp - 1;
+    l.in_rows = l.srows * S;
+    l.box_stride = (d.C * l.in_rows * l.wbox + 127) / 128 * 128;   // (one box, or nwb boxes of wbox columns)
+    l.planar_bytes = l.nwb * l.box_stride;
+    l.staged_bytes = (l.srows * l.pitch + 127) / 128 * 128;
+    // Four panels before the second buffer for input rows, which arrive while the products of the block before run
+    // (with two panels a group of epilogue warps waits for its last tile to leave, a seventh of its time).
+    for (int form = d.OC == 128 ? 2 : 0; form < 4; ++form) {
+      l.panels = form < 2 ? 4 : 2;
+      l.planar_bufs = 2 - (form & 1);
+      l.off_planar = (l.w_bytes + 1023) / 1024 * 1024;
+      l.off_staged = l.off_planar + l.planar_bufs * l.planar_bytes;
+      // rows of a tile past the segment's width read on past the staged row they start in: whatever
+      // follows (the next rows, the panels) is inside this CTA's shared memory
+      l.off_out = (l.off_staged + 2 * l.staged_bytes + 1023) / 1024 * 1024;
+      l.off_bias = l.off_out + l.panels * BLOCK_M * d.OC;
+      l.smem_bytes = l.off_bias + d.OC * 4 + 1024;
+      if (l.smem_bytes <= STEM_SMEM_MAX) break;
+    }
+    if (l.smem_bytes > STEM_SMEM_MAX || l.in_rows > 256) continue;
+    const int64_t blocks = (int64_t)d.N * ((d.OH + rpb - 1) / rpb), rounds = (blocks + 2 * sms - 1) / (2 * sms);
+    const double cost = rounds * (rpb + 0.2 * (l.khp - 1) + 0.4);
+    if (found && cost >= best) continue;
+    found = true;
+    best = cost;
+    *L = l;
   }
-  return false;
+  return found;
 }
 
 }  // namespace
@@ -715,9 +763,12 @@ extern "C" int cvmk_conv2d_stem_launch(const cvmk_stem_conv_plan* plan, cvmk_str
   p.lpad = L.lpad; p.fold_words = L.fold_words;
   p.planar_bytes = L.planar_bytes; p.staged_bytes = L.staged_bytes; p.w_bytes = L.w_bytes;
   p.off_planar = L.off_planar; p.off_staged = L.off_staged; p.off_out = L.off_out; p.off_bias = L.off_bias;
-  int cols = 2 * d.OC, pow2 = 32;
-  while (pow2 < cols) pow2 *= 2;
-  p.tmem_cols = pow2;
+  // Accumulators: half of the SM's TMEM, two CTAs share it (OC is 32, 64 or 128).
+  p.tmem_cols = 256;
+  p.accs = 256 / d.OC; p.panels = L.panels; p.planar_bufs = L.planar_bufs;
+  p.fd_quads = make_fastdiv(L.xw / 4);
+  while ((1 << p.accs_log2) < p.accs) ++p.accs_log2;
+  while ((1 << p.panels_log2) < p.panels) ++p.panels_log2;
   p.status = d.status;
   int rc = lower_chain(d.ep, &p.chain);
   if (rc != CVMK_OK) return rc;
@@ -757,7 +808,7 @@ extern "C" int cvmk_conv2d_stem_launch(const cvmk_stem_conv_plan* plan, cvmk_str
   CUtensorMap tx, ty;
   memcpy(&tx, plan->tmap_x, sizeof(tx));
   memcpy(&ty, plan->tmap_y, sizeof(ty));
-  conv_stem_kernel<<<plan->grid, STEM_THREADS, plan->smem_bytes, (cudaStream_t)stream>>>(tx, ty, p);
+  launch_pdl(conv_stem_kernel, dim3((unsigned)plan->grid), dim3(STEM_THREADS), (size_t)plan->smem_bytes, (cudaStream_t)stream, tx, ty, p);
   return check_cuda(cudaGetLastError(), "conv_stem_kernel launch");
 }
 
