@@ -4,7 +4,7 @@
 // them (about 23 an element), at a third of the memory rate.  Here a group of 32 channels is multiplied by
 // block-diagonal weights: D[pixel, o] = sum_t A_t[pixel, 32 channels] x diag(w_t), one tcgen05.mma kind::i8 of K = 32
 // a filter tap, whose A operand is a window of the staged input.  Such a product reads 4 KB of A and 32 bytes for each
-// column from shared memory, and takes 66 cycles with 32 columns, 67 with 64 and 71 with 128.  So, with stride 1, a row
+// column from shared memory, at 128 bytes a cycle: 40 cycles with 32 columns, 48 with 64 and 64 with 128.  So, with stride 1, a row
 // of the tile is not one output pixel but a block of 2 x 2, whose 4 x 4 input pixels are multiplied once each, by the
 // weights of the up to four outputs that they belong to side by side: 16 products where four times nine were.  With
 // stride 2 a row is one output pixel, and the input, four times the output, sets the time.
@@ -69,9 +69,9 @@ struct DwParams {
 // The products of one channel group: the input pixel of the block, the columns and the first of them, and where their
 // weights begin in a row of blocks of 32 x 32 bytes, each with one filter tap on its diagonal (9: none).  Stride 1: the
 // outputs of a block are 32 columns each, in the order (0,0), (0,1), (1,1), (1,0); a product of an edge has a zero
-// block where it meets an output that it does not belong to.  One product after another of the same columns
-// takes 67 to 71 cycles whatever it is, so there are three shapes only, and the rows of blocks that the products need
-// overlap: 35 KB instead of 48.
+// block where it meets an output that it does not belong to.  There are three shapes only, and the rows
+// of blocks that the products need overlap, 35 KB where 48 blocks would stand alone: what shared memory has left is
+// the ring's.
 struct Product { int iy, ix, n, col, first; };
 constexpr int NUM_PRODUCTS1 = 16, NUM_BLOCKS1 = 35;
 __host__ __device__ constexpr Product product1(int i) {
@@ -261,7 +261,6 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         if (!ensure(&bar_full[unit], phase, 3)) { live = false; break; }
         tc_fence_after();
         const uint32_t al = a_lo + (uint32_t)(unit * (UNIT / 16));
-        // (the lane is chosen at each instruction: conv_tc.cu says why)
 #pragma unroll
         for (int g = 0; g < G; ++g) {
           int issued = 0;
@@ -270,9 +269,8 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const Product q = S == 1 ? product1(i) : product2(i);
             if (!PAIRS && (q.ix & 1) != u) continue;   // a tap of the other plane
             const int at = PAIRS ? ((q.ix + 1) >> 1) * ROW + ((q.ix + 1) & 1) * P : (q.ix >> 1) * P;
-            if (leader)
-              mma_i8_k<1>(d + (uint32_t)(g * Sh::COLS + q.col), al + (uint32_t)((q.iy * LINE + at + g * 32) >> 4), a_hi,
-                          w_lo + (uint32_t)((g * Sh::BLOCKS + q.first) * 64), w_hi, umma_idesc_i8(q.n), u == 0 && issued == 0 ? 0u : 1u);
+            mma_i8_if(leader, d + (uint32_t)(g * Sh::COLS + q.col), al + (uint32_t)((q.iy * LINE + at + g * 32) >> 4), a_hi,
+                      w_lo + (uint32_t)((g * Sh::BLOCKS + q.first) * 64), w_hi, umma_idesc_i8(q.n), u == 0 && issued == 0 ? 0u : 1u);
             if (g == 0 && issued == 2) flush();
             ++issued;
           }

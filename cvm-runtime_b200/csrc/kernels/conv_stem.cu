@@ -269,7 +269,7 @@ __device__ __forceinline__ uint4 staged_order(const uint4& v) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// The products of one tile.  The lane is chosen at each instruction: conv_tc.cu says why.
+// The products of one tile.
 template <int KH, int NJ>
 __device__ __forceinline__ void stem_products(bool leader, uint32_t d_tmem, uint32_t al, uint32_t row_step, uint32_t a_hi, uint32_t bl,
                                               uint32_t b_step, uint32_t b_hi, uint32_t idesc) {
@@ -277,7 +277,7 @@ __device__ __forceinline__ void stem_products(bool leader, uint32_t d_tmem, uint
   for (int ky = 0; ky < KH; ++ky, al += row_step)
 #pragma unroll
     for (int j = 0; j < NJ; ++j, bl += b_step)
-      if (leader) mma_i8_k<1>(d_tmem, al + 2u * (uint32_t)j, a_hi, bl, b_hi, idesc, (uint32_t)(ky | j));
+      mma_i8_if(leader, d_tmem, al + 2u * (uint32_t)j, a_hi, bl, b_hi, idesc, (uint32_t)(ky | j));
 }
 
 __global__ void __launch_bounds__(STEM_THREADS, 2)

@@ -217,6 +217,23 @@ __device__ __forceinline__ void mma_i8_k(uint32_t d_tmem, uint32_t a_lo, uint32_
   }
 }
 #undef CVMK_MMA_I8
+// One instruction of one CTA, issued by the lane for which `leader` holds.  The predicate is in the instruction: a branch
+// around each one takes the issuing warp some ten cycles more (conv_dw.cu: MobileNet, 256 images 664 -> 656 us on the device).
+__device__ __forceinline__ void mma_i8_if(bool leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                          uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 da, db;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "setp.ne.b32 q, %7, 0;\n"
+      "mov.b64 da, {%1, %2};\n"
+      "mov.b64 db, {%3, %4};\n"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+      : "memory");
+}
 // Arrive on `bar` once every tcgen05.mma issued so far by this thread has finished; CG = 2: on the
 // barriers at this place in both CTAs of the pair.
 template <int CG = 1>
