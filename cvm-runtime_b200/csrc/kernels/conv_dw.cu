@@ -23,9 +23,9 @@
 //
 // One B200, 256 images, launched between events (some 6 us of it the launch), the kernels before -> this one: 32
 // channels at 112 x 112 78 -> 47 us (210 MB, 32 us at the copy rate), 128 at 56 x 56 76 -> 52 (32), 256 at 28 x 28
-// 47 -> 30 (16), 512 at 14 x 14 29 -> 20 (8); stride 2: 64 at 112 x 112 86 -> 51 (40), 128 at 56 x 56 47 -> 33 (20).  What
-// bounds stride 1 is shared memory: a tile of 64 channels reads 128 KB of A and 96 KB of weights, and 104 KB go in and
-// out, 2600 cycles of the 2900 that it takes; seven eighths of a tile's rows a side lie inside such images.
+// 47 -> 30 (16), 512 at 14 x 14 29 -> 20 (8); stride 2: 64 at 112 x 112 86 -> 51 (40), 128 at 56 x 56 47 -> 33 (20).  No one
+// thing bounds stride 1: 128 channels at 56 x 56 take 47 us without the products, 49 without the input, 51 without the
+// requantisation, all of them 53; a quarter of the rows of such tiles lies outside the images.
 //
 // Reproduces groupwise_conv2d with groups = C (src/runtime/cpu/ops/ops.cc:333-366) and the chain of bias, shift and clip.
 // Every wait is bounded, as in conv_tc.cu.
