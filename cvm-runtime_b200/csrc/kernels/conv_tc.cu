@@ -257,6 +257,27 @@ __device__ long long g_conv_trace[17 * 512];
 #define TFLUSH(slot) do {} while (0)
 #endif
 
+// The commits that free the last lap of the ring arrive in both CTAs of the pair, and nothing else waits for them in the
+// second: before a CTA may leave, its producers wait for every one.  A producer whose next stage is `turn` stages away
+// (0 or 1, with one producer 0) has so many waits left, `producers` stages apart.
+constexpr __host__ __device__ int drain_waits(int stages, int turn, int producers) { return (stages - turn + producers - 1) / producers; }
+constexpr bool drain_complete() {   // after any number of stages filled, the waits are for the stages of the last lap, each once
+  for (int producers = 1; producers <= 2; ++producers)
+    for (int stages = 2; stages <= MAX_STAGES; ++stages)
+      for (int filled = 0; filled < 3 * MAX_STAGES; ++filled) {
+        int waits[MAX_STAGES] = {};
+        for (int which = 0; which < producers; ++which) {
+          const int turn = producers == 2 ? (filled ^ which) & 1 : 0;
+          int next = filled + turn;
+          for (int k = drain_waits(stages, turn, producers); k > 0; --k, next += producers) ++waits[next % stages];
+        }
+        for (int s = 0; s < stages; ++s)
+          if (waits[s] != 1) return false;
+      }
+  return true;
+}
+static_assert(drain_complete(), "waits before a pair leaves");
+
 // TMA loads into this CTA's shared memory that report to `bar`, a barrier of the pair's first CTA.
 __device__ __forceinline__ void load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::
@@ -605,6 +626,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
           }
         }
+      }
+      for (int k = live ? drain_waits(p.stages, two_issuers ? 0 : turn, two_issuers ? 1 : 2) : 0; k > 0; --k) {
+        if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) break;
+        stage += two_issuers ? 1 : 2;
+        if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
       }
       TADD(12, tk);
 #ifdef CVMK_CONV_TIMING
@@ -1022,7 +1048,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   // ------------------------------------------------------------------ teardown
   // Every warp leaves on its own.  The TMEM columns of both CTAs go back, and the CTAs with them, once every warp that
-  // reads them, reads the other's operands or reports to its barriers has arrived here.
+  // reads them, reads the other's operands, reports to its barriers or waits for its commits has arrived here: the
+  // epilogue has waited for every accumulator, the producers for the last lap of the ring.
   __syncwarp();
   if (threadIdx.x == 0) TRACE(16, 3);
   if (abort_flag) {
