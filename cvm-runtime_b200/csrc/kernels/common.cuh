@@ -127,7 +127,7 @@ __device__ __forceinline__ void apply_chain(const DevChain& c, int32_t (&v)[V], 
           if (V % 16 == 0 && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
 #pragma unroll
             for (int q = 0; q < V / 16; ++q) {
-              int4 raw = __ldg(reinterpret_cast<const int4*>(p) + q);
+              int4 raw = reinterpret_cast<const int4*>(p)[q];
               const int w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
               for (int k = 0; k < 16; ++k) t[q * 16 + k] = (int32_t)(int8_t)(w[k >> 2] >> ((k & 3) * 8));
@@ -141,7 +141,7 @@ __device__ __forceinline__ void apply_chain(const DevChain& c, int32_t (&v)[V], 
           if (V % 4 == 0 && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
 #pragma unroll
             for (int q = 0; q < V / 4; ++q) {
-              int4 raw = __ldg(reinterpret_cast<const int4*>(p) + q);
+              int4 raw = reinterpret_cast<const int4*>(p)[q];
               t[q * 4 + 0] = raw.x; t[q * 4 + 1] = raw.y; t[q * 4 + 2] = raw.z; t[q * 4 + 3] = raw.w;
             }
           } else {
@@ -163,7 +163,7 @@ __device__ __forceinline__ void apply_chain(const DevChain& c, int32_t (&v)[V], 
       case K_ADD_C: {
         const int32_t* p = reinterpret_cast<const int32_t*>(st.ptr);
 #pragma unroll
-        for (int j = 0; j < V; ++j) v[j] += __ldg(p + ch0 + j * cstride);
+        for (int j = 0; j < V; ++j) v[j] += p[ch0 + j * cstride];
       } break;
       case K_MUL_S:
 #pragma unroll
@@ -228,6 +228,10 @@ __device__ __forceinline__ uint32_t pack4(int32_t a, int32_t b, int32_t c, int32
 // Programmatic dependent launch: a kernel launched this way may start while the previous kernel of
 // the stream drains, so it calls pdl_wait() before it touches memory that kernels write, and
 // pdl_trigger() early, which lets the kernel after it do the same.
+// Whatever a kernel may have written is read with ordinary loads.  Loads that promise that nothing writes the memory while
+// this kernel runs (the read-only intrinsic, const pointers declared as unaliased) promise what is not so before pdl_wait(),
+// and the compiler moves them to before it: a depthwise layer whose bias was computed on the way took the bias of the
+// inference before.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -102,13 +102,13 @@ __global__ void __launch_bounds__(128) depthwise_kernel(const __grid_constant__ 
       const int iy = oy * p.sh + fy * p.dh - p.ph;
       if (iy < 0 || iy >= p.H) continue;
       for (int fx = 0; fx < p.KW; ++fx) {
-        const int4 wv = __ldg(reinterpret_cast<const int4*>(p.w + ((int64_t)fy * p.KW + fx) * p.C) + cv);
+        const int4 wv = *(reinterpret_cast<const int4*>(p.w + ((int64_t)fy * p.KW + fx) * p.C) + cv);
         const int ww[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
         for (int q = 0; q < PX; ++q) {
           const int ix = (ox0 + q) * p.sw + fx * p.dw - p.pw;
           if (ix < 0 || ix >= p.W || ox0 + q >= p.OW) continue;
-          const int4 xv = __ldg(reinterpret_cast<const int4*>(reinterpret_cast<const int8_t*>(p.x) +
+          const int4 xv = *(reinterpret_cast<const int4*>(reinterpret_cast<const int8_t*>(p.x) +
                                                                 (((int64_t)n * p.H + iy) * p.W + ix) * p.C) + cv);
           const int xw[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
@@ -166,13 +166,13 @@ __global__ void __launch_bounds__(256) depthwise3x3_kernel(const __grid_constant
     int32_t wgt[9][4];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
-      const int w = __ldg(reinterpret_cast<const int*>(p.w + (int64_t)t * p.C) + cv);
+      const int w = *(reinterpret_cast<const int*>(p.w + (int64_t)t * p.C) + cv);
 #pragma unroll
       for (int k = 0; k < 4; ++k) wgt[t][k] = (int32_t)(int8_t)(w >> (k * 8));
     }
     int32_t bias[4] = {0, 0, 0, 0};
     if (has_bias) {
-      const int4 b4 = __ldg(reinterpret_cast<const int4*>(p.chain.s[0].ptr) + cv);
+      const int4 b4 = *(reinterpret_cast<const int4*>(p.chain.s[0].ptr) + cv);
       bias[0] = b4.x; bias[1] = b4.y; bias[2] = b4.z; bias[3] = b4.w;
     }
     // Rows and columns outside the image are read from a clamped (valid) address and masked to
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) depthwise3x3_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < IN; ++j) {
           const int ix = ix0 + j;
-          const int v = __ldg(rows[fy] + min(max(ix, 0), p.W - 1) * cw);
+          const int v = rows[fy][min(max(ix, 0), p.W - 1) * cw];
           xin[fy][j] = (row_ok[fy] && ix >= 0 && ix < p.W) ? v : 0;
         }
       }
@@ -336,13 +336,13 @@ __global__ void __launch_bounds__(256) dw3x3_tile_kernel(const __grid_constant__
     uint32_t w3[3];
 #pragma unroll
     for (int fx = 0; fx < 3; ++fx)
-      w3[fx] = (uint32_t)__ldg(reinterpret_cast<const int*>(p.w + (int64_t)(fy * 3 + fx) * p.C + c0) + cw);
+      w3[fx] = (uint32_t)*(reinterpret_cast<const int*>(p.w + (int64_t)(fy * 3 + fx) * p.C + c0) + cw);
     transpose4x4(w3[0], w3[1], w3[2], 0u, wrow[fy]);
   }
   int bq[4] = {0, 0, 0, 0};   // (bias + rounding addend) * mul
   {
     int4 b4 = make_int4(0, 0, 0, 0);
-    if (p.bias) b4 = __ldg(reinterpret_cast<const int4*>(p.bias + c0) + cw);
+    if (p.bias) b4 = *(reinterpret_cast<const int4*>(p.bias + c0) + cw);
     bq[0] = (b4.x + p.add) * p.mul; bq[1] = (b4.y + p.add) * p.mul;
     bq[2] = (b4.z + p.add) * p.mul; bq[3] = (b4.w + p.add) * p.mul;
   }
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(256) im2col_pack_kernel(const __grid_constant_
         const int e = lut[k];
         const int iy = iy0 + (e >> 20), ix = ix0 + ((e >> 8) & 0xfff), c = e & 0xff;
         if (iy >= 0 && iy < p.H && ix >= 0 && ix < p.W) {
-          const uint32_t b = (uint8_t)__ldg(xn + ((int64_t)iy * p.W + ix) * p.C + c);
+          const uint32_t b = (uint8_t)xn[((int64_t)iy * p.W + ix) * p.C + c];
           w[j >> 2] |= b << ((j & 3) * 8);
         }
       }
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(512) stem_pack_kernel(const __grid_constant__ 
       const int r = i / (vpr * p.C);
       const int iy = iy0 + r * p.dh;
       if (iy < 0 || iy >= p.H) continue;
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p.x + (((int64_t)n * p.C + c) * p.H + iy) * p.W) + vx);
+      const uint4 raw = *(reinterpret_cast<const uint4*>(p.x + (((int64_t)n * p.C + c) * p.H + iy) * p.W) + vx);
       const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
       int8_t* dst = srow + (r * p.C + c) * p.wp + p.pw + vx * 16;
 #pragma unroll
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(512) stem_pack_kernel(const __grid_constant__ 
       const int iy = iy0 + (i / (p.wp * p.C)) * p.dh;
       int v = 0;
       if (xx >= 0 && xx < p.W && iy >= 0 && iy < p.H) {
-        v = __ldg(p.x + (((int64_t)n * p.C + c) * p.H + iy) * p.W + xx);
+        v = p.x[(((int64_t)n * p.C + c) * p.H + iy) * p.W + xx];
         v = max(min(v, p.clamp), -p.clamp);
       }
       srow[i] = (int8_t)v;

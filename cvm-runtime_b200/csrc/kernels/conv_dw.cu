@@ -181,13 +181,13 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const int tap = S == 1 ? block_taps1.t[b] : b;
         if (tap == 9) continue;
         const uint32_t at = (uint32_t)(c * 33);   // row c, byte c
-        smem[(size_t)blk * 1024 + (at ^ (((at >> 7) & 1u) << 4))] = (uint8_t)__ldg(p.w + (size_t)tap * p.C + c0 + g * 32 + c);
+        smem[(size_t)blk * 1024 + (at ^ (((at >> 7) & 1u) << 4))] = (uint8_t)p.w[(size_t)tap * p.C + c0 + g * 32 + c];
       }
       fence_async_smem();
       if (!p.bias_static) pdl_wait();
       const int g = G == 2 ? (warp - 2) >> (S == 1 ? 3 : 2) : 0;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) bias[j] = (int32_t)((uint32_t)((p.bias ? __ldg(p.bias + c0 + g * 32 + j) : 0) + p.add) * (uint32_t)p.mul);
+      for (int j = 0; j < 32; ++j) bias[j] = (int32_t)((uint32_t)((p.bias ? p.bias[c0 + g * 32 + j] : 0) + p.add) * (uint32_t)p.mul);
     }
     if (warp == Sh::IO_WARP && lane < 2)
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &tmap_y : &tmap_x)) : "memory");

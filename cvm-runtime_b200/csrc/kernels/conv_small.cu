@@ -247,7 +247,7 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (!early) pdl_wait();
     const int ch0 = SWAP ? m0 : n0, channels = SWAP ? BLOCK_M : p.block_n;
     for (int i = (int)threadIdx.x - 64; i < channels; i += THREADS - 64) {
-      const int32_t b = (p.bias && ch0 + i < p.oc) ? __ldg(p.bias + ch0 + i) : 0;
+      const int32_t b = (p.bias && ch0 + i < p.oc) ? p.bias[ch0 + i] : 0;
       // packed requantisation: (bias + rounding addend) pre-multiplied, see fast_requant()
       bias_s[i] = (p.fast_variant >= 0 && p.fast_variant < 8) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
     }

@@ -313,7 +313,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   }
   // weights -> shared memory, the 16 bytes of a tap in the order of the staged pixels
   for (int i = threadIdx.x; i < p.w_bytes / 16; i += STEM_THREADS) {
-    uint4 v = __ldg(reinterpret_cast<const uint4*>(p.w) + i);
+    uint4 v = reinterpret_cast<const uint4*>(p.w)[i];
     if (p.S == 2) v = p.C == 1 ? v : (p.C == 2 ? staged_order<2>(v) : (p.C == 3 ? staged_order<3>(v) : staged_order<4>(v)));
     reinterpret_cast<uint4*>(wq)[i] = v;
   }
@@ -321,7 +321,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   if (warp == MMA_WARP) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
   pdl_wait();      // (so far only parameters were read)
   for (int i = threadIdx.x; i < p.OC; i += STEM_THREADS) {
-    const int32_t b = p.bias ? __ldg(p.bias + i) : 0;
+    const int32_t b = p.bias ? p.bias[i] : 0;
     bias_s[i] = p.fast_mode ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
   }
   tc_fence_before();

@@ -450,7 +450,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   auto stage_bias = [&]() {
     const int padded = min(MAX_BIAS, (p.oc + 31) & ~31);
     for (int i = (int)threadIdx.x - 32; i < padded; i += NUM_THREADS - 64) {   // warps 1..10
-      const int32_t b = i < p.oc && p.bias ? __ldg(p.bias + i) : 0;
+      const int32_t b = i < p.oc && p.bias ? p.bias[i] : 0;
       // fast path: (bias + rounding addend) pre-multiplied by 2^(16 - shift), see fast_row()
       bias_s[i] = (p.fast_mode && !p.fast_wide) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
     }
@@ -922,7 +922,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               }
             } else {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += (col0 + j < p.oc) ? __ldg(p.bias + col0 + j) : 0;
+              for (int j = 0; j < 32; ++j) v[j] += (col0 + j < p.oc) ? p.bias[col0 + j] : 0;
             }
           }
           const size_t lin = (size_t)row * p.oc + col0;

@@ -47,7 +47,7 @@ __device__ __forceinline__ int4 pack16(const int32_t* v) {
 
 // y = chain(x), 16 elements per thread per step.
 template <int XD, int YD>
-__global__ void __launch_bounds__(256) elemwise_kernel(const void* __restrict__ x, void* __restrict__ y,
+__global__ void __launch_bounds__(256) elemwise_kernel(const void* x, void* y,
                                                        int64_t n, const __grid_constant__ DevChain chain) {
   pdl_trigger();
   pdl_wait();
@@ -56,11 +56,11 @@ __global__ void __launch_bounds__(256) elemwise_kernel(const void* __restrict__ 
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
     int32_t v[16];
     if (XD == CVMK_I8) {
-      unpack16(__ldg(reinterpret_cast<const int4*>(x) + i), v);
+      unpack16(reinterpret_cast<const int4*>(x)[i], v);
     } else {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        int4 r = __ldg(reinterpret_cast<const int4*>(x) + i * 4 + q);
+        int4 r = reinterpret_cast<const int4*>(x)[i * 4 + q];
         v[4 * q] = r.x; v[4 * q + 1] = r.y; v[4 * q + 2] = r.z; v[4 * q + 3] = r.w;
       }
     }
@@ -209,7 +209,7 @@ __device__ __forceinline__ void strided_vec_body(const StridedVecParams& p, int6
         }
       }
     }
-    p.y[yo] = __ldg(p.a + ao);
+    p.y[yo] = p.a[ao];
   }
 }
 __global__ void __launch_bounds__(256) strided_vec_kernel(const __grid_constant__ StridedVecParams p) {
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(256) reduce_vec16_kernel(const __grid_constant
       const int64_t step = p.rs[0];
 #pragma unroll 8
       for (int r = slice; r < (int)p.red_total; r += RED_SLICES) {
-        const int4 raw = __ldg(reinterpret_cast<const int4*>(src + r * step));
+        const int4 raw = *(reinterpret_cast<const int4*>(src + r * step));
         const int w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(256) pool_vec_kernel(const __grid_constant__ P
         for (int fx = 0; fx < p.KW; ++fx) {
           const int ix = ox * p.sw + fx - p.pw;
           const bool ok = row_ok && ix >= 0 && ix < p.W;
-          int4 v = __ldg(row + (int64_t)min(max(ix, 0), p.W - 1) * p.cvec);
+          int4 v = row[(int64_t)min(max(ix, 0), p.W - 1) * p.cvec];
           if (!ok) v = make_int4(0x80808080, 0x80808080, 0x80808080, 0x80808080);
           const uint32_t w[4] = {(uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w};
 #pragma unroll
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(256) pool_vec_kernel(const __grid_constant__ P
         for (int fx = 0; fx < p.KW; ++fx) {
           const int ix = ox * p.sw + fx - p.pw;
           const bool ok = row_ok && ix >= 0 && ix < p.W;
-          int4 v = __ldg(row + (int64_t)min(max(ix, 0), p.W - 1) * p.cvec);
+          int4 v = row[(int64_t)min(max(ix, 0), p.W - 1) * p.cvec];
           if (!ok) v = make_int4(INT32_MIN, INT32_MIN, INT32_MIN, INT32_MIN);
           m.x = max(m.x, v.x); m.y = max(m.y, v.y); m.z = max(m.z, v.z); m.w = max(m.w, v.w);
         }
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(256) pool_window_kernel(const __grid_constant_
       uint32_t te[K][4], to[K][4];
 #pragma unroll
       for (int fx = 0; fx < K; ++fx) {
-        const int4 v = __ldg(row + xo[fx]);
+        const int4 v = row[xo[fx]];
         const uint32_t w[4] = {(uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {   // (0, b0, 0, b2) and (0, b1, 0, b3)

@@ -102,8 +102,8 @@ __device__ __forceinline__ int clampv(int v, int clamp) { return max(min(v, clam
 __device__ __forceinline__ int2 clamp2(int2 v, int clamp) { return make_int2(clampv(v.x, clamp), clampv(v.y, clamp)); }
 
 template <bool CLAMP>
-__global__ void __launch_bounds__(THREADS, 1) gvc6_kernel(const int32_t* __restrict__ x, int32_t* __restrict__ y,
-                                                          int32_t* __restrict__ valid_count, int N, int thr,
+__global__ void __launch_bounds__(THREADS, 1) gvc6_kernel(const int32_t* x, int32_t* y,
+                                                          int32_t* valid_count, int N, int thr,
                                                           int chunk_rows, int clamp) {
   pdl_trigger();
   pdl_wait();
@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(THREADS, 1) gvc6_kernel(const int32_t* __restr
   PHASE(11);
 }
 
-__global__ void __launch_bounds__(THREADS) gvc_kernel(const int32_t* __restrict__ x, int32_t* __restrict__ y,
-                                                      int32_t* __restrict__ valid_count, int N, int K,
+__global__ void __launch_bounds__(THREADS) gvc_kernel(const int32_t* x, int32_t* y,
+                                                      int32_t* valid_count, int N, int K,
                                                       int thr, int clamp) {
   pdl_trigger();
   pdl_wait();

@@ -8,7 +8,7 @@ namespace {
 
 __device__ __forceinline__ int32_t load_any(const void* p, int dt, int64_t off) {
   return dt == CVMK_I8 ? (int32_t) reinterpret_cast<const int8_t*>(p)[off]
-                       : __ldg(reinterpret_cast<const int32_t*>(p) + off);
+                       : reinterpret_cast<const int32_t*>(p)[off];
 }
 __device__ __forceinline__ void store_any(void* p, int dt, int64_t off, int32_t v) {
   if (dt == CVMK_I8) reinterpret_cast<int8_t*>(p)[off] = (int8_t)v;
@@ -142,7 +142,7 @@ __global__ void signal_kernel(volatile int* flag) {
 
 // Rows of a packed byte matrix moved to a pitch that TMA can take, 16 bytes a thread: five aligned words
 // and a funnel shift (13 images of 3 x 197 x 197: 1.5 MB, under 3 us).
-__global__ void __launch_bounds__(256) repitch_kernel(const uint32_t* __restrict__ src, uint4* __restrict__ dst, int64_t total, int chunks,
+__global__ void __launch_bounds__(256) repitch_kernel(const uint32_t* src, uint4* dst, int64_t total, int chunks,
                                                       int row_bytes, int64_t last_word) {
   pdl_trigger();
   pdl_wait();
