@@ -916,17 +916,19 @@ struct Lowering {
       d.status = ex.status_dev_;
       d.ep = ch.ep;
       add_step(label + (depthwise ? "[dw]" : "[direct]"), [d](cudaStream_t s) { return cvmk_conv2d_direct(&d, s); });
-      // The parts of the batch (batch-major operands: a part is a contiguous slice), when no step of
-      // the chain indexes another tensor.
+      // The parts of the batch (batch-major operands: a part is a contiguous slice).
       ex.steps_.back().images = d.N;
-      bool sliceable = xin.nhwc && out.nhwc;
-      for (int i = 0; i < d.ep.n; ++i)
-        sliceable &= !(d.ep.s[i].op == CVMK_EP_ADD_T || d.ep.s[i].op == CVMK_EP_SUB_T || d.ep.s[i].op == CVMK_EP_RSUB_T);
-      for (const Range& r : sliceable ? batch_ranges(d.N) : std::vector<Range>()) {
+      for (const Range& r : xin.nhwc && out.nhwc ? batch_ranges(d.N) : std::vector<Range>()) {
         cvmk_conv_direct_desc cd = d;
+        const size_t out_first = (size_t)r.begin * d.OH * d.OW * d.OC;
         cd.N = (int)(r.end - r.begin);
         cd.x = (const char*)d.x + (size_t)r.begin * d.H * d.W * d.C * d.x_dtype;
-        cd.y = (char*)d.y + (size_t)r.begin * d.OH * d.OW * d.OC * d.y_dtype;
+        cd.y = (char*)d.y + out_first * d.y_dtype;
+        for (int i = 0; i < cd.ep.n; ++i) {
+          cvmk_ep_step& st = cd.ep.s[i];
+          if ((st.op == CVMK_EP_ADD_T || st.op == CVMK_EP_SUB_T || st.op == CVMK_EP_RSUB_T) && st.ptr)
+            st.ptr = (const char*)st.ptr + out_first * st.ptr_dtype;
+        }
         ex.steps_.back().chunk.push_back([cd](cudaStream_t s) { return cvmk_conv2d_direct(&cd, s); });
       }
     }

@@ -117,6 +117,43 @@ int lower_chain(const cvmk_epilogue& in, DevChain* out) {
   return CVMK_OK;
 }
 
+bool pack_chain(const DevChain& c, int first, int64_t acc_bound, PackedChain* out) {
+  const int left = c.n - first;
+  if (acc_bound <= 0 || (left != 1 && left != 3) || c.s[first].op != K_RS_CLAMP) return false;
+  const DevStep& rs = c.s[first];
+  const int64_t add = rs.c;
+  const int sh = rs.d;
+  // The packed form clamps after the shift, the chain clamps the sum to [rs.a, rs.b] first: the same value, because
+  // the shift is monotone.
+  const int64_t lo = ((int64_t)rs.a + add) >> sh, hi = ((int64_t)rs.b + add) >> sh;
+  if (acc_bound + add >= (int64_t)INT32_MAX || lo < -32767 || hi > 32767 || lo > hi || sh > 16) return false;
+  // A sum that does not fit 16 bits after the shift is clamped to [rs.a, rs.b] before it is scaled; with the rounding
+  // addend it then stays below 2^(15 + shift).
+  out->wide = ((acc_bound + add) >> sh) >= 32767;
+  if (out->wide && ((int64_t)rs.b + add >= ((int64_t)1 << (15 + sh)) || (int64_t)rs.a + add <= -((int64_t)1 << (15 + sh)))) return false;
+  out->kind = 0;
+  out->step = -1;
+  out->lo2 = out->hi2 = 0;
+  if (left == 3) {
+    const DevStep &t = c.s[first + 1], &clip = c.s[first + 2];
+    if ((t.op != K_ADD_T && t.op != K_SUB_T) || t.dt != CVMK_I8 || clip.op != K_CLIP || clip.a < -32767 || clip.b > 32767 ||
+        (-lo > hi ? -lo : hi) + 128 >= 32767)
+      return false;
+    out->kind = t.op == K_SUB_T ? 3 : 2;
+    out->step = first + 1;
+    out->lo2 = clip.a;
+    out->hi2 = clip.b;
+  }
+  out->shift = sh;
+  out->mul = 1 << (16 - sh);
+  out->add = (int)add;
+  out->pre_lo = rs.a;
+  out->pre_hi = rs.b;
+  out->lo = (int)lo;
+  out->hi = (int)hi;
+  return true;
+}
+
 }  // namespace cvmk
 
 extern "C" const char* cvmk_last_error(void) { return cvmk::g_err; }

@@ -47,6 +47,20 @@ struct DevChain {
 // Host: translate the public chain into the device form.  Returns CVMK_OK or CVMK_ERR_ARG.
 int lower_chain(const cvmk_epilogue& in, DevChain* out);
 
+// A chain, from step `first` on, that can be run on packed 16-bit words (fast_requant in tc_common.cuh): rs_clamp, alone or
+// followed by the sum with (or difference from) an int8 tensor and a clip, after a sum of at most `acc_bound`.
+struct PackedChain {
+  int kind;             // 0: rs_clamp alone, 2: + tensor, 3: - tensor
+  int step;             // the tensor's step
+  int shift, mul, add;  // ((sum + add) * mul) >> 16
+  int wide;             // the sum may exceed what the product holds: it is first clamped to [pre_lo, pre_hi]
+  int pre_lo, pre_hi;
+  int lo, hi;           // clamp after the shift
+  int lo2, hi2;         // clamp after the tensor
+};
+bool pack_chain(const DevChain& c, int first, int64_t acc_bound, PackedChain* out);
+inline uint32_t both_halves(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; }
+
 // Bit length of |x| with the reference's x = 0 -> 1 rule (cpu/ops/ops.cc:525-542).
 __device__ __forceinline__ int32_t precision_of(int32_t x) {
   uint32_t a = x < 0 ? (uint32_t)(-(int64_t)x) : (uint32_t)x;

@@ -526,38 +526,17 @@ __global__ void __launch_bounds__(512) stem_pack_kernel(const __grid_constant__ 
   }
 }
 
-// The chain of a depthwise layer in the packed form, if it has one: [bias] rs_clamp, with a sum that cannot overflow
-// and fits 16 bits after the shift.
-bool dw_requant(const cvmk_conv_direct_desc* d, const DevChain& chain, DwRequant* rq) {
-  if (d->y_dtype != CVMK_I8 || d->acc_bound <= 0) return false;
-  int i0 = 0;
-  rq->bias = nullptr;
-  if (chain.n > 0 && chain.s[0].op == K_ADD_C) { rq->bias = reinterpret_cast<const int32_t*>(chain.s[0].ptr); i0 = 1; }
-  if (chain.n - i0 != 1 || chain.s[i0].op != K_RS_CLAMP) return false;
-  const DevStep& rs = chain.s[i0];
-  const int64_t add = rs.c;
-  const int sh = rs.d;
-  const int64_t lo1 = ((int64_t)rs.a + add) >> sh, hi1 = ((int64_t)rs.b + add) >> sh;
-  if (sh > 16 || d->acc_bound + add >= (int64_t)INT32_MAX || ((d->acc_bound + add) >> sh) >= 32767 ||
-      lo1 < -32767 || hi1 > 32767 || lo1 > hi1)
-    return false;
-  // The kernels clamp after the shift; the chain clamps the sum to [rs.a, rs.b] first.  Both give
-  // the same value because the shift is monotone (the argument of the tensor-core kernels).
-  rq->mul = 1 << (16 - sh);
-  rq->add = (int)add;
-  rq->lo = (int)lo1;
-  rq->hi = (int)hi1;
-  return true;
-}
-
 // Plans and launches dw3x3_tile_kernel when the layer qualifies; returns -1 when it does not (the caller then uses
 // the register kernel).
-int try_dw3x3_tile(const cvmk_conv_direct_desc* d, const DwRequant& rq, cudaStream_t s) {
-  if (d->C % 32 != 0 || d->OW < 1) return -1;
+int try_dw3x3_tile(const cvmk_conv_direct_desc* d, const DevChain& chain, cudaStream_t s) {
+  if (d->C % 32 != 0 || d->OW < 1 || d->y_dtype != CVMK_I8) return -1;
+  const int first = chain.n > 0 && chain.s[0].op == K_ADD_C;
+  PackedChain pc;
+  if (!pack_chain(chain, first, d->acc_bound, &pc) || pc.kind || pc.wide) return -1;
   if (d->pad_h > 1 || d->pad_w > 1) return -1;
   Dw3Params p;
   memset(&p, 0, sizeof(p));
-  p.x = reinterpret_cast<const int8_t*>(d->x); p.w = d->w; p.bias = rq.bias; p.y = reinterpret_cast<int8_t*>(d->y);
+  p.x = reinterpret_cast<const int8_t*>(d->x); p.w = d->w; p.bias = first ? reinterpret_cast<const int32_t*>(chain.s[0].ptr) : nullptr; p.y = reinterpret_cast<int8_t*>(d->y);
   p.N = d->N; p.H = d->H; p.W = d->W; p.C = d->C; p.OH = d->OH; p.OW = d->OW; p.ph = d->pad_h; p.pw = d->pad_w;
   const int S = d->stride_h;
   const int cb = d->C % 128 == 0 ? 128 : (d->C % 64 == 0 ? 64 : 32);
@@ -585,11 +564,10 @@ int try_dw3x3_tile(const cvmk_conv_direct_desc* d, const DwRequant& rq, cudaStre
   p.div_per_row = make_dw_div(p.xw * (p.cb_words / 4));
   p.div_strips = make_dw_div(p.strips);
   p.vec_log2 = p.cb_words == 8 ? 1 : (p.cb_words == 16 ? 2 : 3);
-  p.mul = rq.mul;
-  p.add = rq.add;
-  auto x2 = [](int64_t v) { return (uint32_t)((uint32_t)(uint16_t)(int16_t)v | ((uint32_t)(uint16_t)(int16_t)v << 16)); };
-  p.lo = x2(rq.lo); p.hi = x2(rq.hi);
-  p.relu = rq.lo == 0;
+  p.mul = pc.mul;
+  p.add = pc.add;
+  p.lo = both_halves(pc.lo); p.hi = both_halves(pc.hi);
+  p.relu = pc.lo == 0;
   const int64_t tiles = (int64_t)d->N * p.tiles_y * p.tiles_c;
   if (tiles > INT32_MAX) return -1;
   const int smem = smem_of(R);
@@ -649,12 +627,9 @@ extern "C" int cvmk_conv2d_direct(const cvmk_conv_direct_desc* d, cvmk_stream_t 
     }
     if (d->KH == 3 && d->KW == 3 && d->dil_h == 1 && d->dil_w == 1 && d->stride_h == d->stride_w &&
         (d->stride_h == 1 || d->stride_h == 2)) {
-      DwRequant rq;
-      if (dw_requant(d, p.chain, &rq)) {
-        int rc3 = launch_conv_dw(*d, rq, s);
-        if (rc3 == -1) rc3 = try_dw3x3_tile(d, rq, s);
-        if (rc3 != -1) return rc3;
-      }
+      int rc3 = launch_conv_dw(*d, p.chain, s);
+      if (rc3 == -1) rc3 = try_dw3x3_tile(d, p.chain, s);
+      if (rc3 != -1) return rc3;
       const int64_t work3 = (int64_t)d->N * d->OH * (d->C / 4);
       if (d->stride_h == 1) launch_pdl(depthwise3x3_kernel<1>, dim3((unsigned)(grid_sized(work3, 256))), dim3(256), 0, s, p);
       else launch_pdl(depthwise3x3_kernel<2>, dim3((unsigned)(grid_sized(work3, 256))), dim3(256), 0, s, p);

@@ -27,7 +27,13 @@
 // thing bounds stride 1: 128 channels at 56 x 56 take 47 us without the products, 49 without the input, 51 without the
 // requantisation, all of them 53; a quarter of the rows of such tiles lies outside the images.
 //
-// Reproduces groupwise_conv2d with groups = C (src/runtime/cpu/ops/ops.cc:333-366) and the chain of bias, shift and clip.
+// Any chain behind the products: [bias] shift clamp has forms of its own; a wide sum, and the sum with another tensor (whose
+// tile TMA brings into the output buffer before the result), run packed too, everything else step by step.  128 channels at
+// 28 x 28, 150 images, in a chain of such layers: 9.4 us with shift and clamp, 15.4 with a wide sum, 15.9 with a tensor, 18.9
+// with a clip alone (depthwise3x3_kernel 39.0, 57.2, 34.8; the tensor loaded by the threads that need it 18.4: a
+// row's 32 bytes lie in a cache line of their own).
+//
+// Reproduces groupwise_conv2d with groups = C (src/runtime/cpu/ops/ops.cc:333-366) and the chain behind it.
 // Every wait is bounded, as in conv_tc.cu.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -64,7 +70,17 @@ struct DwParams {
   int mul, add;
   uint32_t lo, hi;
   int bias_static;
+  // chains that are not just [bias] shift clamp
+  int out_w, out_h;        // of an image, in pixels
+  int kind;                // of the packed form (PackedChain), or -1: step by step
+  int out_box_bytes;       // of one image's part of an output tile
+  int wide, pre_lo, pre_hi;
+  uint32_t lo2, hi2;
+  DevChain chain;
 };
+
+// How the sums become bytes: shift and clamp with a lower bound of any kind, or of 0, or any other chain.
+enum { PACKED = 0, PACKED_RELU = 1, OTHER = 2 };
 
 // The products of one channel group: the input pixel of the block, the columns and the first of them, and where their
 // weights begin in a row of blocks of 32 x 32 bytes, each with one filter tap on its diagonal (9: none).  Stride 1: the
@@ -127,9 +143,10 @@ struct Shape {
 
 // G: channel groups of a tile, 1 or 2 (P = 32 G channels).  PAIRS: a tile's input is one box of pixel pairs, not two
 // planes; where an image has P channels, an even width and padding 1.
-template <int S, int G, int PAIRS, int RELU>
+template <int S, int G, int PAIRS, int FORM>
 __global__ void __launch_bounds__(Shape<S>::THREADS, 1)
-conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ DwParams p) {
+conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_r,
+               const __grid_constant__ DwParams p) {
   using Sh = Shape<S>;
   constexpr int P = 32 * G;                               // bytes of a staged pixel
   constexpr int ROW = PAIRS ? 2 * P : P, LINE = (PAIRS ? TILE_X + 2 : TILE_X + 1) * ROW;   // a row of the operand, a line of them
@@ -142,6 +159,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2], bar_staged[2], bar_out_free[2];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
+  __shared__ __align__(16) int32_t bias_s[P];   // (other chains; the two others keep it in registers)
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* const ring = smem + W_BYTES;
   uint8_t* const out = ring + p.units * UNIT;
@@ -185,9 +203,13 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
       fence_async_smem();
       if (!p.bias_static) pdl_wait();
+      if (FORM == OTHER && t < P) {
+        const int32_t b = p.bias ? p.bias[c0 + t] : 0;
+        bias_s[t] = p.wide ? b : (int32_t)((uint32_t)(b + p.add) * (uint32_t)p.mul);
+      }
       const int g = G == 2 ? (warp - 2) >> (S == 1 ? 3 : 2) : 0;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) bias[j] = (int32_t)((uint32_t)((p.bias ? p.bias[c0 + g * 32 + j] : 0) + p.add) * (uint32_t)p.mul);
+      for (int j = 0; j < (FORM == OTHER ? 0 : 32); ++j) bias[j] = (int32_t)((uint32_t)((p.bias ? p.bias[c0 + g * 32 + j] : 0) + p.add) * (uint32_t)p.mul);
     }
     if (warp == Sh::IO_WARP && lane < 2)
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &tmap_y : &tmap_x)) : "memory");
@@ -205,6 +227,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     *n0 = i * p.per_tile;
   };
   const int step = (int)gridDim.x;
+  const bool has_operand = FORM == OTHER && p.kind > 0;   // its tile lies in the output buffer before the result does
 
   if (warp == 0) {
     // ---------------------------------------------------------------- input
@@ -292,7 +315,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     const bool works = !(G == 1 && S == 2 && sub == 1);
     const int bx = lane & 7, by = quarter * 4 + (lane >> 3);
     const int img = p.per_tile > 1 ? fdiv(by, p.fd_pitch) : 0, ly = by - img * p.pitch_y;
-    const FastQ fq = {p.lo, p.hi, 0, 0};
+    const FastQ fq = {p.lo, p.hi, FORM == OTHER ? p.lo2 : 0, FORM == OTHER ? p.hi2 : 0};
     const int mul = p.mul;
     const uint32_t base = smem_u32(out);
     int k = 0;
@@ -304,7 +327,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       const uint32_t use = (uint32_t)(k >> 1) & 1u;
       // (a warp whose 32 rows all lie outside the images has nothing to write)
       const bool any = __any_sync(0xffffffffu, x0 + bx < p.rows_x && y0 + ly < p.rows_y && img < p.per_tile && n0 + img < p.images);
-      if (!mbar_wait(&bar_out_free[acc], use ^ 1u, &abort_flag, 5)) break;
+      if (!mbar_wait(&bar_out_free[acc], has_operand ? use : use ^ 1u, &abort_flag, 5)) break;
       if (!mbar_wait(&bar_acc_full[acc], use, &abort_flag, 4)) break;
       tc_fence_after();
       if (works && any) {
@@ -314,16 +337,50 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           int32_t v[32];
           tmem_ld32(t0 + (uint32_t)(c * 32), v);
           const int q = first + c, oy = S == 1 ? q >> 1 : 0, ox = S == 1 ? (q ^ (q >> 1)) & 1 : 0;   // (0,0), (0,1), (1,1), (1,0)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = v[j] * mul + bias[j];
-          uint4 a, b;
-          const uint4 none = make_uint4(0, 0, 0, 0);
-          fast_requant<RELU, 0>(fq, v, none, none, &a, &b);
           // the output tile lies as the store takes it: lines of pixels, swizzled
           const uint32_t lin = base + (uint32_t)(acc * OUT_BYTES + (by * Sh::OUT + oy) * OUT_LINE + (bx * Sh::OUT + ox) * P + g * 32);
-          const uint32_t key = ((lin >> 7) & p.out_mask) << 4;
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lin ^ key), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w) : "memory");
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"((lin + 16u) ^ key), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+          const uint32_t key = ((lin >> 7) & p.out_mask) << 4, at0 = lin ^ key, at1 = (lin + 16u) ^ key;
+          uint4 a, b;
+          const uint4 none = make_uint4(0, 0, 0, 0);
+          if (FORM == OTHER) {
+            if (p.kind < 0) {
+              const int x = (x0 + bx) * Sh::OUT + ox, y = (y0 + ly) * Sh::OUT + oy;
+              const bool inside = img < p.per_tile && n0 + img < p.images && x < p.out_w && y < p.out_h;
+              const size_t at = (((size_t)(n0 + img) * p.out_h + y) * p.out_w + x) * p.C + c0 + g * 32;
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {   // (16 columns at a time: with a tensor operand 32 do not fit the registers)
+                int32_t u[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = v[16 * h + j];
+                if (inside) apply_chain<16>(p.chain, u, at + 16 * h, c0 + g * 32 + 16 * h);
+                (h ? b : a) = make_uint4(pack4(u[0], u[1], u[2], u[3]), pack4(u[4], u[5], u[6], u[7]), pack4(u[8], u[9], u[10], u[11]), pack4(u[12], u[13], u[14], u[15]));
+              }
+            } else {
+              const int4* bp = reinterpret_cast<const int4*>(bias_s + g * 32);
+              const int am = p.add * mul;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const int4 b4 = bp[j];
+                const int32_t bj[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[4 * j + i] = p.wide ? min(max(v[4 * j + i] + bj[i], p.pre_lo), p.pre_hi) * mul + am : v[4 * j + i] * mul + bj[i];
+              }
+              uint4 r0 = none, r1 = none;
+              if (has_operand) {
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r0.x), "=r"(r0.y), "=r"(r0.z), "=r"(r0.w) : "r"(at0));
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r1.x), "=r"(r1.y), "=r"(r1.z), "=r"(r1.w) : "r"(at1));
+              }
+              if (p.kind == 0) fast_requant<0, 0>(fq, v, none, none, &a, &b);
+              else if (p.kind == 2) fast_requant<0, 2>(fq, v, r0, r1, &a, &b);
+              else fast_requant<0, 3>(fq, v, r0, r1, &a, &b);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = v[j] * mul + bias[j];
+            fast_requant<FORM == PACKED_RELU, 0>(fq, v, none, none, &a, &b);
+          }
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at0), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at1), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
         }
       }
       tc_fence_before();
@@ -338,7 +395,22 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     // ---------------------------------------------------------------- output
     const bool leader = elect_one();
     int k = 0;
+    auto hand_back = [&](int buf, int tile) {   // buffer `buf`, to the requantisation of tile `tile`
+      if (FORM == OTHER && has_operand) {
+        if (tile >= p.num_tiles) return;
+        int x0, y0, n0;
+        origin(tile, &x0, &y0, &n0);
+        const int count = min(p.per_tile, p.images - n0);
+        mbar_expect_tx(&bar_out_free[buf], (uint32_t)(count * p.out_box_bytes));
+        for (int i = 0; i < count; ++i)
+          tma_load_4d(out + buf * OUT_BYTES + (size_t)(i * p.pitch_y * Sh::OUT) * OUT_LINE, &tmap_r, &bar_out_free[buf], c0,
+                      p.out_pairs ? x0 * Sh::OUT / 2 : x0 * Sh::OUT, y0 * Sh::OUT, n0 + i);
+      } else {
+        mbar_arrive(&bar_out_free[buf]);
+      }
+    };
     pdl_wait();
+    if (has_operand && leader) { hand_back(0, blockIdx.x); hand_back(1, blockIdx.x + step); }
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += step, ++k) {
       int x0, y0, n0;
       origin(tile, &x0, &y0, &n0);
@@ -350,7 +422,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           tma_store_4d(&tmap_y, src + (size_t)(i * p.pitch_y * Sh::OUT) * OUT_LINE, c0, p.out_pairs ? x0 * Sh::OUT / 2 : x0 * Sh::OUT, y0 * Sh::OUT, n0 + i);
         tma_store_commit();
         tma_store_wait_read();
-        mbar_arrive(&bar_out_free[buf]);
+        hand_back(buf, tile + 2 * step);
       }
       __syncwarp();
     }
@@ -381,27 +453,31 @@ CUresult encode(EncodeTiledFn enc, CUtensorMap* map, const void* base, int64_t n
              box_c == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (box_c == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B), promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-template <int S, int G, int PAIRS, int RELU>
-int launch(const CUtensorMap& tx, const CUtensorMap& ty, const DwParams& p, int grid, int smem, int dev, cudaStream_t stream) {
+template <int S, int G, int PAIRS, int FORM>
+int launch(const CUtensorMap& tx, const CUtensorMap& ty, const CUtensorMap& tr, const DwParams& p, int grid, int smem, int dev, cudaStream_t stream) {
   static bool attr_set_dev[64] = {false};
   bool& attr_set = attr_set_dev[dev & 63];
   if (!attr_set) {
-    if (check_cuda(cudaFuncSetAttribute(conv_dw_kernel<S, G, PAIRS, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX), "cudaFuncSetAttribute(conv_dw_kernel)"))
+    if (check_cuda(cudaFuncSetAttribute(conv_dw_kernel<S, G, PAIRS, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX), "cudaFuncSetAttribute(conv_dw_kernel)"))
       return CVMK_ERR_CUDA;
     attr_set = true;
   }
-  launch_pdl(conv_dw_kernel<S, G, PAIRS, RELU>, dim3((unsigned)grid), dim3(Shape<S>::THREADS), smem, stream, tx, ty, p);
+  launch_pdl(conv_dw_kernel<S, G, PAIRS, FORM>, dim3((unsigned)grid), dim3(Shape<S>::THREADS), smem, stream, tx, ty, tr, p);
   return check_cuda(cudaGetLastError(), "conv_dw_kernel launch");
 }
 
-typedef int (*LaunchFn)(const CUtensorMap&, const CUtensorMap&, const DwParams&, int, int, int, cudaStream_t);
-const LaunchFn launches[16] = {   // [stride - 1][groups - 1][pairs][relu]
-    launch<1, 1, 0, 0>, launch<1, 1, 0, 1>, launch<1, 1, 1, 0>, launch<1, 1, 1, 1>, launch<1, 2, 0, 0>, launch<1, 2, 0, 1>, launch<1, 2, 1, 0>, launch<1, 2, 1, 1>,
-    launch<2, 1, 0, 0>, launch<2, 1, 0, 1>, launch<2, 1, 1, 0>, launch<2, 1, 1, 1>, launch<2, 2, 0, 0>, launch<2, 2, 0, 1>, launch<2, 2, 1, 0>, launch<2, 2, 1, 1>};
+typedef int (*LaunchFn)(const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const DwParams&, int, int, int, cudaStream_t);
+template <int S, int G, int PAIRS>
+LaunchFn of_form(int form) { return form == OTHER ? launch<S, G, PAIRS, OTHER> : (form == PACKED ? launch<S, G, PAIRS, PACKED> : launch<S, G, PAIRS, PACKED_RELU>); }
+template <int S>
+LaunchFn of_shape(int groups, bool pairs, int form) {
+  if (groups == 1) return pairs ? of_form<S, 1, 1>(form) : of_form<S, 1, 0>(form);
+  return pairs ? of_form<S, 2, 1>(form) : of_form<S, 2, 0>(form);
+}
 
 }  // namespace
 
-int launch_conv_dw(const cvmk_conv_direct_desc& d, const DwRequant& rq, cudaStream_t stream) {
+int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaStream_t stream) {
   const int S = d.stride_h;
   if (d.C % 32 != 0 || d.x_dtype != CVMK_I8 || d.y_dtype != CVMK_I8 || d.KH != 3 || d.KW != 3 || d.dil_h != 1 || d.dil_w != 1 ||
       (S != 1 && S != 2) || d.stride_w != S || d.pad_h > 1 || d.pad_w > 1 || d.N < 1 || d.OH < 1 || d.OW < 1)
@@ -412,7 +488,7 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DwRequant& rq, cudaStre
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   DwParams p;
   memset(&p, 0, sizeof(p));
-  p.w = d.w; p.bias = rq.bias; p.status = d.status;
+  p.w = d.w; p.status = d.status;
   p.C = d.C; p.images = d.N;
   p.pad_h = d.pad_h; p.pad_w = d.pad_w;
   p.rows_x = (d.OW + out - 1) / out;
@@ -453,10 +529,19 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DwRequant& rq, cudaStre
   p.units = std::min(MAX_UNITS, (SMEM_MAX - 1024 - w_bytes - 2 * out_bytes) / unit_bytes);
   p.out_pairs = out_pairs;
   p.out_mask = (uint32_t)((out_pairs ? 2 * P : P) / 16 - 1);
-  p.mul = rq.mul; p.add = rq.add;
-  auto x2 = [](int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; };
-  p.lo = x2(rq.lo); p.hi = x2(rq.hi);
+  const int first = chain.n > 0 && chain.s[0].op == K_ADD_C;
+  PackedChain pc;
+  memset(&pc, 0, sizeof(pc));
+  const bool packed = pack_chain(chain, first, d.acc_bound, &pc) && (!pc.kind || ((uintptr_t)chain.s[pc.step].ptr & 15) == 0);
+  p.bias = first ? reinterpret_cast<const int32_t*>(chain.s[0].ptr) : nullptr;
+  p.mul = pc.mul; p.add = pc.add;
+  p.lo = both_halves(pc.lo); p.hi = both_halves(pc.hi);
+  p.kind = packed ? pc.kind : -1;
+  p.wide = pc.wide; p.pre_lo = pc.pre_lo; p.pre_hi = pc.pre_hi;
+  p.lo2 = both_halves(pc.lo2); p.hi2 = both_halves(pc.hi2);
   p.bias_static = d.bias_static;
+  p.out_w = d.OW; p.out_h = d.OH;
+  p.chain = chain;
   // (206 KB and more: beside a CTA of this kernel, which has all TMEM columns of its SM, no CTA of conv_tc_kernel starts)
   const int smem = std::max(1024 + w_bytes + p.units * unit_bytes + 2 * out_bytes, 206 * 1024);
 
@@ -467,15 +552,22 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DwRequant& rq, cudaStre
     return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? (EncodeTiledFn)fn : (EncodeTiledFn) nullptr;
   }();
   if (!enc) { set_error("conv_dw: cuTensorMapEncodeTiled not found"); return CVMK_ERR_CUDA; }
-  CUtensorMap tx, ty;
-  const int f = pairs ? 2 : 1, fo = out_pairs ? 2 : 1;
+  CUtensorMap tx, ty, tr;
+  const int f = pairs ? 2 : 1, fo = out_pairs ? 2 : 1, out_h = (p.per_tile > 1 ? p.pitch_y : TILE_Y) * out;
+  p.out_box_bytes = TILE_X * out * P * out_h;
+  auto encode_out = [&](CUtensorMap* map, const void* base, CUtensorMapL2promotion promo) {
+    return encode(enc, map, base, d.N, d.OH, d.OW / fo, d.C * fo, P * fo, TILE_X * out / fo, out_h, 1, 1, promo);
+  };
   if (encode(enc, &tx, d.x, d.N, d.H, d.W / f, d.C * f, row, pairs ? box_w : 2 * box_w, box_h, p.per_tile, pairs ? 1 : 2, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) != CUDA_SUCCESS ||
-      encode(enc, &ty, d.y, d.N, d.OH, d.OW / fo, d.C * fo, P * fo, TILE_X * out / fo, (p.per_tile > 1 ? p.pitch_y : TILE_Y) * out, 1, 1, CU_TENSOR_MAP_L2_PROMOTION_NONE) != CUDA_SUCCESS) {
+      encode_out(&ty, d.y, CU_TENSOR_MAP_L2_PROMOTION_NONE) != CUDA_SUCCESS ||
+      encode_out(&tr, p.kind > 0 ? chain.s[pc.step].ptr : d.y, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) != CUDA_SUCCESS) {
     set_error("conv_dw: tensor map rejected");
     return CVMK_ERR_CUDA;
   }
   const int grid = (int)(std::min<int64_t>(tiles, sms) / p.c_tiles * p.c_tiles);
-  return launches[8 * (S - 1) + 4 * (G - 1) + 2 * pairs + (rq.lo == 0)](tx, ty, p, grid, smem, dev, stream);
+  const int form = p.kind != 0 || p.wide ? OTHER : (pc.lo == 0 ? PACKED_RELU : PACKED);
+  const LaunchFn launch_form = S == 1 ? of_shape<1>(G, pairs, form) : of_shape<2>(G, pairs, form);
+  return launch_form(tx, ty, tr, p, grid, smem, dev, stream);
 }
 
 }  // namespace cvmk

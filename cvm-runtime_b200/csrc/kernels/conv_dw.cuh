@@ -5,14 +5,7 @@
 
 namespace cvmk {
 
-// The chain of a depthwise layer in the packed form: [bias,] then ((sum + bias + add) * mul) >> 16 clamped to [lo, hi].
-struct DwRequant {
-  const int32_t* bias;
-  int mul, add;
-  int lo, hi;
-};
-
-// Launches the layer, or returns -1 when it is not one for this kernel.
-int launch_conv_dw(const cvmk_conv_direct_desc& d, const DwRequant& rq, cudaStream_t stream);
+// Launches the layer with its chain, or returns -1 when it is not one for this kernel.
+int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaStream_t stream);
 
 }  // namespace cvmk

@@ -779,22 +779,14 @@ extern "C" int cvmk_conv2d_stem_launch(const cvmk_stem_conv_plan* plan, cvmk_str
     p.first_step = 1;
   }
   // packed requantisation: chain = [bias] rs_clamp, same proof obligations as the general kernel
-  if (d.acc_bound > 0 && p.chain.n - p.first_step == 1 && p.chain.s[p.first_step].op == K_RS_CLAMP &&
-      !dev_env("CVM_B200_NO_FAST_REQUANT")) {
-    const DevStep& rs = p.chain.s[p.first_step];
-    const int64_t add = rs.c;
-    const int sh = rs.d;
-    const int64_t lo1 = ((int64_t)rs.a + add) >> sh, hi1 = ((int64_t)rs.b + add) >> sh;
-    if (d.acc_bound + add < (int64_t)INT32_MAX && ((d.acc_bound + add) >> sh) < 32767 && lo1 >= -32767 &&
-        hi1 <= 32767 && lo1 <= hi1 && sh <= 16) {
-      auto x2 = [](int64_t v) { return (uint32_t)((uint32_t)(uint16_t)(int16_t)v | ((uint32_t)(uint16_t)(int16_t)v << 16)); };
-      p.fast_mode = 1;
-      p.fast_variant = lo1 == 0 ? 1 : 0;
-      p.f_mul = 1 << (16 - sh);
-      p.f_add = (int)add;
-      p.f_lo1 = x2(lo1);
-      p.f_hi1 = x2(hi1);
-    }
+  PackedChain pc;
+  if (pack_chain(p.chain, p.first_step, d.acc_bound, &pc) && pc.kind == 0 && !pc.wide && !dev_env("CVM_B200_NO_FAST_REQUANT")) {
+    p.fast_mode = 1;
+    p.fast_variant = pc.lo == 0 ? 1 : 0;
+    p.f_mul = pc.mul;
+    p.f_add = pc.add;
+    p.f_lo1 = both_halves(pc.lo);
+    p.f_hi1 = both_halves(pc.hi);
   }
   static bool attr_set_dev[64] = {false};
   int dev = 0;

@@ -97,12 +97,10 @@ struct ConvParams {
   int ring_bytes;       // bytes of the operand ring (the staging buffers follow it)
   // Requantisation fast path (see fast_requant below): 0 off, 1 shift+clamp, 2 + tensor add/sub + clamp
   int fast_mode;
-  int f_shift;          // rounding shift (<= 16); its addend 2^(shift-1) is folded into the staged bias
   int f_mul;            // 2^(16 - shift)
-  int f_add;
+  int f_add;            // the shift's rounding addend, folded into the staged bias
   uint32_t f_lo1, f_hi1;  // first clamp, both halves of an s16x2 word
   uint32_t f_lo2, f_hi2;  // clamp after the tensor step
-  int f_sub;            // tensor step subtracts its operand
   int dbg;              // development builds: bit 0 skips the weight loads (timing experiments only)
   int fast_wide;        // the biased sum may exceed the multiply-add's range: clamp it first (f_pre_lo / f_pre_hi)
   int f_pre_lo, f_pre_hi;
@@ -1645,46 +1643,17 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   p.fast_mode = 0;
   const bool small = plan->small_split > 0;
   const bool packed_out = small ? (!plan->small_swap && d.y_dtype == CVMK_I8 && d.OC % 32 == 0) : (p.tma_out && d.OC <= MAX_BIAS);
-  if (packed_out && d.acc_bound > 0 && !dev_env("CVM_B200_NO_FAST_REQUANT")) {
-    const int i0 = p.first_step;
-    const int left = p.chain.n - i0;
-    if (left >= 1 && p.chain.s[i0].op == K_RS_CLAMP) {
-      const DevStep& rs = p.chain.s[i0];
-      const int64_t add = rs.c;
-      const int sh = rs.d;
-      const int64_t lo1 = ((int64_t)rs.a + add) >> sh, hi1 = ((int64_t)rs.b + add) >> sh;
-      const bool no_overflow = d.acc_bound + add < (int64_t)INT32_MAX;
-      const bool fits16 = ((d.acc_bound + add) >> sh) < 32767;
-      const bool clamp_ok = lo1 >= -32767 && hi1 <= 32767 && lo1 <= hi1 && sh <= 16;
-      // Without fits16 the sum is clamped to [rs.a, rs.b] before it is scaled (fast_wide); the
-      // clamped value plus the rounding addend then stays below 2^(15 + shift).
-      const bool wide_ok = (int64_t)rs.b + add < ((int64_t)1 << (15 + sh)) && (int64_t)rs.a + add > -((int64_t)1 << (15 + sh));
-      p.fast_wide = 0;
-      if (no_overflow && (fits16 || wide_ok) && clamp_ok) {
-        if (!fits16) { p.fast_wide = 1; p.f_pre_lo = rs.a; p.f_pre_hi = rs.b; }
-        auto x2 = [](int64_t v) { return (uint32_t)((uint32_t)(uint16_t)(int16_t)v | ((uint32_t)(uint16_t)(int16_t)v << 16)); };
-        if (left == 1) {
-          p.fast_mode = 1;
-        } else if (left == 3 && p.res_step == i0 + 1 && p.chain.s[i0 + 2].op == K_CLIP &&
-                   (p.chain.s[i0 + 1].op == K_ADD_T || p.chain.s[i0 + 1].op == K_SUB_T) &&
-                   p.chain.s[i0 + 2].a >= -32767 && p.chain.s[i0 + 2].b <= 32767 &&
-                   std::max(std::abs(lo1), std::abs(hi1)) + 128 < 32767) {
-          p.fast_mode = 2;
-          p.f_sub = p.chain.s[i0 + 1].op == K_SUB_T;
-          p.f_lo2 = x2(p.chain.s[i0 + 2].a);
-          p.f_hi2 = x2(p.chain.s[i0 + 2].b);
-        }
-        if (p.fast_mode) {
-          const int kind = p.fast_mode == 1 ? 0 : (p.f_sub ? 3 : (p.chain.s[i0 + 2].a == 0 ? 1 : 2));
-          p.fast_variant = (lo1 == 0 ? 1 : 0) + 2 * kind;
-          p.f_shift = sh;
-          p.f_mul = 1 << (16 - sh);
-          p.f_add = (int)add;
-          p.f_lo1 = x2(lo1);
-          p.f_hi1 = x2(hi1);
-        }
-      }
-    }
+  PackedChain pc;
+  if (packed_out && !dev_env("CVM_B200_NO_FAST_REQUANT") && pack_chain(p.chain, p.first_step, d.acc_bound, &pc) &&
+      (pc.kind == 0 || pc.step == p.res_step)) {
+    p.fast_mode = pc.kind ? 2 : 1;
+    p.fast_variant = (pc.lo == 0 ? 1 : 0) + 2 * (pc.kind == 2 && pc.lo2 == 0 ? 1 : pc.kind);
+    p.fast_wide = pc.wide;
+    p.f_pre_lo = pc.pre_lo; p.f_pre_hi = pc.pre_hi;
+    p.f_mul = pc.mul;
+    p.f_add = pc.add;
+    p.f_lo1 = both_halves(pc.lo); p.f_hi1 = both_halves(pc.hi);
+    p.f_lo2 = both_halves(pc.lo2); p.f_hi2 = both_halves(pc.hi2);
   }
 
   if (small) {

@@ -24,3 +24,34 @@ SHAPES = [(80, 64, 32, 16, 1, 1), (75, 64, 33, 17, 1, 1), (40, 64, 33, 18, 1, 1)
 def test_depthwise(n, c, h, w, stride, pad, relu, bias, gpu_run, oracle, wl):
     js, pb, x = cases.conv_case(c + h + n, n, c, h, w, c, 3, stride, pad, groups=c, bias=bias, relu=relu, shift=wl.GraphBuilder.default_shift(9))
     assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
+
+
+# chains without a packed form, run step by step: a clip without a shift, a shift that leaves more than 16 bits, a tensor
+# operand (whole batches and parts of them), a bias that is computed on the way; a tile an SM and more, and fewer
+CHAINS = ["clip", "wide", "residual", "activation_bias"]
+
+
+@pytest.mark.parametrize("n,c,h,w,stride", [(80, 64, 33, 17, 1), (40, 128, 28, 28, 1), (75, 64, 34, 18, 2), (151, 96, 14, 14, 1), (41, 32, 56, 56, 1), (2, 128, 28, 28, 1)])
+@pytest.mark.parametrize("chain", CHAINS)
+def test_depthwise_chain(n, c, h, w, stride, chain, gpu_run, oracle, wl):
+    g = wl.GraphBuilder(c + h)
+    x = cases.rnd(np.random.RandomState(n), (n, c, h, w), 8)
+    d = g.var("data", x.shape, 8)
+    if chain == "activation_bias":
+        one = g.op("cvm_right_shift", [d], x.shape, {"precision": 4, "shift_bit": 4})
+        b = g.op("sum", [one], (c,), {"axis": (0, 2, 3), "keepdims": False, "exclude": False})
+        wt = g.var("w", (c, 1, 3, 3), 8, g.weight8((c, 1, 3, 3)))
+        oh, ow = (h - 1) // stride + 1, (w - 1) // stride + 1
+        y = g.op("conv2d", [d, wt, b], (n, c, oh, ow), {"channels": c, "kernel_size": (3, 3), "strides": (stride, stride), "padding": (1, 1),
+                 "dilation": (1, 1), "groups": c, "layout": "NCHW", "kernel_layout": "OIHW", "use_bias": True})
+        y = g.op("cvm_right_shift", [y], g.shape_of(y), {"precision": 8, "shift_bit": 7})
+    else:
+        y = g.conv(d, c, 3, stride, 1, groups=c, relu=chain == "wide", shift={"clip": 0, "wide": 2, "residual": None}[chain])
+    if chain == "clip":
+        y = g.op("cvm_clip", [y], g.shape_of(y), {"precision": 8})
+    if chain == "residual":
+        z = g.conv(d, c, 1, stride, 0, relu=False)
+        y = g.op("elemwise_sub", [y, z], g.shape_of(y))
+        y = g.op("cvm_clip", [y], g.shape_of(y), {"precision": 8})
+    js, pb = g.finish(y)
+    assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
