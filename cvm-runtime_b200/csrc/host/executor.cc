@@ -707,6 +707,7 @@ struct Lowering {
       sd.clamp = data_range;
       sd.status = ex.status_dev_;
       sd.acc_bound = probe.acc_bound;
+      sd.bias_static = probe.bias_static;
       sd.ep = ch.ep;
       if (W % 16 != 0) sd.x_pitch = (W + 15) / 16 * 16;   // TMA rows start on 16-byte boundaries: the rows are moved apart first
       if (cvmk_conv2d_stem_supported(&sd)) {

@@ -194,6 +194,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       const int t = (int)threadIdx.x - 64;
       for (int i = t; i < W_BYTES / 16; i += 32 * Sh::EPI_WARPS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
       asm volatile("bar.sync 2, %0;" ::"n"(32 * Sh::EPI_WARPS) : "memory");
+      if (!p.bias_static) pdl_wait();
       for (int i = t; i < G * Sh::BLOCKS * 32; i += 32 * Sh::EPI_WARPS) {
         const int c = i & 31, blk = i >> 5, g = blk / Sh::BLOCKS, b = blk - g * Sh::BLOCKS;
         const int tap = S == 1 ? block_taps1.t[b] : b;
@@ -202,7 +203,6 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         smem[(size_t)blk * 1024 + (at ^ (((at >> 7) & 1u) << 4))] = (uint8_t)p.w[(size_t)tap * p.C + c0 + g * 32 + c];
       }
       fence_async_smem();
-      if (!p.bias_static) pdl_wait();
       if (FORM == OTHER && t < P) {
         const int32_t b = p.bias ? p.bias[c0 + t] : 0;
         bias_s[t] = p.wide ? b : (int32_t)((uint32_t)(b + p.add) * (uint32_t)p.mul);

@@ -71,6 +71,7 @@ struct StemConvParams {
   int off_planar, off_staged, off_out, off_bias;  // byte offsets of the shared-memory regions after the weights
   int* status;
   const int32_t* bias;
+  int bias_static;      // the weights and the bias are parameters
   int first_step;
   int fast_mode, fast_variant, f_mul, f_add;
   uint32_t f_lo1, f_hi1;
@@ -311,6 +312,7 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (!p.bias_static) pdl_wait();
   // weights -> shared memory, the 16 bytes of a tap in the order of the staged pixels
   for (int i = threadIdx.x; i < p.w_bytes / 16; i += STEM_THREADS) {
     uint4 v = reinterpret_cast<const uint4*>(p.w)[i];
@@ -770,6 +772,7 @@ extern "C" int cvmk_conv2d_stem_launch(const cvmk_stem_conv_plan* plan, cvmk_str
   while ((1 << p.accs_log2) < p.accs) ++p.accs_log2;
   while ((1 << p.panels_log2) < p.panels) ++p.panels_log2;
   p.status = d.status;
+  p.bias_static = d.bias_static;
   int rc = lower_chain(d.ep, &p.chain);
   if (rc != CVMK_OK) return rc;
   p.bias = nullptr;

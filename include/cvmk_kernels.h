@@ -269,7 +269,8 @@ typedef struct {
   int32_t N, H, W, C, OC, KH, KW, OH, OW, groups;
   int32_t stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
   int32_t depthwise;
-  /* Non-zero: the bias (a leading ADD_C step) is a parameter, which no kernel in flight writes. */
+  /* Non-zero: the weights and the bias (a leading ADD_C step) are parameters, which no kernel in flight writes; they may
+   * be read before the previous kernel of the stream has finished. */
   int32_t bias_static;
   /* Upper bound on |sum + bias| over every output element (0 = unknown), as in cvmk_conv_desc: lets
    * the depthwise kernels requantise with packed 16-bit arithmetic. */
@@ -365,7 +366,7 @@ typedef struct {
   int64_t acc_bound;   /* as in cvmk_conv_desc */
   cvmk_epilogue ep;
   int32_t x_pitch;     /* bytes from one input row to the next; 0: W */
-  int32_t reserved;
+  int32_t bias_static; /* as in cvmk_conv_direct_desc */
 } cvmk_stem_conv_desc;
 
 typedef struct __attribute__((aligned(64))) {
