@@ -62,6 +62,7 @@ struct DwParams {
   int pad_h, pad_w;
   int per_tile;           // images of a tile
   int pitch_y;            // operand lines from one image of a tile to the next
+  int band;               // operand lines of an image in a tile
   int tiles_x, tiles_y, c_tiles, num_tiles;
   FastDiv fd_c, fd_x, fd_y, fd_pitch;
   int units, box_bytes;    // of the ring; bytes of a box
@@ -223,7 +224,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   auto origin = [&](int tile, int* x0, int* y0, int* n0) {
     const int m = fdiv(tile, p.fd_c), r = fdiv(m, p.fd_x), i = fdiv(r, p.fd_y);
     *x0 = (m - r * p.tiles_x) * TILE_X;
-    *y0 = (r - i * p.tiles_y) * TILE_Y;
+    *y0 = (r - i * p.tiles_y) * p.band;
     *n0 = i * p.per_tile;
   };
   const int step = (int)gridDim.x;
@@ -326,7 +327,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       const int acc = k & 1;
       const uint32_t use = (uint32_t)(k >> 1) & 1u;
       // (a warp whose 32 rows all lie outside the images has nothing to write)
-      const bool any = __any_sync(0xffffffffu, x0 + bx < p.rows_x && y0 + ly < p.rows_y && img < p.per_tile && n0 + img < p.images);
+      const bool any = __any_sync(0xffffffffu, x0 + bx < p.rows_x && ly < p.band && y0 + ly < p.rows_y && img < p.per_tile && n0 + img < p.images);
       if (!mbar_wait(&bar_out_free[acc], has_operand ? use : use ^ 1u, &abort_flag, 5)) break;
       if (!mbar_wait(&bar_acc_full[acc], use, &abort_flag, 4)) break;
       tc_fence_after();
@@ -345,7 +346,7 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           if (FORM == OTHER) {
             if (p.kind < 0) {
               const int x = (x0 + bx) * Sh::OUT + ox, y = (y0 + ly) * Sh::OUT + oy;
-              const bool inside = img < p.per_tile && n0 + img < p.images && x < p.out_w && y < p.out_h;
+              const bool inside = img < p.per_tile && ly < p.band && n0 + img < p.images && x < p.out_w && y < p.out_h;
               const size_t at = (((size_t)(n0 + img) * p.out_h + y) * p.out_w + x) * p.C + c0 + g * 32;
 #pragma unroll
               for (int h = 0; h < 2; ++h) {   // (16 columns at a time: with a tensor operand 32 do not fit the registers)
@@ -495,32 +496,43 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   p.rows_y = (d.OH + out - 1) / out;
   p.c_tiles = d.C / P;
   if (p.c_tiles > sms) return -1;
-  // Images of at most seven operand lines are stacked: each takes one line more than it has (what its last taps read),
-  // rounded up so that its part of the output tile starts on a multiple of 1024 bytes.
-  p.per_tile = 1;
-  p.pitch_y = TILE_Y;
-  if (p.rows_y + 1 <= TILE_Y / 2) {
-    const int whole = 1024 / (8 * out * out * P) > 1 ? 1024 / (8 * out * out * P) : 1;
-    p.pitch_y = (p.rows_y + 1 + whole - 1) / whole * whole;
-    p.per_tile = TILE_Y / p.pitch_y;
-    if (p.per_tile < 2) { p.per_tile = 1; p.pitch_y = TILE_Y; }
-  }
+  // A tile holds TILE_Y operand lines of one image, or as many of several as are stacked in it, each with one line more
+  // (what its last taps read), rounded up so that its part of the output tile starts on a multiple of 1024 bytes.  Images
+  // of at most seven lines are stacked whole; higher ones in bands of fewer lines where that takes fewer rounds of
+  // tiles (a band's last line is loaded again with the next, 16 % more input at seven lines).  Stride 1, in a chain of such
+  // layers, whole images -> bands: 256 channels at 16 x 16, 256 images 12.4 -> 10.0 us; 128 at 38 x 38, 128 images 24.3 ->
+  // 13.5 (on the CUDA cores before), 256 at 36 x 36, 128 images 39.5 -> 22.1 (likewise).
+  const int whole = std::max(1, 1024 / (8 * out * out * P));
   p.tiles_x = (p.rows_x + TILE_X - 1) / TILE_X;
-  p.tiles_y = (p.rows_y + TILE_Y - 1) / TILE_Y;
-  const int64_t tiles = (int64_t)p.tiles_x * p.tiles_y * ((d.N + p.per_tile - 1) / p.per_tile) * p.c_tiles;
+  const int64_t grid_max = sms / p.c_tiles * p.c_tiles;
+  int64_t tiles = 0, rounds = 0;
+  for (int band = std::min(p.rows_y, TILE_Y); band >= 1; --band) {
+    int pitch = (band + 1 + whole - 1) / whole * whole, images = TILE_Y / pitch;
+    if (images < 2) { pitch = TILE_Y; images = 1; }
+    if (images == 1 && band < std::min(p.rows_y, TILE_Y)) continue;
+    const int bands = (p.rows_y + band - 1) / band;
+    const int64_t t = (int64_t)p.tiles_x * bands * ((d.N + images - 1) / images) * p.c_tiles, r = (t + grid_max - 1) / grid_max;
+    if (tiles && r >= rounds) continue;
+    tiles = t; rounds = r;
+    p.band = band; p.pitch_y = pitch; p.per_tile = images; p.tiles_y = bands;
+  }
   if (tiles > INT32_MAX / 2) return -1;
   // One box of pixel pairs has half the rows of twice the bytes, and a store of pairs too, where the two pixels lie
   // side by side (C channels a tile).
   const bool pairs = d.C == P && d.W % 2 == 0 && d.pad_w == 1, out_pairs = d.C == P && d.OW % 2 == 0;
-  // The CUDA-core kernel stays the better one where the tiles do not give every SM one, and where half of the rows of
-  // the tiles lie outside the images (7 x 7, stride 1).  Device time with the line at 0, 96, 150, 296 and 592 tiles:
-  // MobileNet, one image 123, 99, 99, 99, 99 us; 20 images 182, 172, 170, 170, 176; 256 images 692 each (of 828 with
-  // none); SSD-512 on 3 images 328, 328, 329, 339, 350; on 8 images 450, 449, 440, 444, 455.  Pairs of pixels are worth
-  // it from half as many tiles on (SSD-512, one image: 293 -> 276 us).
-  if (tiles < (pairs ? sms / 2 : sms) || 2LL * p.rows_x * p.rows_y * p.per_tile < (int64_t)TILE_X * TILE_Y * p.tiles_x * p.tiles_y) return -1;
+  // The CUDA-core kernel stays the better one where the tiles do not give every SM one, and where five eighths of their
+  // rows lie outside the images.  Device time with the line at 0, 96, 150, 296 and 592 tiles: MobileNet, one image 123, 99,
+  // 99, 99, 99 us; 20 images 182, 172, 170, 170, 176; 256 images 692 each (of 828 with none); SSD-512 on 3 images 328, 328,
+  // 329, 339, 350; on 8 images 450, 449, 440, 444, 455.  Pairs of pixels are worth it from half as many tiles on (SSD-512, one
+  // image: 293 -> 276 us).  By the share of rows inside the images, a layer on the CUDA cores -> here: 0.47, 256 channels at 15 x
+  // 20, 256 images 23.8 -> 14.9 us; 0.42, 256 at 18 x 18, 128 images 14.0 -> 10.3; 0.39, 128 at 19 x 19, 128 images 10.0 -> 8.5,
+  // but 40 images of 20 x 20 5.4 -> 5.9, so the rows inside have to fill tiles for half of the SMs; 0.375, 512 at 8 x 8, 256
+  // images 9.6 -> 10.0, 1024 at 7 x 7 16.6 -> 15.1, 512 at 7 x 7 with a clip alone 16.6 -> 19.4.
+  const int64_t least = pairs ? sms / 2 : sms, used = (int64_t)p.rows_x * p.rows_y * d.N * p.c_tiles;
+  if (tiles < least || 2 * used < least * TILE_X * TILE_Y || 8 * used <= 3 * tiles * TILE_X * TILE_Y) return -1;
   p.num_tiles = (int)tiles;
   p.fd_c = make_fastdiv(p.c_tiles); p.fd_x = make_fastdiv(p.tiles_x); p.fd_y = make_fastdiv(p.tiles_y); p.fd_pitch = make_fastdiv(p.pitch_y);
-  const int box_h = p.per_tile > 1 ? 2 * p.pitch_y : std::min(BOX_H, 2 * (p.rows_y + 1));
+  const int box_h = p.per_tile > 1 ? 2 * p.pitch_y : std::min(BOX_H, 2 * (p.band + 1));
   const int row = pairs ? 2 * P : P, box_w = pairs ? TILE_X + 2 : TILE_X + 1;
   p.box_bytes = box_w * row * box_h * p.per_tile;
   const int unit_bytes = (box_w * row * BOX_H + 1023) & ~1023;   // (rows of a tile outside its images read the rest of a unit)
@@ -553,7 +565,7 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   }();
   if (!enc) { set_error("conv_dw: cuTensorMapEncodeTiled not found"); return CVMK_ERR_CUDA; }
   CUtensorMap tx, ty, tr;
-  const int f = pairs ? 2 : 1, fo = out_pairs ? 2 : 1, out_h = (p.per_tile > 1 ? p.pitch_y : TILE_Y) * out;
+  const int f = pairs ? 2 : 1, fo = out_pairs ? 2 : 1, out_h = p.band * out;
   p.out_box_bytes = TILE_X * out * P * out_h;
   auto encode_out = [&](CUtensorMap* map, const void* base, CUtensorMapL2promotion promo) {
     return encode(enc, map, base, d.N, d.OH, d.OW / fo, d.C * fo, P * fo, TILE_X * out / fo, out_h, 1, 1, promo);

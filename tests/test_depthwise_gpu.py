@@ -16,7 +16,11 @@ SHAPES = [(80, 64, 32, 16, 1, 1), (75, 64, 33, 17, 1, 1), (40, 64, 33, 18, 1, 1)
           (75, 64, 30, 31, 1, 1), (41, 32, 56, 56, 1, 1), (301, 128, 14, 14, 1, 1), (60, 32, 57, 63, 1, 1), (3, 32, 256, 254, 1, 1),
           (80, 64, 32, 16, 2, 1), (75, 64, 34, 18, 2, 1), (150, 64, 31, 15, 2, 1), (9, 96, 29, 93, 2, 1), (151, 128, 14, 14, 2, 1),
           (99, 192, 11, 16, 2, 1), (148, 32, 8, 16, 2, 1), (34, 64, 13, 141, 2, 0), (20, 1024, 14, 14, 2, 1), (41, 32, 112, 56, 2, 1),
-          (301, 128, 14, 14, 2, 1), (30, 128, 28, 56, 2, 1)]
+          (301, 128, 14, 14, 2, 1), (30, 128, 28, 56, 2, 1),
+          # images cut into bands of lines, several images' bands in a tile: 16, 15, 18 and 38 lines, the last band shorter, the
+          # last tile not full; 32 channels; stride 2
+          (151, 64, 16, 24, 1, 1), (200, 128, 15, 16, 1, 1), (299, 64, 18, 14, 1, 1), (75, 128, 38, 21, 1, 1), (299, 32, 16, 32, 1, 1),
+          (150, 128, 15, 20, 1, 1), (99, 192, 19, 19, 1, 1), (200, 64, 40, 16, 1, 0), (301, 64, 16, 48, 2, 1), (151, 128, 37, 31, 2, 1)]
 
 
 @pytest.mark.parametrize("n,c,h,w,stride,pad", SHAPES)
