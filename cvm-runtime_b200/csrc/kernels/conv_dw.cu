@@ -29,9 +29,9 @@
 //
 // Any chain behind the products: [bias] shift clamp has forms of its own; a wide sum, and the sum with another tensor (whose
 // tile TMA brings into the output buffer before the result), run packed too, everything else step by step.  128 channels at
-// 28 x 28, 150 images, in a chain of such layers: 9.4 us with shift and clamp, 15.4 with a wide sum, 15.9 with a tensor, 18.9
-// with a clip alone (depthwise3x3_kernel 39.0, 57.2, 34.8; the tensor loaded by the threads that need it 18.4: a
-// row's 32 bytes lie in a cache line of their own).
+// 28 x 28, 150 images, in a chain of such layers: 9.4 us with shift and clamp, 15.4 with a wide sum or a clip alone, 15.9 with a
+// tensor (depthwise3x3_kernel 39.0, 34.8, 57.2; the clip step by step 18.9; the tensor loaded by the threads that need it 18.4:
+// a row's 32 bytes lie in a cache line of their own).
 //
 // Reproduces groupwise_conv2d with groups = C (src/runtime/cpu/ops/ops.cc:333-366) and the chain behind it.
 // Every wait is bounded, as in conv_tc.cu.
@@ -527,7 +527,7 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   // image: 293 -> 276 us).  By the share of rows inside the images, a layer on the CUDA cores -> here: 0.47, 256 channels at 15 x
   // 20, 256 images 23.8 -> 14.9 us; 0.42, 256 at 18 x 18, 128 images 14.0 -> 10.3; 0.39, 128 at 19 x 19, 128 images 10.0 -> 8.5,
   // but 40 images of 20 x 20 5.4 -> 5.9, so the rows inside have to fill tiles for half of the SMs; 0.375, 512 at 8 x 8, 256
-  // images 9.6 -> 10.0, 1024 at 7 x 7 16.6 -> 15.1, 512 at 7 x 7 with a clip alone 16.6 -> 19.4.
+  // images 9.6 -> 10.0, 1024 at 7 x 7 16.6 -> 15.1.
   const int64_t least = pairs ? sms / 2 : sms, used = (int64_t)p.rows_x * p.rows_y * d.N * p.c_tiles;
   if (tiles < least || 2 * used < least * TILE_X * TILE_Y || 8 * used <= 3 * tiles * TILE_X * TILE_Y) return -1;
   p.num_tiles = (int)tiles;
@@ -544,7 +544,13 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   const int first = chain.n > 0 && chain.s[0].op == K_ADD_C;
   PackedChain pc;
   memset(&pc, 0, sizeof(pc));
-  const bool packed = pack_chain(chain, first, d.acc_bound, &pc) && (!pc.kind || ((uintptr_t)chain.s[pc.step].ptr & 15) == 0);
+  bool packed = pack_chain(chain, first, d.acc_bound, &pc) && (!pc.kind || ((uintptr_t)chain.s[pc.step].ptr & 15) == 0);
+  if (chain.n - first == 1 && chain.s[first].op == K_CLIP && chain.s[first].a >= -32767 && chain.s[first].b <= 32767) {   // a shift by 0
+    packed = true;
+    pc.wide = 1; pc.mul = 1 << 16;
+    pc.pre_lo = pc.lo = chain.s[first].a;
+    pc.pre_hi = pc.hi = chain.s[first].b;
+  }
   p.bias = first ? reinterpret_cast<const int32_t*>(chain.s[0].ptr) : nullptr;
   p.mul = pc.mul; p.add = pc.add;
   p.lo = both_halves(pc.lo); p.hi = both_halves(pc.hi);

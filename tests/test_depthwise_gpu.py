@@ -30,9 +30,10 @@ def test_depthwise(n, c, h, w, stride, pad, relu, bias, gpu_run, oracle, wl):
     assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
 
 
-# chains without a packed form, run step by step: a clip without a shift, a shift that leaves more than 16 bits, a tensor
-# operand (whole batches and parts of them), a bias that is computed on the way; a tile an SM and more, and fewer
-CHAINS = ["clip", "wide", "residual", "activation_bias"]
+# chains that are not just a shift: a clip without one, a shift that leaves more than 16 bits, a tensor operand (whole batches
+# and parts of them), a bias that is computed on the way, and a chain that is run step by step with a tensor operand in it;
+# a tile an SM and more, and fewer
+CHAINS = ["clip", "wide", "residual", "activation_bias", "steps"]
 
 
 @pytest.mark.parametrize("n,c,h,w,stride", [(80, 64, 33, 17, 1), (40, 128, 28, 28, 1), (75, 64, 34, 18, 2), (151, 96, 14, 14, 1), (41, 32, 56, 56, 1), (2, 128, 28, 28, 1)])
@@ -50,12 +51,14 @@ def test_depthwise_chain(n, c, h, w, stride, chain, gpu_run, oracle, wl):
                  "dilation": (1, 1), "groups": c, "layout": "NCHW", "kernel_layout": "OIHW", "use_bias": True})
         y = g.op("cvm_right_shift", [y], g.shape_of(y), {"precision": 8, "shift_bit": 7})
     else:
-        y = g.conv(d, c, 3, stride, 1, groups=c, relu=chain == "wide", shift={"clip": 0, "wide": 2, "residual": None}[chain])
+        y = g.conv(d, c, 3, stride, 1, groups=c, relu=chain == "wide", shift={"clip": 0, "wide": 2}.get(chain))
     if chain == "clip":
         y = g.op("cvm_clip", [y], g.shape_of(y), {"precision": 8})
-    if chain == "residual":
+    if chain in ("residual", "steps"):
         z = g.conv(d, c, 1, stride, 0, relu=False)
-        y = g.op("elemwise_sub", [y, z], g.shape_of(y))
+        y = g.op("elemwise_sub", [y, z] if chain == "residual" else [z, y], g.shape_of(y))
+        if chain == "steps":
+            y = g.op("abs", [y], g.shape_of(y))
         y = g.op("cvm_clip", [y], g.shape_of(y), {"precision": 8})
     js, pb = g.finish(y)
     assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
