@@ -4,55 +4,13 @@ import ctypes as ct
 import numpy as np
 import pytest
 
+from kernel_desc import (ADD_C, I8, I32, RSHIFT, Conv, ConvPlan, Direct, Reduce, Stem, chain, conv_sums, int8, right_shift, shape)
+
 pytestmark = pytest.mark.gpu
-
-RSHIFT, ADD_C = 2, 8
-
-
-class Step(ct.Structure):
-    _fields_ = [("op", ct.c_int32), ("a", ct.c_int32), ("b", ct.c_int32), ("ptr_dtype", ct.c_int32), ("ptr", ct.c_void_p)]
-
-
-class Epilogue(ct.Structure):
-    _fields_ = [("n", ct.c_int32), ("reserved", ct.c_int32), ("s", Step * 8)]
-
-
-def ints(names):
-    return [(n, ct.c_int32) for n in names.split()]
-
-
-class Direct(ct.Structure):
-    _fields_ = ([("x", ct.c_void_p)] + ints("x_dtype narrow_x") + [("w", ct.c_void_p), ("y", ct.c_void_p)] +
-                ints("y_dtype N H W C OC KH KW OH OW groups stride_h stride_w pad_h pad_w dil_h dil_w depthwise bias_static") +
-                [("acc_bound", ct.c_int64), ("ep", Epilogue), ("status", ct.c_void_p)])
-
-
-class Stem(ct.Structure):
-    _fields_ = ([("x", ct.c_void_p), ("w", ct.c_void_p), ("y", ct.c_void_p)] +
-                ints("N H W C OC KH KW OH OW stride_h stride_w pad_h pad_w clamp") +
-                [("status", ct.c_void_p), ("acc_bound", ct.c_int64), ("ep", Epilogue)] + ints("x_pitch bias_static"))
-
-
-class Reduce(ct.Structure):
-    _fields_ = (ints("is_max init_zero n_keep n_red") + [(n, ct.c_int64 * 6) for n in ("keep_extent", "keep_stride", "red_extent", "red_stride")] +
-                [("x", ct.c_void_p)] + ints("x_dtype pad0") + [("y", ct.c_void_p)] + ints("y_dtype pad1") + [("ep", Epilogue)])
 
 
 def shift_clip(desc, shift, bias=None):
-    steps = ([(ADD_C, 0, 0, 4, bias)] if bias else []) + [(RSHIFT, shift, 8, 0, None)]
-    desc.ep.n = len(steps)
-    for i, s in enumerate(steps):
-        desc.ep.s[i] = Step(*s)
-
-
-def conv(torch, x, w, bias, shift, stride, pad, groups):
-    """int8 NCHW in, int8 NHWC out: the sums in 64 bits, exact, then cvm_right_shift to 8 bits."""
-    s = torch.nn.functional.conv2d(x.double(), w.double(), bias.double() if bias is not None else None, stride, pad, 1, groups).long()
-    return (((s >> (shift - 1)) + 1) >> 1).clamp(-127, 127).to(torch.int8).permute(0, 2, 3, 1).contiguous()
-
-
-def int8(torch, rng, *shape):
-    return torch.from_numpy(rng.randint(-127, 128, size=shape).astype(np.int8)).cuda()
+    chain(desc, ([(ADD_C, 0, 0, I32, bias)] if bias else []) + [(RSHIFT, shift, 8, 0, None)])
 
 
 # Weights and a bias that the kernel in front of the launch writes, with bias_static left 0.  That kernel is a sum of many rows
@@ -72,8 +30,7 @@ def test_weights_written_by_the_kernel_before(kind, rt):
     else:
         d, xin, wk = Stem(), x, None
         d.clamp = 127
-    for name, value in dict(N=n, H=h, W=h, C=c, OC=oc, KH=k, KW=k, OH=oh, OW=oh, stride_h=step, stride_w=step, pad_h=k // 2, pad_w=k // 2).items():
-        setattr(d, name, value)
+    shape(d, n, c, h, h, oc, k, step, k // 2)
     d.acc_bound = (c // groups) * k * k * 128 * 128 + 5000
     if wk is None:
         packed = np.zeros(lib.cvmk_conv2d_stem_weight_bytes(ct.byref(d)), np.int8)
@@ -103,4 +60,38 @@ def test_weights_written_by_the_kernel_before(kind, rt):
         assert lib.cvmk_reduce(ct.byref(total), at) == 0
         assert (lib.cvmk_conv2d_stem_launch(plan, at) if plan else lib.cvmk_conv2d_direct(ct.byref(d), at)) == 0
         torch.cuda.synchronize()
-    assert torch.equal(y, conv(torch, x, w, bias, shift, step, k // 2, groups))
+    want = conv_sums(torch, x, w, step, k // 2, groups) + bias.long()
+    assert torch.equal(y, right_shift(want, shift).to(torch.int8))
+
+
+# The grouped form of the persistent kernel, which the executor does not launch.  (n, channels, h, w, fold), sizes of the
+# real image: one to three N tiles of 4, 2 and 1 groups of 32 channels; folded pixels, 2 of 64 channels and 4 of 32; an odd
+# number of 128-row tiles, and patches that end outside the image
+@pytest.mark.parametrize("n,c,h,w,fold", [(171, 128, 16, 24, 1), (129, 256, 15, 24, 1), (75, 96, 16, 24, 1), (33, 192, 31, 23, 1), (1, 128, 16, 8, 1),
+                                          (171, 64, 16, 48, 2), (75, 64, 30, 46, 2), (171, 32, 16, 96, 4), (75, 32, 30, 92, 4)])
+@pytest.mark.parametrize("packed", [True, False])
+def test_grouped(n, c, h, w, fold, packed, rt):
+    import torch
+    lib, rng = rt.lib(), np.random.RandomState(n + c)
+    x, wt = int8(torch, rng, n, c, h, w), int8(torch, rng, c, 32, 3, 3)
+    bias = torch.from_numpy(rng.randint(-5000, 5000, size=c).astype(np.int32)).cuda()
+    d, shift = Conv(), 11
+    shape(d, n, c * fold, h, w // fold, c * fold, 3, 1, 1)
+    d.dil_h = d.dil_w = 1
+    d.groups, d.group_fold = c * fold // 32, fold
+    d.acc_bound = 32 * 9 * 127 * 127 + 5000 if packed else 0
+    xin, y = x.permute(0, 2, 3, 1).contiguous(), torch.zeros(n, h, w, c, dtype=torch.int8, device="cuda")
+    wk, bias_k = wt.permute(0, 2, 3, 1).contiguous().repeat(fold, 1, 1, 1), bias.repeat(fold)   # (once per sub-pixel)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    d.x, d.w, d.y, d.y_dtype, d.status = xin.data_ptr(), wk.data_ptr(), y.data_ptr(), I8, status.data_ptr()
+    shift_clip(d, shift, bias_k.data_ptr())
+    raw = ct.create_string_buffer(4096)
+    plan = ConvPlan.from_buffer(raw, (-ct.addressof(raw)) % 64)
+    assert lib.cvmk_conv2d_tc_supported(ct.byref(d)) == 1
+    assert lib.cvmk_conv2d_tc_prepare(ct.byref(d), ct.byref(plan)) == 0 and plan.a_im2col == 4
+    torch.cuda.synchronize()
+    assert lib.cvmk_conv2d_tc_launch(ct.byref(plan), ct.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    want = conv_sums(torch, x, wt, 1, 1, c // 32) + bias.long()
+    assert int(status) == 0
+    assert torch.equal(y, right_shift(want, shift).to(torch.int8))

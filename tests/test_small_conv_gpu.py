@@ -4,13 +4,14 @@ import numpy as np
 import pytest
 
 import cases
+import kernel_desc
 
 pytestmark = pytest.mark.gpu
 
 
 # (n, c, h, w, oc, k, stride): one unit of 32 channels (a ring smaller than the tile it stages on the way
 # out), 64- and 32-column tiles, channels that end inside a tile, ragged last tiles, two to four units behind one
-# barrier, rings that turn, reductions cut over two to eight CTAs with rows the cut does not divide,
+# barrier, rings that turn, reductions whole and cut over four CTAs with rows the cut does not divide,
 # strided filters (im2col loads), patches of several images; two and three CTAs an SM whose rings turn, one unit
 # behind each of eight barriers
 @pytest.mark.parametrize("n,c,h,w,oc,k,stride", [
@@ -33,3 +34,18 @@ def test_dense(rows, k, units, gpu_run, oracle, wl):
     js, pb = g.finish(y)
     x = np.random.RandomState(rows).randint(-127, 128, size=(rows, k)).astype(np.int8)
     assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
+
+
+# The cut that the rule gives for 148 SMs, straight through the kernel interface: reductions over one, two, four and eight CTAs, of
+# tiles of 9, 25, 35, 49, 105 (361 in three tiles) and 128 rows, channels that end inside a tile, im2col loads and patches
+@pytest.mark.parametrize("n,c,h,w,oc,k,stride,split,block_n", [
+    (1, 256, 19, 19, 512, 3, 1, 2, 32), (1, 256, 19, 19, 520, 3, 1, 2, 32), (1, 2048, 19, 19, 512, 1, 1, 2, 32), (2, 256, 19, 19, 264, 3, 1, 2, 32),
+    (1, 512, 7, 7, 512, 3, 1, 4, 32), (1, 512, 13, 13, 512, 3, 2, 4, 32), (3, 256, 7, 7, 128, 3, 1, 4, 32), (1, 2048, 7, 7, 512, 1, 1, 4, 32),
+    (1, 512, 3, 3, 64, 3, 1, 8, 32), (1, 512, 5, 5, 72, 3, 1, 8, 32), (1, 512, 7, 7, 40, 3, 1, 8, 32), (1, 1024, 5, 7, 72, 3, 1, 8, 32),
+    (3, 256, 27, 27, 264, 3, 1, 1, 64), (10, 1024, 14, 14, 520, 1, 1, 1, 64)])
+@pytest.mark.parametrize("packed,join", [(True, False), (False, False), (True, True)])
+def test_cut(n, c, h, w, oc, k, stride, split, block_n, packed, join, rt):
+    import torch
+    plan = kernel_desc.run_conv(rt, n, c, h, w, oc, k, stride, packed, join, seed=n + oc)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (plan.small_split, plan.block_n) == (split, block_n)
