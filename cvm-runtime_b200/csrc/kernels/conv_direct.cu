@@ -644,6 +644,10 @@ extern "C" int cvmk_conv2d_direct(const cvmk_conv_direct_desc* d, cvmk_stream_t 
   return check_cuda(cudaGetLastError(), "conv_direct_kernel launch");
 }
 
+extern "C" int cvmk_conv2d_direct_tensor_cores(const cvmk_conv_direct_desc* d) {
+  return d && d->depthwise && d->groups == d->C && d->OC == d->C && conv_dw_takes(*d);
+}
+
 extern "C" int cvmk_im2col_pack(const cvmk_im2col_desc* d, cvmk_stream_t stream) {
   if (!d || !d->x || !d->a || d->Kp % 16 || d->C > 255 || (d->KW - 1) * d->dil_w > 4095 ||
       (d->KH - 1) * d->dil_h > 2047 || d->KH * d->KW * d->C > d->Kp || d->KH * d->KW * d->C > 8192 ||

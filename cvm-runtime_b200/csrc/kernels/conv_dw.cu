@@ -66,7 +66,7 @@ struct DwParams {
   int tiles_x, tiles_y, c_tiles, num_tiles;
   FastDiv fd_c, fd_x, fd_y, fd_pitch;
   int units, box_bytes;    // of the ring; bytes of a box
-  int out_pairs;           // the output is stored as pairs of pixels
+  int pairs, out_pairs;    // the input is staged, the output stored as pairs of pixels
   uint32_t out_mask;       // the output tile's swizzle: address bits 4.. ^= bits 7.. & out_mask
   int mul, add;
   uint32_t lo, hi;
@@ -476,26 +476,24 @@ LaunchFn of_shape(int groups, bool pairs, int form) {
   return pairs ? of_form<S, 2, 1>(form) : of_form<S, 2, 0>(form);
 }
 
-}  // namespace
-
-int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaStream_t stream) {
+// The shape and the tiles of a layer, or false when it is not one for this kernel.
+bool plan_tiles(const cvmk_conv_direct_desc& d, DwParams* params, int* sm_count) {
   const int S = d.stride_h;
   if (d.C % 32 != 0 || d.x_dtype != CVMK_I8 || d.y_dtype != CVMK_I8 || d.KH != 3 || d.KW != 3 || d.dil_h != 1 || d.dil_w != 1 ||
       (S != 1 && S != 2) || d.stride_w != S || d.pad_h > 1 || d.pad_w > 1 || d.N < 1 || d.OH < 1 || d.OW < 1)
-    return -1;
-  const int G = d.C % 64 == 0 ? 2 : 1, P = 32 * G, out = S == 1 ? 2 : 1;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  DwParams p;
+    return false;
+  const int P = d.C % 64 == 0 ? 64 : 32, out = S == 1 ? 2 : 1;
+  int dev = 0, sms = 148;   // (without a device, of the part this library is built for)
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  else cudaGetLastError();
+  DwParams& p = *params;
   memset(&p, 0, sizeof(p));
-  p.w = d.w; p.status = d.status;
   p.C = d.C; p.images = d.N;
   p.pad_h = d.pad_h; p.pad_w = d.pad_w;
   p.rows_x = (d.OW + out - 1) / out;
   p.rows_y = (d.OH + out - 1) / out;
   p.c_tiles = d.C / P;
-  if (p.c_tiles > sms) return -1;
+  if (p.c_tiles > sms) return false;
   // A tile holds TILE_Y operand lines of one image, or as many of several as are stacked in it, each with one line more
   // (what its last taps read), rounded up so that its part of the output tile starts on a multiple of 1024 bytes.  Images
   // of at most seven lines are stacked whole; higher ones in bands of fewer lines where that takes fewer rounds of
@@ -505,22 +503,24 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   const int whole = std::max(1, 1024 / (8 * out * out * P));
   p.tiles_x = (p.rows_x + TILE_X - 1) / TILE_X;
   const int64_t grid_max = sms / p.c_tiles * p.c_tiles;
-  int64_t tiles = 0, rounds = 0;
+  int64_t tiles = 0, rounds = 0, of_images = 0;
   for (int band = std::min(p.rows_y, TILE_Y); band >= 1; --band) {
     int pitch = (band + 1 + whole - 1) / whole * whole, images = TILE_Y / pitch;
     if (images < 2) { pitch = TILE_Y; images = 1; }
     if (images == 1 && band < std::min(p.rows_y, TILE_Y)) continue;
     const int bands = (p.rows_y + band - 1) / band;
     const int64_t t = (int64_t)p.tiles_x * bands * ((d.N + images - 1) / images) * p.c_tiles, r = (t + grid_max - 1) / grid_max;
-    if (tiles && r >= rounds) continue;
+    if (!tiles) of_images = t;
+    else if (r >= rounds) continue;
     tiles = t; rounds = r;
     p.band = band; p.pitch_y = pitch; p.per_tile = images; p.tiles_y = bands;
   }
-  if (tiles > INT32_MAX / 2) return -1;
+  if (tiles > INT32_MAX / 2) return false;
   // One box of pixel pairs has half the rows of twice the bytes, and a store of pairs too, where the two pixels lie
   // side by side (C channels a tile).
-  const bool pairs = d.C == P && d.W % 2 == 0 && d.pad_w == 1, out_pairs = d.C == P && d.OW % 2 == 0;
-  // The CUDA-core kernel stays the better one where the tiles do not give every SM one, and where five eighths of their
+  p.pairs = d.C == P && d.W % 2 == 0 && d.pad_w == 1;
+  p.out_pairs = d.C == P && d.OW % 2 == 0;
+  // The CUDA-core kernel stays the better one where whole images do not give every SM a tile, and where five eighths of their
   // rows lie outside the images.  Device time with the line at 0, 96, 150, 296 and 592 tiles: MobileNet, one image 123, 99,
   // 99, 99, 99 us; 20 images 182, 172, 170, 170, 176; 256 images 692 each (of 828 with none); SSD-512 on 3 images 328, 328,
   // 329, 339, 350; on 8 images 450, 449, 440, 444, 455.  Pairs of pixels are worth it from half as many tiles on (SSD-512, one
@@ -528,9 +528,22 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   // 20, 256 images 23.8 -> 14.9 us; 0.42, 256 at 18 x 18, 128 images 14.0 -> 10.3; 0.39, 128 at 19 x 19, 128 images 10.0 -> 8.5,
   // but 40 images of 20 x 20 5.4 -> 5.9, so the rows inside have to fill tiles for half of the SMs; 0.375, 512 at 8 x 8, 256
   // images 9.6 -> 10.0, 1024 at 7 x 7 16.6 -> 15.1.
-  const int64_t least = pairs ? sms / 2 : sms, used = (int64_t)p.rows_x * p.rows_y * d.N * p.c_tiles;
-  if (tiles < least || 2 * used < least * TILE_X * TILE_Y || 8 * used <= 3 * tiles * TILE_X * TILE_Y) return -1;
+  const int64_t least = p.pairs ? sms / 2 : sms, used = (int64_t)p.rows_x * p.rows_y * d.N * p.c_tiles;
+  if (of_images < least || 2 * used < least * TILE_X * TILE_Y || 8 * used <= 3 * tiles * TILE_X * TILE_Y) return false;
   p.num_tiles = (int)tiles;
+  *sm_count = sms;
+  return true;
+}
+
+}  // namespace
+
+int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaStream_t stream) {
+  DwParams p;
+  int sms = 0;
+  if (!plan_tiles(d, &p, &sms)) return -1;
+  const int S = d.stride_h, G = d.C % 64 == 0 ? 2 : 1, P = 32 * G, out = S == 1 ? 2 : 1;
+  const bool pairs = p.pairs, out_pairs = p.out_pairs;
+  p.w = d.w; p.status = d.status;
   p.fd_c = make_fastdiv(p.c_tiles); p.fd_x = make_fastdiv(p.tiles_x); p.fd_y = make_fastdiv(p.tiles_y); p.fd_pitch = make_fastdiv(p.pitch_y);
   const int box_h = p.per_tile > 1 ? 2 * p.pitch_y : std::min(BOX_H, 2 * (p.band + 1));
   const int row = pairs ? 2 * P : P, box_w = pairs ? TILE_X + 2 : TILE_X + 1;
@@ -539,7 +552,6 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
   const int w_bytes = G * (S == 1 ? NUM_BLOCKS1 : NUM_BLOCKS2) * 1024;
   const int out_bytes = TILE_X * TILE_Y * out * out * P;
   p.units = std::min(MAX_UNITS, (SMEM_MAX - 1024 - w_bytes - 2 * out_bytes) / unit_bytes);
-  p.out_pairs = out_pairs;
   p.out_mask = (uint32_t)((out_pairs ? 2 * P : P) / 16 - 1);
   const int first = chain.n > 0 && chain.s[0].op == K_ADD_C;
   PackedChain pc;
@@ -582,10 +594,18 @@ int launch_conv_dw(const cvmk_conv_direct_desc& d, const DevChain& chain, cudaSt
     set_error("conv_dw: tensor map rejected");
     return CVMK_ERR_CUDA;
   }
-  const int grid = (int)(std::min<int64_t>(tiles, sms) / p.c_tiles * p.c_tiles);
+  const int grid = std::min(p.num_tiles, sms) / p.c_tiles * p.c_tiles;
   const int form = p.kind != 0 || p.wide ? OTHER : (pc.lo == 0 ? PACKED_RELU : PACKED);
+  int dev = 0;
+  cudaGetDevice(&dev);
   const LaunchFn launch_form = S == 1 ? of_shape<1>(G, pairs, form) : of_shape<2>(G, pairs, form);
   return launch_form(tx, ty, tr, p, grid, smem, dev, stream);
+}
+
+bool conv_dw_takes(const cvmk_conv_direct_desc& d) {
+  DwParams p;
+  int sms = 0;
+  return plan_tiles(d, &p, &sms);
 }
 
 }  // namespace cvmk

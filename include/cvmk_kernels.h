@@ -279,7 +279,9 @@ typedef struct {
   int32_t* status;   /* nullptr, or the word that a kernel whose bounded wait ran out marks, as in cvmk_conv_desc */
 } cvmk_conv_direct_desc;
 CVMK_API int cvmk_conv2d_direct(const cvmk_conv_direct_desc* d, cvmk_stream_t stream);
-
+/* 1 if cvmk_conv2d_direct() runs the layer on the tensor cores of the current device (without one, of
+ * the part this library is built for); looks at sizes and types only. */
+CVMK_API int cvmk_conv2d_direct_tensor_cores(const cvmk_conv_direct_desc* d);
 
 /* ------------------------------------------------------------------------------------------------
  * Patch gather for convolutions whose channel count is not a multiple of 32 (image stems):

@@ -1,11 +1,12 @@
 /* Host-side functions of the kernel C-ABI that need no device: the shapes the tensor-core
- * convolution takes and the scratch they want (none), and the operand order the stem convolution
+ * convolutions take and the scratch they want (none), and the operand order the stem convolution
  * packs its filter into.  Compiled as plain C against include/cvmk_kernels.h (which is therefore
  * checked to be a C header) and linked with the runtime library; the test reads the lines printed
  * here and the packed bytes written to the file named on the command line.
  *
  *   host_fns workspace N H W C OC KH KW        -> "@supported=.. @workspace=.."
  *   host_fns grouped N H W C groups K stride   -> "@supported=.." (OC = C, padding K / 2)
+ *   host_fns depthwise N H W C stride pad      -> "@tensor_cores=.."   (3 x 3, int8 to int8)
  *   host_fns stem N H W C OC KH KW stride pad out.bin
  *                                              -> "@supported=.. @weight_bytes=.. @pack=.."
  * The stem filter is w[oc][c][ky][kx] = ((oc * 131 + c * 31 + ky * 7 + kx) mod 255) - 127.
@@ -43,6 +44,20 @@ int main(int argc, char** argv) {
     d.OH = (d.H + 2 * d.pad_h - d.KH) / d.stride_h + 1;
     d.OW = (d.W + 2 * d.pad_w - d.KW) / d.stride_w + 1;
     printf("@supported=%d\n", cvmk_conv2d_tc_supported(&d));
+    return 0;
+  }
+  if (argc >= 8 && strcmp(argv[1], "depthwise") == 0) {
+    cvmk_conv_direct_desc d;
+    memset(&d, 0, sizeof(d));
+    d.x_dtype = d.y_dtype = CVMK_I8;
+    d.depthwise = 1;
+    d.N = arg(argv, 2); d.H = arg(argv, 3); d.W = arg(argv, 4); d.C = d.OC = d.groups = arg(argv, 5);
+    d.KH = d.KW = 3;
+    d.stride_h = d.stride_w = arg(argv, 6); d.dil_h = d.dil_w = 1;
+    d.pad_h = d.pad_w = arg(argv, 7);
+    d.OH = (d.H + 2 * d.pad_h - 3) / d.stride_h + 1;
+    d.OW = (d.W + 2 * d.pad_w - 3) / d.stride_w + 1;
+    printf("@tensor_cores=%d\n", cvmk_conv2d_direct_tensor_cores(&d));
     return 0;
   }
   if (argc >= 12 && strcmp(argv[1], "stem") == 0) {

@@ -1,9 +1,12 @@
 """The tensor-core kernel for depthwise 3 x 3 layers (csrc/kernels/conv_dw.cu): edges of its tiles of 16 x 32 output pixels
 (8 x 16 with stride 2), images stacked in one tile, 32 and 64 channels a tile, more tiles than CTAs."""
+import ctypes as ct
+
 import numpy as np
 import pytest
 
 import cases
+from kernel_desc import I8, Direct, shape
 
 pytestmark = pytest.mark.gpu
 
@@ -27,6 +30,21 @@ SHAPES = [(80, 64, 32, 16, 1, 1), (75, 64, 33, 17, 1, 1), (40, 64, 33, 18, 1, 1)
 @pytest.mark.parametrize("relu,bias", [(True, True), (False, False)])
 def test_depthwise(n, c, h, w, stride, pad, relu, bias, gpu_run, oracle, wl):
     js, pb, x = cases.conv_case(c + h + n, n, c, h, w, c, 3, stride, pad, groups=c, bias=bias, relu=relu, shift=wl.GraphBuilder.default_shift(9))
+    assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
+
+
+# one output pixel, one operand line and one operand row more than whole tiles (33 x 25 rows of 16 x 8 a tile), in planes and in
+# pairs of pixels, of 32 and 64 channels; every layer runs on the tensor cores
+@pytest.mark.parametrize("n,c,h,w,stride", [(10, 64, 66, 50, 1), (10, 64, 65, 50, 1), (14, 64, 65, 49, 1), (7, 128, 66, 50, 1), (7, 128, 65, 49, 1), (10, 32, 66, 50, 1),
+                                            (5, 96, 66, 49, 1), (10, 64, 65, 50, 2), (10, 64, 66, 50, 2), (14, 64, 65, 49, 2), (7, 128, 66, 50, 2), (7, 128, 65, 49, 2),
+                                            (10, 32, 65, 50, 2), (5, 96, 66, 49, 2), (50, 64, 33, 32, 1), (37, 128, 33, 31, 1)])
+def test_depthwise_edges(n, c, h, w, stride, gpu_run, oracle, wl, rt):
+    d = Direct()
+    shape(d, n, c, h, w, c, 3, stride, 1)
+    d.x_dtype = d.y_dtype = I8
+    d.groups, d.depthwise, d.dil_h, d.dil_w = c, 1, 1, 1
+    assert rt.lib().cvmk_conv2d_direct_tensor_cores(ct.byref(d)) == 1
+    js, pb, x = cases.conv_case(c + h + n, n, c, h, w, c, 3, stride, 1, groups=c, relu=bool(n % 2), shift=wl.GraphBuilder.default_shift(9))
     assert np.array_equal(gpu_run(js, pb, x), oracle.run_model(js, pb, x))
 
 

@@ -109,3 +109,13 @@ def test_stem_refuses_what_it_cannot_run(host_fns, tmp_path, shape):
                                       ((256, 7, 7, 1024, 32, 3, 1), "0")])   # a 7 x 7 image wastes most of an 8 x 16 tile
 def test_grouped_convolutions_the_tensor_core_kernel_takes(host_fns, shape, ok):
     assert host_fns("grouped", *shape)["supported"] == ok
+
+
+@pytest.mark.parametrize("shape,ok", [((256, 56, 56, 128, 1, 1), "1"), ((256, 112, 112, 64, 2, 1), "1"), ((41, 56, 56, 32, 1, 1), "1"),
+                                      ((151, 16, 24, 256, 1, 1), "1"),       # images in bands, several in a tile
+                                      ((1, 56, 56, 128, 1, 1), "0"),         # too few tiles
+                                      ((14, 65, 49, 64, 1, 1), "1"),         # a tile for every SM as images, in bands fewer
+                                      ((256, 8, 8, 512, 1, 1), "0"),         # three eighths of the rows inside images
+                                      ((256, 56, 56, 48, 1, 1), "0"), ((256, 56, 56, 64, 3, 1), "0"), ((256, 56, 56, 64, 1, 2), "0")])
+def test_depthwise_layers_on_the_tensor_cores(host_fns, shape, ok):
+    assert host_fns("depthwise", *shape)["tensor_cores"] == ok
