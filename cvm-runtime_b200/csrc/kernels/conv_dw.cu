@@ -251,6 +251,11 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         if (++unit == p.units) { unit = 0; phase ^= 1; }
       }
     }
+    // nothing else waits for the last commits of the units, which must not come when the CTA has gone
+    for (int u = 0; live && u < p.units; ++u) {
+      live = mbar_wait(&bar_empty[unit], phase ^ 1, &abort_flag, 1);
+      if (++unit == p.units) { unit = 0; phase ^= 1; }
+    }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- products
     const bool leader = elect_one();

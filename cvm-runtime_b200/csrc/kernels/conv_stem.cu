@@ -435,7 +435,9 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             STADD(5, tw);
           }
         }
-        if (leader) mma_commit(&staged_empty[sbuf]);   // all MMAs that read this block's rows have finished
+        // all MMAs that read this block's rows have finished (nobody waits for the last two blocks' commits, which could come
+        // when the CTA has gone)
+        if (leader && blk + 2 * (int)gridDim.x < p.num_blocks) mma_commit(&staged_empty[sbuf]);
       }
 #ifdef CVMK_STEM_TIMING
       if (leader) { stacc[11] = tile; STFLUSH(3); STFLUSH(4); STFLUSH(5); STFLUSH(11); }

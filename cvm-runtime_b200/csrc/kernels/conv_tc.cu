@@ -108,6 +108,7 @@ struct ConvParams {
   int bias_static;      // the bias vector is a parameter: it may be read before the previous kernel has finished
   const int8_t* w;      // the weight matrix [oc, kh * kw * c] and its size, for the L2 warm-up
   unsigned w_bytes;
+  int tiles_each, tiles_left;   // tiles of every pair, and how many pairs have one more
   DevChain chain;
 };
 
@@ -254,27 +255,6 @@ __device__ long long g_conv_trace[17 * 512];
 #define TDECL do {} while (0)
 #define TFLUSH(slot) do {} while (0)
 #endif
-
-// The commits that free the last lap of the ring arrive in both CTAs of the pair, and nothing else waits for them in the
-// second: before a CTA may leave, its producers wait for every one.  A producer whose next stage is `turn` stages away
-// (0 or 1, with one producer 0) has so many waits left, `producers` stages apart.
-constexpr __host__ __device__ int drain_waits(int stages, int turn, int producers) { return (stages - turn + producers - 1) / producers; }
-constexpr bool drain_complete() {   // after any number of stages filled, the waits are for the stages of the last lap, each once
-  for (int producers = 1; producers <= 2; ++producers)
-    for (int stages = 2; stages <= MAX_STAGES; ++stages)
-      for (int filled = 0; filled < 3 * MAX_STAGES; ++filled) {
-        int waits[MAX_STAGES] = {};
-        for (int which = 0; which < producers; ++which) {
-          const int turn = producers == 2 ? (filled ^ which) & 1 : 0;
-          int next = filled + turn;
-          for (int k = drain_waits(stages, turn, producers); k > 0; --k, next += producers) ++waits[next % stages];
-        }
-        for (int s = 0; s < stages; ++s)
-          if (waits[s] != 1) return false;
-      }
-  return true;
-}
-static_assert(drain_complete(), "waits before a pair leaves");
 
 // TMA loads into this CTA's shared memory that report to `bar`, a barrier of the pair's first CTA.
 __device__ __forceinline__ void load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
@@ -625,11 +605,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           }
         }
       }
-      for (int k = live ? drain_waits(p.stages, two_issuers ? 0 : turn, two_issuers ? 1 : 2) : 0; k > 0; --k) {
-        if (!mbar_wait(&bar_empty[stage], phase ^ 1, &abort_flag, 1)) break;
-        stage += two_issuers ? 1 : 2;
-        if (stage >= p.stages) { stage -= p.stages; phase ^= 1; }
-      }
       TADD(12, tk);
 #ifdef CVMK_CONV_TIMING
       if (which == 0 && leader) { TFLUSH(0); TFLUSH(12); }
@@ -676,6 +651,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // have to block on a barrier it pays its debts first (flush), so that an epilogue group or a
       // producer never waits for a commit that waits for them.
       int owed_stage = -1, owed_acc = -1;
+      // A stage's commit arrives in both CTAs, and there only a producer that fills the stage again waits for it.  So it is
+      // left out where none will: an arrival that nobody waits for could reach a CTA that has gone.  `refills`: how many
+      // stages, this one included, are filled again.  (The host divides: it takes 0.2 us here, in front of the first product.)
+      int refills = (p.tiles_each + (first_own < p.tiles_left ? 1 : 0) - me) * num_kb - p.stages;
       auto flush = [&]() {
         if (leader) {
           if (owed_acc >= 0) mma_commit<CG>(&bar_acc_full[owed_acc]);
@@ -721,9 +700,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               } else {
                 for (int u = 0; u < in_stage; ++u, al += unit_q, bl += b_step) mma_i8_k<1, CG>(d_tmem, al, a_hi, bl, a_hi, idesc, (uint32_t)(unit + u));
               }
-              mma_commit<CG>(&bar_empty[stage]);
+              mma_commit_pair_if(refills > 0, &bar_empty[stage]);
               TRACE(5, mseq);
             }
+            --refills;
             unit += in_stage;
             ++mseq;
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -803,7 +783,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 if (fy == 0) flush();
               }
             }
-            owed_stage = stage;
+            owed_stage = refills > 0 ? stage : -1;
+            --refills;
             if (leader) TRACE(5, mseq);
             ++mseq;
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -815,6 +796,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (++acc == p.acc_bufs) { acc = 0; acc_phase ^= 1; }
           for (int k = 0; k < (issuers - 1) * num_kb; ++k)
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          refills -= (issuers - 1) * num_kb;
         }
       }
       if (live) flush();
@@ -1047,7 +1029,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   // ------------------------------------------------------------------ teardown
   // Every warp leaves on its own.  The TMEM columns of both CTAs go back, and the CTAs with them, once every warp that
   // reads them, reads the other's operands, reports to its barriers or waits for its commits has arrived here: the
-  // epilogue has waited for every accumulator, the producers for the last lap of the ring.
+  // epilogue waits for every accumulator, the producers for every stage that is committed.
   __syncwarp();
   if (threadIdx.x == 0) TRACE(16, 3);
   if (abort_flag) {
@@ -1588,6 +1570,9 @@ extern "C" int cvmk_conv2d_tc_launch(const cvmk_conv_plan* plan, cvmk_stream_t s
   if (d.groups > 1) { p.grouped = 1; p.c = d.C / d.groups; p.group_fold = d.group_fold > 1 ? d.group_fold : 1; }
   p.num_units = p.grouped ? d.KH * d.KW : d.KH * d.KW * (p.c / plan->block_k);
   p.num_kb = p.a_mode >= 3 ? (p.grouped ? 1 : p.c / plan->block_k) : (p.num_units + p.units - 1) / p.units;
+  const int pair_tiles = (p.num_m_tiles + 1) / 2 * p.num_n_tiles, walkers = std::max(1, plan->grid / 2);
+  p.tiles_each = pair_tiles / walkers;
+  p.tiles_left = pair_tiles % walkers;
   p.fd_n_tiles = make_fastdiv(p.num_n_tiles);
   p.fd_tiles_w = make_fastdiv(p.tiles_w);
   p.fd_tiles_h = make_fastdiv(p.tiles_h);

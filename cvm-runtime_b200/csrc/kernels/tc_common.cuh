@@ -245,6 +245,17 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   else
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The same for CG = 2 where `go` holds, without a branch.
+__device__ __forceinline__ void mma_commit_pair_if(bool go, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %2, 0;\n"
+      "@p tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+      "}\n" ::"r"(smem_u32(bar)),
+      "h"((uint16_t)3), "r"((uint32_t)go)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
