@@ -19,17 +19,17 @@
 // descriptors that overlap stand in for the patch matrix.
 //
 // One CTA works on blocks of consecutive output rows of one image:
-//   warps 0-3  one of their threads has TMA bring the planar input rows of a block (all channels),
-//              zero-filled above and below the image, two blocks ahead; all of them fold the rows
-//              that have landed: clamp, interleave channels and the S x S neighbours, zero left /
-//              right of the image -> staged rows, 16 bytes per staged pixel;
-//   warp 4     issues KH' * ceil(KW' / 2) tcgen05.mma (M = 128 pixels, N = OC, K = 32) per output row
-//              segment into one of two TMEM accumulators;
-//   warps 5-8  drain the accumulator, apply the fused chain (or the packed requantisation), write
-//              int8 into a swizzled staging panel;
-//   warp 9     stores the panels with TMA.
-// Planar rows, staged rows, accumulators and panels are all double buffered; every mbarrier wait
-// is bounded.
+//   warps 0-3   one of their threads has TMA bring the planar input rows of a block (all channels),
+//               zero-filled above and below the image, one or two blocks ahead; all of them fold the
+//               rows that have landed: clamp, interleave channels and the S x S neighbours, zero left /
+//               right of the image -> staged rows, 16 bytes per staged pixel;
+//   warp 4      issues KH' * ceil(KW' / 2) tcgen05.mma (M = 128 pixels, N = OC, K = 32) per output row
+//               segment into the next of 256 / OC TMEM accumulators (half of the SM's columns);
+//   warps 5-12  in two groups of four that take the tiles in turn: drain an accumulator, apply the fused
+//               chain (or the packed requantisation), write int8 into a swizzled staging panel;
+//   warp 13     stores the panels with TMA.
+// Staged rows are double buffered, planar rows single or double, panels two or four; every mbarrier
+// wait is bounded.
 #include <stdlib.h>
 #include <string.h>
 #include <algorithm>
@@ -149,8 +149,8 @@ __device__ __forceinline__ uint4 fold_pixel(const StemConvParams& p, const uint8
 // The same on words, four staged pixels (X0 .. X0 + 3, X0 a multiple of 4) per call, for a single
 // box that carries zero columns left and right of the image (so that no column needs a test) and a
 // clamp to +-127 (only -128 moves).  Per sub-row and channel the 4 * S input bytes the pixels
-// take come out of two or three aligned words and a funnel shift.  The integer pipe is what the CTAs of an SM
-// run out of, so the bytes move two (stride 2) or, as a 4 x 4 transpose, four at a time: 12 or 8 permutes for four
+// take come out of two or three aligned words and a funnel shift.  The folding warps share their issue slots with
+// the epilogue's, so the bytes move two (stride 2) or, as a 4 x 4 transpose, four at a time: 12 or 8 permutes for four
 // pixels of 12 or 3 bytes, where one for each byte took 48 or 12.
 __device__ __forceinline__ uint32_t clamp127(uint32_t x) {
   const uint32_t t = (x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu;    // top bits: the lower seven are not all zero
@@ -281,6 +281,7 @@ __device__ __forceinline__ void stem_products(bool leader, uint32_t d_tmem, uint
       mma_i8_if(leader, d_tmem, al + 2u * (uint32_t)j, a_hi, bl, b_hi, idesc, (uint32_t)(ky | j));
 }
 
+// (72 registers for two CTAs an SM: the step-by-step chain spills some 250 bytes, everything else fits)
 __global__ void __launch_bounds__(STEM_THREADS, 2)
 conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
                  const __grid_constant__ StemConvParams p) {
@@ -292,9 +293,9 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* wq = smem;                        // [KH' * nj][2][OC][16]: two taps per MMA, no swizzle
-  uint8_t* planar = smem + p.off_planar;     // [2][nwb][C][in_rows][wbox]
+  uint8_t* planar = smem + p.off_planar;     // [planar_bufs][nwb][C][in_rows][wbox]
   uint8_t* staged = smem + p.off_staged;     // [2][srows][pitch]
-  uint8_t* out_panels = smem + p.off_out;    // [2][128][OC], swizzle of width OC
+  uint8_t* out_panels = smem + p.off_out;    // [panels][128][OC], swizzle of width OC
   int32_t* bias_s = reinterpret_cast<int32_t*>(smem + p.off_bias);
   // warp index through a shuffle: provably uniform, so that the loops of the single-issuer roles
   // (loads, MMA, output stores) run on the uniform datapath with one elected lane issuing

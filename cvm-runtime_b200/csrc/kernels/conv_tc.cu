@@ -1,5 +1,5 @@
 // conv2d (groups = 1) and dense as an implicit GEMM on the sm_100a tensor cores; grouped 3 x 3
-// convolutions with 32 channels per group as well (how depthwise layers are given to it).
+// convolutions with 32 channels per group as well.
 //
 //   D[pixel, oc] = sum_{kh,kw,c} X[n, oh*s-p+kh*d, ow*s-p+kw*d, c] * Wt[oc, kh, kw, c]
 //

@@ -89,8 +89,8 @@ typedef struct {
 
 /* ------------------------------------------------------------------------------------------------
  * conv2d, groups = 1, and dense, on the tcgen05 int8 tensor cores; grouped 3 x 3 convolutions with
- * 32 channels per group as well (`groups` below; depthwise layers, i.e. the groups > 1 branch
- * cpu/ops/ops.cc:417-425 with depthwise_conv2d :248-277, are given to it with block-diagonal weights).
+ * 32 channels per group as well (`groups` below), which the runtime does not launch: depthwise
+ * layers go to cvmk_conv2d_direct().
  * Reproduces cvm.runtime.cpu.conv2d (src/runtime/cpu/ops/ops.cc:368-456: im2col_cpu :204-246 +
  * matrix_mul :148-200) and cvm.runtime.cpu.dense (:34-75) followed by the fused chain.
  *
@@ -124,18 +124,15 @@ typedef struct {
   int32_t bias_static;
   /* 0 or 1: an ordinary convolution.  > 1: a grouped convolution whose groups are C / groups = OC /
    * groups = 32 channels wide, 3 x 3, stride 1, no dilation, int8 output; w is then
-   * [OC, KH, KW, 32].  A depthwise layer runs this way with block-diagonal weights (channel c of a
-   * group multiplies only row c of that group): an N tile is up to four groups side by side, one
-   * input halo serves all of them and each group is nine M128 N32 K32 instructions into its own
-   * accumulator columns.  Only the diagonal of every 32 x 32 block is used, and it is still faster
-   * than the CUDA-core form for 128 channels and more, which is bound by instruction issue.
-   * cvmk_conv2d_tc_supported() says whether the 8 x 16 pixel tiles fit the image. */
+   * [OC, KH, KW, 32]: an N tile is up to four groups side by side, one input halo serves all of
+   * them and each group is nine M256 N32 K32 instructions of the pair into its own accumulator
+   * columns.  cvmk_conv2d_tc_supported() says whether the 8 x 16 pixel tiles fit the image. */
   int32_t groups;
   /* Grouped mode only, 0 or 1 = off.  F = 2 or 4: x and y are views of tensors F times as wide with
    * C / F channels: a pixel here is F neighbouring pixels ("sub-pixels") of the real image side by
    * side, and the 3 x 3 filter of an output channel moves in sub-pixel steps (C = OC = 128,
-   * pad_w = 1 real pixel; W and OW count folded pixels).  That is how a depthwise layer over 32 or
-   * 64 channels fills 128-column tiles: the group of sub-pixel a reads the 32-channel groups of
+   * pad_w = 1 real pixel; W and OW count folded pixels).  That is how groups over 32 or 64 channels
+   * in all fill 128-column tiles: the group of sub-pixel a reads the 32-channel groups of
    * sub-pixels a - 1, a, a + 1, the outer ones from the neighbouring folded pixel at the edges. */
   int32_t group_fold;
   int32_t reserved1;
@@ -253,8 +250,10 @@ typedef struct {
 CVMK_API int cvmk_max_pool2d(const cvmk_pool_desc* d, cvmk_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------
- * conv2d on CUDA cores for the shapes the tensor-core path does not take: groups > 1
- * (groupwise_conv2d, cpu/ops/ops.cc:333-366), depthwise, and small or odd channel counts.
+ * conv2d for the shapes cvmk_conv2d_tc_* does not take: groups > 1 (groupwise_conv2d,
+ * cpu/ops/ops.cc:333-366), depthwise, and small or odd channel counts.  Depthwise 3 x 3 layers of
+ * stride 1 and 2 whose tiles fill the GPU run on the tensor cores (conv_dw.cu), with any chain; all
+ * others on the CUDA cores.
  *   x : NHWC [N,H,W,C], int8 or int32 (x_dtype)
  *   w : int8 [OC, KH, KW, C/groups]   (depthwise = 1: int8 [KH, KW, C])
  *   y : NHWC [N,OH,OW,OC] int8 or int32, chain applied (ADD_C carries the bias)
