@@ -29,9 +29,10 @@
 //
 // Any chain behind the products: [bias] shift clamp has forms of its own; a wide sum, and the sum with another tensor (whose
 // tile TMA brings into the output buffer before the result), run packed too, everything else step by step.  128 channels at
-// 28 x 28, 150 images, in a chain of such layers: 9.4 us with shift and clamp, 15.4 with a wide sum or a clip alone, 15.9 with a
+// 28 x 28, 150 images, in a chain of such layers: 9.7 us with shift and clamp, 14.5 with a wide sum or a clip alone, 15.4 with a
 // tensor (depthwise3x3_kernel 39.0, 34.8, 57.2; the clip step by step 18.9; the tensor loaded by the threads that need it 18.4:
-// a row's 32 bytes lie in a cache line of their own).
+// a row's 32 bytes lie in a cache line of their own).  The wide sum's clamp is three more integer instructions an element, the
+// tensor waits in one of the two output buffers, which it takes from the tile two before.
 //
 // Reproduces groupwise_conv2d with groups = C (src/runtime/cpu/ops/ops.cc:333-366) and the chain behind it.
 // Every wait is bounded, as in conv_tc.cu.
@@ -363,13 +364,23 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
               }
             } else {
               const int4* bp = reinterpret_cast<const int4*>(bias_s + g * 32);
-              const int am = p.add * mul;
+              if (p.wide) {   // (two loops: a choice an element costs both)
+                const int am = p.add * mul;
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const int4 b4 = bp[j];
-                const int32_t bj[4] = {b4.x, b4.y, b4.z, b4.w};
+                for (int j = 0; j < 8; ++j) {
+                  const int4 b4 = bp[j];
+                  const int32_t bj[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[4 * j + i] = p.wide ? min(max(v[4 * j + i] + bj[i], p.pre_lo), p.pre_hi) * mul + am : v[4 * j + i] * mul + bj[i];
+                  for (int i = 0; i < 4; ++i) v[4 * j + i] = min(max(v[4 * j + i] + bj[i], p.pre_lo), p.pre_hi) * mul + am;
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const int4 b4 = bp[j];
+                  const int32_t bj[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) v[4 * j + i] = v[4 * j + i] * mul + bj[i];
+                }
               }
               uint4 r0 = none, r1 = none;
               if (has_operand) {
