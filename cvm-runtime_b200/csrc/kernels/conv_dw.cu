@@ -193,25 +193,32 @@ conv_dw_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     asm volatile("bar.arrive 1, %0;" ::"n"(Sh::THREADS) : "memory");
   } else {
     if (warp >= 2 && warp < Sh::IO_WARP) {
+      // all of a thread's weights and its bias set out before anything is stored, behind which ordinary loads would stay
+      constexpr int WORKERS = 32 * Sh::EPI_WARPS, MINE = (G * Sh::BLOCKS * 32 + WORKERS - 1) / WORKERS;
       const int t = (int)threadIdx.x - 64;
-      for (int i = t; i < W_BYTES / 16; i += 32 * Sh::EPI_WARPS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-      asm volatile("bar.sync 2, %0;" ::"n"(32 * Sh::EPI_WARPS) : "memory");
+      const int g = G == 2 ? (warp - 2) >> (S == 1 ? 3 : 2) : 0;
       if (!p.bias_static) pdl_wait();
-      for (int i = t; i < G * Sh::BLOCKS * 32; i += 32 * Sh::EPI_WARPS) {
-        const int c = i & 31, blk = i >> 5, g = blk / Sh::BLOCKS, b = blk - g * Sh::BLOCKS;
-        const int tap = S == 1 ? block_taps1.t[b] : b;
-        if (tap == 9) continue;
-        const uint32_t at = (uint32_t)(c * 33);   // row c, byte c
-        smem[(size_t)blk * 1024 + (at ^ (((at >> 7) & 1u) << 4))] = (uint8_t)p.w[(size_t)tap * p.C + c0 + g * 32 + c];
+      const int32_t my_bias = !p.bias ? 0 : (FORM == OTHER ? (t < P ? p.bias[c0 + t] : 0) : p.bias[c0 + g * 32 + lane]);
+      uint8_t w[MINE];
+#pragma unroll
+      for (int k = 0; k < MINE; ++k) {
+        const int i = t + k * WORKERS, c = i & 31, blk = i >> 5, bg = blk / Sh::BLOCKS, b = blk - bg * Sh::BLOCKS;
+        const int tap = blk < G * Sh::BLOCKS ? (S == 1 ? block_taps1.t[b] : b) : 9;
+        w[k] = tap == 9 ? (uint8_t)0 : (uint8_t)p.w[(size_t)tap * p.C + c0 + bg * 32 + c];
+      }
+      for (int i = t; i < W_BYTES / 16; i += WORKERS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+      asm volatile("bar.sync 2, %0;" ::"n"(WORKERS) : "memory");
+#pragma unroll
+      for (int k = 0; k < MINE; ++k) {
+        const int i = t + k * WORKERS;
+        const uint32_t at = (uint32_t)((i & 31) * 33);   // row c, byte c
+        if ((i >> 5) < G * Sh::BLOCKS) smem[(size_t)(i >> 5) * 1024 + (at ^ (((at >> 7) & 1u) << 4))] = w[k];
       }
       fence_async_smem();
-      if (FORM == OTHER && t < P) {
-        const int32_t b = p.bias ? p.bias[c0 + t] : 0;
-        bias_s[t] = p.wide ? b : (int32_t)((uint32_t)(b + p.add) * (uint32_t)p.mul);
-      }
-      const int g = G == 2 ? (warp - 2) >> (S == 1 ? 3 : 2) : 0;
+      if (FORM == OTHER && t < P) bias_s[t] = p.wide ? my_bias : (int32_t)((uint32_t)(my_bias + p.add) * (uint32_t)p.mul);
 #pragma unroll
-      for (int j = 0; j < (FORM == OTHER ? 0 : 32); ++j) bias[j] = (int32_t)((uint32_t)((p.bias ? p.bias[c0 + g * 32 + j] : 0) + p.add) * (uint32_t)p.mul);
+      for (int j = 0; j < (FORM == OTHER ? 0 : 32); ++j)
+        bias[j] = (int32_t)((uint32_t)(__shfl_sync(0xffffffffu, my_bias, j) + p.add) * (uint32_t)p.mul);
     }
     if (warp == Sh::IO_WARP && lane < 2)
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &tmap_y : &tmap_x)) : "memory");
