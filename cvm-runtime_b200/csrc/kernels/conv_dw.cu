@@ -29,7 +29,7 @@
 //
 // Any chain behind the products: [bias] shift clamp has forms of its own; a wide sum, and the sum with another tensor (whose
 // tile TMA brings into the output buffer before the result), run packed too, everything else step by step.  128 channels at
-// 28 x 28, 150 images, in a chain of such layers: 9.7 us with shift and clamp, 14.5 with a wide sum or a clip alone, 15.4 with a
+// 28 x 28, 150 images, in a chain of such layers: 9.1 us with shift and clamp, 14.5 with a wide sum or a clip alone, 15.3 with a
 // tensor (depthwise3x3_kernel 39.0, 34.8, 57.2; the clip step by step 18.9; the tensor loaded by the threads that need it 18.4:
 // a row's 32 bytes lie in a cache line of their own).  The wide sum's clamp is three more integer instructions an element, the
 // tensor waits in one of the two output buffers, which it takes from the tile two before.
