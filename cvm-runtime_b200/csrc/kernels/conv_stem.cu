@@ -315,10 +315,19 @@ conv_stem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   }
   if (!p.bias_static) pdl_wait();
   // weights -> shared memory, the 16 bytes of a tap in the order of the staged pixels
-  for (int i = threadIdx.x; i < p.w_bytes / 16; i += STEM_THREADS) {
-    uint4 v = reinterpret_cast<const uint4*>(p.w)[i];
-    if (p.S == 2) v = p.C == 1 ? v : (p.C == 2 ? staged_order<2>(v) : (p.C == 3 ? staged_order<3>(v) : staged_order<4>(v)));
-    reinterpret_cast<uint4*>(wq)[i] = v;
+  // (three chunks a thread set out before the first is stored, behind which ordinary loads would stay)
+  const int w_chunks = p.w_bytes / 16;
+  for (int i0 = threadIdx.x; i0 < w_chunks; i0 += 3 * STEM_THREADS) {
+    uint4 v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (i0 + k * STEM_THREADS < w_chunks) v[k] = reinterpret_cast<const uint4*>(p.w)[i0 + k * STEM_THREADS];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (i0 + k * STEM_THREADS >= w_chunks) break;
+      if (p.S == 2) v[k] = p.C == 1 ? v[k] : (p.C == 2 ? staged_order<2>(v[k]) : (p.C == 3 ? staged_order<3>(v[k]) : staged_order<4>(v[k])));
+      reinterpret_cast<uint4*>(wq)[i0 + k * STEM_THREADS] = v[k];
+    }
   }
   fence_async_smem();
   if (warp == MMA_WARP) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);

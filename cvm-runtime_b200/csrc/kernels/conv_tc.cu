@@ -427,10 +427,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   auto stage_bias = [&]() {
     const int padded = min(MAX_BIAS, (p.oc + 31) & ~31);
-    for (int i = (int)threadIdx.x - 32; i < padded; i += NUM_THREADS - 64) {   // warps 1..10
-      const int32_t b = i < p.oc && p.bias ? p.bias[i] : 0;
+    constexpr int T = NUM_THREADS - 64;   // warps 1..10
+    for (int i0 = (int)threadIdx.x - 32; i0 < padded; i0 += 4 * T) {   // (ordinary loads stay behind stores: four set out first)
+      int32_t b[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) b[k] = i0 + k * T < p.oc && p.bias ? p.bias[i0 + k * T] : 0;
       // fast path: (bias + rounding addend) pre-multiplied by 2^(16 - shift), see fast_row()
-      bias_s[i] = (p.fast_mode && !p.fast_wide) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i0 + k * T < padded) bias_s[i0 + k * T] = (p.fast_mode && !p.fast_wide) ? (int32_t)((uint32_t)(b[k] + p.f_add) * (uint32_t)p.f_mul) : b[k];
     }
   };
   uint32_t tmem_base = 0;
