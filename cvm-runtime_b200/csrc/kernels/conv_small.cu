@@ -184,6 +184,12 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int mt = uniform(fdiv(tile, p.fd_n_tiles));
   const int n0 = (tile - mt * p.num_n_tiles) * p.block_n;
   const int m0 = mt * BLOCK_M;
+  // a channel's bias a thread (warps 2 and on), if it is a parameter as early as its place is known
+  static_assert(THREADS - 64 >= BLOCK_M, "a thread for every channel");
+  const int ch0 = SWAP ? m0 : n0, channels = SWAP ? BLOCK_M : p.block_n, bias_at = (int)threadIdx.x - 64;
+  int32_t bias = 0;
+  auto load_bias = [&]() { if (p.bias && bias_at < channels && ch0 + bias_at < p.oc) bias = p.bias[ch0 + bias_at]; };
+  if (warp >= 2 && p.bias_static) load_bias();
   int cw = 0, ch = 0, cn = 0;
   if (p.a_mode == 2) {
     const int r = uniform(fdiv(mt, p.fd_tiles_w));
@@ -243,14 +249,12 @@ conv_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
     pdl_trigger();
   } else {
-    const bool early = p.bias_static != 0;
-    if (!early) pdl_wait();
-    const int ch0 = SWAP ? m0 : n0, channels = SWAP ? BLOCK_M : p.block_n;
-    for (int i = (int)threadIdx.x - 64; i < channels; i += THREADS - 64) {
-      const int32_t b = (p.bias && ch0 + i < p.oc) ? p.bias[ch0 + i] : 0;
-      // packed requantisation: (bias + rounding addend) pre-multiplied, see fast_requant()
-      bias_s[i] = (p.fast_variant >= 0 && p.fast_variant < 8) ? (int32_t)((uint32_t)(b + p.f_add) * (uint32_t)p.f_mul) : b;
+    if (!p.bias_static) {
+      pdl_wait();
+      load_bias();
     }
+    // packed requantisation: (bias + rounding addend) pre-multiplied, see fast_requant()
+    if (bias_at < channels) bias_s[bias_at] = (p.fast_variant >= 0 && p.fast_variant < 8) ? (int32_t)((uint32_t)(bias + p.f_add) * (uint32_t)p.f_mul) : bias;
   }
   tc_fence_before();
   __syncthreads();
